@@ -47,40 +47,40 @@ PAGE = 16
 def listed():
     return [
         # the smallest calls: two short prompts of a tiny model in float32, greedy; launches and host work are all of it
-        dict(name="tiny a, float32, generate", model="gpt2-tiny-a", dtype="float32", work="generate", requests=2, tokens=13,
+        dict(name="tiny generate float32", model="gpt2-tiny-a", dtype="float32", work="generate", requests=2, tokens=13,
              steps=16, ragged=True, temp=0.0),
         # one user's chat
-        dict(name="medium, decode, 1 request", model="gpt2-medium", dtype="bfloat16", work="decode", requests=1, tokens=512,
+        dict(name="medium decode 1", model="gpt2-medium", dtype="bfloat16", work="decode", requests=1, tokens=512,
              steps=16, ragged=False),
         # a few users at once: the repository's headline
-        dict(name="medium, decode, 8 requests", model="gpt2-medium", dtype="bfloat16", work="decode", requests=8, tokens=512,
+        dict(name="medium decode 8", model="gpt2-medium", dtype="bfloat16", work="decode", requests=8, tokens=512,
              steps=16, ragged=False),
         # a full batch, every request at a length of its own
-        dict(name="medium, decode, 64 requests", model="gpt2-medium", dtype="bfloat16", work="decode", requests=64,
+        dict(name="medium decode 64", model="gpt2-medium", dtype="bfloat16", work="decode", requests=64,
              tokens=900, steps=12, ragged=True),
         # reading: two prompts of the full context
-        dict(name="medium, prefill, 2 x 1024", model="gpt2-medium", dtype="bfloat16", work="prefill", requests=2,
+        dict(name="medium prefill", model="gpt2-medium", dtype="bfloat16", work="prefill", requests=2,
              tokens=1024, ragged=False),
         # the all-32-bit path: three prompts of odd lengths
-        dict(name="medium, float32, prefill", model="gpt2-medium", dtype="float32", work="prefill", requests=3, tokens=301,
+        dict(name="medium prefill float32", model="gpt2-medium", dtype="float32", work="prefill", requests=3, tokens=301,
              ragged=True),
         # a server: a prompt in portions of 256 tokens beside 31 requests that decode
-        dict(name="large, mixed, 31 requests", model="gpt2-large", dtype="bfloat16", work="mixed", requests=31, tokens=700,
+        dict(name="large mixed", model="gpt2-large", dtype="bfloat16", work="mixed", requests=31, tokens=700,
              steps=4, portion=256, ragged=True),
         # the largest dense model
-        dict(name="xl, prefill, 2 x 1024", model="gpt2-xl", dtype="bfloat16", work="prefill", requests=2, tokens=1024,
+        dict(name="xl prefill", model="gpt2-xl", dtype="bfloat16", work="prefill", requests=2, tokens=1024,
              ragged=False),
         # reading with recurrent layers
-        dict(name="lelatar, prefill, 2 x 1024", model="lelatar-1024", dtype="bfloat16", work="prefill", requests=2,
+        dict(name="lelatar prefill", model="lelatar-1024", dtype="bfloat16", work="prefill", requests=2,
              tokens=1024, ragged=False),
         # short questions and their answers with recurrent layers
-        dict(name="lelatar, generate, 8 requests", model="lelatar-1024", dtype="bfloat16", work="generate", requests=8,
+        dict(name="lelatar generate", model="lelatar-1024", dtype="bfloat16", work="generate", requests=8,
              tokens=100, steps=16, ragged=True),
         # reading prompts of odd lengths with mixed scores, latent rows and a recurrence
-        dict(name="nufetar, prefill, 3 prompts", model="nufetar-1024", dtype="bfloat16", work="prefill", requests=3,
+        dict(name="nufetar prefill", model="nufetar-1024", dtype="bfloat16", work="prefill", requests=3,
              tokens=731, ragged=True),
         # prompts and their answers, twice as wide
-        dict(name="nufetar 2048, generate, 4", model="nufetar-2048", dtype="bfloat16", work="generate", requests=4,
+        dict(name="nufetar 2048 generate", model="nufetar-2048", dtype="bfloat16", work="generate", requests=4,
              tokens=400, steps=8, ragged=True),
     ]
 
