@@ -548,6 +548,33 @@ def attention_generic(q, positions, token_req, block_table, k_pool, v_pool, out,
           _sinks(sinks, n_heads, "attention"), stream)
 
 
+_PORTIONS_F32_ARGS = [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float,
+                      c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p]
+
+
+def attention_portions_f32_supported(q, k_pool, tiles) -> bool:
+    """Whether float32 portions run in tiles (``attention_portions_f32``) and not row by row (``attention_generic``, which
+    reads every key again for every query): heads of up to 128 in whole 16 bytes, tiles of at most 128 queries."""
+    return (k_pool.dtype == torch.float32 and k_pool.shape[3] <= 128 and k_pool.shape[3] % 4 == 0 and PREFILL_TILE <= 128
+            and tiles is not None and _rows(q, "attention q") % 4 == 0
+            and all(t.data_ptr() % 16 == 0 for t in (q, k_pool, tiles)))
+
+
+def attention_portions_f32(q, tiles, n_tiles: int, block_table, k_pool, v_pool, out, n_heads: int, scale: float, window: int,
+                           status, stream, sinks=None) -> None:
+    """``attention_generic`` for the queries of ``tiles`` (int32 ``[n_tiles, 4]``, as ``attention_portions`` takes them) of a
+    float32 model: the same mathematics, 64 queries by 64 keys at a time."""
+    n_pages, Hkv, page, Dh = _attn_shapes(q, out, k_pool, n_heads, "attention")
+    if not attention_portions_f32_supported(q, k_pool, tiles) or v_pool.shape != k_pool.shape:
+        raise KernelError(f"attention (float32 portions): heads of {Dh}, pools {tuple(k_pool.shape)} and {tuple(v_pool.shape)}")
+    _need(tiles, torch.int32, "attention tiles")
+    if tiles.numel() < 4 * n_tiles:
+        raise KernelError(f"attention: {tiles.numel()} integers for {n_tiles} tiles")
+    _call("attention", "mlxb_attention_portions_f32", _PORTIONS_F32_ARGS, _p(q), _rows(q, "attention q"), _p(tiles), n_tiles,
+          _p(block_table), block_table.shape[1], n_pages, page, n_heads, Hkv, Dh, window, scale, _p(k_pool), _p(v_pool), _p(out),
+          _rows(out, "attention out"), _p(status), _sinks(sinks, n_heads, "attention"), stream)
+
+
 _PRE_ARGS = [c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float,
              c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p]
 

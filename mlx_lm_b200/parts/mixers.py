@@ -111,6 +111,9 @@ def paged_attention(ctx, q, cache, o, n_heads: int, head_dim: int, scale: float,
             ops.attention_portions(q, ctx.portion_tiles, ctx.n_portion_tiles, cache.block_table, cache.k,
                                    cache.v, o, n_heads, scale, window, ctx.status, ctx.stream, sinks=sinks,
                                    first_positions=ctx.req_first_position)
+        elif cache.v.shape == cache.k.shape and ops.attention_portions_f32_supported(q, cache.k, ctx.portion_tiles):
+            ops.attention_portions_f32(q, ctx.portion_tiles, ctx.n_portion_tiles, cache.block_table, cache.k, cache.v, o,
+                                       n_heads, scale, window, ctx.status, ctx.stream, sinks=sinks)
         else:
             ops.attention_generic(q, ctx.positions, ctx.token_req, cache.block_table, cache.k, cache.v, o,
                                   n_heads, scale, window, ctx.status, ctx.stream,

@@ -37,3 +37,35 @@ def test_float32_linear(ops, M, N, K):
     for x2 in (wide[:, 4:], wide[:, 1:K + 1]):
         ops.linear_generic(x2, w, None, out, stream())
         assert rel_err(out, x2.double() @ w.double().T) <= 1e-6
+
+
+@pytest.mark.parametrize("Hq,Hkv,Dh,page,window,sink", [(4, 4, 16, 16, 0, False), (3, 3, 36, 4, 0, True), (6, 2, 64, 16, 0, False),
+                                                        (2, 1, 64, 32, 70, True), (2, 2, 100, 16, 1, False), (2, 2, 128, 64, 200, False)])
+def test_float32_attention_of_portions(ops, Hq, Hkv, Dh, page, window, sink):
+    """Portions around the kernel's 64 queries and the step's tiles of 128, contexts around a block of 64 keys, behind pages that
+    a window gave back; rows of no tile keep what they held."""
+    lens, new = [0, 63, 64, 130, 5, 300], [1, 129, 64, 35, 200, 2]
+    c = paged_case(torch.float32, lens=lens, new=new, Hq=Hq, Hkv=Hkv, Dh=Dh, page=page, seed=Dh)
+    # pool rows of this step's own tokens hold what paged_case put there: both sides read the pools
+    if window:
+        for r, n in enumerate(lens):
+            for p in range(max(0, n - window + 1) // page):
+                c["bt"][r, p] = -1
+    dev = {k: (v.cuda() if torch.is_tensor(v) else v) for k, v in c.items()}
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    sinks = torch.randn(Hq, generator=torch.Generator().manual_seed(1)).cuda() if sink else None
+    first = [sum(new[:r]) for r in range(len(new))]
+    tiles = [(first[r] + a, min(128, n - a), r, lens[r] + a) for r, n in enumerate(new) if r for a in range(0, n, 128)]
+    tiles = torch.tensor(tiles + [(0, 0, 0, 0)], dtype=torch.int32).cuda()
+    scale = Dh ** -0.5
+    q, out = dev["qkv"][:, :Hq * Dh], torch.full((c["T"], Hq * Dh), 7.0, device="cuda")
+    args = (dev["bt"], dev["k_pool"], dev["v_pool"])
+    ops.attention_portions_f32(q, tiles, len(tiles), *args, out, Hq, scale, window, status, stream(), sinks=sinks)
+    assert int(status.item()) == 0
+    assert bool((out[:1] == 7.0).all())
+    row_by_row = torch.empty_like(out)
+    ops.attention_generic(q, dev["positions"], dev["token_req"], *args, row_by_row, Hq, scale, window, status, stream(), sinks=sinks)
+    assert rel_err(out[1:], row_by_row[1:]) <= 3e-6
+    if not sink and not window:
+        want = R.attention(c["qkv"][:, :Hq * Dh], c["positions"], c["token_req"], c["bt"], c["k_pool"], c["v_pool"], Hq, scale, window)
+        assert rel_err(out[1:], want[1:]) <= 3e-6
