@@ -2,8 +2,8 @@
 //   C[M,N] = epilogue(A[M,K] . W[N,K]^T + bias[N]) (+ residual[M,N])
 // A, W bfloat16 (both operands K-major: the K index is contiguous), C bfloat16 or float32, the residual has C's dtype.
 //
-// The kernel is persistent: one CTA per SM walks over the 128 x BN output tiles (BN = 128, 192 or 256,
-// chosen so that the last wave of tiles is as full as possible).  Warp 0 is the TMA producer: it fills a
+// The kernel is persistent: one CTA per SM walks over the 128 x BN output tiles (BN = 32 to 256,
+// see tile_choice).  Warp 0 is the TMA producer: it fills a
 // ring of shared-memory stages with 128x64 tiles of A and BNx64 tiles of W (cp.async.bulk.tensor,
 // 128-byte swizzle, completion counted on an mbarrier per stage; rows and columns outside the
 // matrices arrive as zeros).  Warp 1 allocates tensor memory and issues tcgen05.mma (kind::f16, bf16
@@ -46,6 +46,8 @@ MLXB_DEFINE_LAST_ERROR()
 constexpr int BM = 128, BK = 64;
 constexpr int EPI_WARPS = 16;                     // four per quadrant of TMEM lanes, each a quarter of the columns
 constexpr int THREADS = 64 + 32 * EPI_WARPS;
+// slices of a tile's columns over the epilogue warps of a quadrant; a tile narrower than 128 leaves warps without work
+constexpr int epi_slices(int bn) { return bn >= 128 ? EPI_WARPS / 4 : bn / 32; }
 // Polls of a barrier before a wait gives up (about a second).  A test builds this file with
 // MLXB_TEST_WAIT_TIMEOUT defined: the limit is then short, and mlxb_test_withhold_arrival(1) makes the MMA thread
 // leave out the arrival that tells the epilogue warps that a CTA's first accumulator is complete, so that their
@@ -66,7 +68,7 @@ struct Smem {
   uint64_t drained;       // abort path only: every tensor-core operation issued so far has completed
   uint32_t tmem_base;
   int abort_flag;
-  alignas(16) uint4 stage[EPI_WARPS][32 * 4];   // per epilogue warp: 32 rows x 32 bfloat16 results on their way out
+  alignas(16) uint4 stage[EPI_WARPS][32 * 4];   // per epilogue warp: 64 bytes of results of each of its 32 rows on their way out
 };
 
 
@@ -77,82 +79,23 @@ struct NormFoldRows {
   const float2* stats;    // [M]
 };
 
-__device__ __forceinline__ void unfold8(float (&v)[8], int n8, int N, const float* __restrict__ colsum, float mean,
-                                        float rstd) {
-  if (n8 + 8 <= N && (((uintptr_t)(colsum + n8)) & 15) == 0) {   // the same 32 bytes for every lane: two broadcast loads
-    const float4 c0 = *reinterpret_cast<const float4*>(colsum + n8), c1 = *reinterpret_cast<const float4*>(colsum + n8 + 4);
-    const float cs[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-    const float nm = -mean * rstd;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = fmaf(nm, cs[i], rstd * v[i]);
-    return;
-  }
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-    if (n8 + i < N) v[i] = rstd * (v[i] - mean * colsum[n8 + i]);
-}
-
-// One 8-column group of an output row: the folded norm's correction, bias, activation, residual; the eight
-// float32 results stay in v.
-template <int EPI>
-__device__ __forceinline__ void finish8(float (&v)[8], const uint32_t* r, int n8, int N, size_t row,
-                                        const float* __restrict__ bias, bool bias_vec, const __nv_bfloat16* residual,
-                                        bool have_fetched, uint4 fetched, const float* __restrict__ colsum, float mean,
-                                        float rstd) {
-  const bool whole = n8 + 8 <= N;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
-  if (colsum) unfold8(v, n8, N, colsum, mean, rstd);
-  if (bias) {
-    if (whole && bias_vec) {   // the same 32 bytes for every lane of the warp: two broadcast loads
-      const float4 b0 = *reinterpret_cast<const float4*>(bias + n8), b1 = *reinterpret_cast<const float4*>(bias + n8 + 4);
-      v[0] += b0.x; v[1] += b0.y; v[2] += b0.z; v[3] += b0.w;
-      v[4] += b1.x; v[5] += b1.y; v[6] += b1.z; v[7] += b1.w;
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (n8 + i < N) v[i] += bias[n8 + i];
-    }
-  }
-  if (EPI != EPI_NONE) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = activate<EPI, true>(v[i]);
-  }
-  if (residual) {
-    if (have_fetched || (whole && ((row + n8) & 7) == 0)) {
-      const uint4 u = have_fetched ? fetched : *reinterpret_cast<const uint4*>(residual + row + n8);
-      const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        v[2 * i] += __uint_as_float(w[i] << 16);
-        v[2 * i + 1] += __uint_as_float(w[i] & 0xffff0000u);
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (n8 + i < N) v[i] += __bfloat162float(residual[row + n8 + i]);
-    }
-  }
-}
-
-// float32 results go out as they are: 32 bytes a lane and group, a whole sector.
-__device__ __forceinline__ void store8_f32(const float (&v)[8], int n8, int N, size_t row, float* C) {
-  float* out = C + row + n8;
-  if (n8 + 8 <= N && ((row + n8) & 3) == 0) {
-    *reinterpret_cast<float4*>(out) = make_float4(v[0], v[1], v[2], v[3]);
-    *reinterpret_cast<float4*>(out + 4) = make_float4(v[4], v[5], v[6], v[7]);
-  } else {
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-      if (n8 + i < N) out[i] = v[i];
-  }
-}
-
-// bfloat16 results are 16 bytes a lane and group.  Written by the lane that holds them (one lane per row) they
-// would be half sectors 32 rows apart; so a warp first puts its 32 rows x 32 columns into shared memory (64 bytes
-// a row, the 16-byte pieces of a row XORed with bits of the row number against bank conflicts) and writes them out
-// from there with four lanes on the 64 contiguous bytes of a row: whole sectors, half as many.
+// Results leave through shared memory: a lane holds a row, and written by the lanes that hold them they would be pieces of
+// rows 32 rows apart.  A warp puts 64 bytes of each of its 32 rows there (the 16-byte pieces of a row XORed with bits of the row
+// number against bank conflicts) and writes them out with four lanes on a row: whole sectors.
 __device__ __forceinline__ int stage_index(int row, int piece) { return row * 4 + (piece ^ ((row >> 1) & 3)); }
+
+// 16 bytes of row `row` (an element offset) at column n, from a staged piece.
+__device__ __forceinline__ void store_piece(uint4 u, int n, int N, size_t row, float* C) {
+  float* out = C + row + n;
+  if (n + 4 <= N && ((row + n) & 3) == 0) {
+    *reinterpret_cast<uint4*>(out) = u;
+  } else {
+    const float* e = reinterpret_cast<const float*>(&u);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (n + i < N) out[i] = e[i];
+  }
+}
 
 // Eight bfloat16 of row `row` (an element offset) at column n8, from a staged piece.
 __device__ __forceinline__ void store_piece(uint4 u, int n8, int N, size_t row, __nv_bfloat16* C) {
@@ -200,11 +143,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   auto tile_n0 = [&](int t) { return (t / tiles_m) * BN; };                          // the tile's first column
   constexpr int W_ROWS = BN / CG;                          // W rows per copy
   constexpr uint32_t STAGE_BYTES = CG * (BM + W_ROWS) * BK * sizeof(__nv_bfloat16);   // counted on a stage's barrier
-  constexpr uint32_t TMEM_COLS = BN <= 128 ? 256 : 512;   // two accumulators; a power of two
+  constexpr uint32_t TMEM_COLS = BN <= 128 ? 2 * BN : 512;   // two accumulators; a power of two
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&sm.acc_full[b], 1); mbar_init(&sm.acc_empty[b], CG * 32 * EPI_WARPS); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&sm.acc_full[b], 1); mbar_init(&sm.acc_empty[b], CG * 32 * 4 * epi_slices(BN)); }
     mbar_init(&sm.drained, 1);
     sm.abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -253,124 +196,127 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   residual = after_wait(residual);
 
   if (warp == 0) {
-    if (lane == 0) {
-      int issued = 0;   // stages filled so far, over all tiles
-      bool ok = true;
-      for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step) {
-        const int m0 = tile_m0(tile), n0 = tile_n0(tile);
-        for (int kt = 0; kt < k_tiles; ++kt, ++issued) {
-          const int s = issued % STAGES;
-          const uint32_t ph = (issued / STAGES) & 1;
-          if (issued < early) {   // a fresh stage, armed, whose W rows are on their way already
-            load_a(s, kt, m0);
-            continue;
-          }
+    int issued = 0;   // stages filled so far, over all tiles
+    int s = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step) {
+      const int m0 = tile_m0(tile), n0 = tile_n0(tile);
+      for (int kt = 0; kt < k_tiles; ++kt) {
+        if (issued < early) {   // a fresh stage, armed, whose W rows are on their way already
+          if (elect_one()) load_a(s, kt, m0);
+        } else {
           // free once the products that read it have completed (in a pair: the commit arrives in both CTAs)
-          if (!mbar_wait(&sm.empty[s], ph ^ 1, abort_flag, peer_abort)) { ok = false; break; }
-          if (leader) mbar_expect_tx(&sm.full[s], STAGE_BYTES);
-          load_a(s, kt, m0);
-          load_w(s, kt, n0);
-        }
-      }
-      if (*abort_flag && leader) {   // gave up: let the copies already issued land before the CTA exits
-        for (int i = issued > STAGES ? issued - STAGES : 0; i < issued; ++i) {
-          const uint32_t addr = smem_u32(&sm.full[i % STAGES]);
-          for (uint32_t p = 0; p < (1u << 20); ++p) {
-            uint32_t done;
-            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                         "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(addr), "r"((uint32_t)((i / STAGES) & 1))
-                         : "memory");
-            if (done) break;
+          ok = mbar_wait_warp(&sm.empty[s], ph ^ 1, abort_flag, peer_abort);
+          if (!ok) break;
+          if (elect_one()) {
+            if (leader) mbar_expect_tx(&sm.full[s], STAGE_BYTES);
+            load_a(s, kt, m0);
+            load_w(s, kt, n0);
           }
+        }
+        ++issued;
+        if (++s == STAGES) { s = 0; ph ^= 1; }
+      }
+    }
+    if (lane == 0 && *abort_flag && leader) {   // gave up: let the copies already issued land before the CTA exits
+      for (int i = issued > STAGES ? issued - STAGES : 0; i < issued; ++i) {
+        const uint32_t addr = smem_u32(&sm.full[i % STAGES]);
+        for (uint32_t p = 0; p < (1u << 20); ++p) {
+          uint32_t done;
+          asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                       "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(addr), "r"((uint32_t)((i / STAGES) & 1))
+                       : "memory");
+          if (done) break;
         }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && leader) {   // one thread issues the products, for both CTAs of a pair
+    if (leader) {   // one thread issues the products, for both CTAs of a pair
       constexpr uint32_t idesc = umma_idesc(CG * BM, BN);
-      int consumed = 0, it = 0;
+      // the same offsets in both CTAs of a pair: the descriptors name them in each CTA's own shared memory
+      const uint64_t da0 = umma_desc(smem_u32(sm.a[0])), db0 = umma_desc(smem_u32(sm.b[0]));
+      constexpr uint32_t A_STEP = BM * BK * 2 / 16, B_STEP = W_ROWS * BK * 2 / 16;   // a stage, in units of 16 bytes
+      int s = 0, it = 0;
+      uint32_t ph = 0;
       bool ok = true;
       for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step, ++it) {
         const int b = it & 1;
         // the epilogue (of both CTAs) must have drained this accumulator (its previous use was tile it-2)
-        ok = mbar_wait(&sm.acc_empty[b], ((it >> 1) & 1) ^ 1, abort_flag, peer_abort);
+        ok = mbar_wait_warp(&sm.acc_empty[b], ((it >> 1) & 1) ^ 1, abort_flag, peer_abort);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t tmem_acc = tmem_base + (uint32_t)(b * BN);
-        for (int kt = 0; kt < k_tiles; ++kt, ++consumed) {
-          const int s = consumed % STAGES;
-          const uint32_t ph = (consumed / STAGES) & 1;
-          ok = mbar_wait(&sm.full[s], ph, abort_flag, peer_abort);
+        for (int kt = 0; kt < k_tiles; ++kt) {
+          ok = mbar_wait_warp(&sm.full[s], ph, abort_flag, peer_abort);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          // the same offsets in both CTAs of a pair: the descriptors name them in each CTA's own shared memory
-          const uint64_t da = umma_desc(smem_u32(sm.a[s])), db = umma_desc(smem_u32(sm.b[s]));
+          const uint64_t da = da0 + (uint32_t)s * A_STEP, db = db0 + (uint32_t)s * B_STEP;
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {   // 16 bf16 = 32 bytes = 2 units of the descriptor's start address
-            if (CG == 2) umma_bf16_pair(tmem_acc, da + 2 * k, db + 2 * k, idesc, (kt > 0 || k > 0) ? 1u : 0u);
-            else umma_bf16(tmem_acc, da + 2 * k, db + 2 * k, idesc, (kt > 0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < BK / 16; ++k) {   // 16 bf16 = 32 bytes = 2 units of the descriptor's start address
+              if (CG == 2) umma_bf16_pair(tmem_acc, da + 2 * k, db + 2 * k, idesc, (kt > 0 || k > 0) ? 1u : 0u);
+              else umma_bf16(tmem_acc, da + 2 * k, db + 2 * k, idesc, (kt > 0 || k > 0) ? 1u : 0u);
+            }
+            // the stage is free once these MMAs have read it
+            if (CG == 2) umma_commit_both(&sm.empty[s]);
+            else umma_commit(&sm.empty[s]);
           }
-          // the stage is free once these MMAs have read it
-          if (CG == 2) umma_commit_both(&sm.empty[s]);
-          else umma_commit(&sm.empty[s]);
+          __syncwarp();
+          if (++s == STAGES) { s = 0; ph ^= 1; }
         }
 #ifdef MLXB_TEST_WAIT_TIMEOUT
         if (g_test_withhold_arrival && it == 0) continue;   // the test's missing arrival
 #endif
-        if (ok) {   // arrives when every MMA of this tile has completed
+        if (ok && elect_one()) {   // arrives when every MMA of this tile has completed
           if (CG == 2) umma_commit_both(&sm.acc_full[b]);
           else umma_commit(&sm.acc_full[b]);
         }
+        __syncwarp();
       }
     }
-  } else {
+  } else if (((warp - 2) >> 2) < epi_slices(BN)) {
     // epilogue: warps 2..17; warp w may touch TMEM lanes 32*(w%4) .. +31; the four warps of a quadrant
     // split the tile's columns
     const int q = warp & 3;
     const int half = (warp - 2) >> 2;          // which slice of the columns (0 .. EPI_WARPS/4 - 1)
-    constexpr int HALF_COLS = BN / (EPI_WARPS / 4);   // 32, 48 or 64 columns per warp
-    const bool bias_vec = bias && (((uintptr_t)bias & 15) == 0);
+    constexpr int HALF_COLS = BN / epi_slices(BN);    // 32, 48 or 64 columns per warp
     const uint32_t acc_empty_leader[2] = {CG == 2 ? peer_addr(&sm.acc_empty[0], 0) : 0u,
                                           CG == 2 ? peer_addr(&sm.acc_empty[1], 0) : 0u};
+    const TO* res = reinterpret_cast<const TO*>(residual);
+    constexpr int PER = 16 / sizeof(TO);               // columns of a 16-byte piece of the output
+    uint4* stg = sm.stage[warp - 2];
+    const int o_row = lane >> 2, o_piece = lane & 3;   // what this lane writes out: rows o_row + 8 j
     int it = 0;
     for (int tile = first_tile; tile < n_tiles; tile += tile_step, ++it) {
       const int b = it & 1;
-      const int m0 = tile_m0(tile), n0 = tile_n0(tile);
-      const int m = m0 + q * 32 + lane;
+      const int m0 = tile_m0(tile) + q * 32, n0 = tile_n0(tile) + half * HALF_COLS;     // this warp's first row and column
+      const int m = m0 + lane;
+      const bool in = m < M;
       const size_t row = (size_t)m * ldc;
-      // The residual of this lane's row, 32 columns at a time (64 contiguous bytes), is fetched a chunk ahead:
-      // the first chunk while the tile's products are still running, each further one while the chunk before
-      // it is worked on.  Bit g of `have` says that group g of the chunk was fetched (whole and aligned).
+      // While the tile's products run: all that the epilogue needs from memory besides them.  Lane l keeps (bias, column
+      // sum) of columns l and l + 32 and hands them around through shared memory chunk by chunk; read from global memory
+      // between the steps of the epilogue they cost it a latency each (2048 x 4096 x 1024 with bias, folded norm and
+      // gelu_new: 24.3 us, 17.4 without any of them, 19.5 this way).
       float mean = 0.f, rstd = 1.f;
-      if (fold.colsum != nullptr && m < M) {
+      if (fold.colsum != nullptr && in) {
         const float2 st = fold.stats[m];
         mean = st.x;
         rstd = st.y;
       }
-      uint4 res0, res1, res2, res3, nx0, nx1, nx2, nx3;
-      res0 = res1 = res2 = res3 = nx0 = nx1 = nx2 = nx3 = make_uint4(0u, 0u, 0u, 0u);
-      unsigned have = 0, have_next = 0;
-#define FETCH_RESIDUAL(C0, D0, D1, D2, D3, HAVE)                                                        \
-      {                                                                                                   \
-        HAVE = 0;                                                                                         \
-        if (sizeof(TO) == 2 && residual != nullptr && m < M) {                                            \
-          const int nb = n0 + half * HALF_COLS + (C0);                                                    \
-          const __nv_bfloat16* rp = residual + row + nb;                                                  \
-          const bool al = ((row + nb) & 7) == 0;                                                          \
-          if (al && (C0) + 0 < HALF_COLS && nb + 8 <= N) { D0 = *reinterpret_cast<const uint4*>(rp); HAVE |= 1u; }          \
-          if (al && (C0) + 8 < HALF_COLS && nb + 16 <= N) { D1 = *reinterpret_cast<const uint4*>(rp + 8); HAVE |= 2u; }     \
-          if (al && (C0) + 16 < HALF_COLS && nb + 24 <= N) { D2 = *reinterpret_cast<const uint4*>(rp + 16); HAVE |= 4u; }   \
-          if (al && (C0) + 24 < HALF_COLS && nb + 32 <= N) { D3 = *reinterpret_cast<const uint4*>(rp + 24); HAVE |= 8u; }   \
-        }                                                                                                 \
+      const float shift = -mean * rstd;
+      float2 col_a, col_b;
+      {
+        const int na = n0 + lane, nb = n0 + 32 + lane;
+        const bool oka = na < N && lane < HALF_COLS, okb = nb < N && 32 + lane < HALF_COLS;
+        col_a = make_float2(bias != nullptr && oka ? bias[na] : 0.f, fold.colsum != nullptr && oka ? fold.colsum[na] : 0.f);
+        col_b = make_float2(bias != nullptr && okb ? bias[nb] : 0.f, fold.colsum != nullptr && okb ? fold.colsum[nb] : 0.f);
       }
-      FETCH_RESIDUAL(0, res0, res1, res2, res3, have)
-      if (!mbar_wait(&sm.acc_full[b], (it >> 1) & 1, abort_flag, peer_abort)) break;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       // fused cache write: this row's slot in its page (an element offset before the head and dim are added);
       // -1 for a padding row or an index out of range
       long long slot = -1;
       int in_page = 0;
-      if (SCATTER && m < M && n0 + BN > kv.q_width) {
+      if (SCATTER && in && n0 + HALF_COLS > kv.q_width && n0 < N) {
         const int r = kv.token_req[m];
         if (r >= 0) {
           const int pos = kv.positions[m];
@@ -381,6 +327,29 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           else if (pg >= 0) { slot = (long long)pg * kv.Hkv * kv.page; in_page = pos % kv.page; }
         }
       }
+      // The residual, four 16-byte pieces a lane.  bfloat16: 32 columns of this lane's row (added before the sum is
+      // rounded), a chunk ahead.  float32: the pieces that this lane writes out of 16 columns (added on the way out, four
+      // lanes on a row's 64 bytes), half a chunk ahead (2048 x 4096 x 1024: 28.3 us; by rows and in place 40.1).  Bit i of
+      // `have`: piece i was fetched (whole and aligned).
+      uint4 rp[4];
+      unsigned have = 0;
+      auto fetch = [&](int c) {       // columns c .. of this warp's
+        have = 0;
+        if (res == nullptr) return;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int mm = sizeof(TO) == 2 ? m : m0 + o_row + 8 * i;
+          const int off = c + (sizeof(TO) == 2 ? i : o_piece) * PER, n = n0 + off;
+          const size_t at = (size_t)mm * ldc + n;
+          if (mm < M && n + PER <= N && off < HALF_COLS && (at & (PER - 1)) == 0) {
+            rp[i] = *reinterpret_cast<const uint4*>(res + at);
+            have |= 1u << i;
+          }
+        }
+      };
+      fetch(0);
+      if (!mbar_wait(&sm.acc_full[b], (it >> 1) & 1, abort_flag, peer_abort)) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BN + half * HALF_COLS);
 #pragma unroll 1
       for (int c0 = 0; c0 < HALF_COLS; c0 += 32) {
@@ -390,80 +359,109 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         } else {                                // 48 columns per warp (BN = 192): the last 16
           tmem_ld16(taddr + (uint32_t)c0, r);
         }
-        if (c0 + 32 < HALF_COLS) FETCH_RESIDUAL(c0 + 32, nx0, nx1, nx2, nx3, have_next)
+        reinterpret_cast<float2*>(stg)[lane] = c0 == 0 ? col_a : col_b;
+        __syncwarp();
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         if (c0 + 32 >= HALF_COLS) {   // this warp's part of the accumulator is in registers: hand it back
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           if (CG == 2) mbar_arrive_cluster(acc_empty_leader[b]);   // the leader issues the products into both halves
           else mbar_arrive(&sm.acc_empty[b]);
         }
-        if (sizeof(TO) == 4) {
-          if (m < M) {
+        float v[32];
 #pragma unroll
-            for (int g8 = 0; g8 < 4; ++g8) {
-              const int n8 = n0 + half * HALF_COLS + c0 + g8 * 8;
-              if (c0 + g8 * 8 < HALF_COLS && n8 < N) {
-                float v[8];
-                finish8<EPI>(v, r + g8 * 8, n8, N, row, bias, bias_vec, nullptr, false, res0, fold.colsum, mean, rstd);
-                if (residual != nullptr) {   // a float32 result takes a float32 residual
-                  const float* rf = reinterpret_cast<const float*>(residual) + row + n8;
-                  if (n8 + 8 <= N && ((row + n8) & 3) == 0) {
-                    const float4 a = *reinterpret_cast<const float4*>(rf), b = *reinterpret_cast<const float4*>(rf + 4);
-                    v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w; v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
-                  } else {
+        for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+        const float4* cp = reinterpret_cast<const float4*>(stg);      // (bias, column sum) of two columns: the same for every lane
+        if (fold.colsum != nullptr) {
 #pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                      if (n8 + i < N) v[i] += rf[i];
-                  }
-                }
-                store8_f32(v, n8, N, row, reinterpret_cast<float*>(C));
+          for (int i = 0; i < 16; ++i) {
+            const float4 c = cp[i];
+            v[2 * i] = fmaf(shift, c.y, rstd * v[2 * i]) + c.x;
+            v[2 * i + 1] = fmaf(shift, c.w, rstd * v[2 * i + 1]) + c.z;
+          }
+        } else if (bias != nullptr) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const float4 c = cp[i];
+            v[2 * i] += c.x;
+            v[2 * i + 1] += c.z;
+          }
+        }
+        if (EPI != EPI_NONE) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = activate<EPI, true>(v[i]);
+        }
+        if (sizeof(TO) == 2 && res != nullptr && in) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if ((have >> i) & 1) {
+              const uint32_t w[4] = {rp[i].x, rp[i].y, rp[i].z, rp[i].w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                v[8 * i + 2 * e] += __uint_as_float(w[e] << 16);
+                v[8 * i + 2 * e + 1] += __uint_as_float(w[e] & 0xffff0000u);
               }
+            } else if (c0 + 8 * i < HALF_COLS) {
+#pragma unroll
+              for (int e = 0; e < 8; ++e)
+                if (n0 + c0 + 8 * i + e < N) v[8 * i + e] += to_f(res[row + n0 + c0 + 8 * i + e]);
             }
           }
-        } else {
-          uint4* stg = sm.stage[warp - 2];
+          if (c0 + 32 < HALF_COLS) fetch(c0 + 32);
+        }
+        __syncwarp();                     // the columns' constants are read before results overwrite them
 #pragma unroll
-          for (int g8 = 0; g8 < 4; ++g8) {
-            const int n8 = n0 + half * HALF_COLS + c0 + g8 * 8;
-            uint4 u = make_uint4(0u, 0u, 0u, 0u);
-            if (m < M && c0 + g8 * 8 < HALF_COLS && n8 < N) {
-              float v[8];
-              if (SCATTER && n8 >= kv.q_width)   // keys and values: no activation, no residual
-                finish8<EPI_NONE>(v, r + g8 * 8, n8, N, row, bias, bias_vec, nullptr, false, u, fold.colsum, mean, rstd);
-              else
-                finish8<EPI>(v, r + g8 * 8, n8, N, row, bias, bias_vec, residual, (have >> g8) & 1,
-                             g8 == 0 ? res0 : (g8 == 1 ? res1 : (g8 == 2 ? res2 : res3)), fold.colsum, mean, rstd);
-              u = pack8(v);
+        for (int p0 = 0; p0 < 32; p0 += 4 * PER) {      // 64 bytes of each row at a time
+#pragma unroll
+          for (int p = 0; p < 4; ++p) {
+            uint4 u;
+            if (sizeof(TO) == 2) {
+              float w[8];
+#pragma unroll
+              for (int i = 0; i < 8; ++i) w[i] = v[(p * 8 + i) & 31];
+              u = pack8(w);
+            } else {
+              const int i = (p0 + p * 4) & 31;
+              u = make_uint4(__float_as_uint(v[i]), __float_as_uint(v[i + 1]), __float_as_uint(v[i + 2]), __float_as_uint(v[i + 3]));
             }
-            stg[stage_index(lane, g8)] = u;
+            stg[stage_index(lane, p)] = u;
           }
           __syncwarp();
+          const int n = n0 + c0 + p0 + o_piece * PER;
+          const bool n_in = c0 + p0 + o_piece * PER < HALF_COLS && n < N;
 #pragma unroll
           for (int j = 0; j < 4; ++j) {   // four lanes on a row's 64 bytes, eight rows an instruction
-            const int rr = 8 * j + (lane >> 2), piece = lane & 3;
-            const uint4 u = stg[stage_index(rr, piece)];
-            const int mm = m0 + q * 32 + rr;
-            const int n8 = n0 + half * HALF_COLS + c0 + piece * 8;
+            const int rr = 8 * j + o_row;
+            uint4 u = stg[stage_index(rr, o_piece)];
+            const int mm = m0 + rr;
+            if (sizeof(TO) == 4 && res != nullptr && mm < M && n_in) {
+              float* e = reinterpret_cast<float*>(&u);
+              if ((have >> j) & 1) {
+                e[0] += __uint_as_float(rp[j].x); e[1] += __uint_as_float(rp[j].y);
+                e[2] += __uint_as_float(rp[j].z); e[3] += __uint_as_float(rp[j].w);
+              } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                  if (n + i < N) e[i] += to_f(res[(size_t)mm * ldc + n + i]);
+              }
+            }
             long long slot_r = -1;
             int in_page_r = 0;
             if (SCATTER) {   // the row's page, from the lane that looked it up
               slot_r = __shfl_sync(0xffffffffu, slot, rr);
               in_page_r = __shfl_sync(0xffffffffu, in_page, rr);
             }
-            if (mm < M && c0 + piece * 8 < HALF_COLS && n8 < N) {
-              if (SCATTER && n8 >= kv.q_width) {
-                if (slot_r >= 0) scatter_piece(u, n8, kv, slot_r, in_page_r);
+            if (mm < M && n_in) {
+              if (SCATTER && n >= kv.q_width) {
+                if (slot_r >= 0) scatter_piece(u, n, kv, slot_r, in_page_r);
               } else {
-                store_piece(u, n8, N, (size_t)mm * ldc, reinterpret_cast<__nv_bfloat16*>(C));
+                store_piece(u, n, N, (size_t)mm * ldc, C);
               }
             }
           }
-          __syncwarp();   // the pieces are read before the next chunk overwrites them
+          if (sizeof(TO) == 4) fetch(c0 + p0 + 16);
+          __syncwarp();   // the pieces are read before the next ones overwrite them
         }
-        res0 = nx0; res1 = nx1; res2 = nx2; res3 = nx3;
-        have = have_next;
       }
-#undef FETCH_RESIDUAL
     }
   }
 
@@ -475,7 +473,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   const bool aborted = sm.abort_flag != 0;     // the same in both CTAs of a pair from here on
   if (threadIdx.x == 0 && aborted) atomicOr(status, MLXB_ST_WAIT_TIMEOUT);
   if (warp == 1 && leader) {
-    if (lane == 0 && aborted) {
+    if (aborted && elect_one()) {
       // Somebody gave up.  Products this thread issued may still be running on the tensor memory that is freed
       // below: one more commit arrives when all of them have completed; wait for it, bounded.
       if (CG == 2) umma_commit_pair_local(&sm.drained);
@@ -539,10 +537,9 @@ static int sm_count() {
   return n;
 }
 
-template <int BN, int STAGES, typename TO, bool SCATTER = false, int CG = 1>
+template <int BN, int STAGES, typename TO, bool SCATTER, int CG>
 static int launch(const void* A, const void* W, const float* bias, const void* residual, void* C, int M, int N, int K,
-                  int lda, int ldc, int epi, int* status, cudaStream_t stream, const KvScatter& kv = KvScatter{},
-                  const NormFoldRows& fold = NormFoldRows{}) {
+                  int lda, int ldc, int epi, int* status, cudaStream_t stream, const KvScatter& kv, const NormFoldRows& fold) {
   static_assert((BN / CG) % 8 == 0 && BN % (16 * CG) == 0, "a CTA's W rows are whole 8-row swizzle groups");
   static_assert(sizeof(Smem<BN, STAGES, CG>) + 1024 <= 227 * 1024, "stages and staging buffers fit a CTA's shared memory");
   CUtensorMap ma, mw;
@@ -587,31 +584,59 @@ static int launch(const void* A, const void* W, const float* bias, const void* r
   });
 }
 
-// Tile shape.  The width is the one whose waves of tiles over the SMs cost least, a tile's cost being the rows it
-// streams per K step (128 rows of A plus BN rows of W).  Pairs of CTAs on 256 x BN tiles are taken where they were
-// measured faster: long inner dimensions (their gain is in the main loop: 8192 x 8192 x 8192 runs at 1.50 against
-// 1.39 PFLOP/s) with at least three waves of tiles to work on; with short inner dimensions or few tiles the pair's
-// set-up and its hand-overs across the cluster cost more than the main loop gains (2048 x 4096 x 1024: 31.7 against
-// 29.7 us).
+// Tile shape and pairs or not: the form whose time, as a sum of what was measured, is least.  A step of 64 of K takes a CTA
+// 0.95 ns a row of A or W that it brings (128 + BN rows; 1.15 in a pair, whose CTAs bring 128 + BN / 2) or, in a pair, what its
+// products take (1.08 ns a column), and never less than 215 ns; a launch costs 4.5 us besides (set-up, the first copies,
+// the last tile's results; 0.35 for every 32 columns less than 128), a pair's 6.0, and every further wave of tiles 0.8.
+// This gives each form's time within 10 % at M from 288 to 2048, N from 1024 to 6400 and K from 1024 to 6400.  Single
+// CTAs are best for short K (2048 x 1024 x 1024: 8.3 us against 9.5), pairs for many products (2048 x 1600 x 6400: 32.7
+// against 37.3; 2048 x 6400 x 1600: 31.5 against 34.2), and tiles of 64 or 32 columns where wider ones leave SMs idle anyway,
+// for their shorter end (288 x 1280 x 1280: 7.1 against 8.4; 288 x 1280 x 5120: 20.1 against 22.6).
+// A share of K for each of several CTAs would do more there, but then a row's sums would be added in an order that depends on
+// how many rows the call has.
 struct TileChoice { int bn, cg; };
-static TileChoice tile_choice(int M, int N, int K, bool pairs_built) {
-  const int sms = sm_count();
-  const char* want_pair = getenv("MLXB_TC_PAIR");   // experiments and tests: 0 = never, 1 = wherever a pair has two row tiles
-  int cg = 1;
-  if (pairs_built && M > BM) {
-    if (want_pair) cg = want_pair[0] == '1' ? 2 : 1;
-    else if (K >= 2048 && (long long)((M + 2 * BM - 1) / (2 * BM)) * ((N + 255) / 256) >= 3 * (sms / 2)) cg = 2;
+static TileChoice tile_choice(int M, int N, int K) {
+  // experiments and tests: pairs 0 = never, 1 = wherever there are two row tiles; the width
+  const char *want_pair = getenv("MLXB_TC_PAIR"), *want_bn = getenv("MLXB_TC_BN");
+  const int sms = sm_count(), steps = (K + BK - 1) / BK;
+  TileChoice best = {128, 1};
+  double best_cost = -1.;
+  for (int cg = 1; cg <= 2; ++cg) {
+    if (cg == 2 && M <= BM) break;
+    if (want_pair && M > BM && (want_pair[0] == '1') != (cg == 2)) continue;
+    for (int bn : {256, 192, 128, 64, 32}) {
+      if (want_bn ? atoi(want_bn) != bn : (cg == 2 && bn < 128)) continue;
+      const long long tiles = (long long)((M + cg * BM - 1) / (cg * BM)) * ((N + bn - 1) / bn);
+      const int units = sms / cg;
+      const long long waves = (tiles + units - 1) / units;
+      double step = cg == 1 ? 0.95 * (BM + bn) : (1.15 * (BM + bn / 2) > 1.08 * bn ? 1.15 * (BM + bn / 2) : 1.08 * bn);
+      if (step < 215.) step = 215.;
+      const double cost = waves * steps * step + 800. * (waves - 1) + (cg == 1 ? 4500. - (bn < 128 ? 11. * (128 - bn) : 0.) : 6000.);
+      if (best_cost < 0. || cost < best_cost) { best = {bn, cg}; best_cost = cost; }
+    }
   }
-  const int tiles_m = (M + cg * BM - 1) / (cg * BM), units = sms / cg;
-  TileChoice best = {128, cg};
-  long long best_cost = -1;
-  for (int bn : {256, 192, 128}) {
-    const long long tiles = (long long)tiles_m * ((N + bn - 1) / bn);
-    const long long cost = ((tiles + units - 1) / units) * (cg * BM + bn);
-    if (best_cost < 0 || cost < best_cost) { best = {bn, cg}; best_cost = cost; }
-  }
-  if (const char* force = getenv("MLXB_TC_BN")) best.bn = atoi(force);   // experiments and tests
   return best;
+}
+
+// Runs the form that tile_choice took.
+template <typename TO, bool SCATTER>
+static int launch_choice(const void* A, const void* W, const float* bias, const void* residual, void* C, int M, int N, int K,
+                         int lda, int ldc, int epi, int* status, cudaStream_t stream, const KvScatter& kv,
+                         const NormFoldRows& fold) {
+  const TileChoice t = tile_choice(M, N, K);
+#define GO(BN_, ST_, CG_) \
+  return launch<BN_, ST_, TO, SCATTER, CG_>(A, W, bias, residual, C, M, N, K, lda, ldc, epi, status, stream, kv, fold);
+  if (t.cg == 2) {
+    if (t.bn == 256) GO(256, 6, 2)
+    if (t.bn == 192) GO(192, 6, 2)
+    GO(128, 8, 2)
+  }
+  if (t.bn == 256) GO(256, 4, 1)
+  if (t.bn == 192) GO(192, 4, 1)
+  if (t.bn == 128) GO(128, 6, 1)
+  if (t.bn == 64) GO(64, 7, 1)
+  GO(32, 8, 1)
+#undef GO
 }
 
 // A: bfloat16 [M, K] at row stride lda; W: bfloat16 [N, K] contiguous; bias float32[N] or null; residual of C's dtype
@@ -648,28 +673,9 @@ static int linear_tcgen05(int out_f32, const void* A, const void* W, const float
   if (((uintptr_t)A & 15) || ((uintptr_t)W & 15))
     return mlxb_fail(MLXB_BAD_ARG, "linear (tensor cores): operands must be 16-byte aligned");
   if (!activation_known(epi)) return mlxb_fail(MLXB_BAD_ARG, "linear: epilogue code %d", epi);
-  const TileChoice best = tile_choice(M, N, K, !out_f32);   // pairs are built for bfloat16 results
-#define GO(BN_, ST_)                                                                                              \
-  {                                                                                                               \
-    if (out_f32)                                                                                                  \
-      return launch<BN_, ST_, float>(A, W, bias, residual, C, M, N, K, lda, ldc, epi, status, stream, KvScatter{}, \
-                                     fold);                                                                       \
-    return launch<BN_, ST_, __nv_bfloat16>(A, W, bias, residual, C, M, N, K, lda, ldc, epi, status, stream,        \
-                                           KvScatter{}, fold);                                                    \
-  }
-#define GO2(BN_, ST_)                                                                                             \
-  return launch<BN_, ST_, __nv_bfloat16, false, 2>(A, W, bias, residual, C, M, N, K, lda, ldc, epi, status, stream, \
-                                                   KvScatter{}, fold);
-  if (best.cg == 2) {
-    if (best.bn == 256) GO2(256, 6)
-    if (best.bn == 192) GO2(192, 6)
-    GO2(128, 8)
-  }
-  if (best.bn == 256) GO(256, 4)
-  if (best.bn == 192) GO(192, 4)
-  GO(128, 6)
-#undef GO
-#undef GO2
+  if (out_f32)
+    return launch_choice<float, false>(A, W, bias, residual, C, M, N, K, lda, ldc, epi, status, stream, KvScatter{}, fold);
+  return launch_choice<__nv_bfloat16, false>(A, W, bias, residual, C, M, N, K, lda, ldc, epi, status, stream, KvScatter{}, fold);
 }
 
 
@@ -716,17 +722,5 @@ static int linear_tcgen05_qkv(const void* A, const void* W, const float* bias, v
     return mlxb_fail(MLXB_BAD_ARG, "linear (q|k|v): %d outputs for %d query columns and 2 x %d x %d", N, q_width, Hkv, Dh);
   const KvScatter kv = {positions, token_req, block_table, (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, status,
                         max_pages, n_pages, page, Hkv, Dh, q_width};
-  const TileChoice best = tile_choice(M, N, K, true);
-  if (best.cg == 2) {
-    if (best.bn == 256)
-      return launch<256, 6, __nv_bfloat16, true, 2>(A, W, bias, nullptr, C, M, N, K, lda, ldc, EPI_NONE, status, stream, kv, fold);
-    if (best.bn == 192)
-      return launch<192, 6, __nv_bfloat16, true, 2>(A, W, bias, nullptr, C, M, N, K, lda, ldc, EPI_NONE, status, stream, kv, fold);
-    return launch<128, 8, __nv_bfloat16, true, 2>(A, W, bias, nullptr, C, M, N, K, lda, ldc, EPI_NONE, status, stream, kv, fold);
-  }
-  if (best.bn == 256)
-    return launch<256, 4, __nv_bfloat16, true>(A, W, bias, nullptr, C, M, N, K, lda, ldc, EPI_NONE, status, stream, kv, fold);
-  if (best.bn == 192)
-    return launch<192, 4, __nv_bfloat16, true>(A, W, bias, nullptr, C, M, N, K, lda, ldc, EPI_NONE, status, stream, kv, fold);
-  return launch<128, 6, __nv_bfloat16, true>(A, W, bias, nullptr, C, M, N, K, lda, ldc, EPI_NONE, status, stream, kv, fold);
+  return launch_choice<__nv_bfloat16, true>(A, W, bias, nullptr, C, M, N, K, lda, ldc, EPI_NONE, status, stream, kv, fold);
 }
