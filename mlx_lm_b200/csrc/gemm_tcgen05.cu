@@ -57,10 +57,11 @@ constexpr int epi_slices(int bn) { return bn >= 128 ? EPI_WARPS / 4 : bn / 32; }
 __device__ int g_test_withhold_arrival = 0;
 #endif
 
-template <int BN, int STAGES, int CG>
+// A stage holds KB blocks of 64 of K, each a tile of its own.
+template <int BN, int STAGES, int KB, int CG>
 struct Smem {
-  alignas(1024) __nv_bfloat16 a[STAGES][BM * BK];
-  alignas(1024) __nv_bfloat16 b[STAGES][(BN / CG) * BK];   // in a pair: this CTA's half of the W rows
+  alignas(1024) __nv_bfloat16 a[STAGES][KB * BM * BK];
+  alignas(1024) __nv_bfloat16 b[STAGES][KB * (BN / CG) * BK];   // in a pair: this CTA's half of the W rows
   alignas(8) uint64_t full[STAGES];
   uint64_t empty[STAGES];
   uint64_t acc_full[2];
@@ -122,16 +123,16 @@ __device__ __forceinline__ void scatter_piece(uint4 u, int n8, const KvScatter& 
   *reinterpret_cast<uint4*>(pool + ((size_t)slot + (size_t)hh * kv.page + in_page) * kv.Dh + d) = u;
 }
 
-template <int BN, int STAGES, typename TO, int EPI, bool SCATTER, int CG>
+template <int BN, int STAGES, int KB, typename TO, int EPI, bool SCATTER, int CG>
 __global__ void __launch_bounds__(THREADS)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                     const float* __restrict__ bias, const __nv_bfloat16* residual, TO* C, int M, int N, int K,
                     int ldc, int* __restrict__ status, KvScatter kv, NormFoldRows fold) {
   extern __shared__ uint8_t smem_raw[];
-  Smem<BN, STAGES, CG>& sm = *reinterpret_cast<Smem<BN, STAGES, CG>*>(
+  Smem<BN, STAGES, KB, CG>& sm = *reinterpret_cast<Smem<BN, STAGES, KB, CG>*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int k_tiles = (K + BK - 1) / BK;
+  const int k_tiles = (K + KB * BK - 1) / (KB * BK);     // stages a tile; blocks beyond K arrive as zeros
   // A tile is (CG * 128) x BN; in a pair the CTA of rank r takes rows 128 r .. 128 r + 127 of it and fetches rows
   // (BN / 2) r .. of the tile's W rows.  Pair (or CTA) c takes tiles c, c + step, ...
   const int rank = CG == 2 ? (int)cluster_rank() : 0;
@@ -142,7 +143,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   auto tile_m0 = [&](int t) { return (t % tiles_m) * (CG * BM) + rank * BM; };      // this CTA's first row
   auto tile_n0 = [&](int t) { return (t / tiles_m) * BN; };                          // the tile's first column
   constexpr int W_ROWS = BN / CG;                          // W rows per copy
-  constexpr uint32_t STAGE_BYTES = CG * (BM + W_ROWS) * BK * sizeof(__nv_bfloat16);   // counted on a stage's barrier
+  constexpr uint32_t STAGE_BYTES = CG * KB * (BM + W_ROWS) * BK * sizeof(__nv_bfloat16);   // counted on a stage's barrier
   constexpr uint32_t TMEM_COLS = BN <= 128 ? 2 * BN : 512;   // two accumulators; a power of two
 
   if (threadIdx.x == 0) {
@@ -183,12 +184,20 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   const uint32_t tmem_base = sm.tmem_base;
   // this CTA's copies of a stage: its rows of A, its rows of W
   auto load_a = [&](int s, int kt, int m0) {
-    if (CG == 2) tma_load_2d_pair(sm.a[s], &map_a, kt * BK, m0, peer_addr(&sm.full[s], 0));
-    else tma_load_2d(sm.a[s], &map_a, kt * BK, m0, &sm.full[s]);
+#pragma unroll
+    for (int kb = 0; kb < KB; ++kb) {
+      __nv_bfloat16* dst = sm.a[s] + kb * (BM * BK);
+      if (CG == 2) tma_load_2d_pair(dst, &map_a, (kt * KB + kb) * BK, m0, peer_addr(&sm.full[s], 0));
+      else tma_load_2d(dst, &map_a, (kt * KB + kb) * BK, m0, &sm.full[s]);
+    }
   };
   auto load_w = [&](int s, int kt, int n0) {
-    if (CG == 2) tma_load_2d_pair(sm.b[s], &map_w, kt * BK, n0 + rank * W_ROWS, peer_addr(&sm.full[s], 0));
-    else tma_load_2d(sm.b[s], &map_w, kt * BK, n0, &sm.full[s]);
+#pragma unroll
+    for (int kb = 0; kb < KB; ++kb) {
+      __nv_bfloat16* dst = sm.b[s] + kb * (W_ROWS * BK);
+      if (CG == 2) tma_load_2d_pair(dst, &map_w, (kt * KB + kb) * BK, n0 + rank * W_ROWS, peer_addr(&sm.full[s], 0));
+      else tma_load_2d(dst, &map_w, (kt * KB + kb) * BK, n0, &sm.full[s]);
+    }
   };
   if (threadIdx.x == 0)
     for (int s = 0; s < early; ++s) load_w(s, s, tile_n0(first_tile));
@@ -236,7 +245,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       constexpr uint32_t idesc = umma_idesc(CG * BM, BN);
       // the same offsets in both CTAs of a pair: the descriptors name them in each CTA's own shared memory
       const uint64_t da0 = umma_desc(smem_u32(sm.a[0])), db0 = umma_desc(smem_u32(sm.b[0]));
-      constexpr uint32_t A_STEP = BM * BK * 2 / 16, B_STEP = W_ROWS * BK * 2 / 16;   // a stage, in units of 16 bytes
+      constexpr uint32_t A_STEP = BM * BK * 2 / 16, B_STEP = W_ROWS * BK * 2 / 16;   // a block, in units of 16 bytes
       int s = 0, it = 0;
       uint32_t ph = 0;
       bool ok = true;
@@ -251,12 +260,14 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           ok = mbar_wait_warp(&sm.full[s], ph, abort_flag, peer_abort);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint64_t da = da0 + (uint32_t)s * A_STEP, db = db0 + (uint32_t)s * B_STEP;
+          const uint64_t da = da0 + (uint32_t)(s * KB) * A_STEP, db = db0 + (uint32_t)(s * KB) * B_STEP;
           if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < BK / 16; ++k) {   // 16 bf16 = 32 bytes = 2 units of the descriptor's start address
-              if (CG == 2) umma_bf16_pair(tmem_acc, da + 2 * k, db + 2 * k, idesc, (kt > 0 || k > 0) ? 1u : 0u);
-              else umma_bf16(tmem_acc, da + 2 * k, db + 2 * k, idesc, (kt > 0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < KB * (BK / 16); ++k) {   // 16 bf16 = 32 bytes = 2 units of the descriptor's start address
+              const uint64_t ak = da + (k / (BK / 16)) * A_STEP + 2 * (k % (BK / 16));
+              const uint64_t bk = db + (k / (BK / 16)) * B_STEP + 2 * (k % (BK / 16));
+              if (CG == 2) umma_bf16_pair(tmem_acc, ak, bk, idesc, (kt > 0 || k > 0) ? 1u : 0u);
+              else umma_bf16(tmem_acc, ak, bk, idesc, (kt > 0 || k > 0) ? 1u : 0u);
             }
             // the stage is free once these MMAs have read it
             if (CG == 2) umma_commit_both(&sm.empty[s]);
@@ -367,9 +378,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           if (CG == 2) mbar_arrive_cluster(acc_empty_leader[b]);   // the leader issues the products into both halves
           else mbar_arrive(&sm.acc_empty[b]);
         }
-        float v[32];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+        float* v = reinterpret_cast<float*>(r);
         const float4* cp = reinterpret_cast<const float4*>(stg);      // (bias, column sum) of two columns: the same for every lane
         if (fold.colsum != nullptr) {
 #pragma unroll
@@ -537,22 +546,22 @@ static int sm_count() {
   return n;
 }
 
-template <int BN, int STAGES, typename TO, bool SCATTER, int CG>
+template <int BN, int STAGES, int KB, typename TO, bool SCATTER, int CG>
 static int launch(const void* A, const void* W, const float* bias, const void* residual, void* C, int M, int N, int K,
                   int lda, int ldc, int epi, int* status, cudaStream_t stream, const KvScatter& kv, const NormFoldRows& fold) {
   static_assert((BN / CG) % 8 == 0 && BN % (16 * CG) == 0, "a CTA's W rows are whole 8-row swizzle groups");
-  static_assert(sizeof(Smem<BN, STAGES, CG>) + 1024 <= 227 * 1024, "stages and staging buffers fit a CTA's shared memory");
+  static_assert(sizeof(Smem<BN, STAGES, KB, CG>) + 1024 <= 227 * 1024, "stages and staging buffers fit a CTA's shared memory");
   CUtensorMap ma, mw;
   if (int e = make_map(&ma, A, M, K, lda, BM)) return e;
   if (int e = make_map(&mw, W, N, K, K, BN / CG)) return e;      // a copy brings this CTA's rows of the tile
-  const size_t smem = sizeof(Smem<BN, STAGES, CG>) + 1024;
+  const size_t smem = sizeof(Smem<BN, STAGES, KB, CG>) + 1024;
   const int n_tiles = ((M + CG * BM - 1) / (CG * BM)) * ((N + BN - 1) / BN);
   const int units = sm_count() / CG;                              // CTAs, or pairs of them
   const dim3 grid(CG * (n_tiles < units ? n_tiles : units));
   // The fused cache write has no activation: only the plain epilogue is built for it.
   return dispatch_activation(SCATTER ? (int)EPI_NONE : epi, [&](auto e) {
     constexpr int EPI = SCATTER ? (int)EPI_NONE : (int)decltype(e)::value;
-    auto kern = gemm_tcgen05_kernel<BN, STAGES, TO, EPI, SCATTER, CG>;
+    auto kern = gemm_tcgen05_kernel<BN, STAGES, KB, TO, EPI, SCATTER, CG>;
     static bool raised = false;   // once per instantiation, and never for the first time inside a stream capture
     if (!raised) {
       cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -584,14 +593,14 @@ static int launch(const void* A, const void* W, const float* bias, const void* r
   });
 }
 
-// Tile shape and pairs or not: the form whose time, as a sum of what was measured, is least.  A step of 64 of K takes a CTA
+// Tile shape and pairs or not: the form whose time, as a sum of what was measured, is least.  A block of 64 of K takes a CTA
 // 0.95 ns a row of A or W that it brings (128 + BN rows; 1.15 in a pair, whose CTAs bring 128 + BN / 2) or, in a pair, what its
-// products take (1.08 ns a column), and never less than 215 ns; a launch costs 4.5 us besides (set-up, the first copies,
-// the last tile's results; 0.35 for every 32 columns less than 128), a pair's 6.0, and every further wave of tiles 0.8.
-// This gives each form's time within 10 % at M from 288 to 2048, N from 1024 to 6400 and K from 1024 to 6400.  Single
-// CTAs are best for short K (2048 x 1024 x 1024: 8.3 us against 9.5), pairs for many products (2048 x 1600 x 6400: 32.7
-// against 37.3; 2048 x 6400 x 1600: 31.5 against 34.2), and tiles of 64 or 32 columns where wider ones leave SMs idle anyway,
-// for their shorter end (288 x 1280 x 1280: 7.1 against 8.4; 288 x 1280 x 5120: 20.1 against 22.6).
+// products take (1.08 ns a column); a launch costs 4.5 us besides (set-up, the first copies, the last tile's results;
+// 1.2 less on tiles of 32, 0.9 on tiles of 64 columns), a pair's 6.0, and every further wave of tiles 0.8.  This gives each
+// form's time within 15 % at M from 128 to 2048, N from 1024 to 6400 and K from 1024 to 6400.  Single CTAs are best for short K
+// (2048 x 1024 x 1024: 7.9 us against 8.9), pairs for many products (2048 x 1600 x 6400: 33.9 against 38.0; 2048 x 6400 x
+// 1600: 31.4 against 34.0), and tiles of 64 or 32 columns where wider ones leave SMs idle (288 x 1280 x 1280: 6.0 against 7.7;
+// 288 x 1280 x 5120: 15.4 against 22.9; 768 x 1024 x 1024: 6.0 against 7.1).
 // A share of K for each of several CTAs would do more there, but then a row's sums would be added in an order that depends on
 // how many rows the call has.
 struct TileChoice { int bn, cg; };
@@ -609,9 +618,8 @@ static TileChoice tile_choice(int M, int N, int K) {
       const long long tiles = (long long)((M + cg * BM - 1) / (cg * BM)) * ((N + bn - 1) / bn);
       const int units = sms / cg;
       const long long waves = (tiles + units - 1) / units;
-      double step = cg == 1 ? 0.95 * (BM + bn) : (1.15 * (BM + bn / 2) > 1.08 * bn ? 1.15 * (BM + bn / 2) : 1.08 * bn);
-      if (step < 215.) step = 215.;
-      const double cost = waves * steps * step + 800. * (waves - 1) + (cg == 1 ? 4500. - (bn < 128 ? 11. * (128 - bn) : 0.) : 6000.);
+      const double step = cg == 1 ? 0.95 * (BM + bn) : (1.15 * (BM + bn / 2) > 1.08 * bn ? 1.15 * (BM + bn / 2) : 1.08 * bn);
+      const double cost = waves * steps * step + 800. * (waves - 1) + (cg == 1 ? (bn == 32 ? 3300. : (bn == 64 ? 3600. : 4500.)) : 6000.);
       if (best_cost < 0. || cost < best_cost) { best = {bn, cg}; best_cost = cost; }
     }
   }
@@ -624,18 +632,21 @@ static int launch_choice(const void* A, const void* W, const float* bias, const 
                          int lda, int ldc, int epi, int* status, cudaStream_t stream, const KvScatter& kv,
                          const NormFoldRows& fold) {
   const TileChoice t = tile_choice(M, N, K);
-#define GO(BN_, ST_, CG_) \
-  return launch<BN_, ST_, TO, SCATTER, CG_>(A, W, bias, residual, C, M, N, K, lda, ldc, epi, status, stream, kv, fold);
+#define GO(BN_, ST_, KB_, CG_) \
+  return launch<BN_, ST_, KB_, TO, SCATTER, CG_>(A, W, bias, residual, C, M, N, K, lda, ldc, epi, status, stream, kv, fold);
+  // stages of two blocks where a block's products take less than what surrounds them (waits, votes and commits, some
+  // 0.18 us a stage): 288 x 1280 x 5120 on tiles of 32 columns 15.4 us against 20.1 with stages of one; wider ones gain
+  // nothing by it and lose the depth of the ring (pairs of 256 x 192, 2048 x 1600 x 6400: 36.2 against 33.9)
   if (t.cg == 2) {
-    if (t.bn == 256) GO(256, 6, 2)
-    if (t.bn == 192) GO(192, 6, 2)
-    GO(128, 8, 2)
+    if (t.bn == 256) GO(256, 6, 1, 2)
+    if (t.bn == 192) GO(192, 6, 1, 2)
+    GO(128, 4, 2, 2)
   }
-  if (t.bn == 256) GO(256, 4, 1)
-  if (t.bn == 192) GO(192, 4, 1)
-  if (t.bn == 128) GO(128, 6, 1)
-  if (t.bn == 64) GO(64, 7, 1)
-  GO(32, 8, 1)
+  if (t.bn == 256) GO(256, 4, 1, 1)
+  if (t.bn == 192) GO(192, 4, 1, 1)
+  if (t.bn == 128) GO(128, 3, 2, 1)
+  if (t.bn == 64) GO(64, 4, 2, 1)
+  GO(32, 4, 2, 1)
 #undef GO
 }
 

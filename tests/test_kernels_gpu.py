@@ -259,6 +259,41 @@ def test_linear_tensor_cores(ops, M, N, K, pairs, monkeypatch):
     assert int(status.item()) == 0
 
 
+@pytest.mark.parametrize("M,N,K", [(65, 7, 8), (129, 33, 72), (288, 160, 1280), (300, 250, 200), (700, 1000, 64)])
+@pytest.mark.parametrize("width", ["32", "64", "128", "192", "256"])
+def test_linear_tensor_cores_forms(ops, M, N, K, width, monkeypatch):
+    """Every tile width, stages of one and of two blocks of K (whole and cut), single CTAs and pairs, float32 and bfloat16
+    results, with folded norm, bias, activation and residual (at a row stride that cuts whole pieces): the same
+    products in the same order, so the same bits whatever the form; and the plain statement within rounding."""
+    g = torch.Generator().manual_seed(M + N + K)
+    x = torch.randn(M, K, generator=g).to(torch.bfloat16).cuda()
+    w = (torch.randn(N, K, generator=g) / math.sqrt(K)).to(torch.bfloat16).cuda()
+    b, colsum = torch.randn(N, generator=g).cuda(), torch.randn(N, generator=g).cuda()
+    stats = torch.stack([torch.randn(M, generator=g), torch.rand(M, generator=g) + 0.5], dim=1).cuda()
+    res = torch.randn(M, N + 3, generator=g).cuda()[:, :N]
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    plain = x.double() @ w.double().t()
+    want = R.gelu_new((stats[:, 1:].double() * (plain - stats[:, :1].double() * colsum.double()) + b.double()).float().cpu())
+    want = want + res.cpu()
+
+    def run(dtype):
+        out = torch.empty(M, N + 3, device="cuda").to(dtype)[:, :N]
+        r = torch.empty(M, N + 3, device="cuda").to(dtype)[:, :N]
+        r.copy_(res)
+        ops.linear_tensor_cores(x, w, b, out, status, stream(), epilogue=ops.EPI_GELU_NEW, residual=r, fold=(colsum, stats))
+        return out.clone()
+    base = {d: run(d) for d in DTYPES}                 # the form that the launcher picks
+    monkeypatch.setenv("MLXB_TC_BN", width)
+    for pairs in ("0", "1"):
+        if pairs == "1" and int(width) < 128:
+            continue
+        monkeypatch.setenv("MLXB_TC_PAIR", pairs)
+        for d in DTYPES:
+            assert torch.equal(run(d), base[d]), (d, pairs)
+    assert rel_err(base[torch.float32], want) <= 2e-5 and rel_err(base[torch.bfloat16], want) <= 6e-3
+    assert int(status.item()) == 0
+
+
 @pytest.mark.parametrize("M,N,K", [(3, 200, 96), (40, 1000, 320), (200, 320, 96)])
 def test_every_activation_of_the_list_in_every_linear_kernel(ops, M, N, K):
     """The epilogue activations are one list (csrc/activations.cuh) that every linear kernel is compiled from
