@@ -287,7 +287,7 @@ mamba2_scan_kernel(const T* xbc, int ldx, int x_off, int b_off, int c_off, const
                    const float* __restrict__ dt_bias, const float* __restrict__ A_log,
                    const float* __restrict__ Dskip, float* state, const int* __restrict__ slots,
                    const int* __restrict__ token_req, const int* __restrict__ req_first_token, float* __restrict__ y,
-                   int ldy, int H, int G, int N, int V, int VB) {
+                   int ldy, int H, int G, int N, int V, int VB, int max_run) {
   extern __shared__ __align__(16) float sm[];
   constexpr int NP = NS * SCAN_SEG;        // floats of a token's staged B (or C)
   float* sB = sm;                          // [CHUNK][NP]
@@ -311,7 +311,7 @@ mamba2_scan_kernel(const T* xbc, int ldx, int x_off, int b_off, int c_off, const
   xbc = after_wait(xbc);
   dt_raw = after_wait(dt_raw);
   const int n = request_rows(token_req, t0, t1, r);
-  if (n == 0) return;
+  if (n == 0 || n > max_run) return;
   const float negA = -expf(A_log[h]), skip = Dskip[h], bias = dt_bias[h];
   for (int c0 = 0; c0 < n; c0 += SCAN_CHUNK) {
     const int nc = min(SCAN_CHUNK, n - c0);
@@ -391,12 +391,12 @@ mamba2_scan_kernel(const T* xbc, int ldx, int x_off, int b_off, int c_off, const
 
 // xbc: the convolution's output [n_tokens, ...] (activation dtype) holding x (H*V columns from x_off), B and C (G*N
 // columns each from b_off / c_off); dt_raw: [n_tokens, >= H] at row stride lddt; state: float32 [slots, H, V, N] (column by column);
-// y: float32 [n_tokens, H*V] at row stride ldy.
+// y: float32 [n_tokens, H*V] at row stride ldy.  max_run: only requests that bring up to so many rows (0: all).
 MLXB_EXPORT int mlxb_mamba2_scan(int dtype, const void* xbc, int ldx, int x_off, int b_off, int c_off,
                                  const void* dt_raw, int lddt, const float* dt_bias, const float* A_log,
                                  const float* Dskip, float* state, const int* slots, const int* token_req,
                                  const int* req_first_token, float* y, int ldy, int H, int G, int N, int V,
-                                 int n_requests, cudaStream_t stream) {
+                                 int n_requests, int max_run, cudaStream_t stream) {
   if (n_requests <= 0) return 0;
   if (H <= 0 || G <= 0 || H % G || N <= 0 || V <= 0 || N > 32 * SCAN_NPT || n_requests > 65535)
     return mlxb_fail(MLXB_BAD_ARG, "mamba2_scan: %d heads in %d groups, state %d x %d (at most %d rows)", H, G, N, V,
@@ -416,7 +416,7 @@ MLXB_EXPORT int mlxb_mamba2_scan(int dtype, const void* xbc, int ldx, int x_off,
     if (e == cudaSuccess)                                                                                                \
       launch_pdl(mamba2_scan_kernel<T_, NS_>, grid, dim3(sh.threads), smem, stream, (const T_*)xbc, ldx, x_off, b_off,   \
                  c_off, (const T_*)dt_raw, lddt, dt_bias, A_log, Dskip, state, slots, token_req, req_first_token, y,     \
-                 ldy, H, G, N, V, sh.VB);                                                                                \
+                 ldy, H, G, N, V, sh.VB, max_run > 0 ? max_run : 1 << 30);                                                                                \
   }
 #define M2_NS(NS_) { if (dtype == MLXB_F32) M2_GO(float, NS_) else M2_GO(__nv_bfloat16, NS_) }
   switch (sh.NS) {
@@ -439,7 +439,7 @@ gated_delta_scan_kernel(const T* qkv, int ldq, int q_off, int k_off, int v_off, 
                         const T* a_raw, int lda, const float* __restrict__ dt_bias, const float* __restrict__ A_log,
                         float* state, const int* __restrict__ slots, const int* __restrict__ token_req,
                         const int* __restrict__ req_first_token, float* __restrict__ o, int ldo, int H, int G, int K,
-                        int V, int VB) {
+                        int V, int VB, int max_run) {
   extern __shared__ __align__(16) float sm[];
   constexpr int NP = NS * SCAN_SEG;        // floats of a token's staged q (or k)
   float* sq = sm;                          // [CHUNK][NP]
@@ -463,7 +463,7 @@ gated_delta_scan_kernel(const T* qkv, int ldq, int q_off, int k_off, int v_off, 
   b_raw = after_wait(b_raw);
   a_raw = after_wait(a_raw);
   const int n = request_rows(token_req, t0, t1, r);
-  if (n == 0) return;
+  if (n == 0 || n > max_run) return;
   const float negA = -expf(A_log[h]), bias = dt_bias[h], q_scale = 1.f / sqrtf((float)K);
   for (int c0 = 0; c0 < n; c0 += SCAN_CHUNK) {
     const int nc = min(SCAN_CHUNK, n - c0);
@@ -568,12 +568,12 @@ gated_delta_scan_kernel(const T* qkv, int ldq, int q_off, int k_off, int v_off, 
 
 // qkv: the convolutions' output [n_tokens, ...] (activation dtype): q and k (G*K columns each from q_off / k_off),
 // v (H*V columns from v_off); b_raw, a_raw: [n_tokens, >= H] at row strides ldb / lda; state: float32 [slots, H, V, K] (column by column);
-// o: float32 [n_tokens, H*V] at row stride ldo.
+// o: float32 [n_tokens, H*V] at row stride ldo.  max_run: as above.
 MLXB_EXPORT int mlxb_gated_delta_scan(int dtype, const void* qkv, int ldq, int q_off, int k_off, int v_off,
                                       const void* b_raw, int ldb, const void* a_raw, int lda, const float* dt_bias,
                                       const float* A_log, float* state, const int* slots, const int* token_req,
                                       const int* req_first_token, float* o, int ldo, int H, int G, int K, int V,
-                                      int n_requests, cudaStream_t stream) {
+                                      int n_requests, int max_run, cudaStream_t stream) {
   if (n_requests <= 0) return 0;
   if (H <= 0 || G <= 0 || H % G || K <= 0 || V <= 0 || K > 32 * SCAN_NPT || n_requests > 65535)
     return mlxb_fail(MLXB_BAD_ARG, "gated_delta_scan: %d heads over %d key heads, state %d x %d (at most %d rows)", H, G,
@@ -593,7 +593,7 @@ MLXB_EXPORT int mlxb_gated_delta_scan(int dtype, const void* qkv, int ldq, int q
     if (e == cudaSuccess)                                                                                                 \
       launch_pdl(gated_delta_scan_kernel<T_, NS_>, grid, dim3(sh.threads), smem, stream, (const T_*)qkv, ldq, q_off,      \
                  k_off, v_off, (const T_*)b_raw, ldb, (const T_*)a_raw, lda, dt_bias, A_log, state, slots, token_req,     \
-                 req_first_token, o, ldo, H, G, K, V, sh.VB);                                                             \
+                 req_first_token, o, ldo, H, G, K, V, sh.VB, max_run > 0 ? max_run : 1 << 30);                                                             \
   }
 #define GD_NS(NS_) { if (dtype == MLXB_F32) GD_GO(float, NS_) else GD_GO(__nv_bfloat16, NS_) }
   switch (sh.NS) {

@@ -49,7 +49,7 @@ _DT = {torch.float32: F32, torch.bfloat16: BF16}
 
 # kernel sources that only a bfloat16 run launches from: a float32 run neither compiles nor loads them
 BF16_ONLY_LIBS = frozenset({"gemm_smallm", "gemm_smallm_fold", "gemm_tcgen05", "attention_prefill",
-                            "attention_prefill_tc", "attention_wide_tc", "moe_tcgen05"})
+                            "attention_prefill_tc", "attention_wide_tc", "moe_tcgen05", "recurrent_chunks"})
 
 # status word bits set by kernels (csrc/common.cuh)
 ST_TOKEN_RANGE, ST_POSITION_RANGE, ST_PAGE_RANGE, ST_WAIT_TIMEOUT = 1, 2, 4, 8
@@ -1029,15 +1029,15 @@ def conv_silu(x, weight, bias, state, slots, positions, token_req, req_first_tok
 
 
 _M2_ARGS = [c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
-            c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]
+            c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]
 
 
 def mamba2_scan(xbc, x_off: int, b_off: int, c_off: int, dt_raw, dt_bias, a_log, d_skip, state, slots, token_req,
-                req_first_token, y, n_heads: int, n_groups: int, stream) -> None:
+                req_first_token, y, n_heads: int, n_groups: int, stream, max_run: int = 0) -> None:
     """The selective state-space recurrence per (request, head): ``S <- exp(-exp(A_log) dt) S + dt B x^T``,
     ``y = S^T C + D x`` with ``dt = softplus(dt_raw + dt_bias)``.  ``xbc [T, .]`` holds x, B, C from the given
     column offsets; ``state`` float32 ``[slots, heads, V, N]`` (a head's ``N x V`` state column by column); ``y``
-    float32 ``[T, heads*V]``."""
+    float32 ``[T, heads*V]``.  ``max_run``: only requests that bring up to so many rows (0: all)."""
     _need(xbc, dt_raw.dtype, "mamba2_scan xbc")
     _need(state, torch.float32, "mamba2_scan state")
     _need(y, torch.float32, "mamba2_scan y")
@@ -1049,19 +1049,46 @@ def mamba2_scan(xbc, x_off: int, b_off: int, c_off: int, dt_raw, dt_bias, a_log,
     _call("recurrent", "mlxb_mamba2_scan", _M2_ARGS, dtype_code(xbc.dtype), _p(xbc), _rows(xbc, "mamba2_scan xbc"), x_off,
           b_off, c_off, _p(dt_raw), _rows(dt_raw, "mamba2_scan dt"), _p(dt_bias), _p(a_log), _p(d_skip), _p(state),
           _p(slots), _p(token_req), _p(req_first_token), _p(y), _rows(y, "mamba2_scan y"), H, n_groups, N, V,
+          slots.numel(), int(max_run), stream)
+
+
+def recurrent_chunks_supported(dtype, state_rows: int, limit: int) -> bool:
+    """Whether runs of several rows go through the chunked kernels: bfloat16 inputs, states of up to ``limit`` rows."""
+    return dtype == torch.bfloat16 and state_rows <= limit
+
+
+MAMBA2_CHUNK_ROWS, DELTA_CHUNK_ROWS = 128, 64      # rows of a state that the chunked kernels take at most
+
+
+def mamba2_chunks(xbc, x_off: int, b_off: int, c_off: int, dt_raw, dt_bias, a_log, d_skip, state, slots, token_req,
+                  req_first_token, y, n_heads: int, n_groups: int, stream) -> None:
+    """``mamba2_scan`` for the requests that bring several rows, 64 rows at a time on tensor cores (bfloat16 inputs,
+    csrc/recurrent_chunks.cu); requests with a single row are left to the scan."""
+    _need(xbc, torch.bfloat16, "mamba2_chunks xbc")
+    _need(dt_raw, torch.bfloat16, "mamba2_chunks dt")
+    _need(state, torch.float32, "mamba2_chunks state")
+    _need(y, torch.float32, "mamba2_chunks y")
+    _, H, V, N = state.shape
+    if H != n_heads or y.shape[1] != H * V or not state.is_contiguous() or N > MAMBA2_CHUNK_ROWS:
+        raise KernelError(f"mamba2_chunks: state {tuple(state.shape)} for {n_heads} heads, y {tuple(y.shape)}")
+    for t in (dt_bias, a_log, d_skip):
+        _need(t, torch.float32, "mamba2_chunks head constants")
+    _call("recurrent_chunks", "mlxb_mamba2_chunks", _M2_ARGS[1:-2] + [c_void_p], _p(xbc), _rows(xbc, "mamba2_chunks xbc"), x_off,
+          b_off, c_off, _p(dt_raw), _rows(dt_raw, "mamba2_chunks dt"), _p(dt_bias), _p(a_log), _p(d_skip), _p(state),
+          _p(slots), _p(token_req), _p(req_first_token), _p(y), _rows(y, "mamba2_chunks y"), H, n_groups, N, V,
           slots.numel(), stream)
 
 
 _GD_ARGS = [c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
-            c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]
+            c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]
 
 
 def gated_delta_scan(qkv, q_off: int, k_off: int, v_off: int, b_raw, a_raw, dt_bias, a_log, state, slots, token_req,
-                     req_first_token, o, n_heads: int, n_key_heads: int, stream) -> None:
+                     req_first_token, o, n_heads: int, n_key_heads: int, stream, max_run: int = 0) -> None:
     """The gated delta rule per (request, head): ``S <- g S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q`` with
     q and k made unit vectors (q also divided by sqrt(dim)), ``beta = sigmoid(b_raw)``,
     ``g = exp(-exp(A_log) softplus(a_raw + dt_bias))``.  ``state`` float32 ``[slots, heads, V, K]`` (a head's
-    ``K x V`` state column by column); ``o`` float32."""
+    ``K x V`` state column by column); ``o`` float32.  ``max_run``: only requests that bring up to so many rows (0: all)."""
     _need(state, torch.float32, "gated_delta_scan state")
     _need(o, torch.float32, "gated_delta_scan o")
     _need(b_raw, qkv.dtype, "gated_delta_scan b")
@@ -1070,6 +1097,23 @@ def gated_delta_scan(qkv, q_off: int, k_off: int, v_off: int, b_raw, a_raw, dt_b
     if H != n_heads or o.shape[1] != H * V or not state.is_contiguous():
         raise KernelError(f"gated_delta_scan: state {tuple(state.shape)} for {n_heads} heads, o {tuple(o.shape)}")
     _call("recurrent", "mlxb_gated_delta_scan", _GD_ARGS, dtype_code(qkv.dtype), _p(qkv), _rows(qkv, "gated_delta qkv"),
+          q_off, k_off, v_off, _p(b_raw), _rows(b_raw, "gated_delta b"), _p(a_raw), _rows(a_raw, "gated_delta a"),
+          _p(dt_bias), _p(a_log), _p(state), _p(slots), _p(token_req), _p(req_first_token), _p(o),
+          _rows(o, "gated_delta o"), H, n_key_heads, K, V, slots.numel(), int(max_run), stream)
+
+
+def gated_delta_chunks(qkv, q_off: int, k_off: int, v_off: int, b_raw, a_raw, dt_bias, a_log, state, slots, token_req,
+                       req_first_token, o, n_heads: int, n_key_heads: int, stream) -> None:
+    """``gated_delta_scan`` for the requests that bring several rows, 64 rows at a time on tensor cores (bfloat16 inputs,
+    csrc/recurrent_chunks.cu); requests with a single row are left to the scan."""
+    _need(state, torch.float32, "gated_delta_chunks state")
+    _need(o, torch.float32, "gated_delta_chunks o")
+    for t in (qkv, b_raw, a_raw):
+        _need(t, torch.bfloat16, "gated_delta_chunks inputs")
+    _, H, V, K = state.shape
+    if H != n_heads or o.shape[1] != H * V or not state.is_contiguous() or K > DELTA_CHUNK_ROWS:
+        raise KernelError(f"gated_delta_chunks: state {tuple(state.shape)} for {n_heads} heads, o {tuple(o.shape)}")
+    _call("recurrent_chunks", "mlxb_gated_delta_chunks", _GD_ARGS[1:-2] + [c_void_p], _p(qkv), _rows(qkv, "gated_delta qkv"),
           q_off, k_off, v_off, _p(b_raw), _rows(b_raw, "gated_delta b"), _p(a_raw), _rows(a_raw, "gated_delta a"),
           _p(dt_bias), _p(a_log), _p(state), _p(slots), _p(token_req), _p(req_first_token), _p(o),
           _rows(o, "gated_delta o"), H, n_key_heads, K, V, slots.numel(), stream)

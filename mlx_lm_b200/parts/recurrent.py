@@ -27,7 +27,7 @@ class Mamba2Mixer(Mixer):
     ``y = S^T C + D x`` with ``dt = softplus(dt + dt_bias)``; ``y * silu(z)`` is RMS-normed in ``norm_groups``
     equal parts, times ``norm``, then ``o``."""
     replayable = True
-    kernel_libs = ("recurrent", "rms")
+    kernel_libs = ("recurrent", "recurrent_chunks", "rms")
 
     def __init__(self, name: str, width: int, n_heads: int, vdim: int, state: int, groups: int, norm_groups: int,
                  taps: int, eps: float, init: Init = Init()):
@@ -79,9 +79,13 @@ class Mamba2Mixer(Mixer):
         # what it has to move: its inputs and outputs, and every live request's state in and out
         ops.label(self.name + ".scan", 6.0 * T * inner * self.state, x.element_size() * T * self.conv_width + 4.0 * T * inner
                   + 8.0 * min(T, ctx.n_requests) * inner * self.state)
-        ops.mamba2_scan(xbc, 0, inner, inner + GN, proj[:, inner + self.conv_width:], self.dt_bias, self.a_log,
-                        self.d_skip, ssm_state.state, ssm_state.slots, ctx.token_req, ctx.req_first_token, y,
-                        self.n_heads, self.groups, ctx.stream)
+        args = (xbc, 0, inner, inner + GN, proj[:, inner + self.conv_width:], self.dt_bias, self.a_log, self.d_skip,
+                ssm_state.state, ssm_state.slots, ctx.token_req, ctx.req_first_token, y, self.n_heads, self.groups, ctx.stream)
+        chunks = ctx.n_portion > 0 and ops.recurrent_chunks_supported(x.dtype, self.state, ops.MAMBA2_CHUNK_ROWS)
+        if chunks:
+            ops.mamba2_chunks(*args)
+        if not chunks or ctx.n_single:
+            ops.mamba2_scan(*args, max_run=1 if chunks else 0)
         g = ctx.ws.get("ssm_gated", T, inner, x.dtype)
         ops.label(self.name + ".norm", 8.0 * T * inner, (4.0 + 2 * x.element_size()) * T * inner)
         ops.rmsnorm(y, self.norm_w, g, self.eps, ctx.stream, groups=self.norm_groups, gate=proj[:, :inner],
@@ -103,7 +107,7 @@ class GatedDeltaMixer(Mixer):
     ``beta = sigmoid(b x)`` and ``g = exp(-exp(A_log) softplus(a x + dt_bias))``; every head's ``o`` is divided by
     its root mean square, times ``norm`` (shared by the heads), times ``silu(g x)``; then ``o``."""
     replayable = True
-    kernel_libs = ("recurrent", "rms")
+    kernel_libs = ("recurrent", "recurrent_chunks", "rms")
 
     def __init__(self, name: str, width: int, n_heads: int, n_kv_heads: int, dim: int, vdim: int, taps: int,
                  eps: float, init: Init = Init()):
@@ -156,9 +160,14 @@ class GatedDeltaMixer(Mixer):
         o = ctx.ws.get("delta_o", T, self.v_width, torch.float32)
         ops.label(self.name + ".scan", 8.0 * T * self.v_width * self.dim, x.element_size() * T * self.conv_width + 4.0 * T * self.v_width
                   + 8.0 * min(T, ctx.n_requests) * self.v_width * self.dim)
-        ops.gated_delta_scan(qkv, 0, self.qk_width, 2 * self.qk_width, proj[:, b_off:b_off + H],
-                             proj[:, b_off + H:b_off + 2 * H], self.dt_bias, self.a_log, rule_state.state,
-                             rule_state.slots, ctx.token_req, ctx.req_first_token, o, H, self.n_kv_heads, ctx.stream)
+        args = (qkv, 0, self.qk_width, 2 * self.qk_width, proj[:, b_off:b_off + H], proj[:, b_off + H:b_off + 2 * H],
+                self.dt_bias, self.a_log, rule_state.state, rule_state.slots, ctx.token_req, ctx.req_first_token, o, H,
+                self.n_kv_heads, ctx.stream)
+        chunks = ctx.n_portion > 0 and ops.recurrent_chunks_supported(x.dtype, self.dim, ops.DELTA_CHUNK_ROWS)
+        if chunks:
+            ops.gated_delta_chunks(*args)
+        if not chunks or ctx.n_single:
+            ops.gated_delta_scan(*args, max_run=1 if chunks else 0)
         g = ctx.ws.get("delta_gated", T, self.v_width, x.dtype)
         ops.label(self.name + ".norm", 8.0 * T * self.v_width, (4.0 + 2 * x.element_size()) * T * self.v_width)
         ops.rmsnorm(o, self.norm_w, g, self.eps, ctx.stream, groups=H, period=self.vdim,
