@@ -1,0 +1,119 @@
+"""The chunked kernels of the state-space layer and of the gated delta rule against the recurrences in 64 bits, token by
+token, and against the scans: runs that end inside and at the edges of chunks of 64 rows, states carried from step to step,
+single rows left out, sizes below and at the kernels' tiles, aligned and not."""
+import pytest
+import torch
+
+import plain_lelatar as plain
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda"
+
+
+def arrays(runs):
+    """(request of each row, first row of each request): request r brings ``runs[r]`` rows; two rows of padding at the end."""
+    token_req = sum(([r] * n for r, n in enumerate(runs)), []) + [-1, -1]
+    first = [0]
+    for n in runs:
+        first.append(first[-1] + n)
+    first[-1] += 2
+    return torch.tensor(token_req, dtype=torch.int32, device=DEV), torch.tensor(first, dtype=torch.int32, device=DEV)
+
+
+def close(got, want, scan):
+    """Within 2e-5 of the result's size everywhere, and as a whole no further off than twice what the scan is, which adds in
+    another order (or 2e-7, a few roundings of 32 bits)."""
+    size = float(want.abs().max())
+    err, of_scan = float((got.double() - want).norm() / want.norm()), float((scan.double() - want).norm() / want.norm())
+    assert float((got.double() - want).abs().max()) < 2e-5 * max(1.0, size)
+    assert err < max(2 * of_scan, 2e-7), (err, of_scan)
+
+
+RUNS = [[(64, 1, 130), (200, 65, 2)], [(2, 63, 1), (1, 300, 128)]]
+
+
+@pytest.mark.parametrize("runs", RUNS)
+@pytest.mark.parametrize("H,G,N,V,shift", [(4, 2, 24, 8, 0), (2, 1, 16, 40, 0), (6, 3, 70, 12, 0), (2, 1, 128, 64, 0), (2, 2, 64, 33, 1),
+                                           (1, 1, 3, 5, 0)])
+def test_state_space_chunks(H, G, N, V, shift, runs):
+    from mlx_lm_b200 import ops
+    torch.manual_seed(H * N + V)
+    R, inner, GN = 3, H * V, G * N
+    dt_bias, a_log, d_skip = torch.randn(H, device=DEV) * 0.5, torch.randn(H, device=DEV) * 0.5, torch.randn(H, device=DEV)
+    slots = torch.tensor([2, 0, 3], dtype=torch.int32, device=DEV)
+    pools = [torch.zeros(4, H, V, N, device=DEV) for _ in range(2)]
+    S = torch.zeros(R, H, N, V, dtype=torch.float64, device=DEV)
+    grp = torch.arange(H, device=DEV) // (H // G)
+    for step in runs:
+        token_req, first = arrays(step)
+        T = token_req.numel()
+        wide = (torch.randn(T, inner + 2 * GN + shift, device=DEV) * 0.7).to(torch.bfloat16)
+        xbc, dt_raw = wide[:, shift:], torch.randn(T, H, device=DEV).to(torch.bfloat16)
+        ys = [torch.zeros(T, inner, device=DEV) for _ in range(2)]
+        args = lambda i: (xbc, 0, inner, inner + GN, dt_raw, dt_bias, a_log, d_skip, pools[i], slots, token_req, first, ys[i], H, G,
+                          ops.current_stream())
+        ops.mamba2_chunks(*args(0))
+        assert all(float(ys[0][int(first[r])].abs().max()) == 0.0 for r, n in enumerate(step) if n == 1)
+        ops.mamba2_scan(*args(0), max_run=1)
+        ops.mamba2_scan(*args(1))
+        want = torch.zeros(T, H, V, dtype=torch.float64, device=DEV)
+        x = xbc.double()
+        dt = plain.softplus(dt_raw.double() + dt_bias.double())
+        a = torch.exp(-torch.exp(a_log.double()) * dt)
+        for t in range(T - 2):
+            r, xt = int(token_req[t]), x[t, :inner].view(H, V)
+            B, C = x[t, inner:inner + GN].view(G, N)[grp], x[t, inner + GN:].view(G, N)[grp]
+            S[r] = a[t, :, None, None] * S[r] + (dt[t, :, None] * B)[:, :, None] * xt[:, None, :]
+            want[t] = torch.einsum("hnv,hn->hv", S[r], C) + d_skip.double()[:, None] * xt
+        close(ys[0].view(T, H, V), want, ys[1].view(T, H, V))
+    state = lambda p: p[slots.long()].transpose(2, 3)
+    close(state(pools[0]), S, state(pools[1]))
+    assert float(pools[0][1].abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("runs", RUNS)
+@pytest.mark.parametrize("H,G,K,V,shift", [(4, 2, 16, 24, 0), (2, 2, 40, 8, 0), (2, 1, 64, 64, 0), (1, 1, 64, 33, 1), (3, 1, 7, 5, 0)])
+@pytest.mark.parametrize("slow", [False, True])
+def test_gated_delta_chunks(H, G, K, V, shift, runs, slow):
+    """``slow``: keys that repeat, strong updates and hardly any decay, so that the triangular system is far from the identity."""
+    from mlx_lm_b200 import ops
+    torch.manual_seed(H * K + V)
+    R, n_in = 3, 2 * G * K + H * V
+    dt_bias, a_log = torch.randn(H, device=DEV) * 0.5 - (6.0 if slow else 0.0), torch.randn(H, device=DEV) * 0.5
+    slots = torch.tensor([2, 0, 3], dtype=torch.int32, device=DEV)
+    pools = [torch.zeros(4, H, V, K, device=DEV) for _ in range(2)]
+    S = torch.zeros(R, H, K, V, dtype=torch.float64, device=DEV)
+    grp = torch.arange(H, device=DEV) // (H // G)
+    for step in runs:
+        token_req, first = arrays(step)
+        T = token_req.numel()
+        wide = torch.randn(T, n_in + shift, device=DEV)
+        if slow:
+            wide[:, shift + G * K:shift + 2 * G * K] = wide[:1, shift + G * K:shift + 2 * G * K] + 0.3 * wide[:, shift + G * K:shift + 2 * G * K]
+        wide = wide.to(torch.bfloat16)
+        qkv = wide[:, shift:]
+        b_raw = (torch.randn(T, H, device=DEV) + (3.0 if slow else 0.0)).to(torch.bfloat16)
+        a_raw = torch.randn(T, H, device=DEV).to(torch.bfloat16)
+        os_ = [torch.zeros(T, H * V, device=DEV) for _ in range(2)]
+        args = lambda i: (qkv, 0, G * K, 2 * G * K, b_raw, a_raw, dt_bias, a_log, pools[i], slots, token_req, first, os_[i], H, G,
+                          ops.current_stream())
+        ops.gated_delta_chunks(*args(0))
+        assert all(float(os_[0][int(first[r])].abs().max()) == 0.0 for r, n in enumerate(step) if n == 1)
+        ops.gated_delta_scan(*args(0), max_run=1)
+        ops.gated_delta_scan(*args(1))
+        want = torch.zeros(T, H, V, dtype=torch.float64, device=DEV)
+        x = qkv.double()
+        unit = lambda t: t / torch.sqrt((t * t).sum(-1, keepdim=True) + 1e-6)
+        q, k = unit(x[:, :G * K].reshape(T, G, K)) * K ** -0.5, unit(x[:, G * K:2 * G * K].reshape(T, G, K))
+        v, beta = x[:, 2 * G * K:].reshape(T, H, V), torch.sigmoid(b_raw.double())
+        decay = torch.exp(-torch.exp(a_log.double()) * plain.softplus(a_raw.double() + dt_bias.double()))
+        for t in range(T - 2):
+            r, kt, qt = int(token_req[t]), k[t, grp], q[t, grp]
+            S[r] = decay[t, :, None, None] * S[r]
+            u = beta[t, :, None] * (v[t] - torch.einsum("hkv,hk->hv", S[r], kt))
+            S[r] = S[r] + kt[:, :, None] * u[:, None, :]
+            want[t] = torch.einsum("hkv,hk->hv", S[r], qt)
+        close(os_[0].view(T, H, V), want, os_[1].view(T, H, V))
+    state = lambda p: p[slots.long()].transpose(2, 3)
+    close(state(pools[0]), S, state(pools[1]))
