@@ -20,7 +20,9 @@
 // this block's softmax.  There are two buffers of 128 columns in tensor memory, block i uses buffer i % 2: first for S, then,
 // when P is written and S no longer needed, for O_b; S(i + 1) goes to the other buffer once O_b(i - 1) has been read from
 // it.  K has two buffers as well and is requested two blocks ahead, V of the next block as soon as P V has been computed; two
-// CTAs fit an SM (97 KB of shared memory, 256 of 512 tensor-memory columns each) and overlap one another's phases.  The order in which a query's keys are added depends only
+// CTAs fit an SM (97 KB of shared memory, 256 of 512 tensor-memory columns each) and overlap one another's phases.  2 x 1024 queries of 16 heads take 25.4 us (31.8 with S behind P V and the
+// scores kept, and spilled, in registers), of 25 heads 37.8 (46.4), 256 queries of 20 heads at position 768 23.7 (30.3).  Even
+// and odd blocks as two chains on a cluster of two CTAs: 34.4, 49.0 and 18.2, and sums in another order.  The order in which a query's keys are added depends only
 // on its position (blocks of 128 positions from block 0 or the window's first block upward).
 //
 // Every mbarrier wait is bounded; a wait that gives up sets an abort flag that all roles see, the CTA frees
@@ -35,8 +37,6 @@
 // softmax), `keep_first` (beside a window the first so many positions of the sequence stay visible: their blocks are
 // walked first, then the window's), `gate` (every output column times the sigmoid of a bfloat16 gate column).
 #include <cuda.h>
-
-#include <type_traits>
 
 #include "common.cuh"
 
@@ -87,20 +87,6 @@ __device__ __forceinline__ bool elect_one() {
   uint32_t is;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(is));
   return is != 0;
-}
-// ---- clusters of two CTAs.  Every thread of both CTAs arrives and waits; roles do it where they are, so not .aligned.
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
-__device__ __forceinline__ uint32_t peer_addr(const void* p, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ float4 ld_cluster(uint32_t addr) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-  return v;
 }
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
   asm volatile(
@@ -162,16 +148,12 @@ struct AtSmem {
   uint64_t o_read;                               // O_b has been read: its buffer is free for the next S
   uint64_t x_full[4];                            // exchange of row maxima (and, at the end, sums) of two warps with the same rows
   float row_max[2][TQ];                          // the two halves' maxima of the current block, per row
-  alignas(16) float4 row_sum[TQ];                // the two halves' sums of the odd and the even blocks
-  float4 ml[TQ];                                 // for the peer: a row's maximum and sum
   uint32_t tmem_base;
   int abort_flag;
 };
 
 // tiles: int32 [n_tiles][4] = (row of the tile's first token among the step's tokens, queries in the tile
 // (1..128), block-table row of the request, position of the tile's first query).
-// RANKS: CTAs that share a tile, as a cluster.
-template <int RANKS>
 __global__ void __launch_bounds__(AT_THREADS, 2)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                             const __grid_constant__ CUtensorMap map_v, const int4* __restrict__ tiles,
@@ -182,8 +164,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   extern __shared__ uint8_t smem_raw[];
   AtSmem& sm = *reinterpret_cast<AtSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int4 tile = tiles[blockIdx.x / RANKS];
-  const int rank = blockIdx.x % RANKS;
+  const int4 tile = tiles[blockIdx.x];
   if (tile.y <= 0) return;                // a tile without queries pads the list to a size seen before: nothing to do
 
   const int row0 = tile.x, n_rows = tile.y, req = tile.z, pos0 = tile.w;
@@ -192,24 +173,12 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   const int last_pos = pos0 + n_rows - 1;
   const int first_key = (window > 0 && pos0 - window + 1 > 0) ? pos0 - window + 1 : 0;
   const int kb_lo = first_key / TK, kb_hi = last_pos / TK;
-  // Blocks with kept first positions that lie before the window's first block are walked first, then the window's; the
-  // even ones in one chain with a maximum, sum and O of its own, the odd ones in another, and the two become one at the end.
-  // A cluster's CTAs take a chain each, a CTA alone walks one after the other: the same additions in the same order.
+  // blocks with kept first positions that lie before the window's first block are walked first: block i of the walk
+  // is block kb_at(i) of the sequence
   const int kept = window > 0 ? (keep_first < last_pos + 1 ? keep_first : last_pos + 1) : 0;
   const int kf_blocks = (window > 0 && kept > 0) ? ((kept + TK - 1) / TK < kb_lo ? (kept + TK - 1) / TK : kb_lo) : 0;
-  auto kept_of = [&](int c) { return (kf_blocks + 1 - c) >> 1; };
-  auto first_of = [&](int c) { return kb_lo + ((kb_lo ^ c) & 1); };
-  auto blocks_of = [&](int c) { return kept_of(c) + (first_of(c) <= kb_hi ? ((kb_hi - first_of(c)) >> 1) + 1 : 0); };
-  const int n_even = blocks_of(0), n_odd = blocks_of(1);
-  const bool both = n_even > 0 && n_odd > 0;
-  const int n_blocks = RANKS == 1 ? n_even + n_odd : (rank == 0 ? n_even : n_odd);
-  if (n_blocks == 0) return;                              // the peer has them all and waits for nobody
-  // block i of this CTA's walk; beyond its end, a block after kb_hi
-  auto kb_at = [&](int i) {
-    int c = rank;
-    if (RANKS == 1 && i >= n_even) { c = 1; i -= n_even; }
-    return i < kept_of(c) ? c + 2 * i : first_of(c) + 2 * (i - kept_of(c));
-  };
+  const int n_blocks = kf_blocks + kb_hi - kb_lo + 1;
+  auto kb_at = [&](int i) { return i < kf_blocks ? i : kb_lo + i - kf_blocks; };
 
   if (threadIdx.x == 0) {
     mbar_init(&sm.q_full, 1);
@@ -328,7 +297,6 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       pg_next = pg_after;
       pg_after = pg_far;
     }
-    if (RANKS == 2 && both) { cluster_arrive(); cluster_wait(); cluster_arrive(); cluster_wait(); }     // see below
   } else {
     // softmax: thread (half, r) owns keys [64 half, 64 half + 64) of every block and output dims
     // [32 half, 32 half + 32) of query row r, which is lane r of tensor memory (warp w may touch lanes 32 (w % 4) ..)
@@ -350,16 +318,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     const float mult = softcap > 0.f ? 1.4426950408889634f : scale_log2e;
     uint8_t* p_row = reinterpret_cast<uint8_t*>(sm.p) + half * (TQ * 64 * 2) + (r >> 3) * 1024 + (r & 7) * 128;
     bool ok = true;
-    float o_even[HD / 2], m_even = -INFINITY, l_even = 0.f;      // a CTA alone: the even chain, put aside
     for (int i = 0; i < n_blocks && ok; ++i) {
-      if (RANKS == 1 && both && i == n_even) {
-#pragma unroll
-        for (int d = 0; d < HD / 2; ++d) { o_even[d] = o[d]; o[d] = 0.f; }
-        m_even = m;
-        l_even = l;
-        m = -INFINITY;
-        l = 0.f;
-      }
       const uint32_t ph = (uint32_t)(i & 1);
       const int kb = kb_at(i);
       const int key_base = kb * TK + half * 64;
@@ -448,62 +407,13 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     }
     // the row's sum is the two halves' sums
     if (ok) {
-      float2* sums = reinterpret_cast<float2*>(&sm.row_sum[r]);
-      sums[half] = make_float2(l, l_even);
+      sm.row_max[half][r] = l;
       __syncwarp();
       if (lane == 0) mbar_arrive(x_full);
       ok = mbar_wait_warp(x_full, (uint32_t)(n_blocks & 1), abort_flag);
-      l += sums[half ^ 1].x;
-      l_even += sums[half ^ 1].y;
+      l += sm.row_max[half ^ 1][r];
     }
-    bool finish = ok;
-    if (both) {
-      // The two chains become one.  In a cluster rank 0 finishes the first 32 dims and rank 1 the others: each leaves what
-      // the other finishes where its keys were (every product and copy has completed), rows of 128 bytes, their pieces
-      // XORed with the row number against bank conflicts.
-      float4* mine = reinterpret_cast<float4*>(sm.k[0]);
-      float m_odd = m, l_odd = l;
-      uint32_t theirs = 0;
-      if (RANKS == 2) {
-        if (half != rank) {
-#pragma unroll
-          for (int d = 0; d < 8; ++d)
-            mine[r * 8 + (d ^ (r & 7))] = make_float4(o[4 * d], o[4 * d + 1], o[4 * d + 2], o[4 * d + 3]);
-          sm.ml[r] = make_float4(m, l, 0.f, 0.f);
-        }
-        cluster_arrive();
-        cluster_wait();
-        finish = finish && half == rank;
-        if (half == rank) {
-          const float4 t = ld_cluster(peer_addr(&sm.ml[r], (uint32_t)(rank ^ 1)));
-          theirs = peer_addr(mine + r * 8, (uint32_t)(rank ^ 1));
-          if (rank == 0) { m_even = m; l_even = l; m_odd = t.x; l_odd = t.y; }
-          else { m_even = t.x; l_even = t.y; }
-        }
-      }
-      if (RANKS == 1 || half == rank) {
-        m = fmaxf(m_even, m_odd);
-        const float base = m == -INFINITY ? 0.f : m;
-        const float w_even = fast_exp2(m_even - base), w_odd = fast_exp2(m_odd - base);
-        l = __fmaf_rn(l_even, w_even, __fmul_rn(l_odd, w_odd));
-#pragma unroll
-        for (int d = 0; d < 8; ++d) {
-          float a[4], b[4];
-          float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (RANKS == 2) p = ld_cluster(theirs + (uint32_t)((d ^ (r & 7)) * 16));
-          const float t[4] = {p.x, p.y, p.z, p.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            a[e] = RANKS == 1 ? o_even[4 * d + e] : (rank == 0 ? o[4 * d + e] : t[e]);
-            b[e] = RANKS == 1 || rank == 1 ? o[4 * d + e] : t[e];
-          }
-#pragma unroll
-          for (int e = 0; e < 4; ++e) o[4 * d + e] = __fmaf_rn(a[e], w_even, __fmul_rn(b[e], w_odd));
-        }
-      }
-      if (RANKS == 2) cluster_arrive();       // the peer's results have been read; this CTA's stay until the peer has read them
-    }
-    if (finish && r < n_rows) {
+    if (ok && r < n_rows) {
       if (sinks && m != -INFINITY) l += fast_exp2(sinks[h] * 1.4426950408889634f - m);   // the sink: no key, no value
       const float inv = l > 0.f ? 1.f / l : 0.f;
       const size_t col = (size_t)(h * VS + vs) * HD + half * (HD / 2);      // this thread's first output column
@@ -528,7 +438,6 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         }
       }
     }
-    if (RANKS == 2 && both) cluster_wait();
   }
 
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -594,39 +503,16 @@ MLXB_EXPORT int mlxb_attention_prefill_tc(const void* q, int ldq, int n_tokens, 
   if (int e = make_map(&mk, k_pool, pool_rows, HD, HD, page, "k pool")) return e;
   if (int e = make_map(&mv, v_pool, (long long)n_pages * Hv * page, Dv, Dv, page, "v pool")) return e;
   const size_t smem = sizeof(AtSmem) + 1024;
-  // Two CTAs a tile where all of them fit the SMs at once (two an SM): the chain of a tile's blocks is then half as long.
-  // Measured, 20 heads, 256 queries at positions 768 on: 18.2 us against 23.7; 16 heads, 128 queries at 896: 14.7 against 22.1.
-  // With more tiles the SMs have work beside a chain's waits anyway (2 x 1024 queries, 16 heads: 34.4 against 25.4).
-  auto go = [&](auto ranks) {
-    constexpr int RANKS = decltype(ranks)::value;
-    auto kern = attention_prefill_tc_kernel<RANKS>;
-    static bool raised = false;
-    if (!raised) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess)
-        return mlxb_fail((int)e, "attention (portions, tcgen05): %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
-      raised = true;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(RANKS * n_tiles, Hq * VS);
-    cfg.blockDim = dim3(AT_THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = mlxb_pdl_enabled() ? 1 : 0;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = RANKS;
-    attr[1].val.clusterDim.y = 1;
-    attr[1].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = RANKS == 1 ? 1 : 2;
-    cudaLaunchKernelEx(&cfg, kern, mq, mk, mv, (const int4*)tiles, block_table, max_pages, n_pages, page, Hq, Hkv, window,
-                       scale * 1.4426950408889634f, (__nv_bfloat16*)out, ldo, status, sinks, window > 0 ? keep_first : 0, softcap,
-                       (const __nv_bfloat16*)gate, ldg, Hv, VS, out_f32);
-    return mlxb_check_launch("attention (portions, tcgen05)");
-  };
-  const char* want = getenv("MLXB_ATTENTION_RANKS");      // experiments and tests: CTAs a tile
-  const bool two = want ? want[0] == '2' : (long long)n_tiles * Hq * VS <= mlxb_sm_count();
-  return two ? go(std::integral_constant<int, 2>{}) : go(std::integral_constant<int, 1>{});
+  static bool raised = false;
+  if (!raised) {
+    cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess)
+      return mlxb_fail((int)e, "attention (portions, tcgen05): %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
+    raised = true;
+  }
+  launch_pdl(attention_prefill_tc_kernel, dim3(n_tiles, Hq * VS), dim3(AT_THREADS), smem, stream, mq, mk, mv,
+             (const int4*)tiles, block_table, max_pages, n_pages, page, Hq, Hkv, window,
+             scale * 1.4426950408889634f, (__nv_bfloat16*)out, ldo, status, sinks, window > 0 ? keep_first : 0, softcap,
+             (const __nv_bfloat16*)gate, ldg, Hv, VS, out_f32);
+  return mlxb_check_launch("attention (portions, tcgen05)");
 }

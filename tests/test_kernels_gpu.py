@@ -594,10 +594,10 @@ def test_attention_portions(ops, Hq, Hkv, Dh, page, window, tile):
 @pytest.mark.parametrize("Hq,Hkv,page,window,keep,softcap,sinks", [(4, 4, 16, 0, 0, 0.0, False), (8, 2, 16, 0, 0, 0.0, True),
                                                                    (2, 1, 32, 300, 0, 0.0, False), (3, 3, 128, 130, 200, 0.0, False),
                                                                    (2, 2, 16, 700, 5, 20.0, True), (1, 1, 8, 1, 0, 0.0, False)])
-def test_attention_portions_chains(ops, Hq, Hkv, page, window, keep, softcap, sinks, monkeypatch):
-    """The tcgen05 kernel walks a tile's even and odd key blocks as two chains, on one CTA or on a cluster of two: the same
-    bits either way, and whatever tile a query lies in (tiles cut elsewhere), with from one to nine blocks of either
-    parity, windows that leave one chain empty, kept first positions, a cap and sinks; and the plain statement."""
+def test_attention_portions_of_many_blocks(ops, Hq, Hkv, page, window, keep, softcap, sinks):
+    """The tcgen05 kernel over one to nine blocks of keys (both buffers of keys and of tensor memory several times over),
+    with windows, kept first positions, a cap and sinks: the same bits whatever tile a query lies in (tiles cut
+    elsewhere), and the plain statement."""
     Dh = 64
     lens, new = [0, 900, 127, 250, 513], [400, 200, 2, 300, 128]
     c = paged_case(torch.bfloat16, lens=lens, new=new, Hq=Hq, Hkv=Hkv, Dh=Dh, page=page, seed=page + window)
@@ -605,16 +605,14 @@ def test_attention_portions_chains(ops, Hq, Hkv, page, window, keep, softcap, si
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
     s = torch.randn(Hq, generator=torch.Generator().manual_seed(1)).cuda() if sinks else None
 
-    def run(ranks, tile):
-        monkeypatch.setenv("MLXB_ATTENTION_RANKS", ranks)
+    def run(tile):
         tiles = make_tiles(lens, new, tile).cuda()
         out = torch.zeros(c["T"], Hq * Dh, dtype=torch.bfloat16, device="cuda")
         ops.attention_portions(dev["qkv"][:, :Hq * Dh], tiles, tiles.numel() // 4, dev["bt"], dev["k_pool"], dev["v_pool"], out,
                                Hq, Dh ** -0.5, window, status, stream(), tile_rows=128, sinks=s, keep_first=keep, softcap=softcap)
         return out
-    base = run("1", 128)
-    for ranks, tile in (("2", 128), ("1", 77), ("2", 77)):
-        assert torch.equal(run(ranks, tile), base), (ranks, tile)
+    base = run(128)
+    assert torch.equal(run(77), base)
     assert int(status.item()) == 0
     if not (keep or softcap or sinks):
         ref = R.attention(c["qkv"][:, :Hq * Dh], c["positions"], c["token_req"], c["bt"], c["k_pool"], c["v_pool"], Hq, Dh ** -0.5,
