@@ -28,6 +28,8 @@
 //            folds that row's partials in chunk order and writes the output.
 //            The chunk length is a constant of the engine, not of the batch,
 //            so a row's result does not depend on its neighbours.
+#include <type_traits>
+
 #include "common.cuh"
 
 MLXB_DEFINE_LAST_ERROR()
@@ -369,17 +371,27 @@ attention_portions_f32_kernel(const float* q, int ldq, const int4* __restrict__ 
     }
     __syncwarp();          // a warp reads back the probabilities of its own queries
     const int nk = min(AP_Q, last - j0 + 1);
-#pragma unroll 4
-    for (int jj = 0; jj < nk; ++jj) {
+    auto add_values = [&](int jj, auto some) {       // some: not every query sees every key of this block
       float a[8], b[VD];
       *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(&sm.p[jj][8 * ty]);
       *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(&sm.p[jj][8 * ty + 4]);
 #pragma unroll
       for (int d = 0; d < VD; d += 2) *reinterpret_cast<float2*>(b + d) = *reinterpret_cast<const float2*>(&sm.v[jj][VD * tx + d]);
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int i = 0; i < 8; ++i) {
+        // a key that a query does not see adds nothing, not zero times its value: the value may be infinite
+        const int ahead = j0 + jj - (pos0 + 8 * ty + i);
+        if (decltype(some)::value && (ahead > 0 || (window > 0 && ahead <= -window))) continue;
 #pragma unroll
         for (int d = 0; d < VD; ++d) o[i][d] = fmaf(a[i], b[d], o[i][d]);
+      }
+    };
+    if (j0 + AP_Q - 1 <= pos0 && (window <= 0 || j0 > last - window)) {
+#pragma unroll 4
+      for (int jj = 0; jj < nk; ++jj) add_values(jj, std::false_type());
+    } else {
+#pragma unroll 1
+      for (int jj = 0; jj < nk; ++jj) add_values(jj, std::true_type());
     }
   }
 #pragma unroll

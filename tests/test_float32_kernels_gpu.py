@@ -69,3 +69,26 @@ def test_float32_attention_of_portions(ops, Hq, Hkv, Dh, page, window, sink):
     if not sink and not window:
         want = R.attention(c["qkv"][:, :Hq * Dh], c["positions"], c["token_req"], c["bt"], c["k_pool"], c["v_pool"], Hq, scale, window)
         assert rel_err(out[1:], want[1:]) <= 3e-6
+
+
+@pytest.mark.parametrize("window", [0, 70])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_float32_portions_keep_values_a_query_does_not_see_out(ops, bad, window):
+    """One value that is not finite: queries before its position, and queries whose window has left it behind, come out as they
+    do with a finite one, bit for bit; queries that see it do not."""
+    H, Dh, n, at = 2, 64, 200, 91
+    c = paged_case(torch.float32, lens=[0], new=[n], Hq=H, Hkv=H, Dh=Dh, page=16, seed=4)
+    dev = {k: (v.cuda() if torch.is_tensor(v) else v) for k, v in c.items()}
+    tiles = torch.tensor([(0, 128, 0, 0), (128, n - 128, 0, 128)], dtype=torch.int32).cuda()
+    status, q = torch.zeros(1, dtype=torch.int32, device="cuda"), dev["qkv"][:, :H * Dh]
+    outs = []
+    for value in (1.0, bad):
+        dev["v_pool"][int(c["bt"][0, at // 16]), :, at % 16] = value
+        out = torch.empty(n, H * Dh, device="cuda")
+        ops.attention_portions_f32(q, tiles, 2, dev["bt"], dev["k_pool"], dev["v_pool"], out, H, Dh ** -0.5, window, status, stream())
+        outs.append(out)
+    sees = torch.arange(n, device="cuda") >= at
+    if window:
+        sees &= torch.arange(n, device="cuda") < at + window
+    assert torch.equal(outs[0][~sees], outs[1][~sees])
+    assert not bool(torch.isfinite(outs[1][sees]).any())
