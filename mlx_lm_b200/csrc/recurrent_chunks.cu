@@ -23,9 +23,12 @@ __device__ __forceinline__ float softplus_f(float v) { return v > 20.f ? v : log
 constexpr int RC_Q = 64;            // rows of a chunk
 constexpr int RC_THREADS = 256;
 
+// x as the sum of three bfloat16 numbers.  What is not finite (and what is above bfloat16's largest number, 0.996 of float32's)
+// is the first of them, beside zeros: a product with it is then what a product with x would be.
 __device__ __forceinline__ void split3(float x, __nv_bfloat16& a, __nv_bfloat16& b, __nv_bfloat16& c) {
   a = __float2bfloat16_rn(x);
-  const float r = x - __bfloat162float(a);
+  float r = x - __bfloat162float(a);
+  r = fabsf(r) < INFINITY ? r : 0.f;
   b = __float2bfloat16_rn(r);
   c = __float2bfloat16_rn(r - __bfloat162float(b));
 }
@@ -91,18 +94,51 @@ __device__ __forceinline__ void stage_rows(const __nv_bfloat16* src, int lds_src
   }
 }
 
-// Inclusive sums over the chunk of one value a row, by one warp: lane l has rows 2 l and 2 l + 1.
+// The logarithm of a row's decay, from minus the rate and the step.  Below -200 a decay is zero in float32 whatever follows, so
+// that an infinite step leaves sums with differences.
+__device__ __forceinline__ double log_decay(float rate, float step) {
+  const float l = rate * step;
+  return (double)(l < -200.f ? -200.f : l);
+}
+
+// Inclusive sums over the chunk of one value a row, by one warp: lane l has rows 2 l and 2 l + 1.  A row's sum has only values
+// of rows up to it (and no differences of later sums), so that a NaN stays behind the rows before it.
 __device__ __forceinline__ void chunk_sums(double& a, double& b, int lane) {
-  b += a;
-  double t = b;
+  double t = a + b;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const double u = __shfl_up_sync(0xffffffffu, t, o);
     if (lane >= o) t += u;
   }
-  const double before = t - b;
-  a += before;
-  b += before;
+  const double before = __shfl_up_sync(0xffffffffu, t, 1);
+  if (lane > 0) a += before;
+  b += a;
+}
+
+// Rows of a chunk that are not finite.  A row's weights for the rows behind it are zeros, and zero times an infinity is not
+// zero: in a diagonal tile of 16 rows by 16 such values leave the product (drop_bad, from a B fragment of two neighbouring
+// values each) and are added to the rows that have them behind them (add_bad).  The other values' sums stay as they are.
+__device__ __forceinline__ void drop_bad(unsigned& u) {
+  if ((u & 0x7f80u) == 0x7f80u) u &= 0xffff0000u;
+  if ((u & 0x7f800000u) == 0x7f800000u) u &= 0x0000ffffu;
+}
+// value(s, c): row s, column c; p: the weights' planes, `plane` elements apart.  This thread's eight results of rows 16 ti ..,
+// columns c16 .., as accumulators of two tiles.
+template <typename Value>
+__device__ __forceinline__ void add_bad(float (&acc)[2][4], const __nv_bfloat16* p, int plane, int ldp, int ti, int c16, int g, int q,
+                                        Value value) {
+#pragma unroll 1
+  for (int s = 16 * ti; s < 16 * ti + 16; ++s)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int t = 16 * ti + g + (e >> 1) * 8;
+        const float v = value(s, c16 + 8 * j + 2 * q + (e & 1));
+        if (s > t || fabsf(v) < INFINITY) continue;
+        const __nv_bfloat16* w = p + t * ldp + s;
+        acc[j][e] = fmaf(to_f(w[0]) + (to_f(w[plane]) + to_f(w[2 * plane])), v, acc[j][e]);
+      }
 }
 
 // ---------------------------------------------------------------- state-space scan (Mamba-2)
@@ -123,7 +159,7 @@ struct Mamba2Memory {
 };
 
 template <int NP>
-__global__ void __launch_bounds__(RC_THREADS)
+__global__ void __launch_bounds__(RC_THREADS, NP > 64 ? 1 : 2)      // as many as their shared memory lets an SM hold
 mamba2_chunks_kernel(const __nv_bfloat16* xbc, int ldx, int x_off, int b_off, int c_off, const __nv_bfloat16* dt_raw, int lddt,
                      const float* __restrict__ dt_bias, const float* __restrict__ A_log, const float* __restrict__ Dskip,
                      float* state, const int* __restrict__ slots, const int* __restrict__ token_req,
@@ -178,7 +214,7 @@ mamba2_chunks_kernel(const __nv_bfloat16* xbc, int ldx, int x_off, int b_off, in
       for (int i = 0; i < 2; ++i) {
         const int t = 2 * lane + i;
         d[i] = t < nc ? softplus_f(to_f(dt_raw[(size_t)(t0 + c0 + t) * lddt + h]) + bias) : 0.f;
-        l[i] = (double)(negA * d[i]);
+        l[i] = log_decay(negA, d[i]);
       }
       chunk_sums(l[0], l[1], lane);
       const double end = __shfl_sync(0xffffffffu, l[1], 31);
@@ -198,10 +234,12 @@ mamba2_chunks_kernel(const __nv_bfloat16* xbc, int ldx, int x_off, int b_off, in
         store_split(sm.state[0] + (16 * vi + g + (e >> 1) * 8) * LN + (NP / 4) * ni + 8 * j + 2 * q, M2_VS * LN, S[j][e], S[j][e + 1]);
     __syncthreads();
     if (c0 + RC_Q < n) fetch(buf ^ 1, c0 + RC_Q);
+    bool bad = false;                        // a value of x that is not finite
     for (int e = tid; e < RC_Q * M2_VS / 2; e += RC_THREADS) {
       const int s = e / (M2_VS / 2), c = 2 * (e - s * (M2_VS / 2));
       const float2 xv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sx + s * LV + c));
       store_split(sm.wx[0] + s * LV + c, RC_Q * LV, sm.left[s] * xv.x, sm.left[s] * xv.y);
+      bad |= !(fabsf(xv.x) < INFINITY && fabsf(xv.y) < INFINITY);
     }
     const int ti = warp >> 1;                // rows 16 ti .. of the chunk, for P and y
     // P: columns 32 (warp & 1) .., up to the diagonal's tile
@@ -230,7 +268,7 @@ mamba2_chunks_kernel(const __nv_bfloat16* xbc, int ldx, int x_off, int b_off, in
           store_split(sm.p[0] + t * LP + s, RC_Q * LP, w[0], w[1]);
         }
     }
-    __syncthreads();
+    bad = __syncthreads_or(bad);
     {   // y: columns 16 (warp & 1) .. of the slice
       const int c16 = 16 * (warp & 1);
       float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, low[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
@@ -254,6 +292,10 @@ mamba2_chunks_kernel(const __nv_bfloat16* xbc, int ldx, int x_off, int b_off, in
       for (int k = 0; k <= 16 * ti; k += 16) {
         unsigned bb[4];
         frag_b_t(bb, sx + k * LV + c16, LV, lane);
+        if (bad && k == 16 * ti) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) drop_bad(bb[i]);
+        }
 #pragma unroll
         for (int pl = 2; pl >= 0; --pl) {
           unsigned a[4];
@@ -262,6 +304,7 @@ mamba2_chunks_kernel(const __nv_bfloat16* xbc, int ldx, int x_off, int b_off, in
           mma_plane(acc[1], low[1], pl, a, bb[2], bb[3]);
         }
       }
+      if (bad) add_bad(acc, sm.p[0], RC_Q * LP, LP, ti, c16, g, q, [&](int s, int c) { return to_f(sx[s * LV + c]); });
 #pragma unroll
       for (int j = 0; j < 2; ++j)
 #pragma unroll

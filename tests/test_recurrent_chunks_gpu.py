@@ -117,3 +117,64 @@ def test_gated_delta_chunks(H, G, K, V, shift, runs, slow):
         close(os_[0].view(T, H, V), want, os_[1].view(T, H, V))
     state = lambda p: p[slots.long()].transpose(2, 3)
     close(state(pools[0]), S, state(pools[1]))
+
+
+BAD = [(70, 40, float("inf")), (3, 90, float("nan")), (64, 15, float("-inf"))]      # row, place among the row's inputs, value
+
+
+@pytest.mark.parametrize("row,place,value", BAD)
+@pytest.mark.parametrize("where", ["x", "B", "C", "dt"])
+def test_state_space_rows_before_one_that_is_not_finite(row, place, value, where):
+    """An infinity or a NaN in one row: the rows before it are those of a finite row, bit for bit, as token by token; where it
+    goes into the state, so are the columns of the state that it does not reach, and those it reaches are not finite."""
+    from mlx_lm_b200 import ops
+    H, N, V, T = 2, 128, 64, 130
+    torch.manual_seed(row)
+    consts = [torch.randn(H, device=DEV) * 0.5 for _ in range(3)]
+    token_req, first = arrays((T,))
+    xbc0 = (torch.randn(T + 2, H * V + 2 * N, device=DEV) * 0.7).to(torch.bfloat16)
+    dt0 = torch.randn(T + 2, H, device=DEV).to(torch.bfloat16)
+    got = {}
+    for kernel in ("chunks", "scan"):
+        for v in (1.0, value):
+            xbc, dt = xbc0.clone(), dt0.clone()
+            if where == "dt":
+                dt[row, 0] = abs(v)
+            else:
+                xbc[row, {"x": 0, "B": H * V, "C": H * V + N}[where] + place % 64] = v
+            S, y = torch.zeros(1, H, V, N, device=DEV), torch.zeros(T + 2, H * V, device=DEV)
+            f = ops.mamba2_chunks if kernel == "chunks" else ops.mamba2_scan
+            f(xbc, 0, H * V, H * V + N, dt, *consts, S, torch.zeros(1, dtype=torch.int32, device=DEV), token_req, first, y, H, 1,
+              ops.current_stream())
+            got[kernel, v == 1.0] = y, S
+    for kernel in ("chunks", "scan"):
+        (y, S), (fy, fS) = got[kernel, False], got[kernel, True]
+        assert torch.equal(y[:row], fy[:row])
+        assert not bool(torch.isfinite(y[row]).all())
+        # what the value does not reach (other columns, other heads), and what it does, as token by token
+        reached = torch.isfinite(got["scan", False][0])
+        assert torch.equal(torch.isfinite(y), reached)
+        assert torch.equal(torch.isfinite(S), torch.isfinite(got["scan", False][1]))
+
+
+def test_state_space_chunks_from_a_state_that_is_not_finite():
+    """What comes out of an infinite entry of the state, or of one near the largest number, is what it is token by token."""
+    from mlx_lm_b200 import ops
+    H, N, V, T = 1, 64, 32, 40
+    torch.manual_seed(9)
+    consts = [torch.full((H,), -6.0, device=DEV), torch.zeros(H, device=DEV), torch.zeros(H, device=DEV)]
+    token_req, first = arrays((T,))
+    xbc = (torch.randn(T + 2, H * V + 2 * N, device=DEV) * 0.7).to(torch.bfloat16)
+    xbc[:, H * V + N + 7] = 2.0 ** -20
+    dt, ys = torch.zeros(T + 2, H, device=DEV, dtype=torch.bfloat16), []
+    for f in (ops.mamba2_scan, ops.mamba2_chunks):
+        S, y = torch.zeros(1, H, V, N, device=DEV), torch.zeros(T + 2, H * V, device=DEV)
+        S[0, 0, 3, 5], S[0, 0, 4, 5], S[0, 0, 5, 7] = float("inf"), float("-inf"), 3.3e38
+        f(xbc, 0, H * V, H * V + N, dt, *consts, S, torch.zeros(1, dtype=torch.int32, device=DEV), token_req, first, y, H, 1,
+          ops.current_stream())
+        ys.append((y[:T], S))
+    for got, want in zip(ys[1], ys[0]):
+        finite = torch.isfinite(want)
+        assert bool(finite.any()) and not bool(finite.all())
+        assert torch.equal(torch.where(finite, 0.0, got), torch.where(finite, 0.0, want))
+        assert float((got - want)[finite].abs().max()) <= 2e-5 * float(want[finite].abs().max())
