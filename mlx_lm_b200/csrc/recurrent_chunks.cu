@@ -448,7 +448,7 @@ gated_delta_chunks_kernel(const __nv_bfloat16* qkv, int ldq, int q_off, int k_of
       for (int i = 0; i < 2; ++i) {
         const int t = 2 * lane + i;
         const size_t row = (size_t)(t0 + c0 + t);
-        l[i] = t < nc ? (double)(negA * softplus_f(to_f(a_raw[row * lda + h]) + bias)) : 0.;
+        l[i] = t < nc ? log_decay(negA, softplus_f(to_f(a_raw[row * lda + h]) + bias)) : 0.;
         beta[i] = t < nc ? 1.f / (1.f + expf(-to_f(b_raw[row * ldb + h]))) : 0.f;
       }
       chunk_sums(l[0], l[1], lane);
@@ -513,7 +513,7 @@ gated_delta_chunks_kernel(const __nv_bfloat16* qkv, int ldq, int q_off, int k_of
 #pragma unroll
           for (int i = 0; i < 2; ++i) {
             const float d = s + i <= t ? expf((float)(sm.sum[t] - sm.sum[s + i])) * sm.rk[s + i] : 0.f;
-            w[i] = d * sm.rq[t] * qk[j][e + i];
+            w[i] = s + i <= t ? d * sm.rq[t] * qk[j][e + i] : 0.f;
             sm.m[t * LM + s + i] = s + i < t ? d * sm.beta[t] * sm.rk[t] * kk[j][e + i] : 0.f;
           }
           store_split(sm.p[0] + t * LP + s, RC_Q * LP, w[0], w[1]);
@@ -564,17 +564,23 @@ gated_delta_chunks_kernel(const __nv_bfloat16* qkv, int ldq, int q_off, int k_of
       float rb[16];
 #pragma unroll
       for (int j = 0; j < 16; ++j) rb[j] = sm.r[(16 * b + j) * GD_VS + lane];
-      float ub[2];
+      // The inverse of a triangular block: row i takes the right sides up to its own and no others (which may not be finite).
+      float ub[2] = {0.f, 0.f};
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const float4* t = reinterpret_cast<const float4*>(sm.inv[b] + (warp + 8 * i) * LI);
-        float s = 0.f;
+      for (int j = 0; j < 4; ++j) {
+        const float4 w = reinterpret_cast<const float4*>(sm.inv[b] + (warp + 8) * LI)[j];
+        const float m[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float4 w = t[j];
-          s = fmaf(w.x, rb[4 * j], fmaf(w.y, rb[4 * j + 1], fmaf(w.z, rb[4 * j + 2], fmaf(w.w, rb[4 * j + 3], s))));
-        }
-        ub[i] = s;
+        for (int e = 3; e >= 0; --e)
+          if (4 * j + e < 8 || 4 * j + e - 8 <= warp) ub[1] = fmaf(m[e], rb[4 * j + e], ub[1]);
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const float4 w = reinterpret_cast<const float4*>(sm.inv[b] + warp * LI)[j];
+        const float m[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int e = 3; e >= 0; --e)
+          if (4 * j + e <= warp) ub[0] = fmaf(m[e], rb[4 * j + e], ub[0]);
       }
       __syncthreads();
 #pragma unroll
@@ -596,14 +602,16 @@ gated_delta_chunks_kernel(const __nv_bfloat16* qkv, int ldq, int q_off, int k_of
       __syncthreads();
     }
     __syncthreads();
+    bool bad = false;                        // an update that is not finite
     for (int e = tid; e < RC_Q * GD_VS / 2; e += RC_THREADS) {
       const int s = e / (GD_VS / 2), c = 2 * (e - s * (GD_VS / 2));
       const float2 u = *reinterpret_cast<const float2*>(sm.r + s * GD_VS + c);
       const float w = sm.left[s] * sm.rk[s];
       store_split(sm.u[0] + s * LV + c, RC_Q * LV, u.x, u.y);
       store_split(sm.wu[0] + s * LV + c, RC_Q * LV, w * u.x, w * u.y);
+      bad |= !(fabsf(u.x) < INFINITY && fabsf(u.y) < INFINITY);
     }
-    __syncthreads();
+    bad = __syncthreads_or(bad);
     float low[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
     for (int k = 0; k <= 16 * ti; k += 16) {      // both sides in three numbers: the six products that reach 24 bits
       unsigned a[3][4], bb[3][4];
@@ -611,6 +619,10 @@ gated_delta_chunks_kernel(const __nv_bfloat16* qkv, int ldq, int q_off, int k_of
       for (int pl = 0; pl < 3; ++pl) {
         frag_a(a[pl], sm.p[pl] + 16 * ti * LP + k, LP, lane);
         frag_b_t(bb[pl], sm.u[pl] + k * LV + c16, LV, lane);
+      }
+      if (bad && k == 16 * ti) {      // not finite: the first of an update's three numbers, beside zeros
+#pragma unroll
+        for (int i = 0; i < 4; ++i) drop_bad(bb[0][i]);
       }
 #pragma unroll
       for (int sum = 2; sum >= 0; --sum)
@@ -620,6 +632,7 @@ gated_delta_chunks_kernel(const __nv_bfloat16* qkv, int ldq, int q_off, int k_of
           mma_plane(acc[1], low[1], sum, a[pl], bb[sum - pl][2], bb[sum - pl][3]);
         }
     }
+    if (bad) add_bad(acc, sm.p[0], RC_Q * LP, LP, ti, c16, g, q, [&](int s, int c) { return sm.r[s * GD_VS + c]; });
 #pragma unroll
     for (int j = 0; j < 2; ++j)
 #pragma unroll

@@ -178,3 +178,56 @@ def test_state_space_chunks_from_a_state_that_is_not_finite():
         assert bool(finite.any()) and not bool(finite.all())
         assert torch.equal(torch.where(finite, 0.0, got), torch.where(finite, 0.0, want))
         assert float((got - want)[finite].abs().max()) <= 2e-5 * float(want[finite].abs().max())
+
+
+@pytest.mark.parametrize("row,place,value", BAD)
+@pytest.mark.parametrize("where", ["v", "k", "q", "a", "b"])
+def test_gated_delta_rows_before_one_that_is_not_finite(row, place, value, where):
+    """As for the state-space layer; a decay's or an update strength's input is a NaN (an infinity gives a finite gate)."""
+    from mlx_lm_b200 import ops
+    H, K, V, T = 2, 64, 64, 130
+    torch.manual_seed(row)
+    consts = [torch.randn(H, device=DEV) * 0.5 for _ in range(2)]
+    token_req, first = arrays((T,))
+    qkv0 = torch.randn(T + 2, 2 * K + H * V, device=DEV).to(torch.bfloat16)
+    ab0 = [torch.randn(T + 2, H, device=DEV).to(torch.bfloat16) for _ in range(2)]
+    got = {}
+    for kernel in ("chunks", "scan"):
+        for v in (1.0, value):
+            qkv, (a, b) = qkv0.clone(), (t.clone() for t in ab0)
+            if where in "ab":
+                (a if where == "a" else b)[row, 0] = v if v == 1.0 else float("nan")
+            else:
+                qkv[row, {"q": 0, "k": K, "v": 2 * K}[where] + place % 64] = v
+            S, o = torch.zeros(1, H, V, K, device=DEV), torch.zeros(T + 2, H * V, device=DEV)
+            f = ops.gated_delta_chunks if kernel == "chunks" else ops.gated_delta_scan
+            f(qkv, 0, K, 2 * K, b, a, *consts, S, torch.zeros(1, dtype=torch.int32, device=DEV), token_req, first, o, H, 1,
+              ops.current_stream())
+            got[kernel, v == 1.0] = o, S
+    for kernel in ("chunks", "scan"):
+        (o, S), (fo, fS) = got[kernel, False], got[kernel, True]
+        assert torch.equal(o[:row], fo[:row])
+        assert not bool(torch.isfinite(o[row]).all())
+        assert torch.equal(torch.isfinite(o), torch.isfinite(got["scan", False][0]))
+        assert torch.equal(torch.isfinite(S), torch.isfinite(got["scan", False][1]))
+
+
+def test_gated_delta_chunks_forget_at_an_infinite_step():
+    """A decay of zero: what the state held is gone, and what follows is finite and as token by token."""
+    from mlx_lm_b200 import ops
+    H, K, V, T = 1, 32, 32, 70
+    torch.manual_seed(5)
+    consts = [torch.randn(H, device=DEV) * 0.5 for _ in range(2)]
+    token_req, first = arrays((T,))
+    qkv = torch.randn(T + 2, 2 * K + V, device=DEV).to(torch.bfloat16)
+    a, b = (torch.randn(T + 2, H, device=DEV).to(torch.bfloat16) for _ in range(2))
+    a[21, 0] = a[22, 0] = float("inf")
+    outs = []
+    for f in (ops.gated_delta_scan, ops.gated_delta_chunks):
+        S, o = torch.ones(1, H, V, K, device=DEV), torch.zeros(T + 2, V, device=DEV)
+        f(qkv, 0, K, 2 * K, b, a, *consts, S, torch.zeros(1, dtype=torch.int32, device=DEV), token_req, first, o, H, 1,
+          ops.current_stream())
+        outs.append((o[:T], S))
+    for got, want in zip(outs[1], outs[0]):
+        assert bool(torch.isfinite(want).all())
+        assert float((got - want).abs().max()) <= 2e-5 * float(want.abs().max())
