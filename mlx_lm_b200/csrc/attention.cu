@@ -315,7 +315,14 @@ attention_portions_f32_kernel(const float* q, int ldq, const int4* __restrict__ 
       sm.k[d][key] = kq[i].x; sm.k[d + 1][key] = kq[i].y; sm.k[d + 2][key] = kq[i].z; sm.k[d + 3][key] = kq[i].w;
       *reinterpret_cast<float4*>(&sm.v[key][d]) = vq[i];
     }
-    __syncthreads();
+    // Where some query does not see some key (a weight of zero), a value that is not finite must not reach it.
+    bool bad = false;
+    if (j0 + AP_Q - 1 > pos0 || (window > 0 && j0 <= last - window)) {
+#pragma unroll
+      for (int i = 0; i < PIECES; ++i)
+        bad |= !(fabsf(vq[i].x) < INFINITY && fabsf(vq[i].y) < INFINITY && fabsf(vq[i].z) < INFINITY && fabsf(vq[i].w) < INFINITY);
+    }
+    bad = __syncthreads_or(bad);
     float s[8][4];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
@@ -371,7 +378,7 @@ attention_portions_f32_kernel(const float* q, int ldq, const int4* __restrict__ 
     }
     __syncwarp();          // a warp reads back the probabilities of its own queries
     const int nk = min(AP_Q, last - j0 + 1);
-    auto add_values = [&](int jj, auto some) {       // some: not every query sees every key of this block
+    auto add_values = [&](int jj, auto some) {       // some: only to the queries that see the key
       float a[8], b[VD];
       *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(&sm.p[jj][8 * ty]);
       *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(&sm.p[jj][8 * ty + 4]);
@@ -379,14 +386,13 @@ attention_portions_f32_kernel(const float* q, int ldq, const int4* __restrict__ 
       for (int d = 0; d < VD; d += 2) *reinterpret_cast<float2*>(b + d) = *reinterpret_cast<const float2*>(&sm.v[jj][VD * tx + d]);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        // a key that a query does not see adds nothing, not zero times its value: the value may be infinite
         const int ahead = j0 + jj - (pos0 + 8 * ty + i);
         if (decltype(some)::value && (ahead > 0 || (window > 0 && ahead <= -window))) continue;
 #pragma unroll
         for (int d = 0; d < VD; ++d) o[i][d] = fmaf(a[i], b[d], o[i][d]);
       }
     };
-    if (j0 + AP_Q - 1 <= pos0 && (window <= 0 || j0 > last - window)) {
+    if (!bad) {
 #pragma unroll 4
       for (int jj = 0; jj < nk; ++jj) add_values(jj, std::false_type());
     } else {
