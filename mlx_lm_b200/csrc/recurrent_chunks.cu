@@ -174,7 +174,10 @@ mamba2_chunks_kernel(const __nv_bfloat16* xbc, int ldx, int x_off, int b_off, in
   const int grp = h / (H / G);
   pdl_trigger();
   const int n = run_length(token_req, t0, t1, r);
-  if (n < 2) return;                      // single rows go through the scan
+  if (n < 2) {                            // single rows go through the scan
+    pdl_wait();                           // dependents were let go above: a grid without runs must not end before its predecessor
+    return;
+  }
   // This warp's part of the state, as accumulators: columns v0 + 16 vi .., rows NP / 4 * ni .. of the state, in tiles of 8.
   constexpr int NT = NP / 32;
   const int vi = warp & 1, ni = warp >> 1;
@@ -409,7 +412,10 @@ gated_delta_chunks_kernel(const __nv_bfloat16* qkv, int ldq, int q_off, int k_of
   const int grp = h / (H / G);
   pdl_trigger();
   const int n = run_length(token_req, t0, t1, r);
-  if (n < 2) return;
+  if (n < 2) {
+    pdl_wait();
+    return;
+  }
   // this warp's part of the state, as accumulators: columns v0 + 16 vi .., rows 16 ni .. of the state, in tiles of 8
   const int vi = warp & 1, ni = warp >> 1;
   float S[2][4];

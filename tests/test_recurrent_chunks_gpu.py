@@ -231,3 +231,27 @@ def test_gated_delta_chunks_forget_at_an_infinite_step():
     for got, want in zip(outs[1], outs[0]):
         assert bool(torch.isfinite(want).all())
         assert float((got - want).abs().max()) <= 2e-5 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("kind", ["state space", "delta rule"])
+def test_steps_of_single_rows_keep_the_order_of_kernels(kind):
+    """A grid that finds no run of several rows ends no earlier than the kernel before it, whose result the kernel behind reads."""
+    from mlx_lm_b200 import ops
+    H, R = 4, 16
+    a, w = torch.randn(128, 8192, device=DEV), torch.randn(2048, 8192, device=DEV)
+    c, got, stream = torch.zeros(128, 2048, device=DEV), torch.zeros(128, 2048, device=DEV), ops.current_stream()
+    rows = torch.arange(128, dtype=torch.int32, device=DEV)
+    req, first = torch.arange(R, dtype=torch.int32, device=DEV), torch.arange(R + 1, dtype=torch.int32, device=DEV)
+    x, g = torch.randn(R, 3 * H * 32, device=DEV).to(torch.bfloat16), torch.randn(R, H, device=DEV).to(torch.bfloat16)
+    consts, S, y = [torch.zeros(H, device=DEV) for _ in range(3)], torch.zeros(R, H, 32, 32, device=DEV), torch.zeros(R, H * 32, device=DEV)
+    for _ in range(10):
+        c.zero_()
+        ops.linear_generic(a, w, None, c, stream)
+        if kind == "state space":
+            ops.mamba2_chunks(x, 0, H * 32, 2 * H * 32, g, *consts, S, req, req, first, y, H, H, stream)
+        else:
+            ops.gated_delta_chunks(x, 0, H * 32, 2 * H * 32, g, g, *consts[:2], S, req, req, first, y, H, H, stream)
+        ops.gather_rows(c, rows, got, stream)
+        torch.cuda.synchronize()
+        assert torch.equal(got, c) and float(c[-1].abs().max()) > 0
+    assert float(y.abs().max()) == 0.0
