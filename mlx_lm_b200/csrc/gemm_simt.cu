@@ -16,6 +16,8 @@
 //                 single tile.  1024 rows: 1024 x 1024 245 -> 70 us, 3072 x 1024 300 -> 208, 1024 x 4096 973 -> 264 (the
 //                 64 x 64 tiles of 4 x 4 a thread that this replaces, which read global memory between two barriers):
 //                 31 to 35 TFLOP/s of the 74 that the FMA pipes have.
+//   linear_small  any M, N; one segment, or few outputs.  64 x 64 outputs a block of 256 threads, 4 x 4 a thread, the next K step on
+//                 its way during this one's FMAs.  64 rows, 512 x 64: 6.0 us in float32, 6.2 in bfloat16.
 //   linear_rows   float32, up to 16 rows, 16-byte rows: bound by the stream of W (one row: 206 MB in 70 us) and by latency.
 //                 A warp takes 8 columns and a segment at a time; its W and A pieces travel by cp.async into memory of its
 //                 own, the first of W before the wait for the kernel before.  One row: 1024 x 1024 70 -> 2.7 us,
@@ -43,21 +45,49 @@ __device__ __forceinline__ f32x2 twice(float v) {
   return d;
 }
 
-// Four neighbouring k of one row as float32; zeros outside the matrix.
-template <typename T, bool VEC>
-__device__ __forceinline__ float4 load_k4(const T* p, bool row_ok, int k, int K) {
-  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (!row_ok) return v;
-  if (VEC) {                      // float32 rows of 16-byte pieces: K % 4 == 0
-    if (k < K) v = *reinterpret_cast<const float4*>(p + k);
-  } else {
-    if (k < K) v.x = to_f(p[k]);
-    if (k + 1 < K) v.y = to_f(p[k + 1]);
-    if (k + 2 < K) v.z = to_f(p[k + 2]);
-    if (k + 3 < K) v.w = to_f(p[k + 3]);
+// Four neighbouring k of one row as they lie in memory, zeros outside the matrix; made float32 when they are stored, so that all
+// loads of a thread are on their way together.  VEC: one access (K and the row stride multiples of 4, bases aligned to it).
+template <typename T, bool VEC> struct Quad;
+template <bool VEC>
+struct Quad<float, VEC> {
+  float4 v;
+  __device__ __forceinline__ void load(const float* p, bool row_ok, int k, int K) {
+    if (VEC) {
+      v = row_ok && k < K ? *reinterpret_cast<const float4*>(p + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+    } else {
+      v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (!row_ok) return;
+      if (k < K) v.x = p[k];
+      if (k + 1 < K) v.y = p[k + 1];
+      if (k + 2 < K) v.z = p[k + 2];
+      if (k + 3 < K) v.w = p[k + 3];
+    }
   }
-  return v;
-}
+  __device__ __forceinline__ float4 value() const { return v; }
+};
+template <>
+struct Quad<__nv_bfloat16, true> {
+  uint2 v;
+  __device__ __forceinline__ void load(const __nv_bfloat16* p, bool row_ok, int k, int K) {
+    v = row_ok && k < K ? *reinterpret_cast<const uint2*>(p + k) : make_uint2(0u, 0u);
+  }
+  __device__ __forceinline__ float4 value() const {
+    return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16),
+                       __uint_as_float(v.y & 0xffff0000u));
+  }
+};
+template <>
+struct Quad<__nv_bfloat16, false> {
+  unsigned v[4];
+  __device__ __forceinline__ void load(const __nv_bfloat16* p, bool row_ok, int k, int K) {
+    const unsigned short* u = reinterpret_cast<const unsigned short*>(p);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = row_ok && k + i < K ? u[k + i] : 0u;
+  }
+  __device__ __forceinline__ float4 value() const {
+    return make_float4(__uint_as_float(v[0] << 16), __uint_as_float(v[1] << 16), __uint_as_float(v[2] << 16), __uint_as_float(v[3] << 16));
+  }
+};
 
 // Two groups of BM threads take the segments in turns, each through tiles of its own; the second hands its sums to the
 // first, which adds them up in order.
@@ -83,19 +113,19 @@ linear_tile_kernel(const T* A, const T* __restrict__ W, const float* __restrict_
   const int tx = lane & 7, ty = (lane >> 3) + 4 * warp;
   // A warp fetches 16 rows by 8 k: whole sectors, and stores of 32 different banks.
   const int lr = (lane & 15) + 16 * (warp >> 1), lk = 4 * ((lane >> 4) + 2 * (warp & 1));
-  float4 aq[AQ], wq[WQ];
+  Quad<T, VEC> aq[AQ], wq[WQ];
   auto fetch_w = [&](int k0) {
 #pragma unroll
     for (int i = 0; i < WQ; ++i) {
       const int n = n0 + lr + i * (BM / 4);
-      wq[i] = load_k4<T, VEC>(W + (size_t)n * K, n < N, k0 + lk, K);
+      wq[i].load(W + (size_t)n * K, n < N, k0 + lk, K);
     }
   };
   auto fetch_a = [&](int k0) {
 #pragma unroll
     for (int i = 0; i < AQ; ++i) {
       const int m = m0 + lr + i * (BM / 4);
-      aq[i] = load_k4<T, VEC>(A + (size_t)m * lda, m < M, k0 + lk, K);
+      aq[i].load(A + (size_t)m * lda, m < M, k0 + lk, K);
     }
   };
   auto put = [&](int b) {
@@ -103,13 +133,15 @@ linear_tile_kernel(const T* A, const T* __restrict__ W, const float* __restrict_
     for (int i = 0; i < AQ; ++i) {
       float (*d)[TileMemory<BM>::LDA] = sm.a[group][b];
       const int r = lr + i * (BM / 4);
-      d[lk][r] = aq[i].x; d[lk + 1][r] = aq[i].y; d[lk + 2][r] = aq[i].z; d[lk + 3][r] = aq[i].w;
+      const float4 v = aq[i].value();
+      d[lk][r] = v.x; d[lk + 1][r] = v.y; d[lk + 2][r] = v.z; d[lk + 3][r] = v.w;
     }
 #pragma unroll
     for (int i = 0; i < WQ; ++i) {
       float (*d)[TileMemory<BM>::LDW] = sm.w[group][b];
       const int c = lr + i * (BM / 4);
-      d[lk][c] = wq[i].x; d[lk + 1][c] = wq[i].y; d[lk + 2][c] = wq[i].z; d[lk + 3][c] = wq[i].w;
+      const float4 v = wq[i].value();
+      d[lk][c] = v.x; d[lk + 1][c] = v.y; d[lk + 2][c] = v.z; d[lk + 3][c] = v.w;
     }
   };
   auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "r"(BM) : "memory"); };
@@ -197,6 +229,92 @@ linear_tile_kernel(const T* A, const T* __restrict__ W, const float* __restrict_
         C[(size_t)m * ldc + n] = from_f<TO>(v);
       }
     }
+}
+
+// ---------------------------------------------------------------- small products
+
+// Bound by the chain of K steps.  64 x 64 outputs a block of 256 threads, 4 x 4 a thread, two K steps in shared memory: the tiles
+// above have half of their threads without work when there is one segment, and four times as much for a thread to fetch a step.
+template <typename T, typename TO, int EPI, bool VEC>
+__global__ void __launch_bounds__(256)
+linear_small_kernel(const T* A, const T* __restrict__ W, const float* __restrict__ bias, const TO* residual, TO* C, int M, int N,
+                    int K, int lda, int ldc) {
+  __shared__ __align__(16) float sa[2][BK][64 + 4];
+  __shared__ __align__(16) float sw[2][BK][BN + 4];
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;      // rows 4 ty .., columns 4 tx ..
+  const int m0 = blockIdx.y * 64, n0 = blockIdx.x * BN;
+  const int lr = tid >> 2, lk = (tid & 3) * 4;                    // a thread fetches four k of one row of A and of W
+  const bool m_in = m0 + lr < M, n_in = n0 + lr < N;
+  const T* w_row = W + (size_t)(n_in ? n0 + lr : 0) * K;
+  Quad<T, VEC> aq, wq;
+  wq.load(w_row, n_in, lk, K);
+  pdl_trigger();
+  pdl_wait();
+  A = after_wait(A);
+  residual = after_wait(residual);
+  const T* a_row = A + (size_t)(m_in ? m0 + lr : 0) * lda;
+  auto put = [&](int b) {
+    const float4 a = aq.value(), w = wq.value();
+    sa[b][lk][lr] = a.x; sa[b][lk + 1][lr] = a.y; sa[b][lk + 2][lr] = a.z; sa[b][lk + 3][lr] = a.w;
+    sw[b][lk][lr] = w.x; sw[b][lk + 1][lr] = w.y; sw[b][lk + 2][lr] = w.z; sw[b][lk + 3][lr] = w.w;
+  };
+  float tot[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) tot[i][j] = 0.f;
+  aq.load(a_row, m_in, lk, K);
+  put(0);
+  __syncthreads();
+  int b = 0;
+  for (int s0 = 0; s0 < K; s0 += SEG) {
+    float acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    const int end = min(s0 + SEG, K);
+    for (int k0 = s0; k0 < end; k0 += BK) {
+      const bool more = k0 + BK < K;
+      if (more) {
+        wq.load(w_row, n_in, k0 + BK + lk, K);
+        aq.load(a_row, m_in, k0 + BK + lk, K);
+      }
+#pragma unroll
+      for (int kk = 0; kk < BK; ++kk) {
+        const float4 a = *reinterpret_cast<const float4*>(&sa[b][kk][ty * 4]), w = *reinterpret_cast<const float4*>(&sw[b][kk][tx * 4]);
+        const float av[4] = {a.x, a.y, a.z, a.w}, wv[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
+      }
+      if (more) {
+        b ^= 1;
+        put(b);
+        __syncthreads();
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) tot[i][j] += acc[i][j];
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int m = m0 + 4 * ty + i;
+    if (m >= M) continue;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int n = n0 + 4 * tx + j;
+      if (n >= N) continue;
+      float v = tot[i][j];
+      if (bias) v += bias[n];
+      v = activate<EPI, false>(v);
+      if (residual) v += to_f(residual[(size_t)m * ldc + n]);
+      C[(size_t)m * ldc + n] = from_f<TO>(v);
+    }
+  }
 }
 
 // ---------------------------------------------------------------- few rows
@@ -326,12 +444,27 @@ static int launch_tile(const void* A, const void* W, const float* bias, const vo
 }
 
 template <typename T, typename TO, bool VEC>
+static int launch_small(const void* A, const void* W, const float* bias, const void* residual, void* C, int M, int N, int K,
+                        int lda, int ldc, int epi, cudaStream_t stream) {
+  const dim3 grid((N + BN - 1) / BN, (M + 63) / 64);
+  return dispatch_activation(epi, [&](auto e) {
+    launch_pdl(linear_small_kernel<T, TO, decltype(e)::value, VEC>, grid, dim3(256), 0, stream, (const T*)A, (const T*)W, bias,
+               (const TO*)residual, (TO*)C, M, N, K, lda, ldc);
+    return mlxb_check_launch("linear (generic, small)");
+  });
+}
+
+template <typename T, typename TO, bool VEC>
 static int launch(const void* A, const void* W, const float* bias, const void* residual, void* C, int M, int N,
                   int K, int lda, int ldc, int epi, cudaStream_t stream) {
-  // An SM works through its tiles at a rate that hardly depends on their size, so what counts is the most rows of 64 x 64
+  // Small products first: one segment, or few tiles of up to 320 (64 rows, bfloat16 and float32: 512 x 64 6.2 and 6.0 us here, 10.4
+  // and 9.8 on the tiles; 96 x 320 20.2 and 18.1, on the tiles 22.2 and 20.2; 1024 x 1024 59 and 52, on the tiles 54 and 48).
+  // On the tiles an SM works at a rate that hardly depends on their size, so what counts is the most rows of 64 x 64
   // outputs that one SM gets; at a tie the larger tile reads less.
-  const long long cols = (N + BN - 1) / BN, sms = mlxb_sm_count();
-  const long long large = 2 * (((M + 127) / 128 * cols + sms - 1) / sms), small = ((M + 63) / 64 * cols + sms - 1) / sms;
+  const long long cols = (N + BN - 1) / BN, sms = mlxb_sm_count(), tiles = (M + 63) / 64 * cols;
+  if (K <= SEG || (K <= 320 && tiles <= sms))
+    return launch_small<T, TO, VEC>(A, W, bias, residual, C, M, N, K, lda, ldc, epi, stream);
+  const long long large = 2 * (((M + 127) / 128 * cols + sms - 1) / sms), small = (tiles + sms - 1) / sms;
   if (large <= small) return launch_tile<T, TO, 128, VEC>(A, W, bias, residual, C, M, N, K, lda, ldc, epi, stream);
   return launch_tile<T, TO, 64, VEC>(A, W, bias, residual, C, M, N, K, lda, ldc, epi, stream);
 }
@@ -357,6 +490,9 @@ MLXB_EXPORT int mlxb_linear_simt(int dtype, int out_f32, const void* A, const vo
     return launch<float, float, false>(A, W, bias, residual, C, M, N, K, lda, ldc, epi, stream);
   }
   if (dtype == MLXB_BF16) {
+    const bool vec = K % 4 == 0 && lda % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 7) == 0;
+    if (vec && out_f32) return launch<__nv_bfloat16, float, true>(A, W, bias, residual, C, M, N, K, lda, ldc, epi, stream);
+    if (vec) return launch<__nv_bfloat16, __nv_bfloat16, true>(A, W, bias, residual, C, M, N, K, lda, ldc, epi, stream);
     if (out_f32) return launch<__nv_bfloat16, float, false>(A, W, bias, residual, C, M, N, K, lda, ldc, epi, stream);
     return launch<__nv_bfloat16, __nv_bfloat16, false>(A, W, bias, residual, C, M, N, K, lda, ldc, epi, stream);
   }

@@ -92,3 +92,29 @@ def test_float32_portions_keep_values_a_query_does_not_see_out(ops, bad, window)
         sees &= torch.arange(n, device="cuda") < at + window
     assert torch.equal(outs[0][~sees], outs[1][~sees])
     assert not bool(torch.isfinite(outs[1][sees]).any())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("N,K", [(7, 4), (65, 50), (130, 64), (64, 127), (1030, 128), (70, 132), (96, 319), (40, 320), (40, 324), (64, 1001)])
+def test_linear_on_cuda_cores(ops, dtype, N, K):
+    """The small products' kernel and the tiles', around the sizes where one takes over from the other: sums of exact products (of
+    bfloat16 numbers) in segments of 128, the same bits however many rows the call has, bfloat16 results those sums rounded once."""
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    draw = lambda *s: torch.randn(*s, generator=g, device="cuda").to(dtype)
+    x, w, b = draw(1100, K), draw(N, K) / math.sqrt(K), draw(N).float()
+    w = w.to(dtype)
+    want = x.double() @ w.double().T + b
+    whole = torch.empty(1100, N, device="cuda")
+    ops.linear_generic(x, w, b, whole, stream())
+    assert rel_err(whole, want) <= 1e-6
+    for M in (1, 17, 63, 65, 130, 600):
+        out = torch.empty(M, N, device="cuda")
+        ops.linear_generic(x[:M], w, b, out, stream())
+        assert torch.equal(out, whole[:M])
+        short = torch.empty(M, N, device="cuda", dtype=dtype)
+        ops.linear_generic(x[:M], w, b, short, stream())
+        assert torch.equal(short, out.to(dtype))
+    wide = draw(40, K + 3)                  # a row stride and a first column that no wide access can read
+    out = torch.empty(40, N, device="cuda")
+    ops.linear_generic(wide[:, 1:K + 1], w, None, out, stream())
+    assert rel_err(out, wide[:, 1:K + 1].double() @ w.double().T) <= 1e-6
