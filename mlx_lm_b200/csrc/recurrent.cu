@@ -22,6 +22,7 @@
 // at a time are staged in shared memory by the whole block, laid out so that a thread fetches its 16 values
 // with four 16-byte loads; four tokens at a time go through the recurrence, their read-outs reduced together.
 #include "common.cuh"
+#include "recurrent_tiles.cuh"
 
 MLXB_DEFINE_LAST_ERROR()
 
@@ -287,7 +288,7 @@ mamba2_scan_kernel(const T* xbc, int ldx, int x_off, int b_off, int c_off, const
                    const float* __restrict__ dt_bias, const float* __restrict__ A_log,
                    const float* __restrict__ Dskip, float* state, const int* __restrict__ slots,
                    const int* __restrict__ token_req, const int* __restrict__ req_first_token, float* __restrict__ y,
-                   int ldy, int H, int G, int N, int V, int VB, int max_run) {
+                   int ldy, int H, int G, int N, int V, int VB, int max_run, ChunkRule rule) {
   extern __shared__ __align__(16) float sm[];
   constexpr int NP = NS * SCAN_SEG;        // floats of a token's staged B (or C)
   float* sB = sm;                          // [CHUNK][NP]
@@ -311,7 +312,7 @@ mamba2_scan_kernel(const T* xbc, int ldx, int x_off, int b_off, int c_off, const
   xbc = after_wait(xbc);
   dt_raw = after_wait(dt_raw);
   const int n = request_rows(token_req, t0, t1, r);
-  if (n == 0 || n > max_run) return;
+  if (n == 0 || (max_run > 0 && n > max_run && rule.chunks(n))) return;
   const float negA = -expf(A_log[h]), skip = Dskip[h], bias = dt_bias[h];
   for (int c0 = 0; c0 < n; c0 += SCAN_CHUNK) {
     const int nc = min(SCAN_CHUNK, n - c0);
@@ -391,17 +392,20 @@ mamba2_scan_kernel(const T* xbc, int ldx, int x_off, int b_off, int c_off, const
 
 // xbc: the convolution's output [n_tokens, ...] (activation dtype) holding x (H*V columns from x_off), B and C (G*N
 // columns each from b_off / c_off); dt_raw: [n_tokens, >= H] at row stride lddt; state: float32 [slots, H, V, N] (column by column);
-// y: float32 [n_tokens, H*V] at row stride ldy.  max_run: only requests that bring up to so many rows (0: all).
+// y: float32 [n_tokens, H*V] at row stride ldy.  max_run (0: all runs): of longer ones, only those that the
+// rule does not send through the chunks (recurrent_chunks.cu).
 MLXB_EXPORT int mlxb_mamba2_scan(int dtype, const void* xbc, int ldx, int x_off, int b_off, int c_off,
                                  const void* dt_raw, int lddt, const float* dt_bias, const float* A_log,
                                  const float* Dskip, float* state, const int* slots, const int* token_req,
                                  const int* req_first_token, float* y, int ldy, int H, int G, int N, int V,
-                                 int n_requests, int max_run, cudaStream_t stream) {
+                                 int n_requests, int max_run, int scan_fixed, int scan_row, int chunk_fixed,
+                                 int chunk_each, cudaStream_t stream) {
   if (n_requests <= 0) return 0;
   if (H <= 0 || G <= 0 || H % G || N <= 0 || V <= 0 || N > 32 * SCAN_NPT || n_requests > 65535)
     return mlxb_fail(MLXB_BAD_ARG, "mamba2_scan: %d heads in %d groups, state %d x %d (at most %d rows)", H, G, N, V,
                      32 * SCAN_NPT);
   const ScanShape sh = scan_shape(N, V, (long long)H * n_requests);
+  const ChunkRule rule = {scan_fixed, scan_row, chunk_fixed, chunk_each};
   const size_t smem = (size_t)(SCAN_CHUNK * (2 * sh.NS * SCAN_SEG + sh.VB + 2)) * sizeof(float);
   const dim3 grid(H, n_requests, sh.zblocks);
   if (dtype != MLXB_F32 && dtype != MLXB_BF16) return mlxb_fail(MLXB_BAD_DTYPE, "mamba2_scan: dtype code %d", dtype);
@@ -416,7 +420,7 @@ MLXB_EXPORT int mlxb_mamba2_scan(int dtype, const void* xbc, int ldx, int x_off,
     if (e == cudaSuccess)                                                                                                \
       launch_pdl(mamba2_scan_kernel<T_, NS_>, grid, dim3(sh.threads), smem, stream, (const T_*)xbc, ldx, x_off, b_off,   \
                  c_off, (const T_*)dt_raw, lddt, dt_bias, A_log, Dskip, state, slots, token_req, req_first_token, y,     \
-                 ldy, H, G, N, V, sh.VB, max_run > 0 ? max_run : 1 << 30);                                                                                \
+                 ldy, H, G, N, V, sh.VB, max_run, rule);                                                               \
   }
 #define M2_NS(NS_) { if (dtype == MLXB_F32) M2_GO(float, NS_) else M2_GO(__nv_bfloat16, NS_) }
   switch (sh.NS) {
@@ -439,7 +443,7 @@ gated_delta_scan_kernel(const T* qkv, int ldq, int q_off, int k_off, int v_off, 
                         const T* a_raw, int lda, const float* __restrict__ dt_bias, const float* __restrict__ A_log,
                         float* state, const int* __restrict__ slots, const int* __restrict__ token_req,
                         const int* __restrict__ req_first_token, float* __restrict__ o, int ldo, int H, int G, int K,
-                        int V, int VB, int max_run) {
+                        int V, int VB, int max_run, ChunkRule rule) {
   extern __shared__ __align__(16) float sm[];
   constexpr int NP = NS * SCAN_SEG;        // floats of a token's staged q (or k)
   float* sq = sm;                          // [CHUNK][NP]
@@ -463,7 +467,7 @@ gated_delta_scan_kernel(const T* qkv, int ldq, int q_off, int k_off, int v_off, 
   b_raw = after_wait(b_raw);
   a_raw = after_wait(a_raw);
   const int n = request_rows(token_req, t0, t1, r);
-  if (n == 0 || n > max_run) return;
+  if (n == 0 || (max_run > 0 && n > max_run && rule.chunks(n))) return;
   const float negA = -expf(A_log[h]), bias = dt_bias[h], q_scale = 1.f / sqrtf((float)K);
   for (int c0 = 0; c0 < n; c0 += SCAN_CHUNK) {
     const int nc = min(SCAN_CHUNK, n - c0);
@@ -573,12 +577,14 @@ MLXB_EXPORT int mlxb_gated_delta_scan(int dtype, const void* qkv, int ldq, int q
                                       const void* b_raw, int ldb, const void* a_raw, int lda, const float* dt_bias,
                                       const float* A_log, float* state, const int* slots, const int* token_req,
                                       const int* req_first_token, float* o, int ldo, int H, int G, int K, int V,
-                                      int n_requests, int max_run, cudaStream_t stream) {
+                                      int n_requests, int max_run, int scan_fixed, int scan_row, int chunk_fixed,
+                                      int chunk_each, cudaStream_t stream) {
   if (n_requests <= 0) return 0;
   if (H <= 0 || G <= 0 || H % G || K <= 0 || V <= 0 || K > 32 * SCAN_NPT || n_requests > 65535)
     return mlxb_fail(MLXB_BAD_ARG, "gated_delta_scan: %d heads over %d key heads, state %d x %d (at most %d rows)", H, G,
                      K, V, 32 * SCAN_NPT);
   const ScanShape sh = scan_shape(K, V, (long long)H * n_requests);
+  const ChunkRule rule = {scan_fixed, scan_row, chunk_fixed, chunk_each};
   const size_t smem = (size_t)(SCAN_CHUNK * (2 * sh.NS * SCAN_SEG + sh.VB + 2)) * sizeof(float);
   const dim3 grid(H, n_requests, sh.zblocks);
   if (dtype != MLXB_F32 && dtype != MLXB_BF16) return mlxb_fail(MLXB_BAD_DTYPE, "gated_delta_scan: dtype code %d", dtype);
@@ -593,7 +599,7 @@ MLXB_EXPORT int mlxb_gated_delta_scan(int dtype, const void* qkv, int ldq, int q
     if (e == cudaSuccess)                                                                                                 \
       launch_pdl(gated_delta_scan_kernel<T_, NS_>, grid, dim3(sh.threads), smem, stream, (const T_*)qkv, ldq, q_off,      \
                  k_off, v_off, (const T_*)b_raw, ldb, (const T_*)a_raw, lda, dt_bias, A_log, state, slots, token_req,     \
-                 req_first_token, o, ldo, H, G, K, V, sh.VB, max_run > 0 ? max_run : 1 << 30);                                                             \
+                 req_first_token, o, ldo, H, G, K, V, sh.VB, max_run, rule);                                              \
   }
 #define GD_NS(NS_) { if (dtype == MLXB_F32) GD_GO(float, NS_) else GD_GO(__nv_bfloat16, NS_) }
   switch (sh.NS) {

@@ -163,18 +163,19 @@ __global__ void __launch_bounds__(RC_THREADS, NP > 64 ? 1 : 2)      // as many a
 mamba2_chunks_kernel(const __nv_bfloat16* xbc, int ldx, int x_off, int b_off, int c_off, const __nv_bfloat16* dt_raw, int lddt,
                      const float* __restrict__ dt_bias, const float* __restrict__ A_log, const float* __restrict__ Dskip,
                      float* state, const int* __restrict__ slots, const int* __restrict__ token_req,
-                     const int* __restrict__ req_first_token, float* __restrict__ y, int ldy, int H, int G, int N, int V, int vec) {
+                     const int* __restrict__ req_first_token, const int* __restrict__ requests, ChunkRule rule, float* __restrict__ y,
+                     int ldy, int H, int G, int N, int V, int vec) {
   extern __shared__ __align__(16) char rc_sm[];
   using Mem = Mamba2Memory<NP>;
   Mem& sm = *reinterpret_cast<Mem*>(rc_sm);
   constexpr int LN = Mem::LN, LV = Mem::LV, LP = Mem::LP;
-  const int h = blockIdx.x, r = blockIdx.y, v0 = blockIdx.z * M2_VS;
-  const int t0 = req_first_token[r], t1 = req_first_token[r + 1];
+  const int h = blockIdx.x, r = requests != nullptr ? requests[blockIdx.y] : (int)blockIdx.y, v0 = blockIdx.z * M2_VS;
+  const int t0 = r >= 0 ? req_first_token[r] : 0, t1 = r >= 0 ? req_first_token[r + 1] : 0;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
   const int grp = h / (H / G);
   pdl_trigger();
   const int n = run_length(token_req, t0, t1, r);
-  if (n < 2) {                            // single rows go through the scan
+  if (!rule.chunks(n)) {                  // goes through the scan, or only fills the list of requests up
     pdl_wait();                           // dependents were let go above: a grid without runs must not end before its predecessor
     return;
   }
@@ -353,11 +354,13 @@ mamba2_chunks_kernel(const __nv_bfloat16* xbc, int ldx, int x_off, int b_off, in
     }
 }
 
-// The arguments of mlxb_mamba2_scan (bfloat16 inputs, states of up to 128 rows); requests that bring a single row are left out.
+// The arguments of mlxb_mamba2_scan (bfloat16 inputs, states of up to 128 rows).  requests: the n_requests to look at (-1: none),
+// or null for the first n_requests of the step; of these, the runs that the rule sends here.
 MLXB_EXPORT int mlxb_mamba2_chunks(const void* xbc, int ldx, int x_off, int b_off, int c_off, const void* dt_raw, int lddt,
                                    const float* dt_bias, const float* A_log, const float* Dskip, float* state, const int* slots,
                                    const int* token_req, const int* req_first_token, float* y, int ldy, int H, int G, int N, int V,
-                                   int n_requests, cudaStream_t stream) {
+                                   const int* requests, int n_requests, int scan_fixed, int scan_row, int chunk_fixed, int chunk_each,
+                                   cudaStream_t stream) {
   if (n_requests <= 0) return 0;
   if (H <= 0 || G <= 0 || H % G || N <= 0 || V <= 0 || N > 128 || n_requests > 65535)
     return mlxb_fail(MLXB_BAD_ARG, "mamba2_chunks: %d heads in %d groups, state %d x %d (at most 128 rows)", H, G, N, V);
@@ -368,8 +371,8 @@ MLXB_EXPORT int mlxb_mamba2_chunks(const void* xbc, int ldx, int x_off, int b_of
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return mlxb_fail((int)e, "mamba2_chunks: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
     launch_pdl(kern, grid, dim3(RC_THREADS), smem, stream, (const __nv_bfloat16*)xbc, ldx, x_off, b_off, c_off,
-               (const __nv_bfloat16*)dt_raw, lddt, dt_bias, A_log, Dskip, state, slots, token_req, req_first_token, y, ldy, H, G, N, V,
-               vec);
+               (const __nv_bfloat16*)dt_raw, lddt, dt_bias, A_log, Dskip, state, slots, token_req, req_first_token, requests,
+               ChunkRule{scan_fixed, scan_row, chunk_fixed, chunk_each}, y, ldy, H, G, N, V, vec);
     return mlxb_check_launch("mamba2_chunks");
   };
   if (N <= 64) return go(mamba2_chunks_kernel<64>, sizeof(Mamba2Memory<64>));
@@ -402,17 +405,18 @@ __global__ void __launch_bounds__(RC_THREADS)
 gated_delta_chunks_kernel(const __nv_bfloat16* qkv, int ldq, int q_off, int k_off, int v_off, const __nv_bfloat16* b_raw, int ldb,
                           const __nv_bfloat16* a_raw, int lda, const float* __restrict__ dt_bias, const float* __restrict__ A_log,
                           float* state, const int* __restrict__ slots, const int* __restrict__ token_req,
-                          const int* __restrict__ req_first_token, float* __restrict__ o, int ldo, int H, int G, int K, int V, int vec) {
+                          const int* __restrict__ req_first_token, const int* __restrict__ requests, ChunkRule rule,
+                          float* __restrict__ o, int ldo, int H, int G, int K, int V, int vec) {
   extern __shared__ __align__(16) char rc_sm[];
   DeltaMemory& sm = *reinterpret_cast<DeltaMemory*>(rc_sm);
   constexpr int LK = DeltaMemory::LK, LV = DeltaMemory::LV, LP = DeltaMemory::LP, LM = DeltaMemory::LM, LI = DeltaMemory::LI;
-  const int h = blockIdx.x, r = blockIdx.y, v0 = blockIdx.z * GD_VS;
-  const int t0 = req_first_token[r], t1 = req_first_token[r + 1];
+  const int h = blockIdx.x, r = requests != nullptr ? requests[blockIdx.y] : (int)blockIdx.y, v0 = blockIdx.z * GD_VS;
+  const int t0 = r >= 0 ? req_first_token[r] : 0, t1 = r >= 0 ? req_first_token[r + 1] : 0;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
   const int grp = h / (H / G);
   pdl_trigger();
   const int n = run_length(token_req, t0, t1, r);
-  if (n < 2) {
+  if (!rule.chunks(n)) {
     pdl_wait();
     return;
   }
@@ -678,7 +682,8 @@ gated_delta_chunks_kernel(const __nv_bfloat16* qkv, int ldq, int q_off, int k_of
 MLXB_EXPORT int mlxb_gated_delta_chunks(const void* qkv, int ldq, int q_off, int k_off, int v_off, const void* b_raw, int ldb,
                                         const void* a_raw, int lda, const float* dt_bias, const float* A_log, float* state,
                                         const int* slots, const int* token_req, const int* req_first_token, float* o, int ldo, int H,
-                                        int G, int K, int V, int n_requests, cudaStream_t stream) {
+                                        int G, int K, int V, const int* requests, int n_requests, int scan_fixed, int scan_row,
+                                        int chunk_fixed, int chunk_each, cudaStream_t stream) {
   if (n_requests <= 0) return 0;
   if (H <= 0 || G <= 0 || H % G || K <= 0 || V <= 0 || K > GD_KP || n_requests > 65535)
     return mlxb_fail(MLXB_BAD_ARG, "gated_delta_chunks: %d heads over %d key heads, state %d x %d (at most %d rows)", H, G, K, V, GD_KP);
@@ -689,6 +694,7 @@ MLXB_EXPORT int mlxb_gated_delta_chunks(const void* qkv, int ldq, int q_off, int
   if (e != cudaSuccess) return mlxb_fail((int)e, "gated_delta_chunks: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
   launch_pdl(gated_delta_chunks_kernel, dim3(H, n_requests, (V + GD_VS - 1) / GD_VS), dim3(RC_THREADS), smem, stream,
              (const __nv_bfloat16*)qkv, ldq, q_off, k_off, v_off, (const __nv_bfloat16*)b_raw, ldb, (const __nv_bfloat16*)a_raw, lda,
-             dt_bias, A_log, state, slots, token_req, req_first_token, o, ldo, H, G, K, V, vec);
+             dt_bias, A_log, state, slots, token_req, req_first_token, requests, ChunkRule{scan_fixed, scan_row, chunk_fixed, chunk_each}, o, ldo,
+             H, G, K, V, vec);
   return mlxb_check_launch("gated_delta_chunks");
 }

@@ -14,6 +14,16 @@ __device__ __forceinline__ int run_length(const int* __restrict__ token_req, int
   return n;
 }
 
+// A request's run of rows goes through a recurrence token by token or in chunks of 64 rows, whichever takes less time by this
+// rule (nanoseconds of a launch, from the layer's sizes and the number of requests with runs; what is known of the times
+// stands with the rule's maker, ops.chunk_rule).  A single row never goes in chunks.
+struct ChunkRule {
+  int scan_fixed, scan_row, chunk_fixed, chunk_each;
+  __device__ __forceinline__ bool chunks(int n) const {
+    return n > 1 && chunk_fixed + (long long)chunk_each * ((n + 63) / 64) < scan_fixed + (long long)scan_row * n;
+  }
+};
+
 // Rows of v: columns v0 .. v0 + VS - 1 of one head into [rows, lds]; zeros beyond n rows and beyond V columns.
 template <bool VEC>
 __device__ __forceinline__ void stage_values(const __nv_bfloat16* src, int ld, int row0, int n, int rows, int v0, int V, int VS,

@@ -19,7 +19,7 @@ into one pinned host buffer and reach the device in one copy.
 from __future__ import annotations
 
 from dataclasses import dataclass, field
-from typing import Dict, Hashable, List, Optional, Sequence
+from typing import Dict, Hashable, List, Optional, Sequence, Tuple
 
 import numpy as np
 import torch
@@ -136,8 +136,19 @@ class StepContext:
         # the single-token rows as tiles of one query: int32 [n_single, 4] = (token row, 1, block-table row,
         # position), or (token row, 0, 0, 0) for a row that pads the step
         self.single_tiles = None
+        # the lengths of the entries that bring several tokens (host side)
+        self.runs: Tuple[int, ...] = ()
+        self._rules: Dict[tuple, Optional[ops.ChunkRule]] = {}
         self._tables: List[torch.Tensor] = []
         self._slots: Optional[torch.Tensor] = None
+
+    def chunk_rule(self, recurrence: tuple) -> Optional[ops.ChunkRule]:
+        """How this step's runs go through a part's ``chunked_recurrence`` (see ``ops.chunk_rule``)."""
+        if self.dtype != torch.bfloat16 or not self.runs:
+            return None
+        if recurrence not in self._rules:
+            self._rules[recurrence] = ops.chunk_rule(*recurrence, self.runs, sms=ops.sm_count())
+        return self._rules[recurrence]
 
     def cache_view(self, entry: RunEntry) -> LayerCacheView:
         mgr = self.engine.cache
@@ -207,6 +218,7 @@ class Engine:
         # arguments), which skips the Python of the parts and of the kernel wrappers: possible when every
         # part only launches kernels whose arguments are fixed by the shape (Part.replayable).
         self.use_replay = all(p.all_replayable() for p in d.parts())
+        self._recurrences = sorted(set().union(*(p.all_chunked_recurrences() for p in d.parts())))
         self._plans: Dict[tuple, tuple] = {}
         self.n_replayed = 0
 
@@ -401,6 +413,7 @@ class Engine:
             if n_single_rows:
                 h[off["single_tiles"]: off["single_tiles"] + 4 * n_single_rows] = \
                     np.asarray(single_tiles, dtype=np.int32).reshape(-1)
+            ctx.runs = tuple(len(e.tokens) for e in entries if len(e.tokens) > 1)
             rids = [e.rid for e in entries]
             for g in range(len(mgr.kv_groups)):
                 o = off[f"table{g}"]
@@ -424,7 +437,8 @@ class Engine:
             if n_single_rows:
                 ctx.single_tiles = view("single_tiles", 4 * n_single_rows)
             ctx._tables = [view(f"table{g}", R * W).view(R, W) for g in range(len(mgr.kv_groups))]
-            logits = self._run(ctx, (T, R, L_rows, n_single_rows, n_tiles, ctx.stream, dev.data_ptr()))
+            logits = self._run(ctx, (T, R, L_rows, n_single_rows, n_tiles, ctx.stream, dev.data_ptr())
+                               + tuple(ctx.chunk_rule(c) for c in self._recurrences))
         except BaseException:
             # The step did not run to its end: its positions are not part of the requests.  The pages taken for
             # them go back, and the requests continue from where they were.

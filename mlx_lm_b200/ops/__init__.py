@@ -14,7 +14,7 @@ from __future__ import annotations
 
 import ctypes
 from ctypes import c_float, c_int, c_void_p
-from typing import Optional
+from typing import NamedTuple, Optional
 
 import torch
 
@@ -1028,16 +1028,70 @@ def conv_silu(x, weight, bias, state, slots, positions, token_req, req_first_tok
           _p(req_first_position), _p(out), _rows(out, "conv out"), T, slots.numel(), int(bool(activation)), stream)
 
 
+class ChunkRule(NamedTuple):
+    """Which of two ways a request's run of rows goes through a recurrence: token by token, or in chunks of 64 rows on tensor
+    cores.  Nanoseconds of a launch; whole numbers, so that host and kernels (csrc/recurrent_tiles.cuh) agree."""
+    scan_fixed: int
+    scan_row: int
+    chunk_fixed: int
+    chunk_each: int
+
+    def chunks(self, n: int) -> bool:
+        return n > 1 and self.chunk_fixed + self.chunk_each * ((n + 63) // 64) < self.scan_fixed + self.scan_row * n
+
+
+CHUNKS = ChunkRule(0, 1, 0, 0)      # every run of several rows in chunks
+MAMBA2_CHUNK_ROWS, DELTA_CHUNK_ROWS = 128, 64      # rows of a state that the chunked kernels take at most
+
+
+def chunk_rule(kind: str, n_heads: int, state_rows: int, columns: int, runs, sms: int = 148) -> Optional[ChunkRule]:
+    """How the rows of a step go through a recurrence (``kind``: ``"mamba2"`` or ``"delta"``, ``n_heads`` states of
+    ``state_rows x columns``, bfloat16 inputs), where requests bring the ``runs`` of several rows: None: all token by token;
+    ``CHUNKS``: all in chunks; else the rule that says which.
+
+    A block of the chunked kernels holds an SM (two do for states of up to 64 rows of the state-space layer) for 1.3 us and
+    what its chunks take, however few rows a chunk has; blocks beyond the SMs come in waves.  The scan's blocks share the SMs: a row
+    takes their latency until the SMs are full, then what their threads take.  Measured at 1 to 32 requests of 2 to 256 rows
+    and the sizes of models 1024 and 2048 wide, the state-space layer (32 heads of 128 x 64) breaks even at 20 to 28 rows:
+    one request of 16 rows 7 us by the scan and 9 in a chunk, of 64 rows 21 and 9; 32 requests of 8 rows 53 and 112.  The delta rule (64 x 64)
+    at 23 rows for up to 64 states, at 41 for 128; 256 states are never faster in chunks (96 rows 60 and 81 us), 512 from 122
+    rows on.  Chunks have to win by a twentieth: times of the scan differ by that much with the shapes of its blocks."""
+    if not runs or state_rows > (MAMBA2_CHUNK_ROWS if kind == "mamba2" else DELTA_CHUNK_ROWS):
+        return None
+    pairs = len(runs) * n_heads
+    # the scan's blocks, as csrc/recurrent.cu cuts them: threads an SM gets at most
+    per_column = 1
+    while per_column * 16 < state_rows:
+        per_column *= 2
+    lanes = 32 // per_column
+    wide = min(-(-columns // lanes) * lanes, 512 // per_column)
+    while wide > lanes and pairs * -(-columns // wide) < sms:
+        half = -(-(wide // 2) // lanes) * lanes
+        if half >= wide or half * per_column < 128:
+            break
+        wide = half
+    threads = -(-pairs * -(-columns // wide) // sms) * wide * per_column
+    scan_row = max(360, 460 * threads // 512) if kind == "mamba2" else max(420, 560 * threads // 512)
+    blocks, two = pairs * -(-columns // 32), kind == "mamba2" and state_rows <= 64
+    waves = -(-blocks // (2 * sms if two else sms))
+    each = 10000 if kind != "mamba2" else (6550 if not two else 5600 if blocks <= sms else 6900)
+    rule = ChunkRule(max(1500, 3700 * threads // 512), scan_row, 1365 * waves, each * waves * 21 // 20)
+    ways = [rule.chunks(n) for n in runs]
+    return CHUNKS if all(ways) else rule if any(ways) else None
+
+
 _M2_ARGS = [c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
-            c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]
+            c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int] + [c_int] * 5 + [c_void_p]
+_M2_CHUNKS_ARGS = _M2_ARGS[1:21] + [c_void_p] + [c_int] * 5 + [c_void_p]
 
 
 def mamba2_scan(xbc, x_off: int, b_off: int, c_off: int, dt_raw, dt_bias, a_log, d_skip, state, slots, token_req,
-                req_first_token, y, n_heads: int, n_groups: int, stream, max_run: int = 0) -> None:
+                req_first_token, y, n_heads: int, n_groups: int, stream, max_run: int = 0, rule: ChunkRule = CHUNKS) -> None:
     """The selective state-space recurrence per (request, head): ``S <- exp(-exp(A_log) dt) S + dt B x^T``,
     ``y = S^T C + D x`` with ``dt = softplus(dt_raw + dt_bias)``.  ``xbc [T, .]`` holds x, B, C from the given
     column offsets; ``state`` float32 ``[slots, heads, V, N]`` (a head's ``N x V`` state column by column); ``y``
-    float32 ``[T, heads*V]``.  ``max_run``: only requests that bring up to so many rows (0: all)."""
+    float32 ``[T, heads*V]``.  ``max_run`` (0: all runs): of longer ones, only those that ``rule`` does not send through
+    ``mamba2_chunks``."""
     _need(xbc, dt_raw.dtype, "mamba2_scan xbc")
     _need(state, torch.float32, "mamba2_scan state")
     _need(y, torch.float32, "mamba2_scan y")
@@ -1049,21 +1103,21 @@ def mamba2_scan(xbc, x_off: int, b_off: int, c_off: int, dt_raw, dt_bias, a_log,
     _call("recurrent", "mlxb_mamba2_scan", _M2_ARGS, dtype_code(xbc.dtype), _p(xbc), _rows(xbc, "mamba2_scan xbc"), x_off,
           b_off, c_off, _p(dt_raw), _rows(dt_raw, "mamba2_scan dt"), _p(dt_bias), _p(a_log), _p(d_skip), _p(state),
           _p(slots), _p(token_req), _p(req_first_token), _p(y), _rows(y, "mamba2_scan y"), H, n_groups, N, V,
-          slots.numel(), int(max_run), stream)
+          slots.numel(), int(max_run), *rule, stream)
 
 
-def recurrent_chunks_supported(dtype, state_rows: int, limit: int) -> bool:
-    """Whether runs of several rows go through the chunked kernels: bfloat16 inputs, states of up to ``limit`` rows."""
-    return dtype == torch.bfloat16 and state_rows <= limit
-
-
-MAMBA2_CHUNK_ROWS, DELTA_CHUNK_ROWS = 128, 64      # rows of a state that the chunked kernels take at most
+def _requests(requests, slots, what: str):
+    """(list of the requests to look at, their number): None stands for all of the step."""
+    if requests is None:
+        return None, slots.numel()
+    _need(requests, torch.int32, what + " requests")
+    return _p(requests), requests.numel()
 
 
 def mamba2_chunks(xbc, x_off: int, b_off: int, c_off: int, dt_raw, dt_bias, a_log, d_skip, state, slots, token_req,
-                  req_first_token, y, n_heads: int, n_groups: int, stream) -> None:
-    """``mamba2_scan`` for the requests that bring several rows, 64 rows at a time on tensor cores (bfloat16 inputs,
-    csrc/recurrent_chunks.cu); requests with a single row are left to the scan."""
+                  req_first_token, y, n_heads: int, n_groups: int, stream, requests=None, rule: ChunkRule = CHUNKS) -> None:
+    """``mamba2_scan`` for the requests whose runs ``rule`` sends here, 64 rows at a time on tensor cores (bfloat16 inputs,
+    csrc/recurrent_chunks.cu).  ``requests``: int32, the requests to look at (-1: none); None: all."""
     _need(xbc, torch.bfloat16, "mamba2_chunks xbc")
     _need(dt_raw, torch.bfloat16, "mamba2_chunks dt")
     _need(state, torch.float32, "mamba2_chunks state")
@@ -1073,22 +1127,25 @@ def mamba2_chunks(xbc, x_off: int, b_off: int, c_off: int, dt_raw, dt_bias, a_lo
         raise KernelError(f"mamba2_chunks: state {tuple(state.shape)} for {n_heads} heads, y {tuple(y.shape)}")
     for t in (dt_bias, a_log, d_skip):
         _need(t, torch.float32, "mamba2_chunks head constants")
-    _call("recurrent_chunks", "mlxb_mamba2_chunks", _M2_ARGS[1:-2] + [c_void_p], _p(xbc), _rows(xbc, "mamba2_chunks xbc"), x_off,
+    listed, n_listed = _requests(requests, slots, "mamba2_chunks")
+    _call("recurrent_chunks", "mlxb_mamba2_chunks", _M2_CHUNKS_ARGS, _p(xbc), _rows(xbc, "mamba2_chunks xbc"), x_off,
           b_off, c_off, _p(dt_raw), _rows(dt_raw, "mamba2_chunks dt"), _p(dt_bias), _p(a_log), _p(d_skip), _p(state),
           _p(slots), _p(token_req), _p(req_first_token), _p(y), _rows(y, "mamba2_chunks y"), H, n_groups, N, V,
-          slots.numel(), stream)
+          listed, n_listed, *rule, stream)
 
 
 _GD_ARGS = [c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
-            c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]
+            c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int] + [c_int] * 5 + [c_void_p]
+_GD_CHUNKS_ARGS = _GD_ARGS[1:22] + [c_void_p] + [c_int] * 5 + [c_void_p]
 
 
 def gated_delta_scan(qkv, q_off: int, k_off: int, v_off: int, b_raw, a_raw, dt_bias, a_log, state, slots, token_req,
-                     req_first_token, o, n_heads: int, n_key_heads: int, stream, max_run: int = 0) -> None:
+                     req_first_token, o, n_heads: int, n_key_heads: int, stream, max_run: int = 0,
+                     rule: ChunkRule = CHUNKS) -> None:
     """The gated delta rule per (request, head): ``S <- g S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q`` with
     q and k made unit vectors (q also divided by sqrt(dim)), ``beta = sigmoid(b_raw)``,
     ``g = exp(-exp(A_log) softplus(a_raw + dt_bias))``.  ``state`` float32 ``[slots, heads, V, K]`` (a head's
-    ``K x V`` state column by column); ``o`` float32.  ``max_run``: only requests that bring up to so many rows (0: all)."""
+    ``K x V`` state column by column); ``o`` float32.  ``max_run`` and ``rule`` as for ``mamba2_scan``."""
     _need(state, torch.float32, "gated_delta_scan state")
     _need(o, torch.float32, "gated_delta_scan o")
     _need(b_raw, qkv.dtype, "gated_delta_scan b")
@@ -1099,13 +1156,14 @@ def gated_delta_scan(qkv, q_off: int, k_off: int, v_off: int, b_raw, a_raw, dt_b
     _call("recurrent", "mlxb_gated_delta_scan", _GD_ARGS, dtype_code(qkv.dtype), _p(qkv), _rows(qkv, "gated_delta qkv"),
           q_off, k_off, v_off, _p(b_raw), _rows(b_raw, "gated_delta b"), _p(a_raw), _rows(a_raw, "gated_delta a"),
           _p(dt_bias), _p(a_log), _p(state), _p(slots), _p(token_req), _p(req_first_token), _p(o),
-          _rows(o, "gated_delta o"), H, n_key_heads, K, V, slots.numel(), int(max_run), stream)
+          _rows(o, "gated_delta o"), H, n_key_heads, K, V, slots.numel(), int(max_run), *rule, stream)
 
 
 def gated_delta_chunks(qkv, q_off: int, k_off: int, v_off: int, b_raw, a_raw, dt_bias, a_log, state, slots, token_req,
-                       req_first_token, o, n_heads: int, n_key_heads: int, stream) -> None:
-    """``gated_delta_scan`` for the requests that bring several rows, 64 rows at a time on tensor cores (bfloat16 inputs,
-    csrc/recurrent_chunks.cu); requests with a single row are left to the scan."""
+                       req_first_token, o, n_heads: int, n_key_heads: int, stream, requests=None,
+                       rule: ChunkRule = CHUNKS) -> None:
+    """``gated_delta_scan`` for the requests whose runs ``rule`` sends here, 64 rows at a time on tensor cores (bfloat16 inputs,
+    csrc/recurrent_chunks.cu).  ``requests`` as for ``mamba2_chunks``."""
     _need(state, torch.float32, "gated_delta_chunks state")
     _need(o, torch.float32, "gated_delta_chunks o")
     for t in (qkv, b_raw, a_raw):
@@ -1113,10 +1171,11 @@ def gated_delta_chunks(qkv, q_off: int, k_off: int, v_off: int, b_raw, a_raw, dt
     _, H, V, K = state.shape
     if H != n_heads or o.shape[1] != H * V or not state.is_contiguous() or K > DELTA_CHUNK_ROWS:
         raise KernelError(f"gated_delta_chunks: state {tuple(state.shape)} for {n_heads} heads, o {tuple(o.shape)}")
-    _call("recurrent_chunks", "mlxb_gated_delta_chunks", _GD_ARGS[1:-2] + [c_void_p], _p(qkv), _rows(qkv, "gated_delta qkv"),
+    listed, n_listed = _requests(requests, slots, "gated_delta_chunks")
+    _call("recurrent_chunks", "mlxb_gated_delta_chunks", _GD_CHUNKS_ARGS, _p(qkv), _rows(qkv, "gated_delta qkv"),
           q_off, k_off, v_off, _p(b_raw), _rows(b_raw, "gated_delta b"), _p(a_raw), _rows(a_raw, "gated_delta a"),
           _p(dt_bias), _p(a_log), _p(state), _p(slots), _p(token_req), _p(req_first_token), _p(o),
-          _rows(o, "gated_delta o"), H, n_key_heads, K, V, slots.numel(), stream)
+          _rows(o, "gated_delta o"), H, n_key_heads, K, V, listed, n_listed, *rule, stream)
 
 
 # --------------------------------------------------------------------------

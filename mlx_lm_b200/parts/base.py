@@ -28,7 +28,7 @@ instances directly.
 from __future__ import annotations
 
 from dataclasses import dataclass
-from typing import Callable, Dict, List, Mapping, Optional, Sequence, Tuple
+from typing import Callable, Dict, List, Mapping, Optional, Sequence, Set, Tuple
 
 import torch
 
@@ -89,6 +89,9 @@ class Part:
     # then re-issues a recorded step of the same shape without calling forward() again.  Leave it False
     # for a part that does anything else (host-side loops over requests, torch operators, ...).
     replayable: bool = False
+    # A recurrence that runs in chunks: what ops.chunk_rule needs beside the step's runs.  Which way it takes is then part of
+    # a step's shape.
+    chunked_recurrence: Optional[tuple] = None
 
     def param_specs(self) -> List[ParamSpec]:
         return []
@@ -107,6 +110,10 @@ class Part:
 
     def all_replayable(self) -> bool:
         return self.replayable and all(c.all_replayable() for c in self.children())
+
+    def all_chunked_recurrences(self) -> Set[tuple]:
+        own = {self.chunked_recurrence} if self.chunked_recurrence else set()
+        return own.union(*(c.all_chunked_recurrences() for c in self.children()))
 
     def all_kernel_libs(self) -> List[str]:
         out = list(self.kernel_libs)

@@ -37,6 +37,7 @@ class Mamba2Mixer(Mixer):
         self.n_heads, self.vdim, self.state, self.groups, self.norm_groups = n_heads, vdim, state, groups, norm_groups
         self.taps, self.eps = taps, float(eps)
         self.inner = n_heads * vdim
+        self.chunked_recurrence = ("mamba2", n_heads, state, vdim)
         self.conv_width = self.inner + 2 * groups * state
         self.n_proj = 2 * self.inner + 2 * groups * state + n_heads
         self.proj = Linear(f"{name}.in", width, self.n_proj, bias=False, weight_suffix="", init=init)
@@ -81,11 +82,11 @@ class Mamba2Mixer(Mixer):
                   + 8.0 * min(T, ctx.n_requests) * inner * self.state)
         args = (xbc, 0, inner, inner + GN, proj[:, inner + self.conv_width:], self.dt_bias, self.a_log, self.d_skip,
                 ssm_state.state, ssm_state.slots, ctx.token_req, ctx.req_first_token, y, self.n_heads, self.groups, ctx.stream)
-        chunks = ctx.n_portion > 0 and ops.recurrent_chunks_supported(x.dtype, self.state, ops.MAMBA2_CHUNK_ROWS)
-        if chunks:
-            ops.mamba2_chunks(*args)
-        if not chunks or ctx.n_single:
-            ops.mamba2_scan(*args, max_run=1 if chunks else 0)
+        rule = ctx.chunk_rule(self.chunked_recurrence)
+        if rule is not None:
+            ops.mamba2_chunks(*args, rule=rule)
+        if rule is not ops.CHUNKS or ctx.n_single:
+            ops.mamba2_scan(*args, max_run=0 if rule is None else 1, rule=rule or ops.CHUNKS)
         g = ctx.ws.get("ssm_gated", T, inner, x.dtype)
         ops.label(self.name + ".norm", 8.0 * T * inner, (4.0 + 2 * x.element_size()) * T * inner)
         ops.rmsnorm(y, self.norm_w, g, self.eps, ctx.stream, groups=self.norm_groups, gate=proj[:, :inner],
@@ -116,6 +117,7 @@ class GatedDeltaMixer(Mixer):
         self.name, self.width = name, width
         self.n_heads, self.n_kv_heads, self.dim, self.vdim, self.taps, self.eps = n_heads, n_kv_heads, dim, vdim, taps, float(eps)
         self.qk_width, self.v_width = n_kv_heads * dim, n_heads * vdim
+        self.chunked_recurrence = ("delta", n_heads, dim, vdim)
         self.conv_width = 2 * self.qk_width + self.v_width
         self.proj = FusedLinear(f"{name}.in", width, [(f"{name}.q", self.qk_width), (f"{name}.k", self.qk_width),
                                                       (f"{name}.v", self.v_width), (f"{name}.g", self.v_width),
@@ -163,11 +165,11 @@ class GatedDeltaMixer(Mixer):
         args = (qkv, 0, self.qk_width, 2 * self.qk_width, proj[:, b_off:b_off + H], proj[:, b_off + H:b_off + 2 * H],
                 self.dt_bias, self.a_log, rule_state.state, rule_state.slots, ctx.token_req, ctx.req_first_token, o, H,
                 self.n_kv_heads, ctx.stream)
-        chunks = ctx.n_portion > 0 and ops.recurrent_chunks_supported(x.dtype, self.dim, ops.DELTA_CHUNK_ROWS)
-        if chunks:
-            ops.gated_delta_chunks(*args)
-        if not chunks or ctx.n_single:
-            ops.gated_delta_scan(*args, max_run=1 if chunks else 0)
+        rule = ctx.chunk_rule(self.chunked_recurrence)
+        if rule is not None:
+            ops.gated_delta_chunks(*args, rule=rule)
+        if rule is not ops.CHUNKS or ctx.n_single:
+            ops.gated_delta_scan(*args, max_run=0 if rule is None else 1, rule=rule or ops.CHUNKS)
         g = ctx.ws.get("delta_gated", T, self.v_width, x.dtype)
         ops.label(self.name + ".norm", 8.0 * T * self.v_width, (4.0 + 2 * x.element_size()) * T * self.v_width)
         ops.rmsnorm(o, self.norm_w, g, self.eps, ctx.stream, groups=H, period=self.vdim,

@@ -255,3 +255,92 @@ def test_steps_of_single_rows_keep_the_order_of_kernels(kind):
         torch.cuda.synchronize()
         assert torch.equal(got, c) and float(c[-1].abs().max()) > 0
     assert float(y.abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("kind", ["state space", "delta rule"])
+def test_every_run_goes_one_way(kind):
+    """A rule that sends runs of 20 rows and less through the scan: with the requests that bring several rows listed, both kernels
+    together leave what the scan alone does."""
+    from mlx_lm_b200 import ops
+    torch.manual_seed(2)
+    H, N, V, runs = 4, 32, 48, (1, 20, 70, 2, 21, 1)
+    rule = ops.ChunkRule(0, 10, 205, 0)
+    assert [rule.chunks(n) for n in runs] == [False, False, True, False, True, False]
+    token_req, first = arrays(runs)
+    T, R = token_req.numel(), len(runs)
+    slots = torch.arange(R, dtype=torch.int32, device=DEV)
+    listed = torch.tensor([2, 4, 1, 3, -1, -1], dtype=torch.int32, device=DEV)
+    x, g = torch.randn(T, H * V + 2 * H * N, device=DEV).to(torch.bfloat16), torch.randn(T, H, device=DEV).to(torch.bfloat16)
+    consts = [torch.randn(H, device=DEV) * 0.5 for _ in range(3)]
+    S0, out = torch.randn(R, H, V, N, device=DEV) * 0.1, []
+    for both in (True, False):
+        S, y = S0.clone(), torch.zeros(T, H * V, device=DEV)
+        if kind == "state space":
+            args = (x, 0, H * V, H * V + H * N, g, *consts, S, slots, token_req, first, y, H, H, ops.current_stream())
+            chunks, scan = ops.mamba2_chunks, ops.mamba2_scan
+        else:
+            args = (x, 0, H * N, 2 * H * N, g, g, *consts[:2], S, slots, token_req, first, y, H, H, ops.current_stream())
+            chunks, scan = ops.gated_delta_chunks, ops.gated_delta_scan
+        if both:
+            chunks(*args, requests=listed, rule=rule)
+            assert [bool(y[int(first[r])].any()) for r in range(R)] == [rule.chunks(n) for n in runs]
+            scan(*args, max_run=1, rule=rule)
+        else:
+            scan(*args)
+        out.append((y, S))
+    for got, want in zip(*out):
+        assert float((got - want).abs().max()) <= 2e-5 * float(want.abs().max())
+    for r, n in enumerate(runs):                       # what the scan did, it did as alone
+        if not rule.chunks(n):
+            assert torch.equal(out[0][0][int(first[r]):int(first[r]) + n], out[1][0][int(first[r]):int(first[r]) + n])
+            assert torch.equal(out[0][1][r], out[1][1][r])
+
+
+def test_a_plan_belongs_to_its_runs(tmp_path, monkeypatch):
+    """Steps of the same shape (rows, requests, tiles) whose runs go different ways: each re-issues a plan of its own."""
+    from lelatar_cases import CONFIG_Q, make_dir, tokens
+    from mlx_lm_b200 import ops
+    from mlx_lm_b200.engine import Engine, StepEntry
+    from mlx_lm_b200.weights import load_model
+    make_dir(tmp_path, CONFIG_Q, seed=3)
+    model = load_model(str(tmp_path), dtype="bfloat16")[0]
+    steps = [(50, 14), (40, 24), (47, 17), (60, 3), (33, 18), (50, 14)]
+
+    def go(limit):
+        rule = ops.ChunkRule(0, 10, 10 * limit, 0)
+        monkeypatch.setattr(ops, "chunk_rule", lambda *layer, sms=148: rule if any(rule.chunks(n) for n in layer[-1]) else None)
+        engine, out, calls = Engine(model, page_size=16, n_pages=64, max_requests=4, max_len=512), [], []
+        real = ops.mamba2_chunks
+        monkeypatch.setattr(ops, "mamba2_chunks", lambda *a, **k: (calls.append(1), real(*a, **k)))
+        for i, lengths in enumerate(steps):
+            for r in range(2):
+                engine.add_request((i, r))
+            out.append(engine.step([StepEntry((i, r), tokens(n, CONFIG_Q["vocab"], n), [n - 1]) for r, n in enumerate(lengths)]).clone())
+            for r in range(2):
+                engine.finish((i, r))
+        monkeypatch.setattr(ops, "mamba2_chunks", real)
+        return torch.stack(out), len(calls), engine.n_replayed
+
+    want, n, replayed = go(1 << 20)
+    assert n == 0 and replayed == len(steps) - 1
+    got, n, replayed = go(45)
+    assert n > 0 and replayed == len(steps) - 2
+    assert float((got - want).abs().max()) <= 0.06 * float(want.abs().max())
+    by_rows = [bool((got[i] == want[i]).all()) for i in range(len(steps))]
+    assert by_rows[1] and by_rows[4] and not all(by_rows)
+
+
+def test_short_prompts_launch_no_chunks(tmp_path, monkeypatch):
+    from lelatar_cases import CONFIG_Q, make_dir, tokens
+    from mlx_lm_b200 import ops
+    from mlx_lm_b200.engine import Engine, StepEntry
+    from mlx_lm_b200.weights import load_model
+    make_dir(tmp_path, CONFIG_Q, seed=3)
+    engine = Engine(load_model(str(tmp_path), dtype="bfloat16")[0], page_size=16, n_pages=64, max_requests=4, max_len=512)
+    seen = []
+    for name in ("mamba2_chunks", "gated_delta_chunks"):
+        monkeypatch.setattr(ops, name, lambda *a, name=name, real=getattr(ops, name), **k: (seen.append(name), real(*a, **k)))
+    for rid, n in (("short", 8), ("long", 200)):
+        engine.add_request(rid)
+        engine.step([StepEntry(rid, tokens(n, CONFIG_Q["vocab"], n), [n - 1])])
+        assert bool(seen) == (rid == "long")
