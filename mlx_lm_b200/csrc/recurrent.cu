@@ -302,6 +302,15 @@ mamba2_scan_kernel(const T* xbc, int ldx, int x_off, int b_off, int c_off, const
   const int s = tid % NS, vl = tid / NS, v = vb * VB + vl;
   const bool valid = v < V;
   const int g = h / (H / G);
+  // A run that goes in chunks is left out before its state is asked for.  The span of a request's rows may end in padding.
+  int n = -1;
+  if (max_run > 0 && t1 - t0 > max_run) {
+    n = request_rows(token_req, t0, t1, r);
+    if (n > max_run && rule.chunks(n)) {
+      pdl_wait();
+      return;
+    }
+  }
   // The state was last written by a step before this one (a cache is touched by one launch a step), so it can
   // be on its way before the wait for the kernel that wrote this step's inputs.
   float* st = state + ((size_t)slots[r] * H + h) * N * V + (size_t)(valid ? v : 0) * N;   // this thread's column
@@ -311,8 +320,8 @@ mamba2_scan_kernel(const T* xbc, int ldx, int x_off, int b_off, int c_off, const
   pdl_trigger();
   xbc = after_wait(xbc);
   dt_raw = after_wait(dt_raw);
-  const int n = request_rows(token_req, t0, t1, r);
-  if (n == 0 || (max_run > 0 && n > max_run && rule.chunks(n))) return;
+  if (n < 0) n = request_rows(token_req, t0, t1, r);
+  if (n == 0) return;
   const float negA = -expf(A_log[h]), skip = Dskip[h], bias = dt_bias[h];
   for (int c0 = 0; c0 < n; c0 += SCAN_CHUNK) {
     const int nc = min(SCAN_CHUNK, n - c0);
@@ -457,6 +466,14 @@ gated_delta_scan_kernel(const T* qkv, int ldq, int q_off, int k_off, int v_off, 
   const int s = tid % NS, vl = tid / NS, v = vb * VB + vl;
   const bool valid = v < V;
   const int g = h / (H / G);
+  int n = -1;
+  if (max_run > 0 && t1 - t0 > max_run) {
+    n = request_rows(token_req, t0, t1, r);
+    if (n > max_run && rule.chunks(n)) {
+      pdl_wait();
+      return;
+    }
+  }
   // older than this step (see mamba2_scan_kernel): asked for before the wait
   float* st = state + ((size_t)slots[r] * H + h) * K * V + (size_t)(valid ? v : 0) * K;   // this thread's column
   float S[SCAN_NPT];
@@ -466,8 +483,8 @@ gated_delta_scan_kernel(const T* qkv, int ldq, int q_off, int k_off, int v_off, 
   qkv = after_wait(qkv);
   b_raw = after_wait(b_raw);
   a_raw = after_wait(a_raw);
-  const int n = request_rows(token_req, t0, t1, r);
-  if (n == 0 || (max_run > 0 && n > max_run && rule.chunks(n))) return;
+  if (n < 0) n = request_rows(token_req, t0, t1, r);
+  if (n == 0) return;
   const float negA = -expf(A_log[h]), bias = dt_bias[h], q_scale = 1.f / sqrtf((float)K);
   for (int c0 = 0; c0 < n; c0 += SCAN_CHUNK) {
     const int nc = min(SCAN_CHUNK, n - c0);

@@ -136,8 +136,10 @@ class StepContext:
         # the single-token rows as tiles of one query: int32 [n_single, 4] = (token row, 1, block-table row,
         # position), or (token row, 0, 0, 0) for a row that pads the step
         self.single_tiles = None
-        # the lengths of the entries that bring several tokens (host side)
+        # the lengths of the entries that bring several tokens (host side), and, for a model with recurrences that run in
+        # chunks, those entries' request indexes, longest first, filled up with -1 (int32)
         self.runs: Tuple[int, ...] = ()
+        self.portion_requests = None
         self._rules: Dict[tuple, Optional[ops.ChunkRule]] = {}
         self._tables: List[torch.Tensor] = []
         self._slots: Optional[torch.Tensor] = None
@@ -341,12 +343,13 @@ class Engine:
             if L_rows:
                 L_rows = (L_rows + 7) // 8 * 8
         T = sum(span) + n_fake + n_pad_rows
+        n_listed = R - n_single_rows if n_portions and self._recurrences else 0
         mixed = 0 < n_single_rows < n_real + n_fake
         off, sizes = {}, [("tokens", T), ("positions", T), ("token_req", T), ("logit_rows", L_rows), ("slots", R),
                           ("req_first_token", R + 1), ("req_first_position", R),
                           ("single_rows", n_single_rows if mixed else 0),
                           ("portion_rows", T - n_single_rows if mixed else 0), ("tiles", 4 * n_tiles),
-                          ("single_tiles", 4 * n_single_rows)]
+                          ("single_tiles", 4 * n_single_rows), ("portion_requests", n_listed)]
         sizes += [(f"table{g}", R * W) for g in range(len(mgr.kv_groups))]
         total = 0
         for name, n in sizes:
@@ -414,6 +417,9 @@ class Engine:
                 h[off["single_tiles"]: off["single_tiles"] + 4 * n_single_rows] = \
                     np.asarray(single_tiles, dtype=np.int32).reshape(-1)
             ctx.runs = tuple(len(e.tokens) for e in entries if len(e.tokens) > 1)
+            if n_listed:
+                listed = sorted((r for r, e in enumerate(entries) if len(e.tokens) > 1), key=lambda r: -len(entries[r].tokens))
+                h[off["portion_requests"]: off["portion_requests"] + n_listed] = listed + [-1] * (n_listed - n_portions)
             rids = [e.rid for e in entries]
             for g in range(len(mgr.kv_groups)):
                 o = off[f"table{g}"]
@@ -436,6 +442,8 @@ class Engine:
                 ctx.portion_tiles, ctx.n_portion_tiles = view("tiles", 4 * n_tiles), n_tiles
             if n_single_rows:
                 ctx.single_tiles = view("single_tiles", 4 * n_single_rows)
+            if n_listed:
+                ctx.portion_requests = view("portion_requests", n_listed)
             ctx._tables = [view(f"table{g}", R * W).view(R, W) for g in range(len(mgr.kv_groups))]
             logits = self._run(ctx, (T, R, L_rows, n_single_rows, n_tiles, ctx.stream, dev.data_ptr())
                                + tuple(ctx.chunk_rule(c) for c in self._recurrences))

@@ -84,7 +84,7 @@ class Mamba2Mixer(Mixer):
                 ssm_state.state, ssm_state.slots, ctx.token_req, ctx.req_first_token, y, self.n_heads, self.groups, ctx.stream)
         rule = ctx.chunk_rule(self.chunked_recurrence)
         if rule is not None:
-            ops.mamba2_chunks(*args, rule=rule)
+            ops.mamba2_chunks(*args, requests=ctx.portion_requests, rule=rule)
         if rule is not ops.CHUNKS or ctx.n_single:
             ops.mamba2_scan(*args, max_run=0 if rule is None else 1, rule=rule or ops.CHUNKS)
         g = ctx.ws.get("ssm_gated", T, inner, x.dtype)
@@ -167,7 +167,7 @@ class GatedDeltaMixer(Mixer):
                 self.n_kv_heads, ctx.stream)
         rule = ctx.chunk_rule(self.chunked_recurrence)
         if rule is not None:
-            ops.gated_delta_chunks(*args, rule=rule)
+            ops.gated_delta_chunks(*args, requests=ctx.portion_requests, rule=rule)
         if rule is not ops.CHUNKS or ctx.n_single:
             ops.gated_delta_scan(*args, max_run=0 if rule is None else 1, rule=rule or ops.CHUNKS)
         g = ctx.ws.get("delta_gated", T, self.v_width, x.dtype)
