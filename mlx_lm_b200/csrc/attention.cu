@@ -423,16 +423,17 @@ MLXB_EXPORT int mlxb_attention_portions_f32(const float* q, int ldq, const int* 
   if (int e = check_common("attention", page, Hq, Hkv, Dh)) return e;
   if (Dh > 128 || Dh % 4 || ldq % 4 || (((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)tiles) & 15) || Hq > 65535)
     return mlxb_fail(MLXB_BAD_ARG, "attention (float32 portions): heads of %d (multiples of 4 up to 128), row stride %d", Dh, ldq);
-  auto go = [&](auto kernel, size_t smem) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static SharedLimit limits[3];
+  auto go = [&](auto kernel, size_t smem, SharedLimit& limit) {
+    const cudaError_t e = limit.raise(kernel, smem);
     if (e != cudaSuccess) return mlxb_fail((int)e, "attention: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
     launch_pdl(kernel, dim3(2 * n_tiles, Hq), dim3(128), smem, stream, q, ldq, (const int4*)tiles, block_table, max_pages, n_pages,
                page, Hq, Hkv, Dh, window, scale, k_pool, v_pool, out, ldo, status, sinks);
     return mlxb_check_launch("attention (float32 portions)");
   };
-  if (Dh <= 32) return go(attention_portions_f32_kernel<32>, sizeof(PortionMemory<32>));
-  if (Dh <= 64) return go(attention_portions_f32_kernel<64>, sizeof(PortionMemory<64>));
-  return go(attention_portions_f32_kernel<128>, sizeof(PortionMemory<128>));
+  if (Dh <= 32) return go(attention_portions_f32_kernel<32>, sizeof(PortionMemory<32>), limits[0]);
+  if (Dh <= 64) return go(attention_portions_f32_kernel<64>, sizeof(PortionMemory<64>), limits[1]);
+  return go(attention_portions_f32_kernel<128>, sizeof(PortionMemory<128>), limits[2]);
 }
 
 

@@ -12,6 +12,8 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <atomic>
+
 #define MLXB_EXPORT extern "C" __attribute__((visibility("default")))
 
 // dtype codes shared with mlx_lm_b200/ops (0 = float32, 1 = bfloat16)
@@ -80,6 +82,23 @@ static inline int mlxb_sm_count() {
   }
   return n;
 }
+
+// The shared memory that a kernel's launches may ask for, raised once per device: a call into the driver for every launch costs the
+// host as much as a small launch.  One object a kernel (static), always with the same number of bytes.
+struct SharedLimit {
+  std::atomic<unsigned char> raised[64];      // by device; zero in static storage
+  template <typename Kernel>
+  cudaError_t raise(Kernel kernel, size_t bytes) {
+    int dev = -1;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const bool known = dev >= 0 && dev < 64;
+    if (known && raised[dev].load(std::memory_order_relaxed)) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess && known) raised[dev].store(1, std::memory_order_relaxed);
+    return e;
+  }
+};
 
 static inline bool mlxb_pdl_enabled() {
   static int on = -1;

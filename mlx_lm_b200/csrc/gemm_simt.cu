@@ -413,15 +413,21 @@ linear_rows_kernel(const float* A, const float* __restrict__ W, const float* __r
 // here 6); K: the segments' sums have to fit shared memory beside the pieces.
 constexpr int RW_MAX_ROWS = 16, RW_MAX_K = 16384;
 
+static constexpr size_t rows_memory(int R, int nseg, int warps) {
+  return sizeof(float) * (size_t)(nseg * 4 * R * RW_COLS + warps * 2 * (RW_COLS + 4 * R) * RW_LD);
+}
+
 template <int R>
 static int launch_rows(const float* A, const float* W, const float* bias, const float* residual, float* C, int M, int N, int K,
                        int lda, int ldc, int epi, cudaStream_t stream) {
   const int nseg = (K + SEG - 1) / SEG, warps = nseg < rw_warps(R) ? nseg : rw_warps(R);
-  const size_t smem = sizeof(float) * (size_t)(nseg * 4 * R * RW_COLS + warps * 2 * (RW_COLS + 4 * R) * RW_LD);
+  const size_t smem = rows_memory(R, nseg, warps);
   return dispatch_activation(epi, [&](auto e) {
     auto kernel = linear_rows_kernel<decltype(e)::value, R>;
     if (smem > 48 * 1024) {
-      const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      static SharedLimit limit;
+      constexpr int WARPS = rw_warps(R), SEGS = RW_MAX_K / SEG;
+      const cudaError_t err = limit.raise(kernel, rows_memory(R, SEGS, WARPS));
       if (err != cudaSuccess) return mlxb_fail((int)err, "linear: %zu bytes of shared memory: %s", smem, cudaGetErrorString(err));
     }
     launch_pdl(kernel, dim3((N + RW_COLS - 1) / RW_COLS), dim3(32 * warps), smem, stream, A, W, bias, residual, C, M, N, K, lda, ldc);
@@ -435,7 +441,8 @@ static int launch_tile(const void* A, const void* W, const float* bias, const vo
   dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
   return dispatch_activation(epi, [&](auto e) {
     auto kernel = linear_tile_kernel<T, TO, decltype(e)::value, BM, VEC>;
-    const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileMemory<BM>));
+    static SharedLimit limit;
+    const cudaError_t err = limit.raise(kernel, sizeof(TileMemory<BM>));
     if (err != cudaSuccess) return mlxb_fail((int)err, "linear: %zu bytes of shared memory: %s", sizeof(TileMemory<BM>), cudaGetErrorString(err));
     launch_pdl(kernel, grid, dim3(BM * 2), sizeof(TileMemory<BM>), stream, (const T*)A, (const T*)W, bias, (const TO*)residual,
                (TO*)C, M, N, K, lda, ldc);

@@ -367,16 +367,17 @@ MLXB_EXPORT int mlxb_mamba2_chunks(const void* xbc, int ldx, int x_off, int b_of
   const int vec = (((uintptr_t)xbc & 15) == 0 && ldx % 8 == 0 && x_off % 8 == 0 && b_off % 8 == 0 && c_off % 8 == 0 && N % 8 == 0 &&
                    V % 8 == 0);
   const dim3 grid(H, n_requests, (V + M2_VS - 1) / M2_VS);
-  auto go = [&](auto kern, size_t smem) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static SharedLimit limits[2];
+  auto go = [&](auto kern, size_t smem, SharedLimit& limit) {
+    const cudaError_t e = limit.raise(kern, smem);
     if (e != cudaSuccess) return mlxb_fail((int)e, "mamba2_chunks: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
     launch_pdl(kern, grid, dim3(RC_THREADS), smem, stream, (const __nv_bfloat16*)xbc, ldx, x_off, b_off, c_off,
                (const __nv_bfloat16*)dt_raw, lddt, dt_bias, A_log, Dskip, state, slots, token_req, req_first_token, requests,
                ChunkRule{scan_fixed, scan_row, chunk_fixed, chunk_each}, y, ldy, H, G, N, V, vec);
     return mlxb_check_launch("mamba2_chunks");
   };
-  if (N <= 64) return go(mamba2_chunks_kernel<64>, sizeof(Mamba2Memory<64>));
-  return go(mamba2_chunks_kernel<128>, sizeof(Mamba2Memory<128>));
+  if (N <= 64) return go(mamba2_chunks_kernel<64>, sizeof(Mamba2Memory<64>), limits[0]);
+  return go(mamba2_chunks_kernel<128>, sizeof(Mamba2Memory<128>), limits[1]);
 }
 
 // ---------------------------------------------------------------- gated delta rule
@@ -690,7 +691,8 @@ MLXB_EXPORT int mlxb_gated_delta_chunks(const void* qkv, int ldq, int q_off, int
   const int vec = (((uintptr_t)qkv & 15) == 0 && ldq % 8 == 0 && q_off % 8 == 0 && k_off % 8 == 0 && v_off % 8 == 0 && K % 8 == 0 &&
                    V % 8 == 0);
   const size_t smem = sizeof(DeltaMemory);
-  const cudaError_t e = cudaFuncSetAttribute(gated_delta_chunks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static SharedLimit limit;
+  const cudaError_t e = limit.raise(gated_delta_chunks_kernel, smem);
   if (e != cudaSuccess) return mlxb_fail((int)e, "gated_delta_chunks: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
   launch_pdl(gated_delta_chunks_kernel, dim3(H, n_requests, (V + GD_VS - 1) / GD_VS), dim3(RC_THREADS), smem, stream,
              (const __nv_bfloat16*)qkv, ldq, q_off, k_off, v_off, (const __nv_bfloat16*)b_raw, ldb, (const __nv_bfloat16*)a_raw, lda,
