@@ -593,35 +593,38 @@ static int launch(const void* A, const void* W, const float* bias, const void* r
   });
 }
 
-// Tile shape and pairs or not: the form whose time, as a sum of what was measured, is least.  A block of 64 of K takes a CTA
-// 0.95 ns a row of A or W that it brings (128 + BN rows; 1.15 in a pair, whose CTAs bring 128 + BN / 2) or, in a pair, what its
-// products take (1.08 ns a column); a launch costs 4.5 us besides (set-up, the first copies, the last tile's results;
-// 1.2 less on tiles of 32, 0.9 on tiles of 64 columns), a pair's 6.0, and every further wave of tiles 0.8.  This gives each
-// form's time within 15 % at M from 128 to 2048, N from 1024 to 6400 and K from 1024 to 6400.  Single CTAs are best for short K
-// (2048 x 1024 x 1024: 7.9 us against 8.9), pairs for many products (2048 x 1600 x 6400: 33.9 against 38.0; 2048 x 6400 x
-// 1600: 31.4 against 34.0), and tiles of 64 or 32 columns where wider ones leave SMs idle (288 x 1280 x 1280: 6.0 against 7.7;
-// 288 x 1280 x 5120: 15.4 against 22.9; 768 x 1024 x 1024: 6.0 against 7.1).
+// Tile shape and pairs or not: the form whose time, as a sum of what was measured, is least: a launch (set-up, the first copies, the
+// last tile's results), every block of 64 of K, every further wave of tiles.  The constants are fits to the times of each form
+// at M from 65 to 2048 and N and K from 1024 to 8448, which they give within 5 %.  Single CTAs are best for short K and for up to some
+// 2048 of it on wide outputs (2048 x 1024 x 1024: 7.9 us against 8.9; 2048 x 2048 x 2048: 16.1 against 18.2), pairs for many products
+// (2048 x 1600 x 6400: 33.9 against 38.0; 2048 x 6400 x 1600: 31.4 against 34.0; 768 x 1600 x 6400: 21.6 against 24.1), and tiles of 64
+// or 32 columns where wider ones leave SMs idle (288 x 1280 x 1280: 6.0 against 7.7; 288 x 1280 x 5120: 15.4 against 22.9; 768 x 1024 x
+// 1024: 6.0 against 7.1).
 // A share of K for each of several CTAs would do more there, but then a row's sums would be added in an order that depends on
 // how many rows the call has.
 struct TileChoice { int bn, cg; };
+struct FormCost { int bn, cg; double launch, block, wave; };      // microseconds
+static constexpr FormCost FORMS[] = {{256, 1, 5.35, .288, 2.7}, {192, 1, 5.2, .247, 1.8}, {128, 1, 4.7, .198, 1.4}, {64, 1, 3.9, .174, .6},
+                                     {32, 1, 3.4, .160, .5},   {256, 2, 7.1, .288, .9},  {192, 2, 7.35, .216, 1.2}, {128, 2, 6.55, .149, 1.}};
+// 128 columns in stages of one block of K: nothing waits less often with two of them where K has no more (2048 x 1024 x 64: 4.3 us
+// against 4.8)
+static bool short_k(int K) { return K <= 2 * BK; }
 static TileChoice tile_choice(int M, int N, int K) {
   // experiments and tests: pairs 0 = never, 1 = wherever there are two row tiles; the width
   const char *want_pair = getenv("MLXB_TC_PAIR"), *want_bn = getenv("MLXB_TC_BN");
   const int sms = sm_count(), steps = (K + BK - 1) / BK;
   TileChoice best = {128, 1};
   double best_cost = -1.;
-  for (int cg = 1; cg <= 2; ++cg) {
-    if (cg == 2 && M <= BM) break;
-    if (want_pair && M > BM && (want_pair[0] == '1') != (cg == 2)) continue;
-    for (int bn : {256, 192, 128, 64, 32}) {
-      if (want_bn ? atoi(want_bn) != bn : (cg == 2 && bn < 128)) continue;
-      const long long tiles = (long long)((M + cg * BM - 1) / (cg * BM)) * ((N + bn - 1) / bn);
-      const int units = sms / cg;
-      const long long waves = (tiles + units - 1) / units;
-      const double step = cg == 1 ? 0.95 * (BM + bn) : (1.15 * (BM + bn / 2) > 1.08 * bn ? 1.15 * (BM + bn / 2) : 1.08 * bn);
-      const double cost = waves * steps * step + 800. * (waves - 1) + (cg == 1 ? (bn == 32 ? 3300. : (bn == 64 ? 3600. : 4500.)) : 6000.);
-      if (best_cost < 0. || cost < best_cost) { best = {bn, cg}; best_cost = cost; }
-    }
+  for (const FormCost& f : FORMS) {
+    if (f.cg == 2 && M <= BM) continue;
+    if (want_pair && M > BM && (want_pair[0] == '1') != (f.cg == 2)) continue;
+    if (want_bn && atoi(want_bn) != f.bn) continue;
+    const long long tiles = (long long)((M + f.cg * BM - 1) / (f.cg * BM)) * ((N + f.bn - 1) / f.bn);
+    const int units = sms / f.cg;
+    const long long waves = (tiles + units - 1) / units;
+    const double launch = f.bn == 128 && f.cg == 1 && short_k(K) ? f.launch - .5 : f.launch;
+    const double cost = launch + waves * steps * f.block + (waves - 1) * f.wave;
+    if (best_cost < 0. || cost < best_cost) { best = {f.bn, f.cg}; best_cost = cost; }
   }
   return best;
 }
@@ -644,6 +647,7 @@ static int launch_choice(const void* A, const void* W, const float* bias, const 
   }
   if (t.bn == 256) GO(256, 4, 1, 1)
   if (t.bn == 192) GO(192, 4, 1, 1)
+  if (t.bn == 128 && short_k(K)) GO(128, 4, 1, 1)
   if (t.bn == 128) GO(128, 3, 2, 1)
   if (t.bn == 64) GO(64, 4, 2, 1)
   GO(32, 4, 2, 1)
