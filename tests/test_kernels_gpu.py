@@ -417,6 +417,41 @@ def test_linear_qkv_to_cache_many_rows(ops, Hq, Hkv, Dh, page, K, pairs, monkeyp
     assert float(out[:, qw:].abs().max()) == 0.0                   # key and value columns of the output stay untouched
 
 
+@pytest.mark.parametrize("Hq,Hkv,Dh,page,K", [(3, 3, 32, 16, 96), (16, 16, 64, 16, 1024), (5, 1, 80, 16, 200)])
+@pytest.mark.parametrize("fold", [False, True])
+def test_linear_qkv_to_cache_forms(ops, Hq, Hkv, Dh, page, K, fold, monkeypatch):
+    """The fused cache write in every form of the tcgen05 kernel: each tile width with its own slices of columns for the epilogue's
+    warps (48 of them at 192), single CTAs and pairs, with and without the folded norm: the same bits in queries and pages, and
+    they are those of the plain linear layer's output."""
+    lens, new = [0, 37, 130, 5], [150, 75, 1, 91]
+    c = paged_case(torch.bfloat16, lens=lens, new=new, Hq=Hq, Hkv=Hkv, Dh=Dh, page=page, seed=K + 2)
+    g = torch.Generator().manual_seed(K)
+    n_pad, cut = 7, 150
+    M, N, qw, kw = c["T"] + n_pad, (Hq + 2 * Hkv) * Dh, Hq * Dh, Hkv * Dh
+    x = torch.randn(M, K, generator=g).to(torch.bfloat16).cuda()
+    w = (torch.randn(N, K, generator=g) / math.sqrt(K)).to(torch.bfloat16).cuda()
+    b, colsum = torch.randn(N, generator=g).cuda(), torch.randn(N, generator=g).cuda()
+    stats = torch.stack([torch.randn(M, generator=g), torch.rand(M, generator=g) + 0.5], dim=1).cuda()
+    positions = torch.cat([c["positions"][:cut], torch.zeros(n_pad, dtype=torch.int32), c["positions"][cut:]])
+    token_req = torch.cat([c["token_req"][:cut], torch.full((n_pad,), -1, dtype=torch.int32), c["token_req"][cut:]])
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    plain = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+    ops.linear_tensor_cores(x, w, b, plain, status, stream(), fold=(colsum, stats) if fold else None)
+    rows = plain.cpu()
+    rk, rv = R.kv_write(rows[:, qw:qw + kw], rows[:, qw + kw:], positions, token_req, c["bt"], c["k_pool"], c["v_pool"])
+    for pairs, width in [("0", n) for n in (32, 64, 128, 192, 256)] + [("1", n) for n in (128, 192, 256)]:
+        monkeypatch.setenv("MLXB_TC_PAIR", pairs)
+        monkeypatch.setenv("MLXB_TC_BN", str(width))
+        kp, vp = c["k_pool"].cuda(), c["v_pool"].cuda()
+        out = torch.zeros(M, N, dtype=torch.bfloat16, device="cuda")
+        ops.linear_qkv_to_cache(x, w, b, out, positions.cuda(), token_req.cuda(), c["bt"].cuda(), kp, vp, qw, status, stream(),
+                                fold=(colsum, stats) if fold else None)
+        assert torch.equal(out[:, :qw], plain[:, :qw]), (pairs, width)
+        assert torch.equal(kp.cpu(), rk) and torch.equal(vp.cpu(), rv), (pairs, width)
+        assert float(out[:, qw:].abs().max()) == 0.0
+    assert int(status.item()) == 0
+
+
 def test_linear_few_rows_refuses_odd_inner_size(ops):
     x = torch.zeros(2, 12, dtype=torch.bfloat16, device="cuda")
     w = torch.zeros(5, 12, dtype=torch.bfloat16, device="cuda")
