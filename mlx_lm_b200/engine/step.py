@@ -136,21 +136,30 @@ class StepContext:
         # the single-token rows as tiles of one query: int32 [n_single, 4] = (token row, 1, block-table row,
         # position), or (token row, 0, 0, 0) for a row that pads the step
         self.single_tiles = None
-        # the lengths of the entries that bring several tokens (host side), and, for a model with recurrences that run in
-        # chunks, those entries' request indexes, longest first, filled up with -1 (int32)
-        self.runs: Tuple[int, ...] = ()
+        # the first positions and lengths of the entries that bring several tokens (host side), and, for a model with recurrences
+        # that run in chunks, those entries' request indexes, longest first, filled up with -1 (int32)
+        self.portions: Tuple[Tuple[int, int], ...] = ()
         self.portion_requests = None
-        self._rules: Dict[tuple, Optional[ops.ChunkRule]] = {}
+        self._choices: Dict[tuple, object] = {}
         self._tables: List[torch.Tensor] = []
         self._slots: Optional[torch.Tensor] = None
 
     def chunk_rule(self, recurrence: tuple) -> Optional[ops.ChunkRule]:
         """How this step's runs go through a part's ``chunked_recurrence`` (see ``ops.chunk_rule``)."""
-        if self.dtype != torch.bfloat16 or not self.runs:
+        if self.dtype != torch.bfloat16 or not self.portions:
             return None
-        if recurrence not in self._rules:
-            self._rules[recurrence] = ops.chunk_rule(*recurrence, self.runs, sms=ops.sm_count())
-        return self._rules[recurrence]
+        if recurrence not in self._choices:
+            runs = tuple(n for _, n in self.portions)
+            self._choices[recurrence] = ops.chunk_rule(*recurrence, runs, sms=ops.sm_count())
+        return self._choices[recurrence]
+
+    def attention_in_tiles(self, attention: tuple) -> bool:
+        """Whether float32 portions run in tiles (see ``ops.attention_portions_f32_pays``)."""
+        if not self.portions:
+            return False
+        if attention not in self._choices:
+            self._choices[attention] = ops.attention_portions_f32_pays(*attention, self.portions, sms=ops.sm_count())
+        return self._choices[attention]
 
     def cache_view(self, entry: RunEntry) -> LayerCacheView:
         mgr = self.engine.cache
@@ -220,7 +229,9 @@ class Engine:
         # arguments), which skips the Python of the parts and of the kernel wrappers: possible when every
         # part only launches kernels whose arguments are fixed by the shape (Part.replayable).
         self.use_replay = all(p.all_replayable() for p in d.parts())
-        self._recurrences = sorted(set().union(*(p.all_chunked_recurrences() for p in d.parts())))
+        of = "chunked_recurrence" if model.dtype == torch.bfloat16 else "portion_attention"
+        choices = sorted(set().union(*(p.all_choices(of) for p in d.parts())))
+        self._recurrences, self._attentions = (choices, []) if model.dtype == torch.bfloat16 else ([], choices)
         self._plans: Dict[tuple, tuple] = {}
         self.n_replayed = 0
 
@@ -416,7 +427,7 @@ class Engine:
             if n_single_rows:
                 h[off["single_tiles"]: off["single_tiles"] + 4 * n_single_rows] = \
                     np.asarray(single_tiles, dtype=np.int32).reshape(-1)
-            ctx.runs = tuple(len(e.tokens) for e in entries if len(e.tokens) > 1)
+            ctx.portions = tuple((s.first_position, s.n_tokens) for s in ctx.spans if s.n_tokens > 1)
             if n_listed:
                 listed = sorted((r for r, e in enumerate(entries) if len(e.tokens) > 1), key=lambda r: -len(entries[r].tokens))
                 h[off["portion_requests"]: off["portion_requests"] + n_listed] = listed + [-1] * (n_listed - n_portions)
@@ -446,7 +457,8 @@ class Engine:
                 ctx.portion_requests = view("portion_requests", n_listed)
             ctx._tables = [view(f"table{g}", R * W).view(R, W) for g in range(len(mgr.kv_groups))]
             logits = self._run(ctx, (T, R, L_rows, n_single_rows, n_tiles, ctx.stream, dev.data_ptr())
-                               + tuple(ctx.chunk_rule(c) for c in self._recurrences))
+                               + tuple(ctx.chunk_rule(c) for c in self._recurrences)
+                               + tuple(ctx.attention_in_tiles(a) for a in self._attentions))
         except BaseException:
             # The step did not run to its end: its positions are not part of the requests.  The pages taken for
             # them go back, and the requests continue from where they were.

@@ -560,6 +560,23 @@ def attention_portions_f32_supported(q, k_pool, tiles) -> bool:
             and all(t.data_ptr() % 16 == 0 for t in (q, k_pool, tiles)))
 
 
+def attention_portions_f32_pays(n_heads: int, head_dim: int, window: int, portions, sms: int = 148) -> bool:
+    """Whether tiles take less time than row by row for ``portions`` (first position and rows of each request with several rows).
+
+    Row by row a warp walks the keys of its (row, head), so the longest row counts until the rows fill the SMs; tiles take a
+    fixed time for every 64 keys however few rows they have, in waves of as many blocks as fit their shared memory.  Microseconds, fits
+    to 1456 pairs of times (2 to 64 rows of 1 to 32 requests at positions 0 to 100, heads of 16 to 128; they hold up to position
+    6000): 16 heads of 64, 2 rows at position 0 6.5 row by row and 11.9 in tiles, 12 rows 12.0 and 12.6, 64 rows 47 and 15."""
+    padded, resident = (32, 5) if head_dim <= 32 else (64, 3) if head_dim <= 64 else (128, 1)
+    seen = window or 1 << 30
+    longest = max(min(start + n, seen) for start, n in portions)
+    keys = sum(n * min(start + n / 2, seen) for start, n in portions)
+    rows = 4.6 + longest * (0.295 + 0.0032 * head_dim) + keys * n_heads * (2.8e-6 + 4.7e-6 * head_dim)
+    waves = -(-sum(-(-n // 64) for _, n in portions) * n_heads // (sms * resident))
+    blocks = max(-(-min(start + n, seen + n) // 64) for start, n in portions)
+    return waves * ((5.52 + 0.0748 * padded) * blocks + 4.65) - 1.4 < rows
+
+
 def attention_portions_f32(q, tiles, n_tiles: int, block_table, k_pool, v_pool, out, n_heads: int, scale: float, window: int,
                            status, stream, sinks=None) -> None:
     """``attention_generic`` for the queries of ``tiles`` (int32 ``[n_tiles, 4]``, as ``attention_portions`` takes them) of a

@@ -89,9 +89,11 @@ class Part:
     # then re-issues a recorded step of the same shape without calling forward() again.  Leave it False
     # for a part that does anything else (host-side loops over requests, torch operators, ...).
     replayable: bool = False
-    # A recurrence that runs in chunks: what ops.chunk_rule needs beside the step's runs.  Which way it takes is then part of
-    # a step's shape.
+    # What a part's choice between kernels needs beside the step's portions: of a recurrence that runs in chunks
+    # (ops.chunk_rule), of attention in float32 (heads, head size, window; ops.attention_portions_f32_pays).  The choices are then
+    # part of a step's shape.
     chunked_recurrence: Optional[tuple] = None
+    portion_attention: Optional[tuple] = None
 
     def param_specs(self) -> List[ParamSpec]:
         return []
@@ -111,9 +113,10 @@ class Part:
     def all_replayable(self) -> bool:
         return self.replayable and all(c.all_replayable() for c in self.children())
 
-    def all_chunked_recurrences(self) -> Set[tuple]:
-        own = {self.chunked_recurrence} if self.chunked_recurrence else set()
-        return own.union(*(c.all_chunked_recurrences() for c in self.children()))
+    def all_choices(self, name: str) -> Set[tuple]:
+        """What this part and its children name as ``chunked_recurrence`` or ``portion_attention``."""
+        own = {getattr(self, name)} - {None}
+        return own.union(*(c.all_choices(name) for c in self.children()))
 
     def all_kernel_libs(self) -> List[str]:
         out = list(self.kernel_libs)

@@ -37,6 +37,7 @@ class Attention(Mixer):
             raise ValueError(f"{name}: head size {head_dim} must be a multiple of 16 between 16 and 256")
         self.name, self.width = name, width
         self.n_heads, self.n_kv_heads, self.head_dim, self.window = n_heads, n_kv_heads, head_dim, window
+        self.portion_attention = (n_heads, head_dim, window or 0)
         self.scale = head_dim ** -0.5 if scale is None else float(scale)
         self.position = position
         self.q_width, self.kv_width = n_heads * head_dim, n_kv_heads * head_dim
@@ -111,7 +112,8 @@ def paged_attention(ctx, q, cache, o, n_heads: int, head_dim: int, scale: float,
             ops.attention_portions(q, ctx.portion_tiles, ctx.n_portion_tiles, cache.block_table, cache.k,
                                    cache.v, o, n_heads, scale, window, ctx.status, ctx.stream, sinks=sinks,
                                    first_positions=ctx.req_first_position)
-        elif cache.v.shape == cache.k.shape and ops.attention_portions_f32_supported(q, cache.k, ctx.portion_tiles):
+        elif (cache.v.shape == cache.k.shape and ops.attention_portions_f32_supported(q, cache.k, ctx.portion_tiles)
+              and ctx.attention_in_tiles((n_heads, head_dim, window))):
             ops.attention_portions_f32(q, ctx.portion_tiles, ctx.n_portion_tiles, cache.block_table, cache.k, cache.v, o,
                                        n_heads, scale, window, ctx.status, ctx.stream, sinks=sinks)
         else:
@@ -152,6 +154,7 @@ class SinkAttention(Mixer):
         self.head_dim = (max(dim, vdim) + 15) // 16 * 16
         if self.head_dim > 256:
             raise ValueError(f"{name}: head size {max(dim, vdim)} is beyond 256")
+        self.portion_attention = (n_heads, self.head_dim, window or 0)
         self.scale, self.eps, self.window = float(scale), float(eps), window
         self.rot_dims, self.rot_base, self.qk_norm, self.has_sink = rot_dims, float(rot_base), qk_norm, sink
         self.qkv = FusedLinear(f"{name}.qkv", width, [(f"{name}.q", n_heads * dim), (f"{name}.k", n_kv_heads * dim),

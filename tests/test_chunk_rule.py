@@ -1,5 +1,5 @@
-"""Which runs of rows go through a recurrence token by token and which in chunks (``ops.chunk_rule``), and that a step's plan
-knows it."""
+"""Choices between kernels that depend on a step's portions: which runs of rows go through a recurrence token by token and which in
+chunks (``ops.chunk_rule``), and whether float32 portions run in tiles (``ops.attention_portions_f32_pays``)."""
 import pytest
 
 from mlx_lm_b200 import ops
@@ -33,3 +33,11 @@ def test_what_the_chunked_kernels_do_not_take():
     assert ops.chunk_rule("mamba2", 32, 129, 64, (1024,)) is None
     assert ops.chunk_rule("delta", 16, 65, 64, (1024,)) is None
     assert ops.chunk_rule(*MAMBA, ()) is None
+
+
+@pytest.mark.parametrize("heads,dim", [(4, 16), (16, 64), (16, 128)])
+def test_float32_attention_of_few_keys_goes_row_by_row(heads, dim):
+    pays = lambda portions, window=0: ops.attention_portions_f32_pays(heads, dim, window, portions)
+    assert not pays([(0, 2)]) and not pays([(0, 8)] * 4) and not pays([(8, 2)])
+    assert pays([(0, 64)]) and pays([(0, 300), (0, 5)]) and pays([(1000, 2)]) and pays([(0, 1024)] * 2)
+    assert not pays([(1000, 2)], window=4)              # rows that see four keys

@@ -118,3 +118,31 @@ def test_linear_on_cuda_cores(ops, dtype, N, K):
     out = torch.empty(40, N, device="cuda")
     ops.linear_generic(wide[:, 1:K + 1], w, None, out, stream())
     assert rel_err(out, wide[:, 1:K + 1].double() @ w.double().T) <= 1e-6
+
+
+def test_float32_steps_of_one_shape_choose_their_attention(ops, tmp_path, monkeypatch):
+    """The same number of rows after few and after many positions: each step's plan has the kernel that it was recorded with."""
+    from helpers import CONFIG_A, make_model_dir
+    from mlx_lm_b200.engine import Engine, StepEntry
+    from mlx_lm_b200.weights import load_model
+    make_model_dir(tmp_path, CONFIG_A, seed=2)
+    model = load_model(str(tmp_path), dtype="float32")[0]
+    tokens = torch.randint(0, 512, (128,), generator=torch.Generator().manual_seed(1)).tolist()
+
+    def go():
+        engine, out, calls, real = Engine(model, page_size=16, n_pages=16, max_requests=2), [], [], ops.attention_portions_f32
+        monkeypatch.setattr(ops, "attention_portions_f32", lambda *a, **k: (calls.append(len(out)), real(*a, **k)))
+        for rid in range(2):
+            engine.add_request(rid)
+            for at in range(0, 128, 8):
+                out.append(engine.step([StepEntry(rid, tokens[at:at + 8], list(range(8)))]).clone())
+            engine.finish(rid)
+        monkeypatch.setattr(ops, "attention_portions_f32", real)
+        return torch.cat(out), set(calls), engine.n_replayed
+
+    got, chosen, replayed = go()
+    assert len(chosen) == 1 and 0 < min(chosen) < 15 and replayed == 30      # one plan in tiles, one row by row
+    monkeypatch.setattr(ops, "attention_portions_f32_pays", lambda *a, **k: False)
+    want, chosen, _ = go()
+    assert not chosen
+    assert rel_err(got, want) <= 1e-5 and torch.equal(got[:8], want[:8])
