@@ -16,14 +16,15 @@
 //   O          kept in registers by the softmax threads: O = O * correction + O_b, so nothing is ever
 //              written back to tensor memory
 // What bounds it is the chain of a tile's blocks (a tile of a prompt's end has eight at 1024 tokens, and an SM has only
-// two tiles), so the chain holds the softmax, P V and the adding up, and nothing else: S of the next block is computed during
-// this block's softmax.  There are two buffers of 128 columns in tensor memory, block i uses buffer i % 2: first for S, then,
-// when P is written and S no longer needed, for O_b; S(i + 1) goes to the other buffer once O_b(i - 1) has been read from
-// it.  K has two buffers as well and is requested two blocks ahead, V of the next block as soon as P V has been computed; two
-// CTAs fit an SM (97 KB of shared memory, 256 of 512 tensor-memory columns each) and overlap one another's phases.  2 x 1024 queries of 16 heads take 25.4 us (31.8 with S behind P V and the
-// scores kept, and spilled, in registers), of 25 heads 37.8 (46.4), 256 queries of 20 heads at position 768 23.7 (30.3).  Even
-// and odd blocks as two chains on a cluster of two CTAs: 34.4, 49.0 and 18.2, and sums in another order.  The order in which a query's keys are added depends only
-// on its position (blocks of 128 positions from block 0 or the window's first block upward).
+// two tiles), so the chain holds the softmax, P V and the adding up, and nothing else: S of the next block is computed
+// during this block's softmax.  There are two buffers of 128 columns in tensor memory, block i uses buffer i % 2: first
+// for S, then, when P is written and S no longer needed, for O_b; S(i + 1) goes to the other buffer once O_b(i - 1) has
+// been read from it.  K has two buffers as well and is requested two blocks ahead, V of the next block as soon as P V has
+// been computed; two CTAs fit an SM (97 KB of shared memory, 256 of 512 tensor-memory columns each) and overlap one
+// another's phases.  2 x 1024 queries of 16 heads take 25.4 us (31.8 with S behind P V and the scores kept, and spilled,
+// in registers), of 25 heads 37.8 (46.4), 256 queries of 20 heads at position 768 23.7 (30.3).  The order in which a
+// query's keys are added depends only on its position (blocks of 128 positions from block 0 or the window's first block
+// upward).
 //
 // Every mbarrier wait is bounded; a wait that gives up sets an abort flag that all roles see, the CTA frees
 // its tensor memory and reports MLXB_ST_WAIT_TIMEOUT.  TMA coordinates: x is always 0 or a multiple of 64
@@ -81,12 +82,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
 // that it can meet in __syncwarp afterwards.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
-}
-// One lane of a warp that is together (see tcgen05.cuh).
-__device__ __forceinline__ bool elect_one() {
-  uint32_t is;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(is));
-  return is != 0;
 }
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
   asm volatile(

@@ -73,6 +73,16 @@ __device__ __forceinline__ T* after_wait(T* p) {
   return p;
 }
 
+// One lane of a warp that is together.  Roles of one thread run their loops with the whole warp and let the elected lane
+// issue: stage numbers, coordinates and descriptors are then the same for all lanes as the compiler sees it and can stay
+// in uniform registers, which copies and products take as they are.  With an `if (lane == 0)` around the whole loop a step of
+// four products took 0.285 us whatever their size (0.23 this way; the products of a 128 x 128 tile take 0.14).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t is;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(is));
+  return is != 0;
+}
+
 static inline int mlxb_sm_count() {
   static int n = 0;
   if (n == 0) {

@@ -4,10 +4,10 @@
 //
 // The kernel is persistent: one CTA per SM walks over the 128 x BN output tiles (BN = 32 to 256,
 // see tile_choice).  Warp 0 is the TMA producer: it fills a
-// ring of shared-memory stages with 128x64 tiles of A and BNx64 tiles of W (cp.async.bulk.tensor,
+// ring of shared-memory stages with one or two blocks of 64 of K each, 128x64 tiles of A and BNx64 of W (cp.async.bulk.tensor,
 // 128-byte swizzle, completion counted on an mbarrier per stage; rows and columns outside the
 // matrices arrive as zeros).  Warp 1 allocates tensor memory and issues tcgen05.mma (kind::f16, bf16
-// inputs, float32 accumulator of 128 lanes x BN columns in TMEM), four K=16 steps per stage, and
+// inputs, float32 accumulator of 128 lanes x BN columns in TMEM), four K=16 steps per block, and
 // releases each stage with tcgen05.commit.  There are two accumulators in TMEM: while warps 2-17 (the
 // epilogue, four warps per quadrant of 32 TMEM lanes, each a quarter of the columns) read a finished one
 // with tcgen05.ld, add the bias, apply gelu_new, add the residual and store, the MMA warp already
@@ -34,7 +34,7 @@
 // instead of a hang.
 //
 // K and the row strides must be multiples of 8 elements (16 bytes), base addresses 16-byte aligned.
-// The accumulation order over K is fixed (stage by stage, four steps per stage), independent of M.
+// The accumulation order over K is fixed (block by block, four steps per block), the same in every form, independent of M.
 #include <cuda.h>
 
 #include "activations.cuh"

@@ -4,7 +4,10 @@
 // of request r lives in row slots[r] of a float32 pool, is read at the start of the run and written
 // back at its end, so a sequence may be cut into steps anywhere.  All state and everything that feeds
 // a recurrence (step sizes, decays, gates, unit norms) is float32; inputs arrive in the activation
-// dtype.  The order of additions for a token depends on the layer's sizes only, never on the batch.
+// dtype.  Here the order of additions for a token depends on the layer's sizes only, never on the batch.  Longer bfloat16 runs
+// of the two recurrences go through recurrent_chunks.cu instead (see ChunkRule), whose chunks count from the run's first
+// row: there a token's order, and so its rounding, also depends on where its run begins and how long it is, that is on how
+// a prompt was cut into steps.
 //
 // conv_silu          out[t, c] = silu(bias[c] + sum_j w[c, taps-1-j] * in(t - j, c)),  j = 0 .. taps-1 (act = 0: the sum
 //                    as it is, without the silu),

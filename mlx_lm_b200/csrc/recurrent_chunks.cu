@@ -2,10 +2,11 @@
 //
 // Token by token a scan is a chain as long as the run: 1024 rows of the state-space layer (32 heads of 64 columns, 128 rows of
 // state, two requests) took 387 us and of the gated delta rule (16 heads of 64 x 64) 423, with almost everything idle; in
-// chunks they take 104 and 152 (eight runs of 100 rows: 107 -> 58 and 54 -> 42; one of 70: 24 -> 15 and 33 -> 21).  A block
-// of threads here has a (request, head, slice of VS columns of the state), keeps its state in registers as accumulators and
-// walks the run in chunks of 64 rows; within a chunk everything is a product of small matrices.  What is left is a chain
-// too, of a chunk's phases.
+// chunks they take 107 and 159 (eight runs of 100 rows: 107 -> 59 and 54 -> 43; one of 70: 24 -> 15 and 33 -> 21).  A chunk
+// takes its time however few rows it has, and a block most of an SM's shared memory, so short runs, and many states of the
+// delta rule, stay with the scan (ops.chunk_rule).  A block of threads here has a (request, head, slice of VS columns of the
+// state), keeps its state in registers as accumulators and walks the run in chunks of 64 rows; within a chunk everything is
+// a product of small matrices.  What is left is a chain too, of a chunk's phases.
 //
 // Nothing is held in less than 32 bits.  Inputs are bfloat16 as they come; every float32 operand of a product (the state,
 // decay-weighted scores, weighted inputs) goes in as three bfloat16 numbers whose sum it is, the smallest first.  Decays

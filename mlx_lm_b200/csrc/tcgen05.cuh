@@ -42,19 +42,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
 }
 
 // The same for a whole warp, with one answer for all its lanes (a vote: the compiler then knows that the warp stays
-// together, see elect_one).
+// together, see elect_one in common.cuh).
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                                uint32_t peer_abort = 0) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, peer_abort));
-}
-// One lane of a warp that is together.  Roles of one thread run their loops with the whole warp and let the elected lane
-// issue: stage numbers, coordinates and descriptors are then the same for all lanes as the compiler sees it and can stay
-// in uniform registers, which copies and products take as they are.  With an `if (lane == 0)` around the whole loop a step of
-// four products took 0.285 us whatever their size (0.23 this way; the products of a 128 x 128 tile take 0.14).
-__device__ __forceinline__ bool elect_one() {
-  uint32_t is;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(is));
-  return is != 0;
 }
 
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
