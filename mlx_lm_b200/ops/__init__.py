@@ -1071,8 +1071,9 @@ def chunk_rule(kind: str, n_heads: int, state_rows: int, columns: int, runs, sms
     takes their latency until the SMs are full, then what their threads take.  Measured at 1 to 32 requests of 2 to 256 rows
     and the sizes of models 1024 and 2048 wide, the state-space layer (32 heads of 128 x 64) breaks even at 20 to 28 rows:
     one request of 16 rows 7 us by the scan and 9 in a chunk, of 64 rows 21 and 9; 32 requests of 8 rows 53 and 112.  The delta rule (64 x 64)
-    at 23 rows for up to 64 states, at 41 for 128; 256 states are never faster in chunks (96 rows 60 and 81 us), 512 from 122
-    rows on.  Chunks have to win by a twentieth: times of the scan differ by that much with the shapes of its blocks."""
+    at 23 rows for up to 64 states, at 44 for 128; 256 states are never faster in chunks (96 rows 60 and 81 us), 512 from 122
+    rows on.  Chunks have to win by a twentieth: times of the scan differ by that
+    much with the shapes of its blocks.  Of 430 launches timed both ways none takes 2 % longer than by the scan."""
     if not runs or state_rows > (MAMBA2_CHUNK_ROWS if kind == "mamba2" else DELTA_CHUNK_ROWS):
         return None
     pairs = len(runs) * n_heads
@@ -1087,8 +1088,13 @@ def chunk_rule(kind: str, n_heads: int, state_rows: int, columns: int, runs, sms
         if half >= wide or half * per_column < 128:
             break
         wide = half
-    threads = -(-pairs * -(-columns // wide) // sms) * wide * per_column
-    scan_row = max(360, 460 * threads // 512) if kind == "mamba2" else max(420, 560 * threads // 512)
+    share = -(-pairs * -(-columns // wide) // sms)      # blocks an SM gets at most
+    threads = share * wide * per_column
+    if kind == "mamba2":                                # a row's latency
+        alone = 360 if state_rows > 64 else 290
+    else:
+        alone = 850 if wide * per_column == 32 else 420 if share == 1 else 480
+    scan_row = max(alone, (460 if kind == "mamba2" else 560) * threads // 512)
     blocks, two = pairs * -(-columns // 32), kind == "mamba2" and state_rows <= 64
     waves = -(-blocks // (2 * sms if two else sms))
     each = 10000 if kind != "mamba2" else (6550 if not two else 5600 if blocks <= sms else 6900)
