@@ -340,6 +340,38 @@ def linear_generic(x, w, bias, out, stream, epilogue: int = EPI_NONE, residual=N
           _p(residual), _p(out), M, N, K, lda, ldc, epilogue, stream)
 
 
+def linear_split_supported(x, w, out, residual=None) -> bool:
+    """Whether ``linear_split`` takes these operands: float32, rows that 16-byte accesses can read and write."""
+    if x.dtype != torch.float32 or w.dtype != torch.float32 or out.dtype != torch.float32 or x.dim() != 2 or x.stride(1) != 1:
+        return False
+    if x.shape[1] % 4 or x.stride(0) % 4:
+        return False
+    return not any(t is not None and t.data_ptr() % 16 for t in (x, w, out, residual))
+
+
+def linear_split(x, w, bias, out, status, stream, epilogue: int = EPI_NONE, residual=None) -> None:
+    """``linear_generic``'s contract for float32 and more than a few rows, on tcgen05 tensor cores: every operand in three bfloat16
+    parts, sums at float32's precision (csrc/gemm_split.cu).  Operands as ``linear_split_supported`` says.  ``status`` receives
+    ``ST_WAIT_TIMEOUT`` if a bounded wait gives up."""
+    for t, what in ((x, "x"), (w, "w"), (out, "out")):
+        _need(t, torch.float32, f"linear {what}")
+    M, K = x.shape
+    N = w.shape[0]
+    if w.shape[1] != K or not w.is_contiguous() or out.shape[0] != M or out.shape[1] != N:
+        raise KernelError(f"linear: x {tuple(x.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
+    lda, ldc = _rows(x, "linear x"), _rows(out, "linear out")
+    if bias is not None:
+        _need(bias, torch.float32, "linear bias")
+        if bias.numel() != N:
+            raise KernelError(f"linear: bias of {bias.numel()} for {N} outputs")
+    if residual is not None:
+        _need(residual, torch.float32, "linear residual")
+        if residual.shape != out.shape or _rows(residual, "linear residual") != ldc:
+            raise KernelError("linear: residual must have the output's shape and row stride")
+    _call("gemm_split", "mlxb_linear_split", [c_void_p] * 5 + [c_int] * 6 + [c_void_p, c_void_p], _p(x), _p(w), _p(bias),
+          _p(residual), _p(out), M, N, K, lda, ldc, epilogue, _p(status), stream)
+
+
 _SMALLM_ARGS = [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                 c_void_p]
 

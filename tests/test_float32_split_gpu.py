@@ -1,0 +1,69 @@
+"""The float32 linear kernel on tensor cores (operands in three bfloat16 parts) at the edges of its tiles and blocks, against float64."""
+import math
+
+import pytest
+import torch
+
+from test_kernels_gpu import rel_err, stream
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from mlx_lm_b200 import ops
+    return ops
+
+
+@pytest.mark.parametrize("width", ["64", "128"])
+@pytest.mark.parametrize("M,N,K", [(1, 64, 256), (17, 7, 4), (127, 65, 60), (128, 128, 64), (129, 130, 68), (300, 200, 1000),
+                                   (257, 1030, 260), (1100, 512, 128), (64, 3072, 132), (40, 24, 4100)])
+def test_float32_linear_in_parts(ops, M, N, K, width, monkeypatch):
+    """What is left out of a product is 2^-25 of it, a block of 64 of K takes four cut-off sums of 2^-23 at most, the blocks' sums K / 64
+    roundings of 2^-24: a few 1e-7 over the whole result at most; the same bits for both tile widths and however many rows."""
+    monkeypatch.setenv("MLXB_SPLIT_BN", width)
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    draw = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    x, w, b, res = draw(M, K), draw(N, K) / math.sqrt(K), draw(N), draw(M, N)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    want = x.double() @ w.double().T
+    out = torch.empty(M, N, device="cuda")
+    ops.linear_split(x, w, None, out, status, stream())
+    assert rel_err(out, want) <= 5e-7
+    if M < 130:
+        more = torch.empty(M + 140, N, device="cuda")
+        monkeypatch.setenv("MLXB_SPLIT_BN", "128" if width == "64" else "64")
+        ops.linear_split(torch.cat([x, draw(140, K)]), w, None, more, status, stream())
+        assert torch.equal(more[:M], out)
+    ops.linear_split(x, w, b, out, status, stream(), epilogue=ops.EPI_GELU_NEW, residual=res)
+    plain = torch.empty(M, N, device="cuda")
+    ops.linear_generic(x, w, b, plain, stream(), epilogue=ops.EPI_GELU_NEW, residual=res)
+    assert rel_err(out, plain) <= 1e-6
+    inplace = res.clone()
+    ops.linear_split(x, w, None, inplace, status, stream(), residual=inplace)
+    assert rel_err(inplace, want + res) <= 5e-7
+    wide = draw(M, K + 4)                            # a row stride of its own
+    ops.linear_split(wide[:, 4:], w, b, out, status, stream())
+    assert rel_err(out, wide[:, 4:].double() @ w.double().T + b) <= 1e-6
+    assert int(status.item()) == 0
+
+
+def test_float32_linear_in_parts_of_numbers_at_the_ends(ops):
+    """Infinities, NaN, numbers that bfloat16 rounds to infinity, and tiny ones: as in plain float32."""
+    g = torch.Generator(device="cuda").manual_seed(1)
+    draw = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    x, w = draw(200, 512), draw(130, 512) / 16
+    x[3, 5], x[7, 9], w[11, 20], x[50, 1] = math.inf, math.nan, -math.inf, 3.4e38
+    w[12], w[13, 5], w[14, 5] = w[12].bfloat16().float(), 0.0, 0.5
+    w[:, 1].clamp_(-0.5, 0.5)
+    x[60] *= 1e-30
+    status, out, plain = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.empty(200, 130, device="cuda"), torch.empty(200, 130, device="cuda")
+    ops.linear_split(x, w, None, out, status, stream())
+    ops.linear_generic(x, w, None, plain, stream())
+    assert int(status.item()) == 0
+    assert torch.equal(torch.isnan(out), torch.isnan(plain)) and torch.equal(torch.isinf(out), torch.isinf(plain))
+    assert torch.equal(out[torch.isinf(out)], plain[torch.isinf(plain)])
+    fine = torch.isfinite(plain)
+    assert bool(fine[50].any()) and bool(fine[60].any())
+    for r in (0, 50, 60, 199):
+        assert rel_err(out[r][fine[r]], plain[r][fine[r]]) <= 1e-6
