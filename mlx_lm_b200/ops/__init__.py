@@ -1636,6 +1636,51 @@ def attention_wide_tc_supported(k_pool, v_pool, n_heads: int, key_dim: int, valu
                   int(v_pool.data_ptr() == k_pool.data_ptr())))
 
 
+_WIDE_TCGEN05_ARGS = [c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p] + [c_int] * 11 + [
+    c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_float, c_int, c_int, c_int, c_void_p]
+
+
+def attention_wide_portions_supported(q, q_head_stride: int, k_pool, v_pool, n_heads: int, key_dim: int, value_dim: int,
+                                      talk: bool) -> bool:
+    """Whether ``attention_wide_portions`` serves these sizes (pages of 8 to 64 positions, mixed scores of heads in whole chunks
+    of 64 columns, a tile that fits shared and tensor memory)."""
+    if k_pool.dtype != torch.bfloat16 or any(t.data_ptr() % 16 for t in (q, k_pool, v_pool)):
+        return False
+    if _rows(q, "attention_wide_portions q") % 4 or q_head_stride % 4:
+        return False
+    f, _ = _fn("attention_wide_tcgen05", "mlxb_attention_wide_tcgen05_supported", [c_int] * 10)
+    return bool(f(n_heads, k_pool.shape[1], v_pool.shape[1], key_dim, value_dim, k_pool.shape[3], v_pool.shape[3], k_pool.shape[2],
+                  int(talk), int(v_pool.data_ptr() == k_pool.data_ptr())))
+
+
+def attention_wide_portions(q, q_head_stride: int, tiles, n_tiles: int, tile_queries: int, block_table, k_pool, v_pool, out,
+                            out_head_stride: int, n_heads: int, key_dim: int, value_dim: int, scale: float, status, stream,
+                            window: int = 0, chunk: int = 0, talk=None, gate=None, softcap: float = 0.0,
+                            keep_first: int = 0) -> None:
+    """``attention_wide_tiles`` for prompt portions on tcgen05 tensor cores (csrc/attention_wide_tcgen05.cu): the same contract
+    without the split single rows.  ``status`` receives ``ST_WAIT_TIMEOUT`` if a bounded wait gives up."""
+    what = "attention_wide_portions"
+    _need(q, torch.float32, f"{what} q")
+    _need(k_pool, torch.bfloat16, f"{what} k_pool")
+    _need(v_pool, torch.bfloat16, f"{what} v_pool")
+    _need(tiles, torch.int32, f"{what} tiles")
+    n_pages, Hkv, page, krs = k_pool.shape
+    if not _pools_fit(k_pool, v_pool):
+        raise KernelError(f"{what}: pools {tuple(k_pool.shape)} and {tuple(v_pool.shape)}")
+    if out.dtype not in (torch.bfloat16, torch.float32) or out.shape[0] != q.shape[0] or tiles.numel() < 4 * n_tiles:
+        raise KernelError(f"{what}: out {out.dtype} {tuple(out.shape)} for q {tuple(q.shape)}")
+    if talk is not None:
+        _need(talk, torch.float32, f"{what} talk")
+        if talk.shape != (n_heads, n_heads) or not talk.is_contiguous():
+            raise KernelError(f"{what}: talk {tuple(talk.shape)} for {n_heads} heads")
+    ldg, gate_cols = _wide_gate(gate, torch.bfloat16, n_heads, value_dim, what)
+    _call("attention_wide_tcgen05", "mlxb_attention_wide_tcgen05", _WIDE_TCGEN05_ARGS, int(out.dtype == torch.float32), _p(q),
+          _rows(q, f"{what} q"), q_head_stride, _p(tiles), n_tiles, tile_queries, _p(block_table), block_table.shape[1], n_pages,
+          page, n_heads, Hkv, key_dim, value_dim, krs, v_pool.shape[3], int(window or 0), int(chunk or 0), float(scale), _p(talk),
+          _p(k_pool), _p(v_pool), _p(gate), ldg, _p(out), _rows(out, f"{what} out"), out_head_stride, _p(status),
+          float(softcap or 0.0), int(keep_first or 0), gate_cols, v_pool.shape[1], stream)
+
+
 def attention_wide_scratch(n_rows: int, n_heads: int, value_dim: int, window: int, chunk: int, max_len: int,
                            keep_first: int = 0) -> int:
     """Floats of scratch memory with which ``attention_wide_tiles`` splits the keys of single rows over several
