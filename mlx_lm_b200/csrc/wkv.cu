@@ -16,6 +16,8 @@
 // run and written back at its end.  A thread holds 16 consecutive rows of one column in registers; the NS threads of
 // a column are neighbouring lanes and add their partial sums by shuffles; 16 tokens at a time are staged in shared
 // memory.  The order of additions for a token depends on the layer's sizes only.
+#include <type_traits>
+
 #include "common.cuh"
 
 MLXB_DEFINE_LAST_ERROR()
@@ -322,6 +324,391 @@ wkv_scan_kernel(const T* rkv, int ld, int r_off, int k_off, int v_off, const flo
       if (kk < K) st[kk] = S[i];
     }
   }
+}
+
+// ---------------------------------------------------------------- the recurrence in chunks
+
+// Token by token a run is a chain as long as it is, on as many SMs as there are (request, head) pairs: 731, 683 and 613 rows of 16
+// heads took 440 us.  The state is linear in the state before, channel by channel: over a chunk of rows, S_end = W S_0 + L with W
+// the product of the chunk's decays (one number a key channel) and L the state that the chunk leaves of an empty one.  So the
+// chunks of a run are walked side by side:
+//   first pass   chunk 0 of a run as a scan, with its outputs; of every other chunk but the last L and W
+//   second pass  every chunk after the first: its state from the chunks before, then the scan with its outputs
+// in float32 like the scan, in the same order within a chunk.  What bounds it then is the FMAs and the loads of r, k, w that feed
+// them, so a thread has two columns (32 numbers of the state) and multiplies pairs of channels (fma.rn.f32x2).
+constexpr int WC_Q = 64;       // rows of a chunk
+constexpr int WC_VB = 64;      // columns of a block: NS threads for every two of them
+
+typedef unsigned long long f32x2;      // two float32, the first in the low half
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 twice(float v) {
+  f32x2 d;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(v));
+  return d;
+}
+__device__ __forceinline__ float sum2(f32x2 v) { return __uint_as_float((unsigned)v) + __uint_as_float((unsigned)(v >> 32)); }
+
+// Job `job` of the step: chunk c of request r, in the order of the requests; base: chunks before the request's last ones, of the
+// requests before it (where its states between chunks are kept).  r = -1: there are fewer jobs.  A whole warp calls it.
+struct ChunkJob { int r, c, base; };
+__device__ __forceinline__ ChunkJob find_job(const int* __restrict__ req_first_token, int n_requests, int job) {
+  const int lane = threadIdx.x & 31;
+  ChunkJob out = {-1, 0, 0};
+  int before = 0;
+  for (int r0 = 0; r0 < n_requests; r0 += 32) {
+    const int r = r0 + lane;
+    const int mine = r < n_requests ? (req_first_token[r + 1] - req_first_token[r] + WC_Q - 1) / WC_Q : 0;
+    int jobs = mine, kept = mine > 0 ? mine - 1 : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, jobs, o), w = __shfl_up_sync(0xffffffffu, kept, o);
+      if (lane >= o) { jobs += u; kept += w; }
+    }
+    const unsigned hit = __ballot_sync(0xffffffffu, before + jobs > job);
+    if (hit) {
+      const int src = __ffs(hit) - 1;
+      out.r = r0 + src;
+      out.c = job - before - __shfl_sync(0xffffffffu, jobs - mine, src);
+      out.base += __shfl_sync(0xffffffffu, kept - (mine > 0 ? mine - 1 : 0), src);
+      return out;
+    }
+    before += __shfl_sync(0xffffffffu, jobs, 31);
+    out.base += __shfl_sync(0xffffffffu, kept, 31);
+  }
+  return out;
+}
+
+template <int NS>
+struct WkvMemory {
+  static constexpr int NP = NS * WK_SEG;
+  float r[WK_CHUNK][NP], k[WK_CHUNK][NP], w[WK_CHUNK][NP];
+  float v[WK_CHUNK][WC_VB];
+  float bonus[WK_CHUNK];      // sum_k r u k of the token
+};
+
+// kept: [chunks before last ones][H][V][K] states (W S_0 + L of a run's first chunk, L of the others), then [..][H][K] products W.
+template <typename T, int NS, bool FIRST>
+__global__ void __launch_bounds__(32 * NS)
+wkv_chunks_kernel(const T* rkv, int ld, int r_off, int k_off, int v_off, const float* d_raw, int ldd, const float* __restrict__ u,
+                  float* state, const int* __restrict__ slots, const int* __restrict__ token_req,
+                  const int* __restrict__ req_first_token, int n_requests, float* o, int ldo, int H, int V, float* kept,
+                  float* products) {
+  extern __shared__ __align__(16) char wc_sm[];
+  WkvMemory<NS>* sm = reinterpret_cast<WkvMemory<NS>*>(wc_sm);      // two: the next tokens are staged beside these
+  constexpr int K = NS * WK_NPT, THREADS = 32 * NS, PER_TOK = K / 8;
+  const int h = blockIdx.x, v0 = blockIdx.z * WC_VB, tid = threadIdx.x;
+  const int s = tid % NS, col = 2 * (tid / NS);      // rows 16 s .. of columns col, col + 1 of the slice
+  const bool valid = v0 + col < V;                   // (V is even)
+  pdl_trigger();
+  const ChunkJob job = find_job(req_first_token, n_requests, blockIdx.y);
+  const int t_first = job.r >= 0 ? req_first_token[job.r] : 0, t_end = job.r >= 0 ? req_first_token[job.r + 1] : 0;
+  const int n = run_length(token_req, t_first, t_end, job.r);
+  const bool last = (job.c + 1) * WC_Q >= n;
+  pdl_wait();
+  if (job.c * WC_Q >= n || (FIRST ? job.c > 0 && last : job.c == 0)) return;
+  rkv = after_wait(rkv);
+  d_raw = after_wait(d_raw);
+  state = after_wait(state);
+  kept = after_wait(kept);
+  products = after_wait(products);
+  const bool outputs = !FIRST || job.c == 0;
+  const int t0 = t_first + job.c * WC_Q, rows = min(WC_Q, n - job.c * WC_Q);
+  const size_t at = ((size_t)h * V + (valid ? v0 + col : 0)) * K + s * WK_NPT;      // of this thread's first column in a state
+  const size_t state_size = (size_t)H * V * K;
+  float* pool = state + (size_t)slots[job.r] * state_size + at;
+  f32x2 S[2][8];
+  auto load_state = [&](const float* p) {
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const ulonglong2 x = valid ? *reinterpret_cast<const ulonglong2*>(p + (size_t)c * K + 4 * i) : make_ulonglong2(0ull, 0ull);
+        S[c][2 * i] = x.x;
+        S[c][2 * i + 1] = x.y;
+      }
+  };
+  auto store_state = [&](float* p) {
+    if (!valid) return;
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) *reinterpret_cast<ulonglong2*>(p + (size_t)c * K + 4 * i) = make_ulonglong2(S[c][2 * i], S[c][2 * i + 1]);
+  };
+  // ---- staging: a thread eight key channels of one token; 16-byte pieces of the values
+  const int tok_s = tid / PER_TOK, kk_s = (tid % PER_TOK) * 8;
+  constexpr int V_PIECES = WK_CHUNK * WC_VB / 8, VP = (V_PIECES + THREADS - 1) / THREADS, WORDS = sizeof(T) / 2;
+  float uv[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) uv[i] = u[(size_t)h * K + kk_s + i];
+  uint4 nr[WORDS], nk[WORDS], nv[VP][WORDS];
+  float4 nd[2];
+  const bool vec_v = (V & 7) == 0;
+  auto fetch = [&](int c0) {
+    const int nc = rows - c0;
+    if (tok_s < nc) {
+      const size_t row = (size_t)(t0 + c0 + tok_s);
+      const uint4* kp = reinterpret_cast<const uint4*>(rkv + row * ld + k_off + h * K + kk_s);
+      const uint4* rp = reinterpret_cast<const uint4*>(rkv + row * ld + r_off + h * K + kk_s);
+      const float4* dp = reinterpret_cast<const float4*>(d_raw + row * ldd + h * K + kk_s);
+#pragma unroll
+      for (int i = 0; i < WORDS; ++i) {
+        nk[i] = kp[i];
+        if (outputs) nr[i] = rp[i];
+      }
+      nd[0] = dp[0];
+      nd[1] = dp[1];
+    }
+#pragma unroll
+    for (int i = 0; i < VP; ++i) {
+      const int e = tid + i * THREADS, tok = e / (WC_VB / 8), c = v0 + (e % (WC_VB / 8)) * 8;
+#pragma unroll
+      for (int j = 0; j < WORDS; ++j) nv[i][j] = make_uint4(0u, 0u, 0u, 0u);
+      if (e >= V_PIECES || tok >= nc || c >= V) continue;
+      const T* vp = rkv + (size_t)(t0 + c0 + tok) * ld + v_off + h * V + c;
+      if (vec_v) {
+#pragma unroll
+        for (int j = 0; j < WORDS; ++j) nv[i][j] = reinterpret_cast<const uint4*>(vp)[j];
+      } else {
+        T* d = reinterpret_cast<T*>(nv[i]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (c + j < V) d[j] = vp[j];
+      }
+    }
+  };
+  auto values = [](const uint4 (&raw)[WORDS], float (&f)[8]) {
+    if (sizeof(T) == 2) {
+      unpack8(raw[0], f);
+    } else {
+      *reinterpret_cast<uint4*>(f) = raw[0];
+      *reinterpret_cast<uint4*>(f + 4) = raw[WORDS - 1];
+    }
+  };
+  auto stage = [&](WkvMemory<NS>& m, int c0) {
+    const bool have = tok_s < rows - c0;      // a row beyond the run changes nothing: no decay, nothing added
+    float kv[8], rv[8], b = 0.f;
+    values(nk, kv);
+    values(nr, rv);
+    const float dv[8] = {nd[0].x, nd[0].y, nd[0].z, nd[0].w, nd[1].x, nd[1].y, nd[1].z, nd[1].w};
+    const int p = (kk_s / WK_NPT) * WK_SEG + (kk_s % WK_NPT);
+    float w[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if (!have) kv[i] = 0.f;
+      if (!have || !outputs) rv[i] = 0.f;
+      w[i] = have ? expf(-expf(dv[i])) : 1.f;
+      b = fmaf(rv[i] * uv[i], kv[i], b);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i += 4) {
+      *reinterpret_cast<float4*>(&m.k[tok_s][p + i]) = make_float4(kv[i], kv[i + 1], kv[i + 2], kv[i + 3]);
+      *reinterpret_cast<float4*>(&m.w[tok_s][p + i]) = make_float4(w[i], w[i + 1], w[i + 2], w[i + 3]);
+      if (outputs) *reinterpret_cast<float4*>(&m.r[tok_s][p + i]) = make_float4(rv[i], rv[i + 1], rv[i + 2], rv[i + 3]);
+    }
+#pragma unroll
+    for (int off = PER_TOK >> 1; off > 0; off >>= 1) b += __shfl_xor_sync(0xffffffffu, b, off);
+    if (kk_s == 0) m.bonus[tok_s] = b;
+#pragma unroll
+    for (int i = 0; i < VP; ++i) {
+      const int e = tid + i * THREADS;
+      if (e >= V_PIECES) continue;
+      float f[8];
+      values(nv[i], f);
+      float4* d = reinterpret_cast<float4*>(&m.v[e / (WC_VB / 8)][(e % (WC_VB / 8)) * 8]);
+      d[0] = make_float4(f[0], f[1], f[2], f[3]);
+      d[1] = make_float4(f[4], f[5], f[6], f[7]);
+    }
+  };
+  fetch(0);
+  f32x2 prod[8];      // W, by the threads of the first columns
+#pragma unroll
+  for (int i = 0; i < 8; ++i) prod[i] = twice(1.f);
+  if (FIRST && job.c > 0) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) S[0][i] = S[1][i] = 0ull;
+  } else if (FIRST) {
+    load_state(pool);
+  } else {            // the run's state after its first chunk, then through the chunks up to this one
+    const float* L = kept + (size_t)job.base * state_size + at;
+    const float* W = products + ((size_t)job.base * H + h) * K + s * WK_NPT;
+    load_state(L);
+    for (int c = 1; c < job.c; ++c) {
+      L += state_size;
+      W += (size_t)H * K;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(W + 4 * i);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const ulonglong2 x = valid ? *reinterpret_cast<const ulonglong2*>(L + (size_t)j * K + 4 * i) : make_ulonglong2(0ull, 0ull);
+          S[j][2 * i] = fma2(w.x, S[j][2 * i], x.x);
+          S[j][2 * i + 1] = fma2(w.y, S[j][2 * i + 1], x.y);
+        }
+      }
+    }
+  }
+  for (int c0 = 0, b = 0; c0 < rows; c0 += WK_CHUNK, b ^= 1) {
+    WkvMemory<NS>& m = sm[b];
+    stage(m, c0);
+    __syncthreads();      // (with two buffers one barrier: the tokens before last have been read)
+    if (c0 + WK_CHUNK < rows) fetch(c0 + WK_CHUNK);
+    const int nc = min(WK_CHUNK, rows - c0);
+#pragma unroll 1
+    for (int q = 0; q < nc; q += 4) {
+      float x[4][2];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 v = *reinterpret_cast<const float2*>(&m.v[q + e][col]);
+        const f32x2 vv[2] = {twice(v.x), twice(v.y)};
+        f32x2 acc[2] = {0ull, 0ull};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const ulonglong2 k2 = *reinterpret_cast<const ulonglong2*>(&m.k[q + e][s * WK_SEG + 4 * i]);
+          const ulonglong2 w2 = *reinterpret_cast<const ulonglong2*>(&m.w[q + e][s * WK_SEG + 4 * i]);
+          if (outputs) {
+            const ulonglong2 r2 = *reinterpret_cast<const ulonglong2*>(&m.r[q + e][s * WK_SEG + 4 * i]);
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+              acc[j] = fma2(r2.x, S[j][2 * i], acc[j]);
+              acc[j] = fma2(r2.y, S[j][2 * i + 1], acc[j]);
+            }
+          } else if (tid < NS) {
+            prod[2 * i] = mul2(prod[2 * i], w2.x);
+            prod[2 * i + 1] = mul2(prod[2 * i + 1], w2.y);
+          }
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            S[j][2 * i] = fma2(w2.x, S[j][2 * i], mul2(k2.x, vv[j]));
+            S[j][2 * i + 1] = fma2(w2.y, S[j][2 * i + 1], mul2(k2.y, vv[j]));
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) x[e][j] = sum2(acc[j]);
+      }
+      if (!outputs) continue;
+      // The NS threads of a column add up: four tokens by two columns halved twice, so that a thread ends with one token
+      // (NS of 1 or 2: with four or two).
+      constexpr int HAVE = NS >= 4 ? 1 : NS == 2 ? 2 : 4;
+      int first = 0;
+      if (NS >= 2) {
+        const bool up = s & 1;
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const float give = up ? x[e][j] : x[e + 2][j], keep = up ? x[e + 2][j] : x[e][j];
+            x[e][j] = keep + __shfl_xor_sync(0xffffffffu, give, 1);
+          }
+        first = up ? 2 : 0;
+      }
+      if (NS >= 4) {
+        const bool up = s & 2;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const float give = up ? x[0][j] : x[1][j], keep = up ? x[1][j] : x[0][j];
+          x[0][j] = keep + __shfl_xor_sync(0xffffffffu, give, 2);
+        }
+        first += up ? 1 : 0;
+      }
+#pragma unroll
+      for (int off = 4; off < NS; off <<= 1)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) x[0][j] += __shfl_xor_sync(0xffffffffu, x[0][j], off);
+#pragma unroll
+      for (int e = 0; e < HAVE; ++e) {
+        const int tok = q + first + e;
+        if (s < 4 && valid && tok < nc) {
+          const float2 v = *reinterpret_cast<const float2*>(&m.v[tok][col]);
+          *reinterpret_cast<float2*>(o + (size_t)(t0 + c0 + tok) * ldo + h * V + v0 + col) =
+              make_float2(fmaf(m.bonus[tok], v.x, x[e][0]), fmaf(m.bonus[tok], v.y, x[e][1]));
+        }
+      }
+    }
+  }
+  if (last) {
+    store_state(pool);
+  } else if (FIRST) {
+    store_state(kept + (size_t)(job.base + job.c) * state_size + at);
+    if (job.c > 0 && tid < NS && blockIdx.z == 0) {
+      float* W = products + ((size_t)(job.base + job.c) * H + h) * K + s * WK_NPT;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) *reinterpret_cast<ulonglong2*>(W + 4 * i) = make_ulonglong2(prod[2 * i], prod[2 * i + 1]);
+    }
+  }
+}
+
+// Floats of scratch memory for mlxb_wkv_chunks: states and products of the chunks before a run's last one.
+MLXB_EXPORT long long mlxb_wkv_chunks_scratch(int n_tokens, int H, int K, int V) {
+  return (long long)(n_tokens / WC_Q) * H * K * (V + 1);
+}
+
+// What the kernels take: states of 16, 32, ... 256 rows and an even number of columns, 16-byte rows of r, k and the decay.
+static bool chunks_take(const void* rkv, int size, int ld, int r_off, int k_off, int v_off, const void* d_raw, int ldd, const void* state,
+                        const void* o, int ldo, int K, int V) {
+  const int unit = 16 / size;
+  return K >= 16 && K <= 256 && (K & (K - 1)) == 0 && V % 2 == 0 && ld % unit == 0 && r_off % unit == 0 && k_off % unit == 0 &&
+         (V % 8 != 0 || v_off % unit == 0) && ldd % 4 == 0 && ldo % 2 == 0 && (((uintptr_t)rkv | (uintptr_t)d_raw | (uintptr_t)state) & 15) == 0 &&
+         ((uintptr_t)o & 7) == 0;
+}
+
+MLXB_EXPORT int mlxb_wkv_scan(int dtype, const void* rkv, int ld, int r_off, int k_off, int v_off, const float* d_raw,
+                              int ldd, const float* u, float* state, const int* slots, const int* token_req,
+                              const int* req_first_token, float* o, int ldo, int H, int K, int V, int n_requests,
+                              cudaStream_t stream);
+
+// The arguments of mlxb_wkv_scan, the step's rows, and scratch memory of mlxb_wkv_chunks_scratch floats (16-byte aligned).  Sizes
+// that the kernels do not take go token by token.
+MLXB_EXPORT int mlxb_wkv_chunks(int dtype, const void* rkv, int ld, int r_off, int k_off, int v_off, const float* d_raw, int ldd,
+                                const float* u, float* state, const int* slots, const int* token_req, const int* req_first_token,
+                                float* o, int ldo, int H, int K, int V, int n_requests, int n_tokens, float* scratch,
+                                cudaStream_t stream) {
+  if (n_requests <= 0 || n_tokens <= 0) return 0;
+  const int size = dtype == MLXB_F32 ? 4 : 2;
+  if (!chunks_take(rkv, size, ld, r_off, k_off, v_off, d_raw, ldd, state, o, ldo, K, V) || ((uintptr_t)scratch & 15) || H <= 0)
+    return mlxb_wkv_scan(dtype, rkv, ld, r_off, k_off, v_off, d_raw, ldd, u, state, slots, token_req, req_first_token, o, ldo, H, K, V,
+                         n_requests, stream);
+  const long long jobs = (long long)n_tokens / WC_Q + n_requests;
+  if (jobs > 65535 || (V + WC_VB - 1) / WC_VB > 65535) return mlxb_fail(MLXB_BAD_ARG, "wkv_chunks: %d rows of %d requests, %d columns", n_tokens, n_requests, V);
+  float* products = scratch + (size_t)(n_tokens / WC_Q) * H * V * K;
+  const dim3 grid(H, (unsigned)jobs, (V + WC_VB - 1) / WC_VB);
+  auto run = [&](auto type, auto ns) {
+    using T = decltype(type);
+    constexpr int NS = decltype(ns)::value;
+    static SharedLimit limits[2];
+    const size_t smem = 2 * sizeof(WkvMemory<NS>);
+    auto go = [&](auto kernel, SharedLimit& limit) {
+      const cudaError_t e = limit.raise(kernel, smem);
+      if (e != cudaSuccess) return mlxb_fail((int)e, "wkv_chunks: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
+      launch_pdl(kernel, grid, dim3(32 * NS), smem, stream, (const T*)rkv, ld, r_off, k_off, v_off, d_raw, ldd, u, state, slots,
+                 token_req, req_first_token, n_requests, o, ldo, H, V, scratch, products);
+      return mlxb_check_launch("wkv_chunks");
+    };
+    if (int e = go(wkv_chunks_kernel<T, NS, true>, limits[0])) return e;
+    // a run of more than one chunk: not with fewer rows than that
+    if (n_tokens <= WC_Q) return 0;
+    return go(wkv_chunks_kernel<T, NS, false>, limits[1]);
+  };
+  auto by_rows = [&](auto type) {
+    switch (K) {
+      case 16: return run(type, std::integral_constant<int, 1>{});
+      case 32: return run(type, std::integral_constant<int, 2>{});
+      case 64: return run(type, std::integral_constant<int, 4>{});
+      case 128: return run(type, std::integral_constant<int, 8>{});
+      default: return run(type, std::integral_constant<int, 16>{});
+    }
+  };
+  if (dtype == MLXB_F32) return by_rows(float{});
+  if (dtype == MLXB_BF16) return by_rows(__nv_bfloat16{});
+  return mlxb_fail(MLXB_BAD_DTYPE, "wkv_chunks: dtype code %d", dtype);
 }
 
 // rkv: [n_tokens, .] (activation dtype) holding r and k (H*K columns each from r_off / k_off) and v (H*V columns from

@@ -1848,24 +1848,50 @@ _WKV_ARGS = [c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_voi
              c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p]
 
 
+def _wkv_args(rkv, r_off: int, k_off: int, v_off: int, decay_raw, bonus, state, slots, token_req, req_first_token, o,
+              n_heads: int, what: str):
+    _need(state, torch.float32, f"{what} state")
+    _need(o, torch.float32, f"{what} o")
+    _need(decay_raw, torch.float32, f"{what} decay")
+    _need(bonus, torch.float32, f"{what} bonus")
+    _, H, V, K = state.shape
+    if H != n_heads or o.shape[1] != H * V or not state.is_contiguous() or bonus.numel() != H * K \
+            or not bonus.is_contiguous() or decay_raw.shape[1] != H * K:
+        raise KernelError(f"{what}: state {tuple(state.shape)} for {n_heads} heads, o {tuple(o.shape)}, "
+                          f"decay {tuple(decay_raw.shape)}, bonus {tuple(bonus.shape)}")
+    return (dtype_code(rkv.dtype), _p(rkv), _rows(rkv, f"{what} rkv"), r_off, k_off, v_off, _p(decay_raw),
+            _rows(decay_raw, f"{what} decay"), _p(bonus), _p(state), _p(slots), _p(token_req), _p(req_first_token), _p(o),
+            _rows(o, f"{what} o"), H, K, V, slots.numel())
+
+
 def wkv_scan(rkv, r_off: int, k_off: int, v_off: int, decay_raw, bonus, state, slots, token_req, req_first_token, o,
              n_heads: int, stream) -> None:
     """Per (request, head): ``o_t = (S + diag(u) k_t v_t^T)^T r_t``, then ``S <- diag(w_t) S + k_t v_t^T`` with
     ``w_t = exp(-exp(decay_raw_t))``.  ``rkv [T, .]`` holds r, k, v from the given column offsets; ``decay_raw``
     float32 ``[T, heads*K]``; ``bonus`` (u) float32 ``[heads, K]``; ``state`` float32 ``[slots, heads, V, K]`` (a head's
     ``K x V`` state column by column); ``o`` float32 ``[T, heads*V]``."""
-    _need(state, torch.float32, "wkv_scan state")
-    _need(o, torch.float32, "wkv_scan o")
-    _need(decay_raw, torch.float32, "wkv_scan decay")
-    _need(bonus, torch.float32, "wkv_scan bonus")
-    _, H, V, K = state.shape
-    if H != n_heads or o.shape[1] != H * V or not state.is_contiguous() or bonus.numel() != H * K \
-            or not bonus.is_contiguous() or decay_raw.shape[1] != H * K:
-        raise KernelError(f"wkv_scan: state {tuple(state.shape)} for {n_heads} heads, o {tuple(o.shape)}, "
-                          f"decay {tuple(decay_raw.shape)}, bonus {tuple(bonus.shape)}")
-    _call("wkv", "mlxb_wkv_scan", _WKV_ARGS, dtype_code(rkv.dtype), _p(rkv), _rows(rkv, "wkv_scan rkv"), r_off, k_off,
-          v_off, _p(decay_raw), _rows(decay_raw, "wkv_scan decay"), _p(bonus), _p(state), _p(slots), _p(token_req),
-          _p(req_first_token), _p(o), _rows(o, "wkv_scan o"), H, K, V, slots.numel(), stream)
+    _call("wkv", "mlxb_wkv_scan", _WKV_ARGS,
+          *_wkv_args(rkv, r_off, k_off, v_off, decay_raw, bonus, state, slots, token_req, req_first_token, o, n_heads, "wkv_scan"),
+          stream)
+
+
+def wkv_chunks_scratch(n_tokens: int, n_heads: int, state_rows: int, columns: int) -> int:
+    """Floats of scratch memory for ``wkv_chunks`` over ``n_tokens`` rows."""
+    f, _ = _fn("wkv", "mlxb_wkv_chunks_scratch", [c_int] * 4)
+    f.restype = ctypes.c_longlong
+    return int(f(n_tokens, n_heads, state_rows, columns))
+
+
+def wkv_chunks(rkv, r_off: int, k_off: int, v_off: int, decay_raw, bonus, state, slots, token_req, req_first_token, o,
+               n_heads: int, scratch, stream) -> None:
+    """``wkv_scan`` with the chunks of 64 rows of a request's run side by side (csrc/wkv.cu).  ``scratch``: float32, at least
+    ``wkv_chunks_scratch`` elements."""
+    args = _wkv_args(rkv, r_off, k_off, v_off, decay_raw, bonus, state, slots, token_req, req_first_token, o, n_heads, "wkv_chunks")
+    _need(scratch, torch.float32, "wkv_chunks scratch")
+    T, (_, H, V, K) = rkv.shape[0], state.shape
+    if scratch.numel() < wkv_chunks_scratch(T, H, K, V):
+        raise KernelError(f"wkv_chunks: {scratch.numel()} floats of scratch memory for {T} rows")
+    _call("wkv", "mlxb_wkv_chunks", _WKV_ARGS[:-1] + [c_int, c_void_p, c_void_p], *args, T, _p(scratch), stream)
 
 
 # --------------------------------------------------------------------------
