@@ -7,15 +7,19 @@
 //                  from one (offset 1).  A gate g (activation dtype) may come in: mode 1 multiplies x by
 //                  silu(g) BEFORE the statistics, mode 2 multiplies the normed value by silu(g).
 //                  x is float32 or has the activation dtype, which the result has.  No weight: the normed value as it is
-//                  (times the offset where there is one).  All arithmetic is float32.  Rows or parts of up to
-//                  512 columns without a weight, or in the activation dtype, take a kernel with a warp each.
-// rmsnorm_rows     the same for whole float32 rows with a weight per column, a row kept in registers.
+//                  (times the offset where there is one).  All arithmetic is float32.
+// rmsnorm_rows     the same for whole float32 rows with a weight per column.
 // residual_update  x[r, :] += scale * (f1(y1[r, :]) + f2(y2[r, :])),  f_i = rmsnorm with weight w_i over the
 //                  whole row, or the identity where w_i is null; y2 may be null.  Optionally a copy of the new
 //                  row in the activation dtype is left in `cast_out` for the products that read it next.
 // norm_update      y = scale * (sum of the row's `terms` rows of y1) + y2[r, :];  x[r, :] += y / sqrt(mean(y^2) + eps) * w: a sublayer
 //                  whose result is normed before it joins the stream, with the sum over the experts a token used in the same
 //                  pass, and a copy of the new row as above.
+//
+// Bound by memory where there are many rows and by latency where there are few, so where rows and strides are whole groups of four
+// columns a thread asks for all that it has of a row at once (16-byte accesses, the weights before the wait for the kernel before)
+// and keeps it in registers between the sum and the result; parts of up to 512 columns take a warp each, wider ones a block.  The
+// kernels that read a column at a time, and the row again for the result, serve what is left.
 #include "common.cuh"
 
 MLXB_DEFINE_LAST_ERROR()
@@ -75,6 +79,8 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, const float (&v)[4]) {
   *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const unsigned*>(&a), *reinterpret_cast<const unsigned*>(&b));
 }
 
+__device__ __forceinline__ float squares(const float (&v)[4]) { return (v[0] * v[0] + v[1] * v[1]) + (v[2] * v[2] + v[3] * v[3]); }
+
 // Parts (or whole rows) of at most 128 * RP_STEPS columns (a multiple of 4, accesses of four columns): a warp per part,
 // the part in registers between the sum and the result.
 constexpr int RP_STEPS = 4;
@@ -105,68 +111,102 @@ rmsnorm_parts_kernel(const TI* x, int ldx, const float* __restrict__ w, float of
     }
   }
 #pragma unroll
-  for (int i = 0; i < RP_STEPS; ++i)
+  for (int i = 0; i < RP_STEPS; ++i) {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
+    for (int e = 0; e < 4; ++e)
       if (gate_mode == 1) v[i][e] *= silu_f(gv[i][e]);
-      s = fmaf(v[i][e], v[i][e], s);
-    }
+    s += squares(v[i]);
+  }
   const float rinv = 1.f / sqrtf(warp_sum(s) / (float)Dg + eps);
   TO* o = out + (size_t)r * ldo + (size_t)g * Dg;
 #pragma unroll
   for (int i = 0; i < RP_STEPS; ++i) {
     const int c = (i * 32 + lane) * 4;
     if (c >= Dg) continue;
-    float res[4];
+    float res[4], wv[4] = {0.f, 0.f, 0.f, 0.f};
+    if (w) load4(w + (g * Dg + c) % period, wv);      // (the period is a multiple of four: the four lie side by side)
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      res[e] = v[i][e] * rinv * (w ? offset + w[(g * Dg + c + e) % period] : offset);
+      res[e] = v[i][e] * rinv * (offset + wv[e]);
       if (gate_mode == 2) res[e] *= silu_f(gv[i][e]);
     }
     store4(o + c, res);
   }
 }
 
-// Whole float32 rows with a weight per column, four columns a thread and step: the row stays in registers between the sum and
-// the result, the weights are asked for before the wait.  NV * 4 * blockDim.x columns at most.
-template <typename TO, int NV>
+// Wider parts (or whole rows), four columns a thread and step: a block per part, the part in registers, the weights asked for before
+// the wait.  NV * 4 * blockDim.x columns at most.
+template <typename TI, typename TO, int NV>
 __global__ void __launch_bounds__(512)
-rmsnorm_rows_kernel(const float* x, int ldx, const int* __restrict__ rows, int n_src_rows, const float* __restrict__ w, float offset,
-                    TO* __restrict__ out, int ldo, int D, float eps) {
+rmsnorm_rows_kernel(const TI* x, int ldx, const int* __restrict__ rows, int n_src_rows, const float* __restrict__ w, float offset,
+                    int period, const TO* gate, int ldg, int gate_mode, TO* __restrict__ out, int ldo, int Dg, float eps) {
   __shared__ float red[33];
-  const int r = blockIdx.x;
+  const int r = blockIdx.x, g = blockIdx.y;
   const int src = rows ? rows[r] : r;
   const bool there = src >= 0 && src < n_src_rows;
-  float wv[NV][4], v[NV][4];
+  const int w0 = g * Dg % period;      // (a part's weights are neighbours: the period is the width or the part's)
+  float wv[NV][4], v[NV][4], gv[NV][4];
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int c = (i * blockDim.x + threadIdx.x) * 4;
-    if (c < D) load4(w + c, wv[i]);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) wv[i][e] = v[i][e] = gv[i][e] = 0.f;
+    if (c < Dg && w) load4(w + w0 + c, wv[i]);
   }
   pdl_wait();
   pdl_trigger();
   x = after_wait(x);
+  gate = after_wait(gate);
   float s = 0.f;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int c = (i * blockDim.x + threadIdx.x) * 4;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) v[i][e] = 0.f;
-    if (c < D && there) load4(x + (size_t)src * ldx + c, v[i]);
+    if (c < Dg && there) {
+      load4(x + (size_t)src * ldx + (size_t)g * Dg + c, v[i]);
+      if (gate_mode) load4(gate + (size_t)src * ldg + (size_t)g * Dg + c, gv[i]);
+    }
   }
 #pragma unroll
-  for (int i = 0; i < NV; ++i)
+  for (int i = 0; i < NV; ++i) {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) s = fmaf(v[i][e], v[i][e], s);
-  const float rinv = 1.f / sqrtf(block_sum(s, red) / (float)D + eps);
+    for (int e = 0; e < 4; ++e)
+      if (gate_mode == 1) v[i][e] *= silu_f(gv[i][e]);
+    s += squares(v[i]);
+  }
+  const float rinv = 1.f / sqrtf(block_sum(s, red) / (float)Dg + eps);
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int c = (i * blockDim.x + threadIdx.x) * 4;
-    if (c >= D) continue;
+    if (c >= Dg) continue;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) v[i][e] = v[i][e] * rinv * (offset + wv[i][e]);
-    store4(out + (size_t)r * ldo + c, v[i]);
+    for (int e = 0; e < 4; ++e) {
+      v[i][e] = v[i][e] * rinv * (offset + wv[i][e]);
+      if (gate_mode == 2) v[i][e] *= silu_f(gv[i][e]);
+      if (!there) v[i][e] = 0.f;
+    }
+    store4(out + (size_t)r * ldo + (size_t)g * Dg + c, v[i]);
   }
+}
+
+constexpr int RR_MAX = 4 * 512 * 4;      // columns of a part that a block holds
+
+// Threads of a block with a part of Dg columns: the fewest that have it in two steps each, up to 512.
+static int rows_threads(int Dg) {
+  int threads = 64;
+  while (threads < 512 && Dg / 4 > threads * 2) threads *= 2;
+  return threads;
+}
+template <typename TI, typename TO>
+static void launch_rows(const TI* x, int ldx, const int* rows, int n_src_rows, const float* w, float offset, int period, const TO* gate,
+                        int ldg, int gate_mode, TO* out, int ldo, int R, int Dg, int groups, float eps, cudaStream_t stream) {
+  const int threads = rows_threads(Dg), nv = (Dg / 4 + threads - 1) / threads;
+  auto go = [&](auto kernel) {
+    launch_pdl(kernel, dim3(R, groups), dim3(threads), 0, stream, x, ldx, rows, n_src_rows, w, offset, period, gate, ldg, gate_mode, out,
+               ldo, Dg, eps);
+  };
+  if (nv <= 1) go(rmsnorm_rows_kernel<TI, TO, 1>);
+  else if (nv <= 2) go(rmsnorm_rows_kernel<TI, TO, 2>);
+  else go(rmsnorm_rows_kernel<TI, TO, 4>);
 }
 
 // x_f32: x is float32 (else it has out_dtype); w may be null (the offset is then the factor).
@@ -183,16 +223,28 @@ MLXB_EXPORT int mlxb_rmsnorm(int out_dtype, int x_f32, const void* x, int ldx, c
   if (out_dtype != MLXB_F32 && out_dtype != MLXB_BF16) return mlxb_fail(MLXB_BAD_DTYPE, "rmsnorm: dtype code %d", out_dtype);
   const int Dg = D / groups;
   const int xb = (x_f32 || out_dtype == MLXB_F32) ? 16 : 8, ob = out_dtype == MLXB_F32 ? 16 : 8;   // bytes of four columns
-  // (weighted norms of float32 rows keep the block per row or part and its order of additions)
-  const bool parts = (w == nullptr || (!x_f32 && out_dtype == MLXB_BF16)) && rows == nullptr && Dg % 4 == 0 && Dg <= 128 * RP_STEPS && ldx % 4 == 0 && ldo % 4 == 0 &&
-                     (!gate || ldg % 4 == 0) && (uintptr_t)x % xb == 0 && ((uintptr_t)out | (uintptr_t)gate) % ob == 0;
+  const bool fours = Dg % 4 == 0 && ldx % 4 == 0 && ldo % 4 == 0 && (!gate || ldg % 4 == 0) && (!w || period % 4 == 0) &&
+                     (uintptr_t)x % xb == 0 && (uintptr_t)w % 16 == 0 && ((uintptr_t)out | (uintptr_t)gate) % ob == 0;
+  const bool parts = fours && rows == nullptr && Dg <= 128 * RP_STEPS;
+  const bool wide = fours && !parts && Dg <= RR_MAX && (!w || period == D || period == Dg);
   const int threads = parts ? 256 : (Dg >= 2048 ? 256 : (Dg >= 512 ? 128 : (Dg >= 128 ? 64 : 32)));
   const dim3 grid = parts ? dim3((unsigned)(((long long)R * groups + 7) / 8)) : dim3(R, groups);
-#define RMS_GO(TI, TO)                                                                                                  if (parts)                                                                                                              launch_pdl(rmsnorm_parts_kernel<TI, TO>, grid, dim3(threads), 0, stream, (const TI*)x, ldx, w, offset, period,                   (const TO*)gate, ldg, gate_mode, (TO*)out, ldo, R, Dg, groups, eps);                                     else                                                                                                                    launch_pdl(rmsnorm_kernel<TI, TO>, grid, dim3(threads), 0, stream, (const TI*)x, ldx, rows, n_src_rows, w, offset,                period, (const TO*)gate, ldg, gate_mode, (TO*)out, ldo, D, groups, eps)
-  if (out_dtype == MLXB_F32) { RMS_GO(float, float); }
-  else if (x_f32) { RMS_GO(float, __nv_bfloat16); }
-  else { RMS_GO(__nv_bfloat16, __nv_bfloat16); }
-#undef RMS_GO
+  auto go = [&](auto from, auto to) {
+    using TI = decltype(from);
+    using TO = decltype(to);
+    if (parts)
+      launch_pdl(rmsnorm_parts_kernel<TI, TO>, grid, dim3(threads), 0, stream, (const TI*)x, ldx, w, offset, period, (const TO*)gate, ldg,
+                 gate_mode, (TO*)out, ldo, R, Dg, groups, eps);
+    else if (wide)
+      launch_rows<TI, TO>((const TI*)x, ldx, rows, n_src_rows, w, offset, period, (const TO*)gate, ldg, gate_mode, (TO*)out, ldo, R, Dg,
+                          groups, eps, stream);
+    else
+      launch_pdl(rmsnorm_kernel<TI, TO>, grid, dim3(threads), 0, stream, (const TI*)x, ldx, rows, n_src_rows, w, offset, period,
+                 (const TO*)gate, ldg, gate_mode, (TO*)out, ldo, D, groups, eps);
+  };
+  if (out_dtype == MLXB_F32) go(float{}, float{});
+  else if (x_f32) go(float{}, __nv_bfloat16{});
+  else go(__nv_bfloat16{}, __nv_bfloat16{});
   return mlxb_check_launch("rmsnorm");
 }
 
@@ -202,26 +254,15 @@ MLXB_EXPORT int mlxb_rmsnorm_rows(int out_dtype, const float* x, int ldx, const 
                                   float offset, void* out, int ldo, int R, int D, float eps, cudaStream_t stream) {
   if (R <= 0) return 0;
   const int ob = out_dtype == MLXB_F32 ? 16 : 8;
-  if (D <= 0 || D % 4 || D > 4 * 512 * 4 || ldx % 4 || ldo % 4 || ldx < D || ldo < D || !w || (((uintptr_t)x | (uintptr_t)w) & 15) ||
+  if (D <= 0 || D % 4 || D > RR_MAX || ldx % 4 || ldo % 4 || ldx < D || ldo < D || !w || (((uintptr_t)x | (uintptr_t)w) & 15) ||
       (uintptr_t)out % ob)
     return mlxb_fail(MLXB_BAD_ARG, "rmsnorm_rows: width %d, strides %d / %d", D, ldx, ldo);
-  int threads = 64;
-  while (threads < 512 && D / 4 > threads * 2) threads *= 2;
-  const int nv = (D / 4 + threads - 1) / threads;
-#define RMS_ROWS(TO, NV)                                                                                                \
-  launch_pdl(rmsnorm_rows_kernel<TO, NV>, dim3(R), dim3(threads), 0, stream, x, ldx, rows, n_src_rows, w, offset, (TO*)out, ldo, \
-             D, eps)
-#define RMS_ROWS_NV(TO)                \
-  do {                                 \
-    if (nv <= 1) RMS_ROWS(TO, 1);      \
-    else if (nv <= 2) RMS_ROWS(TO, 2); \
-    else RMS_ROWS(TO, 4);              \
-  } while (0)
-  if (out_dtype == MLXB_F32) RMS_ROWS_NV(float);
-  else if (out_dtype == MLXB_BF16) RMS_ROWS_NV(__nv_bfloat16);
-  else return mlxb_fail(MLXB_BAD_DTYPE, "rmsnorm_rows: dtype code %d", out_dtype);
-#undef RMS_ROWS_NV
-#undef RMS_ROWS
+  if (out_dtype == MLXB_F32)
+    launch_rows<float, float>(x, ldx, rows, n_src_rows, w, offset, D, nullptr, 0, 0, (float*)out, ldo, R, D, 1, eps, stream);
+  else if (out_dtype == MLXB_BF16)
+    launch_rows<float, __nv_bfloat16>(x, ldx, rows, n_src_rows, w, offset, D, nullptr, 0, 0, (__nv_bfloat16*)out, ldo, R, D, 1, eps, stream);
+  else
+    return mlxb_fail(MLXB_BAD_DTYPE, "rmsnorm_rows: dtype code %d", out_dtype);
   return mlxb_check_launch("rmsnorm_rows");
 }
 
@@ -259,21 +300,95 @@ __global__ void residual_update_kernel(float* x, int ldx, const float* y1, const
   }
 }
 
+// Four columns a thread and step, all of a row's operands in registers: NV * 4 * blockDim.x columns at most.
+template <typename TO, int NV>
+__global__ void __launch_bounds__(512)
+residual_update_rows_kernel(float* x, int ldx, const float* y1, const float* __restrict__ w1, const float* y2,
+                            const float* __restrict__ w2, int ldy, float scale, float eps, TO* __restrict__ cast_out, int ldc, int D) {
+  __shared__ float red[33], red2[33];
+  const int r = blockIdx.x;
+  float wa[NV][4], wb[NV][4], a[NV][4], b[NV][4], xv[NV][4];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = (i * blockDim.x + threadIdx.x) * 4;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      wa[i][e] = wb[i][e] = 1.f;
+      a[i][e] = b[i][e] = xv[i][e] = 0.f;
+    }
+    if (c < D && w1) load4(w1 + c, wa[i]);
+    if (c < D && w2) load4(w2 + c, wb[i]);
+  }
+  pdl_wait();
+  pdl_trigger();
+  x = after_wait(x);
+  y1 = after_wait(y1);
+  y2 = after_wait(y2);
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = (i * blockDim.x + threadIdx.x) * 4;
+    if (c >= D) continue;
+    load4(y1 + (size_t)r * ldy + c, a[i]);
+    if (y2) load4(y2 + (size_t)r * ldy + c, b[i]);
+    load4(x + (size_t)r * ldx + c, xv[i]);
+  }
+  auto normed = [&](float (&v)[NV][4], const float (&w)[NV][4], float* memory) {
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s = fmaf(v[i][e], v[i][e], s);
+    const float f = 1.f / sqrtf(block_sum(s, memory) / (float)D + eps);
+#pragma unroll
+    for (int i = 0; i < NV; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[i][e] = v[i][e] * f * w[i][e];
+  };
+  if (w1) normed(a, wa, red);
+  if (y2 && w2) normed(b, wb, red2);
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = (i * blockDim.x + threadIdx.x) * 4;
+    if (c >= D) continue;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) xv[i][e] += scale * (y2 ? a[i][e] + b[i][e] : a[i][e]);
+    store4(x + (size_t)r * ldx + c, xv[i]);
+    if (cast_out) store4(cast_out + (size_t)r * ldc + c, xv[i]);
+  }
+}
+
 MLXB_EXPORT int mlxb_residual_update(int cast_dtype, float* x, int ldx, const float* y1, const float* w1,
                                      const float* y2, const float* w2, int ldy, float scale, float eps, void* cast_out,
                                      int ldc, int R, int D, cudaStream_t stream) {
   if (R <= 0) return 0;
   if (D <= 0 || ldx < D || ldy < D || y1 == nullptr || (cast_out && ldc < D))
     return mlxb_fail(MLXB_BAD_ARG, "residual_update: width %d, strides %d / %d / %d", D, ldx, ldy, ldc);
+  if (cast_dtype != MLXB_F32 && cast_dtype != MLXB_BF16) return mlxb_fail(MLXB_BAD_DTYPE, "residual_update: dtype code %d", cast_dtype);
+  const bool fours = D % 4 == 0 && D <= RR_MAX && ldx % 4 == 0 && ldy % 4 == 0 && (!cast_out || ldc % 4 == 0) &&
+                     (((uintptr_t)x | (uintptr_t)y1 | (uintptr_t)y2 | (uintptr_t)w1 | (uintptr_t)w2) & 15) == 0 &&
+                     (uintptr_t)cast_out % (cast_dtype == MLXB_F32 ? 16 : 8) == 0;
+  if (fours) {
+    const int threads = rows_threads(D), nv = (D / 4 + threads - 1) / threads;
+    auto by = [&](auto to) {
+      using TO = decltype(to);
+      auto go = [&](auto kernel) {
+        launch_pdl(kernel, dim3(R), dim3(threads), 0, stream, x, ldx, y1, w1, y2, w2, ldy, scale, eps, (TO*)cast_out, ldc, D);
+      };
+      if (nv <= 1) go(residual_update_rows_kernel<TO, 1>);
+      else if (nv <= 2) go(residual_update_rows_kernel<TO, 2>);
+      else go(residual_update_rows_kernel<TO, 4>);
+    };
+    if (cast_dtype == MLXB_F32) by(float{});
+    else by(__nv_bfloat16{});
+    return mlxb_check_launch("residual_update");
+  }
   const int threads = D >= 2048 ? 256 : (D >= 512 ? 128 : 64);
   if (cast_dtype == MLXB_F32)
     launch_pdl(residual_update_kernel<float>, dim3(R), dim3(threads), 0, stream, x, ldx, y1, w1, y2, w2, ldy, scale,
                eps, (float*)cast_out, ldc, D);
-  else if (cast_dtype == MLXB_BF16)
+  else
     launch_pdl(residual_update_kernel<__nv_bfloat16>, dim3(R), dim3(threads), 0, stream, x, ldx, y1, w1, y2, w2, ldy,
                scale, eps, (__nv_bfloat16*)cast_out, ldc, D);
-  else
-    return mlxb_fail(MLXB_BAD_DTYPE, "residual_update: dtype code %d", cast_dtype);
   return mlxb_check_launch("residual_update");
 }
 
