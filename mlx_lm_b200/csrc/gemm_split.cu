@@ -1,9 +1,9 @@
 // Linear layer of float32 rows on the 5th-generation tensor cores, at float32's precision:
 //   C[M,N] = epilogue(A[M,K] . W[N,K]^T + bias[N]) (+ residual[M,N]),  all of them float32
 //
-// Every operand is the sum of three bfloat16 numbers, x = h + m + l, each the nearest to what the ones before it leave (24
-// bits together, nothing of x is lost), and a product of two operands is the six products of such parts that reach 24 bits:
-// h h, h m, m h, h l, l h, m m (what is left out is 2^-25 of the product at most).  The tensor core's products are exact; what
+// Every operand is the sum of three bfloat16 numbers, x = h + m + l (24 bits together, nothing of x is lost; h is cut off, m
+// rounded, so that l has either sign), and a product of two operands is the six products of such parts that reach 24 bits:
+// h h, h m, m h, h l, l h, m m (what is left out, m l and l m, is 2^-23 of the product at most and as often above as below).  The tensor core's products are exact; what
 // it adds to its accumulator it cuts off instead of rounding, so no sum is left to it for long: a block of 64 of K starts a
 // fresh accumulator, the five small products of all its steps go in first, when the accumulator is 2^-8 of what it will be,
 // the four steps of h h last, and the block's sum is added, rounded to nearest, to a sum in registers.  One order for every
@@ -53,23 +53,45 @@ struct Smem {
   int abort_flag;
 };
 
-// Four neighbours taken apart, into the three planes at byte offset `at`.
+// Four neighbours taken apart, into the three planes at byte offset `at`: h is the number's upper half as it stands, m the nearest to
+// what that leaves (16 bits), and what is left then (8 bits) is a bfloat16 number as it stands: one conversion for two numbers,
+// and conversions run at an eighth of the rate of other instructions.
+__device__ __forceinline__ uint32_t upper_halves(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x7632); }
 __device__ __forceinline__ void put_parts(const float4& v, char* plane0, uint32_t plane_bytes, uint32_t at) {
-  float r[4] = {v.x, v.y, v.z, v.w};
+  const float x[4] = {v.x, v.y, v.z, v.w};
+  uint32_t u[4], h[2], m[2], l[2];
+  float r[4];
 #pragma unroll
-  for (int p = 0; p < 3; ++p) {
-    const __nv_bfloat162 a = __floats2bfloat162_rn(r[0], r[1]), b = __floats2bfloat162_rn(r[2], r[3]);
-    uint2 u;
-    u.x = *reinterpret_cast<const uint32_t*>(&a);
-    u.y = *reinterpret_cast<const uint32_t*>(&b);
-    *reinterpret_cast<uint2*>(plane0 + p * plane_bytes + at) = u;
-    if (p < 2) {
-      r[0] -= __uint_as_float(u.x << 16);
-      r[1] -= __uint_as_float(u.x & 0xffff0000u);
-      r[2] -= __uint_as_float(u.y << 16);
-      r[3] -= __uint_as_float(u.y & 0xffff0000u);
-    }
+  for (int i = 0; i < 4; ++i) {
+    u[i] = __float_as_uint(x[i]);
+    r[i] = x[i] - __uint_as_float(u[i] & 0xffff0000u);
   }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    h[i] = upper_halves(u[2 * i], u[2 * i + 1]);
+    const __nv_bfloat162 c = __floats2bfloat162_rn(r[2 * i], r[2 * i + 1]);
+    m[i] = *reinterpret_cast<const uint32_t*>(&c);
+    r[2 * i] -= __uint_as_float(m[i] << 16);
+    r[2 * i + 1] -= __uint_as_float(m[i] & 0xffff0000u);
+    l[i] = upper_halves(__float_as_uint(r[2 * i]), __float_as_uint(r[2 * i + 1]));
+  }
+  *reinterpret_cast<uint2*>(plane0 + at) = make_uint2(h[0], h[1]);
+  *reinterpret_cast<uint2*>(plane0 + plane_bytes + at) = make_uint2(m[0], m[1]);
+  *reinterpret_cast<uint2*>(plane0 + 2 * plane_bytes + at) = make_uint2(l[0], l[1]);
+}
+
+// 32 columns of a row's accumulator and the wait for them in one statement: between two the compiler may put additions of
+// registers that the load has not written yet.
+__device__ __forceinline__ void tmem_get32(uint32_t taddr, uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\ttcgen05.wait::ld.sync.aligned;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr) : "memory");
 }
 
 // A row of A times a row of W in plain float32, by a warp; the same in every lane.
@@ -221,8 +243,7 @@ linear_split_kernel(const float* A, const float* __restrict__ W, const float* __
 #pragma unroll
         for (int c = 0; c < COLS; c += 32) {
           uint32_t r[32];
-          tmem_ld32(taddr + (uint32_t)(b * BN + c), r);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          tmem_get32(taddr + (uint32_t)(b * BN + c), r);
 #pragma unroll
           for (int i = 0; i < 32; ++i) sum[c + i] += __uint_as_float(r[i]);
         }

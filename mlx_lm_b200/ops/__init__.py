@@ -51,6 +51,9 @@ _DT = {torch.float32: F32, torch.bfloat16: BF16}
 BF16_ONLY_LIBS = frozenset({"gemm_smallm", "gemm_smallm_fold", "gemm_tcgen05", "attention_prefill",
                             "attention_prefill_tc", "attention_wide_tc", "moe_tcgen05", "recurrent_chunks"})
 
+# ... and those that only a float32 run launches from
+F32_ONLY_LIBS = frozenset({"gemm_split"})
+
 # status word bits set by kernels (csrc/common.cuh)
 ST_TOKEN_RANGE, ST_POSITION_RANGE, ST_PAGE_RANGE, ST_WAIT_TIMEOUT = 1, 2, 4, 8
 
@@ -347,6 +350,12 @@ def linear_split_supported(x, w, out, residual=None) -> bool:
     if x.shape[1] % 4 or x.stride(0) % 4:
         return False
     return not any(t is not None and t.data_ptr() % 16 for t in (x, w, out, residual))
+
+
+def linear_split_pays(M: int, N: int, K: int) -> bool:
+    """Whether ``linear_split`` takes less time than ``linear_generic``: from 17 rows on (up to 16 the few-rows kernel, 6 us at
+    1024 x 1024, to 28) and two blocks of K (20 rows, 512 x 128: 8.2 us to 10.0; 20 and 300 rows with 64 of K 6.9 and 7.7 to 6.4 and 6.9)."""
+    return M > 16 and K >= 128
 
 
 def linear_split(x, w, bias, out, status, stream, epilogue: int = EPI_NONE, residual=None) -> None:

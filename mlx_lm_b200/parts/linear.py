@@ -24,7 +24,7 @@ ACTIVATIONS = {None: ops.EPI_NONE, **ops.ACTIVATION_CODES}
 class Linear(Part):
     replayable = True
     # (the few-rows kernel with a folded norm is a library of its own, named by the block that folds norms)
-    kernel_libs = ("gemm_simt", "gemm_smallm", "gemm_tcgen05")
+    kernel_libs = ("gemm_simt", "gemm_smallm", "gemm_tcgen05", "gemm_split")
 
     def __init__(self, name: str, n_in: int, n_out: int, bias: bool = True, stored: str = "out_in",
                  weight_suffix: str = ".weight", init: Init = Init(), bias_init: Init = Init(),
@@ -107,7 +107,7 @@ class Linear(Part):
         return (f.colsum, stats)
 
     def forward(self, ctx, x, out, activation=None, residual=None) -> torch.Tensor:
-        """float32: the generic kernel (true 32-bit arithmetic).  bfloat16: the weight-streaming kernel for up
+        """float32: the generic kernel (true 32-bit arithmetic), or for more than a few rows the tensor cores at the same precision.  bfloat16: the weight-streaming kernel for up
         to 64 rows, the tcgen05 kernel for more; an inner size that is no multiple of 8 (no 16-byte rows)
         goes to the generic kernel."""
         epi = ACTIVATIONS[activation]
@@ -129,6 +129,8 @@ class Linear(Part):
         elif fast:
             ops.linear_tensor_cores(x, self.weight, self.bias, out, ctx.status, ctx.stream, epilogue=epi,
                                     residual=residual, fold=fold)
+        elif ops.linear_split_supported(x, self.weight, out, residual) and ops.linear_split_pays(M, self.n_out, self.n_in):
+            ops.linear_split(x, self.weight, self.bias, out, ctx.status, ctx.stream, epilogue=epi, residual=residual)
         else:
             ops.linear_generic(x, self.weight, self.bias, out, ctx.stream, epilogue=epi, residual=residual)
         return out
