@@ -39,7 +39,7 @@ constexpr int STALE = 8;                            // powers of two that a row'
 
 struct Control {
   uint64_t full[MAX_SLOTS], empty[MAX_SLOTS];
-  uint64_t s_full[2], p_full, o_full;
+  uint64_t s_full[2], p_full[2], o_full;           // by block & 1: a pair of softmax warps may be a block ahead of another
   uint64_t x_full[4];                               // exchange between the two warps of the same rows
   uint64_t drained;                                 // abort path only
   float row_max[2][2][M];                           // [block & 1][half][row]
@@ -79,7 +79,25 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
       ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
         "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
 }
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// Loads with their wait in one statement: between two statements the compiler may put arithmetic on registers that the load
+// has not written yet.
+#define LD_REGS_16 "%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15"
+__device__ __forceinline__ void tmem_get16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {" LD_REGS_16 "}, [%16];\n\ttcgen05.wait::ld.sync.aligned;"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+                 "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+               : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_get32(uint32_t taddr, uint32_t (&r)[32]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {" LD_REGS_16
+               ", %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\t"
+               "tcgen05.wait::ld.sync.aligned;"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+                 "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+                 "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+                 "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+               : "r"(taddr) : "memory");
+}
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ int stage_index(int row, int piece) { return row * 4 + (piece ^ ((row >> 1) & 3)); }
 
@@ -125,8 +143,7 @@ attention_wide_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const _
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < a.slots; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], 1); }
-    for (int b = 0; b < 2; ++b) mbar_init(&sm.s_full[b], 1);
-    mbar_init(&sm.p_full, SOFT_WARPS);
+    for (int b = 0; b < 2; ++b) { mbar_init(&sm.s_full[b], 1); mbar_init(&sm.p_full[b], SOFT_WARPS); }
     mbar_init(&sm.o_full, 1);
     for (int w = 0; w < 4; ++w) mbar_init(&sm.x_full[w], 2);
     mbar_init(&sm.drained, 1);
@@ -304,7 +321,7 @@ attention_wide_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const _
         issue_s(i + 1);
         if (!ok) break;
       }
-      if (!(ok = mbar_wait_warp(&sm.p_full, (uint32_t)(i & 1), abort_flag))) break;
+      if (!(ok = mbar_wait_warp(&sm.p_full[i & 1], (uint32_t)((i >> 1) & 1), abort_flag))) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       Mark at = v_at;
       for (int c = 0; c < a.v_chunks; ++c) {
@@ -344,8 +361,7 @@ attention_wide_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const _
       if (!(ok = mbar_wait_warp(&sm.s_full[i & 1], (uint32_t)((i >> 1) & 1), abort_flag))) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       uint32_t s[32];
-      tmem_ld32(t_s + 32u * half, s);
-      tmem_wait_ld();
+      tmem_get32(t_s + 32u * half, s);
       const bool open = j0 + KB - 1 <= pos0 && (j0 >= lo_min || j0 + KB <= kept);      // every key is visible to the first token
       // (and to the others, unless the window or the run moves on between them)
       const bool all = open && (a.window <= 0 || j0 >= last_pos - a.window + 1 || j0 + KB <= kept) &&
@@ -357,6 +373,7 @@ attention_wide_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const _
         if (a.softcap > 0.f) f = a.softcap * tanhf(f * a.scale / a.softcap);
         v[e] = f * mult;
       }
+      __syncwarp();
       if (!all) {
 #pragma unroll
         for (int e = 0; e < 32; ++e) {
@@ -379,9 +396,8 @@ attention_wide_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const _
         if (!(ok = mbar_wait_warp(&sm.o_full, (uint32_t)((i - 1) & 1), abort_flag))) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         for (int c = 0; c < o_cols; c += 16) {
-          uint32_t o[32], w[16];
-          tmem_ld16(tmem_o + lanes + (uint32_t)(o_first + c), o);
-          tmem_wait_ld();
+          uint32_t o[16], w[16];
+          tmem_get16(tmem_o + lanes + (uint32_t)(o_first + c), o);
 #pragma unroll
           for (int e = 0; e < 16; ++e) w[e] = __float_as_uint(__uint_as_float(o[e]) * corr);
           tmem_st16(tmem_o + lanes + (uint32_t)(o_first + c), w);
@@ -418,8 +434,10 @@ attention_wide_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const _
       tmem_wait_st();
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) mbar_arrive(&sm.p_full);
+      if (lane == 0) mbar_arrive(&sm.p_full[i & 1]);
     }
+    // (S of the last block says that P V of the last but two is done: a parity tells one block from the next, not two)
+    if (ok && n_blocks > 1) ok = mbar_wait_warp(&sm.o_full, (uint32_t)(n_blocks & 1), abort_flag);
     if (ok) ok = mbar_wait_warp(&sm.o_full, (uint32_t)((n_blocks - 1) & 1), abort_flag);
     if (ok) {
       sm.row_max[n_blocks & 1][half][r] = l;
@@ -442,8 +460,7 @@ attention_wide_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const _
       constexpr int PER = 16 / sizeof(TO), ROUND = 4 * PER;          // columns of a piece, and of the 64 bytes of a row a round
       for (int c = 0; c < o_cols; c += 32) {
         uint32_t o[32];
-        tmem_ld32(tmem_o + lanes + (uint32_t)(o_first + c), o);
-        tmem_wait_ld();
+        tmem_get32(tmem_o + lanes + (uint32_t)(o_first + c), o);
 #pragma unroll
         for (int e = 0; e < 32; ++e) {
           float u = __uint_as_float(o[e]) * f;

@@ -49,7 +49,7 @@ _DT = {torch.float32: F32, torch.bfloat16: BF16}
 
 # kernel sources that only a bfloat16 run launches from: a float32 run neither compiles nor loads them
 BF16_ONLY_LIBS = frozenset({"gemm_smallm", "gemm_smallm_fold", "gemm_tcgen05", "attention_prefill",
-                            "attention_prefill_tc", "attention_wide_tc", "moe_tcgen05", "recurrent_chunks"})
+                            "attention_prefill_tc", "attention_wide_tc", "attention_wide_tcgen05", "moe_tcgen05", "recurrent_chunks"})
 
 # ... and those that only a float32 run launches from
 F32_ONLY_LIBS = frozenset({"gemm_split"})
@@ -1748,6 +1748,12 @@ def attention_wide_step(ctx, q, q_head_stride: int, cache_k, cache_v, block_tabl
             attention_portions(q_rounded, ctx.portion_tiles, ctx.n_portion_tiles, block_table, cache_k, cache_v, out,
                                n_heads, scale, window, ctx.status, ctx.stream, keep_first=keep_first, softcap=softcap,
                                gate=gate)
+        elif (ctx.n_portion and ctx.portion_tiles is not None
+              and attention_wide_portions_supported(q, q_head_stride, cache_k, cache_v, n_heads, key_dim, value_dim, talk is not None)):
+            attention_wide_portions(q, q_head_stride, ctx.portion_tiles, ctx.n_portion_tiles, PREFILL_TILE, block_table,
+                                    cache_k, cache_v, out, out_head_stride, n_heads, key_dim, value_dim, scale, ctx.status,
+                                    ctx.stream, window=window, chunk=chunk, talk=talk, gate=gate, softcap=softcap,
+                                    keep_first=keep_first)
         elif ctx.n_portion and ctx.portion_tiles is not None:
             attention_wide_tiles(q, q_head_stride, ctx.portion_tiles, ctx.n_portion_tiles, PREFILL_TILE, block_table,
                                  cache_k, cache_v, out, out_head_stride, n_heads, key_dim, value_dim, scale, ctx.status,

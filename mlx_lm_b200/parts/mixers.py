@@ -313,7 +313,7 @@ class TalkingHeadsAttention(Mixer):
     Queries go to the kernel in float32; scores, their mix and the softmax are float32.  ``mix`` returns the output
     projection in float32 for a block that adds it to the stream itself; ``forward`` adds it in that product's epilogue."""
     replayable = True
-    kernel_libs = ("attention_wide", "attention_wide_tc", "rotary")
+    kernel_libs = ("attention_wide", "attention_wide_tc", "attention_wide_tcgen05", "rotary")
 
     def __init__(self, name: str, width: int, n_heads: int, n_kv_heads: int, dim: int, vdim: int, scale: float,
                  eps: float, rot_dims: int = 0, rot_base: float = 10000.0, interleaved: bool = False, bias: bool = True,
@@ -478,7 +478,7 @@ class LatentAttention(Mixer):
     output projection in float32 for a block that adds it to the stream itself; ``forward`` adds it in that product's
     epilogue."""
     replayable = True
-    kernel_libs = ("attention_wide", "attention_wide_tc", "latent")
+    kernel_libs = ("attention_wide", "attention_wide_tc", "attention_wide_tcgen05", "latent")
 
     def __init__(self, name: str, width: int, n_heads: int, dim: int, rot_dim: int, vdim: int, kv_rank: int,
                  scale: float, eps: float, rot_base: float = 10000.0, interleaved: bool = True,
@@ -601,7 +601,7 @@ class DifferentialAttention(Mixer):
     weights are bound, by a permutation of the rows of ``q`` and of its convolution) so that the queries of one key
     head lie together: group ``g`` holds ``[map 1 of its heads | map 2 of its heads]``."""
     replayable = True
-    kernel_libs = ("attention_wide", "attention_wide_tc", "rotary", "recurrent", "rms")
+    kernel_libs = ("attention_wide", "attention_wide_tc", "attention_wide_tcgen05", "rotary", "recurrent", "rms")
 
     def __init__(self, name: str, width: int, n_heads: int, n_kv_heads: int, dim: int, vdim: int, scale: float,
                  eps: float, diff: float, taps: int = 0, init: Init = Init()):
