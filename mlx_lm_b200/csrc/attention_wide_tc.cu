@@ -61,7 +61,7 @@ attention_wide_tc_kernel(const float* q, int ldq, int qhs, const int* __restrict
                          int chunk, float scale, const float* __restrict__ talk, const __nv_bfloat16* k_pool,
                          const __nv_bfloat16* v_pool, const __nv_bfloat16* gate, int ldg, TO* __restrict__ out, int ldo,
                          int ohs, int* __restrict__ status, int bps, int n_rel, float* __restrict__ scratch, int nbuf,
-                         float softcap, int keep_first, int gate_cols, int Hv) {
+                         float softcap, int keep_first, int gate_cols, int Hv, int vec_q) {
   constexpr int M = TC_M * MP, THREADS = TC_THREADS * MP;
   extern __shared__ __align__(16) unsigned char tc_smem[];
   const int ldk = DkE + 8, ldv = shared_v ? ldk : Dv + 8;
@@ -158,6 +158,35 @@ attention_wide_tc_kernel(const float* q, int ldq, int qhs, const int* __restrict
 
   // ---- queries: float32 -> hi + lo; with talk, the heads' queries mixed into the key heads' segments
   const int rows_used = nq * HG;                             // rows 0 .. rows_used - 1 carry a (token, head)
+  if (vec_q && !talk) {
+    // four columns an access and four accesses on their way together: one column at a time each store waited for its load
+    // (single rows of 32 heads of 288: 28.1 us a launch, LATENT_ROWS this way)
+    const int per_row = DkE / 4, n = rows_used * per_row;
+    for (int e0 = tid; e0 < n; e0 += 4 * THREADS) {
+      float4 v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int e = e0 + i * THREADS, r = e / per_row, col = (e - r * per_row) * 4;
+        v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (e < n && col < Dk) v[i] = *reinterpret_cast<const float4*>(q + (size_t)(t0 + r / HG) * ldq + (size_t)(h0 + r % HG) * qhs + col);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int e = e0 + i * THREADS, r = e / per_row, col = (e - r * per_row) * 4;
+        if (e >= n) continue;
+        const float f[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+        __nv_bfloat162 hi[2], lo[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          hi[j] = __floats2bfloat162_rn(f[2 * j], f[2 * j + 1]);
+          const float2 b = __bfloat1622float2(hi[j]);
+          lo[j] = __floats2bfloat162_rn(f[2 * j] - b.x, f[2 * j + 1] - b.y);
+        }
+        *reinterpret_cast<uint2*>(sQh + r * ldk + col) = *reinterpret_cast<const uint2*>(hi);
+        *reinterpret_cast<uint2*>(sQl + r * ldk + col) = *reinterpret_cast<const uint2*>(lo);
+      }
+    }
+  } else
   for (int e = tid; e < rows_used * DkE; e += THREADS) {
     const int r = e / DkE, col = e - r * DkE;
     const int tq = r / HG, h = h0 + r % HG;
@@ -365,6 +394,244 @@ attention_wide_tc_kernel(const float* q, int ldq, int qhs, const int* __restrict
   }
 }
 
+// Single rows whose scores are mixed across heads: a CTA takes a row with all its heads and `bps` blocks of 64 keys (0: all of
+// them), so that the scores of every head are made once (a product of a row's queries with its key head: the mixed queries above
+// are as many times wider as there are key heads, once for every group of heads) and mixed in float32 as scores.
+//   raw scores   warp w: keys 8 w .. of every key head; the A tile has the heads' high halves in rows 0-7, the low ones in rows 8-15
+//   mix          a thread a key and every fourth head
+//   softmax      a warp a head; weights rounded to bfloat16 and summed as rounded
+//   values       warp w: every eighth tile of 8 columns of all value heads
+// Bound by latency: loads, four phases and their barriers, then the merge.  4 rows of 32 heads of 64 at 400 positions: 111 us with
+// mixed queries (most of it the mixing, a column at a time), TALK_ROWS us this way with the merge.
+constexpr int TR_MAXH = 64, TR_ITEMS = 16;
+struct TalkRows { int ldq, ldk, ldv, ldp; long long smem; };
+static __host__ __device__ inline TalkRows talk_rows_layout(int Hq, int G, int Dk, int Dv) {
+  TalkRows l;
+  l.ldq = Dk + 8; l.ldk = G * Dk + 8; l.ldv = G * Dv + 8; l.ldp = TC_N + TC_PPAD;
+  l.smem = 4LL * Hq * Hq + 2LL * 4 * Hq * (TC_N + TC_SPAD) + 3LL * 4 * Hq + 2LL * G * 16 * (l.ldq + l.ldp) + 2LL * TC_N * (l.ldk + l.ldv);
+  return l;
+}
+template <typename TO>
+__global__ void __launch_bounds__(TC_THREADS)
+attention_talk_rows_kernel(const float* q, int ldq_g, int qhs, const int* __restrict__ tiles, const int* __restrict__ block_table,
+                           int max_pages, int n_pages, int page, int Hq, int G, int Dk, int Dv, int krs, int vrs, int window, int chunk,
+                           float scale, const float* __restrict__ talk, const __nv_bfloat16* k_pool, const __nv_bfloat16* v_pool,
+                           const __nv_bfloat16* gate, int ldg, TO* __restrict__ out, int ldo, int ohs, int* __restrict__ status, int bps,
+                           int n_rel, float* __restrict__ scratch, int keep_first, int gate_cols) {
+  extern __shared__ __align__(16) unsigned char tc_smem[];
+  const TalkRows L = talk_rows_layout(Hq, G, Dk, Dv);
+  constexpr int LS = TC_N + TC_SPAD;
+  float* sT = reinterpret_cast<float*>(tc_smem);                            // [Hq][Hq]
+  float* sS = sT + Hq * Hq;                                                 // [Hq][LS] raw scores
+  float* sX = sS + Hq * LS;                                                 // [Hq][LS] mixed scores
+  float* sM = sX + Hq * LS;                                                 // [Hq] running maximum, sum, correction
+  float* sL = sM + Hq;
+  float* sC = sL + Hq;
+  __nv_bfloat16* sQ = reinterpret_cast<__nv_bfloat16*>(sC + Hq);            // [G][16][ldq]
+  __nv_bfloat16* sP = sQ + G * 16 * L.ldq;                                  // [G][16][ldp]
+  __nv_bfloat16* sK = sP + G * 16 * L.ldp;                                  // [64][ldk]
+  __nv_bfloat16* sV = sK + TC_N * L.ldk;                                    // [64][ldv]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tq4 = lane & 3;
+  const int tile = blockIdx.x, rep = Hq / G;
+  if (tiles[4 * tile + 1] <= 0) return;
+  const int t = tiles[4 * tile], p = tiles[4 * tile + 3];
+  const int* bt = block_table + (size_t)tiles[4 * tile + 2] * max_pages;
+  int lo = 0;
+  if (window > 0 && p - window + 1 > lo) lo = p - window + 1;
+  if (chunk > 0 && (p / chunk) * chunk > lo) lo = (p / chunk) * chunk;
+  int p_max = p, j_first = (lo / TC_N) * TC_N, kept_end = min((min(keep_first, lo) + TC_N - 1) / TC_N * TC_N, j_first);
+  int j_start = kept_end > 0 ? 0 : j_first;
+  if (bps > 0) {      // the splits of the kernel above
+    const int kz = (kept_end / TC_N + bps - 1) / bps;
+    if ((int)blockIdx.z < kz) {
+      j_start = blockIdx.z * bps * TC_N;
+      p_max = min(kept_end, j_start + bps * TC_N) - 1;
+      kept_end = p_max + 1;
+      j_first = kept_end;
+    } else {
+      const int za = (lo / TC_N) / bps + (blockIdx.z - kz);
+      if (za * bps * TC_N > p_max) return;
+      j_first = max(j_first, za * bps * TC_N);
+      p_max = min(p_max, (za + 1) * bps * TC_N - 1);
+      kept_end = 0;
+      j_start = j_first;
+    }
+  }
+  for (int e = tid; e < Hq * Hq; e += TC_THREADS) sT[e] = talk[e];
+  for (int e = tid; e < Hq; e += TC_THREADS) { sM[e] = -INFINITY; sL[e] = 0.f; sC[e] = 0.f; }
+  pdl_wait();
+  pdl_trigger();
+  q = after_wait(q);
+  k_pool = after_wait(k_pool);
+  v_pool = after_wait(v_pool);
+  gate = after_wait(gate);
+  // a thread a piece of 16 bytes, zeros where the row does not see the key or a page is missing
+  auto load_tile = [&](__nv_bfloat16* dst, int ld, const __nv_bfloat16* pool, int width, int rs, int j0, bool report) {
+    const int per_head = width / 8, per_key = G * per_head;
+    for (int e = tid; e < TC_N * per_key; e += TC_THREADS) {
+      const int jj = e / per_key, x = e - jj * per_key, c = x / per_head, d = (x - c * per_head) * 8, j = j0 + jj;
+      const __nv_bfloat16* src = nullptr;
+      if ((j >= lo || j < keep_first) && j <= p_max) {
+        const int lp = j / page;
+        const int pg = lp < max_pages ? bt[lp] : -1;
+        if (pg >= 0 && pg < n_pages) src = pool + (((size_t)pg * G + c) * page + (j % page)) * rs + d;
+        else if (report) atomicOr(status, pg >= n_pages ? MLXB_ST_PAGE_RANGE : MLXB_ST_POSITION_RANGE);
+      }
+      __nv_bfloat16* to = dst + jj * ld + c * width + d;
+      if (src) cp_async16(to, src);
+      else *reinterpret_cast<uint4*>(to) = make_uint4(0u, 0u, 0u, 0u);
+    }
+  };
+  auto load_block = [&](int j0) {
+    load_tile(sK, L.ldk, k_pool, Dk, krs, j0, true);
+    load_tile(sV, L.ldv, v_pool, Dv, vrs, j0, false);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  load_block(j_start);
+  {
+    const float* qt = q + (size_t)t * ldq_g;
+    const int per_row = Dk / 4;
+    for (int e = tid; e < Hq * per_row; e += TC_THREADS) {
+      const int h = e / per_row, d = (e - h * per_row) * 4, c = h / rep, i = h - c * rep;
+      const float4 v = *reinterpret_cast<const float4*>(qt + (size_t)h * qhs + d);
+      const float f[4] = {v.x, v.y, v.z, v.w};
+      __nv_bfloat162 hi[2], lw[2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        hi[k] = __floats2bfloat162_rn(f[2 * k], f[2 * k + 1]);
+        const float2 b = __bfloat1622float2(hi[k]);
+        lw[k] = __floats2bfloat162_rn(f[2 * k] - b.x, f[2 * k + 1] - b.y);
+      }
+      *reinterpret_cast<uint2*>(sQ + (c * 16 + i) * L.ldq + d) = *reinterpret_cast<const uint2*>(hi);
+      *reinterpret_cast<uint2*>(sQ + (c * 16 + 8 + i) * L.ldq + d) = *reinterpret_cast<const uint2*>(lw);
+    }
+    // (rows of no head: what they give is not read)
+  }
+  float o[TR_ITEMS][2];
+#pragma unroll
+  for (int i = 0; i < TR_ITEMS; ++i) o[i][0] = o[i][1] = 0.f;
+  const int nv = Dv / 8, n_items = G * nv;
+  auto next_block = [&](int j0) { const int n = j0 + TC_N; return (n >= kept_end && n < j_first) ? j_first : n; };
+  for (int j0 = j_start; j0 <= p_max; j0 = next_block(j0)) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    for (int c = 0; c < G; ++c) {
+      float s[4] = {0.f, 0.f, 0.f, 0.f};
+      const unsigned kb = smem_addr(sK + (warp * 8 + (lane & 7)) * L.ldk + c * Dk + ((lane >> 3) & 1) * 8);
+      const unsigned qa = smem_addr(sQ + (c * 16 + (lane & 15)) * L.ldq + (lane >> 4) * 8);
+#pragma unroll 4
+      for (int k0 = 0; k0 < Dk; k0 += 16) {
+        unsigned a[4], b[2];
+        ldmatrix_x4(a, qa + k0 * 2);
+        ldmatrix_x2(b, kb + k0 * 2);
+        mma_bf16(s, a, b);
+      }
+      if (g < rep) {
+        float* d = sS + (c * rep + g) * LS + warp * 8 + tq4 * 2;
+        d[0] = (s[0] + s[2]) * scale;
+        d[1] = (s[1] + s[3]) * scale;
+      }
+    }
+    __syncthreads();
+    {
+      const int key = tid & 63, first = tid >> 6, j = j0 + key;
+      const bool sees = j <= p_max && (j >= lo || j < keep_first);
+      for (int h0 = first; h0 < Hq; h0 += 32) {      // heads h0, h0 + 4, .. h0 + 28
+        float acc[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+        for (int x = 0; x < Hq; x += 4) {
+          const float s0 = sS[x * LS + key], s1 = sS[(x + 1) * LS + key], s2 = sS[(x + 2) * LS + key], s3 = sS[(x + 3) * LS + key];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            if (h0 + 4 * i >= Hq) continue;
+            const float4 w = *reinterpret_cast<const float4*>(sT + (h0 + 4 * i) * Hq + x);
+            acc[i] = fmaf(w.x, s0, acc[i]);
+            acc[i] = fmaf(w.y, s1, acc[i]);
+            acc[i] = fmaf(w.z, s2, acc[i]);
+            acc[i] = fmaf(w.w, s3, acc[i]);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if (h0 + 4 * i < Hq) sX[(h0 + 4 * i) * LS + key] = sees ? acc[i] : -INFINITY;
+      }
+    }
+    __syncthreads();
+    for (int h = warp; h < Hq; h += TC_WARPS) {
+      const float s0 = sX[h * LS + lane], s1 = sX[h * LS + lane + 32], m_old = sM[h];
+      const float m_new = fmaxf(m_old, warp_max(fmaxf(s0, s1)));
+      const __nv_bfloat16 p0 = __float2bfloat16_rn(s0 == -INFINITY ? 0.f : expf(s0 - m_new));
+      const __nv_bfloat16 p1 = __float2bfloat16_rn(s1 == -INFINITY ? 0.f : expf(s1 - m_new));
+      const float sum = warp_sum(__bfloat162float(p0) + __bfloat162float(p1));
+      const int c = h / rep;
+      __nv_bfloat16* d = sP + (c * 16 + h - c * rep) * L.ldp;
+      d[lane] = p0;
+      d[lane + 32] = p1;
+      if (lane == 0) {
+        const float corr = m_old == -INFINITY ? 0.f : expf(m_old - m_new);
+        sM[h] = m_new;
+        sL[h] = sL[h] * corr + sum;
+        sC[h] = corr;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < TR_ITEMS; ++i) {
+      const int it = warp + i * TC_WARPS;
+      if (it >= n_items) continue;
+      const int c = it / nv, nt = it - c * nv;
+      float d[4] = {0.f, 0.f, 0.f, 0.f};
+      const unsigned pa = smem_addr(sP + (c * 16 + (lane & 15)) * L.ldp + (lane >> 4) * 8);
+      const unsigned vb = smem_addr(sV + (lane & 15) * L.ldv + c * Dv + nt * 8);
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) {
+        unsigned a[4], b[2];
+        ldmatrix_x4(a, pa + ks * 16 * 2);
+        ldmatrix_x2_trans(b, vb + ks * 16 * L.ldv * 2);
+        mma_bf16(d, a, b);
+      }
+      const float corr = g < rep ? sC[c * rep + g] : 0.f;
+      o[i][0] = fmaf(o[i][0], corr, d[0]);
+      o[i][1] = fmaf(o[i][1], corr, d[1]);
+    }
+    if (next_block(j0) <= p_max) {
+      __syncthreads();                                       // everybody is done with the tiles before they are refilled
+      load_block(next_block(j0));
+    }
+  }
+  __syncthreads();
+  const size_t stride = (size_t)Dv + 2;
+  float* part = scratch + ((size_t)tile * Hq * n_rel + blockIdx.z) * stride;      // [head] n_rel * stride apart
+  if (bps > 0)
+    for (int h = tid; h < Hq; h += TC_THREADS) {
+      part[(size_t)h * n_rel * stride + Dv] = sM[h];
+      part[(size_t)h * n_rel * stride + Dv + 1] = sL[h];
+    }
+#pragma unroll
+  for (int i = 0; i < TR_ITEMS; ++i) {
+    const int it = warp + i * TC_WARPS;
+    if (it >= n_items || g >= rep) continue;
+    const int c = it / nv, col = (it - c * nv) * 8 + tq4 * 2, h = c * rep + g;
+    if (bps > 0) {
+      float* sp = part + (size_t)h * n_rel * stride + col;
+      sp[0] = o[i][0];
+      sp[1] = o[i][1];
+      continue;
+    }
+    const float l = sL[h], f = l > 0.f ? 1.f / l : 0.f;
+    float g0 = 1.f, g1 = 1.f;
+    if (gate) {
+      const __nv_bfloat16* gp = gate + (size_t)t * ldg + (gate_cols ? (size_t)h * Dv + col : (size_t)h);
+      g0 = 1.f / (1.f + expf(-__bfloat162float(gp[0])));
+      g1 = gate_cols ? 1.f / (1.f + expf(-__bfloat162float(gp[1]))) : g0;
+    }
+    TO* op = out + (size_t)t * ldo + (size_t)h * ohs + col;
+    op[0] = from_f<TO>(o[i][0] * f * g0);
+    op[1] = from_f<TO>(o[i][1] * f * g1);
+  }
+}
+
 // The partial results of a single row's splits, merged in the order of the splits: one block per (tile, head).
 template <typename TO>
 __global__ void attention_wide_merge_kernel(const int* __restrict__ tiles, int Hq, int Dv, int window, int chunk, int bps,
@@ -477,6 +744,38 @@ MLXB_EXPORT int mlxb_attention_wide_tc_supported(int Hq, int Hkv, int Dk, int Dv
   return tc_plan(Hq, Hkv, Dk, Dv, krs, vrs, talk, shared_v, false, &p) ? 1 : 0;
 }
 
+// Whether the kernel of mixed single rows takes these sizes: up to 8 heads a key head (a tile of 16 rows has their halves), whole
+// tiles of 16 query and 8 value columns, tiles that fit the shared memory.
+static bool talk_rows_take(const float* q, int ldq, int qhs, int Hq, int Hkv, int Hv, int Dk, int Dv, int krs, int vrs, float softcap) {
+  return Hq > 0 && Hkv > 0 && Hq % Hkv == 0 && Hv == Hkv && softcap <= 0.f && Hq <= TR_MAXH && Hq % 4 == 0 && Hq / Hkv <= 8 && Dk % 16 == 0 &&
+         Dv % 8 == 0 && krs >= Dk && vrs >= Dv && krs % 8 == 0 && vrs % 8 == 0 && Hkv * Dv <= 8 * TC_WARPS * TR_ITEMS && ldq % 4 == 0 &&
+         qhs % 4 == 0 && ((uintptr_t)q & 15) == 0 && talk_rows_layout(Hq, Hkv, Dk, Dv).smem <= 220 * 1024;
+}
+template <typename TO>
+static int launch_talk_rows(const float* q, int ldq, int qhs, const int* tiles, int n_tiles, const int* block_table, int max_pages,
+                            int n_pages, int page, int Hq, int Hkv, int Dk, int Dv, int krs, int vrs, int window, int chunk, float scale,
+                            const float* talk, const void* k_pool, const void* v_pool, const void* gate, int ldg, void* out, int ldo,
+                            int ohs, int* status, float* scratch, int max_len, int keep_first, int gate_cols, cudaStream_t stream) {
+  // rows that can see more than a few blocks of keys are always split: what a row gives does not depend on how many there are
+  const bool split = scratch != nullptr && tc_splits_rows(window, chunk, max_len, keep_first);
+  const int n_rel = tc_splits(window, chunk, max_len, keep_first), bps = split ? TC_BPS : 0;
+  const long long smem = talk_rows_layout(Hq, Hkv, Dk, Dv).smem;
+  auto kern = attention_talk_rows_kernel<TO>;
+  static SharedLimit limit;
+  const cudaError_t e = limit.raise(kern, 220 * 1024);
+  if (e != cudaSuccess)
+    return mlxb_fail((int)e, "attention (wide, mixed rows): %lld bytes of shared memory: %s", smem, cudaGetErrorString(e));
+  launch_pdl(kern, dim3(n_tiles, 1, split ? n_rel : 1), dim3(TC_THREADS), (size_t)smem, stream, q, ldq, qhs, tiles, block_table, max_pages,
+             n_pages, page, Hq, Hkv, Dk, Dv, krs, vrs, window, chunk, scale, talk, (const __nv_bfloat16*)k_pool,
+             (const __nv_bfloat16*)v_pool, (const __nv_bfloat16*)gate, ldg, (TO*)out, ldo, ohs, status, bps, n_rel, scratch, keep_first,
+             gate_cols);
+  if (int rc = mlxb_check_launch("attention (wide, mixed rows)")) return rc;
+  if (split)
+    launch_pdl(attention_wide_merge_kernel<TO>, dim3(n_tiles, Hq), dim3(Dv >= 128 ? 128 : 64), 0, stream, tiles, Hq, Dv, window, chunk, bps,
+               n_rel, (const float*)scratch, (const __nv_bfloat16*)gate, ldg, (TO*)out, ldo, ohs, keep_first, gate_cols);
+  return mlxb_check_launch("attention (wide, mixed rows)");
+}
+
 // The arguments of mlxb_attention_wide with bfloat16 pools, and instead of the token rows a list of tiles: int32
 // [n_tiles, 4] = (first token row, queries, block-table row, first position), each of at most tile_q queries.  Hv: heads
 // of v_pool (0: Hkv); with fewer, key heads c * Hkv/Hv .. read value head c.
@@ -492,12 +791,20 @@ MLXB_EXPORT int mlxb_attention_wide_tc(int out_f32, const float* q, int ldq, int
     return mlxb_fail(MLXB_BAD_ARG, "attention (wide, tensor cores): %d key heads over %d value heads", Hkv, Hv);
   TcPlan pl;
   const int shared_v = v_pool == k_pool;
+  if (window <= 0) keep_first = 0;           // without a window every earlier position is visible anyway
+  if (talk && tile_q == 1 && !shared_v && page > 0 && (page & (page - 1)) == 0 && qhs >= Dk && ohs >= Dv &&
+      talk_rows_take(q, ldq, qhs, Hq, Hkv, Hv, Dk, Dv, krs, vrs, softcap))
+    return out_f32 ? launch_talk_rows<float>(q, ldq, qhs, tiles, n_tiles, block_table, max_pages, n_pages, page, Hq, Hkv, Dk, Dv, krs, vrs,
+                                             window, chunk, scale, talk, k_pool, v_pool, gate, ldg, out, ldo, ohs, status, scratch, max_len,
+                                             keep_first, gate_cols, stream)
+                   : launch_talk_rows<__nv_bfloat16>(q, ldq, qhs, tiles, n_tiles, block_table, max_pages, n_pages, page, Hq, Hkv, Dk, Dv,
+                                                     krs, vrs, window, chunk, scale, talk, k_pool, v_pool, gate, ldg, out, ldo, ohs, status,
+                                                     scratch, max_len, keep_first, gate_cols, stream);
   if (!tc_plan(Hq, Hkv, Dk, Dv, krs, vrs, talk != nullptr, shared_v, tile_q > 1, &pl) || page <= 0 || (page & (page - 1)) ||
       tile_q <= 0 || qhs < Dk || ohs < Dv)
     return mlxb_fail(MLXB_BAD_ARG, "attention (wide, tensor cores): %d/%d heads, sizes %d/%d in rows of %d/%d", Hq, Hkv,
                      Dk, Dv, krs, vrs);
   // single rows with scratch memory: their keys split over grid.z, then merged
-  if (window <= 0) keep_first = 0;           // without a window every earlier position is visible anyway
   const int n_rel = tc_splits(window, chunk, max_len, keep_first);
   // (only while the rows alone leave SMs idle: with more CTAs than SMs a split adds work and nothing else; a row's
   // result is the same up to the rounding of the merge either way)
@@ -506,6 +813,7 @@ MLXB_EXPORT int mlxb_attention_wide_tc(int out_f32, const float* q, int ldq, int
   const int subs = (tile_q + TQ - 1) / TQ;
   const int bps = split ? TC_BPS : 0;
   const long long smem = pl.smem;
+  const int vec_q = Dk % 4 == 0 && ldq % 4 == 0 && qhs % 4 == 0 && ((uintptr_t)q & 15) == 0;
   const dim3 grid((unsigned)n_tiles * subs, Hq / pl.HG, split ? n_rel : 1), block(TC_THREADS * pl.MP);
 #define TCW_GO(TO, MPV)                                                                                                \
   do {                                                                                                                 \
@@ -519,7 +827,7 @@ MLXB_EXPORT int mlxb_attention_wide_tc(int out_f32, const float* q, int ldq, int
     launch_pdl(kern, grid, block, (size_t)smem, stream, q, ldq, qhs, tiles, subs, TQ, pl.HG, block_table, max_pages,   \
                n_pages, page, Hq, Hkv, Dk, Dv, pl.DkE, pl.seg, pl.n_seg, krs, vrs, shared_v, window, chunk, scale, talk, \
                (const __nv_bfloat16*)k_pool, (const __nv_bfloat16*)v_pool, (const __nv_bfloat16*)gate, ldg, (TO*)out,  \
-               ldo, ohs, status, bps, n_rel, scratch, pl.nbuf, softcap, keep_first, gate_cols, Hv);                        \
+               ldo, ohs, status, bps, n_rel, scratch, pl.nbuf, softcap, keep_first, gate_cols, Hv, vec_q);                 \
     if (split) {                                                                                                       \
       if (int e = mlxb_check_launch("attention (wide, tensor cores)")) return e;                                       \
       launch_pdl(attention_wide_merge_kernel<TO>, dim3(n_tiles, Hq), dim3(Dv >= 128 ? 128 : 64), 0, stream, tiles, Hq, \
