@@ -428,7 +428,7 @@ attention_rows_kernel(const __nv_bfloat16* __restrict__ q, int ldq, const int4* 
                       const int* __restrict__ block_table, int max_pages, int n_pages, int page, int Hq, int Hkv,
                       int window, float scale_log2e, const __nv_bfloat16* __restrict__ k_pool,
                       const __nv_bfloat16* __restrict__ v_pool, __nv_bfloat16* __restrict__ out, int ldo,
-                      int* __restrict__ status, const float* __restrict__ sinks) {
+                      int* __restrict__ status, const float* __restrict__ sinks, bool beside) {
   constexpr int THREADS = RW * 32;
   constexpr int STRIDE = DH + 8;              // elements per shared-memory row (16 bytes of padding)
   constexpr int KS = DH / 16;                 // k steps of q K^T
@@ -442,6 +442,7 @@ attention_rows_kernel(const __nv_bfloat16* __restrict__ q, int ldq, const int4* 
   __nv_bfloat16* sv = sk + RS * BKV * STRIDE;                        // [RS][BKV][STRIDE]
 
   pdl_trigger();
+  const WaitAtEnd end{beside && last_block_thread()};      // beside the portions' kernel, which was launched before this one
   const int4 tile = tiles[blockIdx.x];        // the step's inputs: no kernel writes them
   const int row = tile.x, req = tile.z, pos = tile.w;
   if (tile.y <= 0) return;                    // a row that pads the step
@@ -489,7 +490,8 @@ attention_rows_kernel(const __nv_bfloat16* __restrict__ q, int ldq, const int4* 
     load_block(kb_lo + issued, issued);
     ++issued;
   }
-  pdl_wait();
+  if (beside) __threadfence();
+  else pdl_wait();
   q = after_wait(q);
   k_pool = after_wait(k_pool);
   v_pool = after_wait(v_pool);
@@ -502,8 +504,8 @@ attention_rows_kernel(const __nv_bfloat16* __restrict__ q, int ldq, const int4* 
 #pragma unroll
     for (int ks = 0; ks < KS; ++ks) {
       const int d = ks * 16 + 2 * qd;
-      qa[ks][0] = g == 0 ? *reinterpret_cast<const unsigned*>(qr + d) : 0u;
-      qa[ks][2] = g == 0 ? *reinterpret_cast<const unsigned*>(qr + d + 8) : 0u;
+      qa[ks][0] = g == 0 ? __ldcg(reinterpret_cast<const unsigned*>(qr + d)) : 0u;
+      qa[ks][2] = g == 0 ? __ldcg(reinterpret_cast<const unsigned*>(qr + d + 8)) : 0u;
       qa[ks][1] = qa[ks][3] = 0u;
     }
   }
@@ -615,7 +617,7 @@ attention_rows_kernel(const __nv_bfloat16* __restrict__ q, int ldq, const int4* 
 template <int DH, int RW, int RS>
 static int launch_rows(const void* q, int ldq, const int* tiles, int n_tiles, const int* block_table, int max_pages,
                        int n_pages, int page, int Hq, int Hkv, int window, float scale, const void* k_pool,
-                       const void* v_pool, void* out, int ldo, int* status, cudaStream_t stream, const float* sinks) {
+                       const void* v_pool, void* out, int ldo, int* status, cudaStream_t stream, const float* sinks, bool beside) {
   const size_t smem = (size_t)RS * 2 * BKV * (DH + 8) * sizeof(__nv_bfloat16);    // (the merge needs far less)
   auto kern = attention_rows_kernel<DH, RW, RS>;
   static bool raised = false;
@@ -625,7 +627,7 @@ static int launch_rows(const void* q, int ldq, const int* tiles, int n_tiles, co
   }
   launch_pdl(kern, dim3(n_tiles, Hq), dim3(RW * 32), smem, stream, (const __nv_bfloat16*)q, ldq, (const int4*)tiles,
              block_table, max_pages, n_pages, page, Hq, Hkv, window, scale * 1.4426950408889634f,
-             (const __nv_bfloat16*)k_pool, (const __nv_bfloat16*)v_pool, (__nv_bfloat16*)out, ldo, status, sinks);
+             (const __nv_bfloat16*)k_pool, (const __nv_bfloat16*)v_pool, (__nv_bfloat16*)out, ldo, status, sinks, beside);
   return mlxb_check_launch("attention (single rows)");
 }
 
@@ -634,7 +636,7 @@ static int launch_rows(const void* q, int ldq, const int* tiles, int n_tiles, co
 MLXB_EXPORT int mlxb_attention_rows(const void* q, int ldq, const int* tiles, int n_tiles, const int* block_table,
                                     int max_pages, int n_pages, int page, int Hq, int Hkv, int Dh, int window,
                                     float scale, const void* k_pool, const void* v_pool, void* out, int ldo,
-                                    int* status, const float* sinks, cudaStream_t stream) {
+                                    int* status, const float* sinks, int beside, cudaStream_t stream) {
   if (n_tiles <= 0) return 0;
   if (page <= 0 || (page & (page - 1))) return mlxb_fail(MLXB_BAD_ARG, "attention (single rows): page size %d", page);
   if (Hkv <= 0 || Hq <= 0 || Hq % Hkv || Hq > 65535)
@@ -644,7 +646,7 @@ MLXB_EXPORT int mlxb_attention_rows(const void* q, int ldq, const int* tiles, in
 #define GO(D)                                                                                                         \
   case D:                                                                                                             \
     return launch_rows<D, 4, (D <= 64 ? 3 : 2)>(q, ldq, tiles, n_tiles, block_table, max_pages, n_pages, page, Hq,    \
-                                                Hkv, window, scale, k_pool, v_pool, out, ldo, status, stream, sinks)
+                                                Hkv, window, scale, k_pool, v_pool, out, ldo, status, stream, sinks, beside != 0)
   switch (Dh) {
     GO(16); GO(32); GO(48); GO(64); GO(80); GO(96); GO(112); GO(128);
     default:

@@ -155,7 +155,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                             const int* __restrict__ block_table, int max_pages, int n_pages, int page, int Hq, int Hkv,
                             int window, float scale_log2e, __nv_bfloat16* out, int ldo, int* __restrict__ status,
                             const float* __restrict__ sinks, int keep_first, float softcap,
-                            const __nv_bfloat16* gate, int ldg, int Hv, int VS, int out_f32) {
+                            const __nv_bfloat16* gate, int ldg, int Hv, int VS, int out_f32, bool beside) {
   extern __shared__ uint8_t smem_raw[];
   AtSmem& sm = *reinterpret_cast<AtSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -199,7 +199,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = sm.tmem_base;
   volatile int* abort_flag = &sm.abort_flag;
-  pdl_trigger();
+  if (!beside) pdl_trigger();      // (else after the wait: the kernel that is launched next runs beside this one, see WaitAtEnd)
 
   if (warp == MMA_WARP) {
     // The whole warp takes part in the loads: lane s looks up the page of slot s of a block (one round of
@@ -237,6 +237,10 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     int pg_next = page_of(kb_at(1));      // pages of block i + 1 (for V), one further ahead for K
     int pg_after = page_of(kb_at(2));
     pdl_wait();   // queries, keys and values of this step come from the kernel before; tiles and block table do not
+    if (beside) {
+      __threadfence();
+      pdl_trigger();
+    }
     if (elect_one()) {
       mbar_expect_tx(&sm.q_full, TQ * HD * (uint32_t)sizeof(__nv_bfloat16));
       tma_load_2d(sm.q, &map_q, h * HD, row0, &sm.q_full);
@@ -473,13 +477,14 @@ static int make_map(CUtensorMap* map, const void* base, long long rows, int cols
 // (tiles of at most 128 queries; a tile of 0 queries is skipped); pools [n_pages, Hkv, page, 64], page a power of two from 8 to 128.
 // Hv, Dv (0: Hkv, 64): the value pool is [n_pages, Hv, page, Dv] with Hv a divisor of Hkv (key heads c * Hkv/Hv .. read
 // value head c: several score maps over the same values) and Dv a multiple of 64; a CTA then takes one slice of 64
-// value columns (the scores are formed once per slice) and out is [*, Hq*Dv].  out_f32: out is float32.
+// value columns (the scores are formed once per slice) and out is [*, Hq*Dv].  out_f32: out is float32.  beside: the launch that
+// follows is that of the single rows with `beside`.
 MLXB_EXPORT int mlxb_attention_prefill_tc(const void* q, int ldq, int n_tokens, const int* tiles, int n_tiles,
                                           const int* block_table, int max_pages, int n_pages, int page, int Hq,
                                           int Hkv, int Dh, int window, float scale, const void* k_pool,
                                           const void* v_pool, void* out, int ldo, int* status, const float* sinks,
                                           int keep_first, float softcap, const void* gate, int ldg, int Hv, int Dv,
-                                          int out_f32, cudaStream_t stream) {
+                                          int out_f32, int beside, cudaStream_t stream) {
   if (n_tiles <= 0) return 0;
   if (Hv <= 0) Hv = Hkv;
   if (Dv <= 0) Dv = HD;
@@ -513,6 +518,6 @@ MLXB_EXPORT int mlxb_attention_prefill_tc(const void* q, int ldq, int n_tokens, 
   launch_pdl(attention_prefill_tc_kernel, dim3(n_tiles, Hq * VS), dim3(AT_THREADS), smem, stream, mq, mk, mv,
              (const int4*)tiles, block_table, max_pages, n_pages, page, Hq, Hkv, window,
              scale * 1.4426950408889634f, (__nv_bfloat16*)out, ldo, status, sinks, window > 0 ? keep_first : 0, softcap,
-             (const __nv_bfloat16*)gate, ldg, Hv, VS, out_f32);
+             (const __nv_bfloat16*)gate, ldg, Hv, VS, out_f32, beside != 0);
   return mlxb_check_launch("attention (portions, tcgen05)");
 }

@@ -63,6 +63,19 @@ static inline int mlxb_check_launch(const char* what) {
 // attribute off (every kernel then starts after its predecessor has finished, as usual).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Two kernels that do not depend on each other, one launched right after the other, can run side by side: the first lets its dependents go
+// only after its own wait (every block: the kernel before both is then finished), the second does not wait where it starts but
+// where it ends, in one thread of its grid, so that it is not finished before the first is (what comes next waits for the second).
+// What the kernel before both wrote the second reads past L1.
+struct WaitAtEnd {
+  bool on;
+  __device__ __forceinline__ ~WaitAtEnd() {
+    if (on) pdl_wait();
+  }
+};
+__device__ __forceinline__ bool last_block_thread() {
+  return threadIdx.x == 0 && blockIdx.x + 1 == gridDim.x && blockIdx.y + 1 == gridDim.y && blockIdx.z + 1 == gridDim.z;
+}
 // A pointer to memory the predecessor writes, as seen after pdl_wait().  A `const __restrict__` parameter
 // promises the compiler that nobody writes the memory while the kernel runs, which would allow it to move
 // a load through such a pointer up into the code before the wait; passing the pointer through this (empty)

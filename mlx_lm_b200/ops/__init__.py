@@ -641,7 +641,7 @@ PREFILL_TC = _os.environ.get("MLXB_PREFILL_TC", "1") != "0"         # heads of 6
 
 _PRE_TC_ARGS = [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                 c_float, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_float, c_void_p, c_int, c_int, c_int,
-                c_int, c_void_p]
+                c_int, c_int, c_void_p]
 
 
 def attention_portions_supported(dtype, head_dim: int, scale: float = 1.0) -> bool:
@@ -663,7 +663,7 @@ def attention_portions_tc_supported(q, out, k_pool, v_pool, tile_rows: int = 0) 
 
 def attention_portions(q, tiles, n_tiles: int, block_table, k_pool, v_pool, out, n_heads: int, scale: float,
                        window: int, status, stream, tile_rows: int = 0, sinks=None, first_positions=None,
-                       keep_first: int = 0, softcap: float = 0.0, gate=None) -> None:
+                       keep_first: int = 0, softcap: float = 0.0, gate=None, beside: bool = False) -> None:
     """Causal attention of prompt portions on tensor cores (bfloat16, csrc/attention_prefill.cu).
     ``keep_first``, ``softcap``, ``gate`` (bfloat16 ``[T, n_heads * 64]``, a sigmoid gate per output column): options of
     the tcgen05 kernel only (``attention_portions_tc_supported``).  So are a value pool with fewer heads than the key
@@ -673,7 +673,8 @@ def attention_portions(q, tiles, n_tiles: int, block_table, k_pool, v_pool, out,
     ``tiles``: int32 device tensor ``[n_tiles, 4]``: first token row of the tile, queries in it (1..64),
     block-table row of its request, position of its first query.  ``first_positions``: int32, per block-table
     row the first position this step brings for that request; with it the kernel fetches keys older than the
-    step before it waits for the kernel that wrote this step's."""
+    step before it waits for the kernel that wrote this step's.  ``beside`` (tcgen05 kernel): the launch that follows is
+    ``attention_rows`` or ``attention_decode`` of other rows with ``beside``, and runs beside this one."""
     if first_positions is not None:
         _need(first_positions, torch.int32, "attention_portions first_positions")
         if first_positions.numel() < block_table.shape[0]:
@@ -705,8 +706,10 @@ def attention_portions(q, tiles, n_tiles: int, block_table, k_pool, v_pool, out,
               n_tiles, _p(block_table), block_table.shape[1], n_pages, page, n_heads, Hkv, Dh, window, scale,
               _p(k_pool), _p(v_pool), _p(out), ldo, _p(status), _sinks(sinks, n_heads, "attention_portions"),
               int(keep_first or 0), float(softcap or 0.0), _p(gate), _rows(gate, "attention gate") if gate is not None else 0,
-              Hv, Dv, int(out.dtype == torch.float32), stream)
+              Hv, Dv, int(out.dtype == torch.float32), int(beside), stream)
         return
+    if beside:
+        raise KernelError("attention_portions: only the tcgen05 kernel has others run beside it")
     if keep_first or softcap or gate is not None:
         raise KernelError("attention_portions: kept first positions, a cap and a gate are options of the tcgen05 kernel")
     _call("attention_prefill", "mlxb_attention_prefill", _PRE_ARGS, _p(q), _rows(q, "attention q"), _p(tiles), n_tiles,
@@ -716,7 +719,7 @@ def attention_portions(q, tiles, n_tiles: int, block_table, k_pool, v_pool, out,
 
 
 _ROWS_ARGS = [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float,
-              c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p]
+              c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p]
 
 
 # (row, head) pairs from which single-token rows run on the tensor-core kernel: about seven times the number
@@ -742,22 +745,23 @@ def sm_count() -> int:
 
 
 def attention_rows(q, tiles, n_rows: int, block_table, k_pool, v_pool, out, n_heads: int, scale: float, window: int,
-                   status, stream, sinks=None) -> None:
+                   status, stream, sinks=None, beside: bool = False) -> None:
     """Attention of rows with a single query each (decode steps) on tensor cores (bfloat16,
     csrc/attention_prefill.cu): ``tiles`` is an int32 device tensor ``[n_rows, 4]`` = (token row, 1, block-table
-    row, position), or (token row, 0, 0, 0) for a padding row."""
+    row, position), or (token row, 0, 0, 0) for a padding row.  ``beside``: as in ``attention_decode``."""
     n_pages, Hkv, page, Dh = _attn_shapes(q, out, k_pool, n_heads, "attention_rows")
     _need(tiles, torch.int32, "attention_rows tiles")
     if tiles.numel() < 4 * n_rows:
         raise KernelError(f"attention_rows: {tiles.numel()} integers for {n_rows} rows")
     _call("attention_prefill", "mlxb_attention_rows", _ROWS_ARGS, _p(q), _rows(q, "attention q"), _p(tiles), n_rows,
           _p(block_table), block_table.shape[1], n_pages, page, n_heads, Hkv, Dh, window, scale, _p(k_pool),
-          _p(v_pool), _p(out), _rows(out, "attention out"), _p(status), _sinks(sinks, n_heads, "attention_rows"), stream)
+          _p(v_pool), _p(out), _rows(out, "attention out"), _p(status), _sinks(sinks, n_heads, "attention_rows"),
+          int(beside), stream)
 
 
 _DEC_ARGS = [c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
              c_int, c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p,
-             c_void_p, c_void_p]
+             c_void_p, c_int, c_void_p]
 
 DECODE_CHUNK = 1024   # key positions per CTA of the single-token attention kernel: a constant, never a function of the batch
 
@@ -769,11 +773,13 @@ def attention_decode_scratch(n_rows: int, n_heads: int, head_dim: int, max_len: 
 
 def attention_decode(q, positions, token_req, block_table, k_pool, v_pool, out, n_heads: int, scale: float,
                      window: int, scratch, counters, max_len: int, status, stream, rows=None,
-                     chunk: int = DECODE_CHUNK, sinks=None) -> None:
+                     chunk: int = DECODE_CHUNK, sinks=None, beside: bool = False) -> None:
     """Attention for rows with a single query each (decode steps): keys are cut into chunks of ``chunk``
     positions, one CTA per (chunk, head, row) writes a partial result to ``scratch`` (float32, at least
     ``attention_decode_scratch(...)`` elements) and the CTA that finishes last for a (row, head) combines
-    them.  ``counters``: int32, at least rows x heads, zero before the first call (every call leaves it zero)."""
+    them.  ``counters``: int32, at least rows x heads, zero before the first call (every call leaves it zero).
+    ``beside``: the launch before was ``attention_portions`` with ``beside`` over the same queries, and these rows do not
+    wait for it."""
     n_pages, Hkv, page, Dh = _attn_shapes(q, out, k_pool, n_heads, "attention_decode")
     n = q.shape[0] if rows is None else rows.numel()
     n_chunks = (max_len + chunk - 1) // chunk
@@ -785,7 +791,7 @@ def attention_decode(q, positions, token_req, block_table, k_pool, v_pool, out, 
     _call("attention", "mlxb_attention_decode", _DEC_ARGS, dtype_code(k_pool.dtype), _p(q), _rows(q, "attention q"),
           _p(rows), _p(positions), _p(token_req), _p(block_table), block_table.shape[1], n_pages, page, n_heads, Hkv,
           Dh, window, scale, _p(k_pool), _p(v_pool), _p(scratch), _p(counters), n_chunks, chunk, _p(out),
-          _rows(out, "attention out"), n, _p(status), _sinks(sinks, n_heads, "attention_decode"), stream)
+          _rows(out, "attention out"), n, _p(status), _sinks(sinks, n_heads, "attention_decode"), int(beside), stream)
 
 
 # --------------------------------------------------------------------------

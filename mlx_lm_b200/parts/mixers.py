@@ -96,22 +96,31 @@ def paged_attention(ctx, q, cache, o, n_heads: int, head_dim: int, scale: float,
     of ``o``.  ``sinks``: float32 ``[n_heads]``, one more term of each head's softmax denominator, or None."""
     window = window or 0
     single_tiles = getattr(ctx, "single_tiles", None)
+    portions = (ctx.n_portion and ctx.portion_tiles is not None
+                and ops.attention_portions_supported(q.dtype, head_dim, scale))
+    # rows and portions know nothing of each other: where the portions' kernel lets them, the rows run beside it
+    beside = bool(portions and ctx.n_single and ops.attention_portions_tc_supported(q, o, cache.k, cache.v))
+
+    def in_portions() -> None:
+        ops.attention_portions(q, ctx.portion_tiles, ctx.n_portion_tiles, cache.block_table, cache.k, cache.v, o, n_heads, scale,
+                               window, ctx.status, ctx.stream, sinks=sinks, first_positions=ctx.req_first_position, beside=beside)
+
+    if beside:
+        in_portions()
     if (ctx.n_single and single_tiles is not None
             and ops.attention_rows_supported(q.dtype, head_dim, ctx.n_single, n_heads, scale)):
         ops.attention_rows(q, single_tiles, ctx.n_single, cache.block_table, cache.k, cache.v, o, n_heads,
-                           scale, window, ctx.status, ctx.stream, sinks=sinks)
+                           scale, window, ctx.status, ctx.stream, sinks=sinks, beside=beside)
     elif ctx.n_single:
         scratch = ctx.ws.flat("attn_partial", ops.attention_decode_scratch(
             ctx.n_single, n_heads, head_dim, ctx.max_len), torch.float32)
         counters = ctx.ws.flat("attn_tickets", ctx.n_single * n_heads, torch.int32)
         ops.attention_decode(q, ctx.positions, ctx.token_req, cache.block_table, cache.k, cache.v, o,
                              n_heads, scale, window, scratch, counters, ctx.max_len, ctx.status,
-                             ctx.stream, rows=ctx.single_rows, sinks=sinks)
-    if ctx.n_portion:
-        if ops.attention_portions_supported(q.dtype, head_dim, scale) and ctx.portion_tiles is not None:
-            ops.attention_portions(q, ctx.portion_tiles, ctx.n_portion_tiles, cache.block_table, cache.k,
-                                   cache.v, o, n_heads, scale, window, ctx.status, ctx.stream, sinks=sinks,
-                                   first_positions=ctx.req_first_position)
+                             ctx.stream, rows=ctx.single_rows, sinks=sinks, beside=beside)
+    if ctx.n_portion and not beside:
+        if portions:
+            in_portions()
         elif (cache.v.shape == cache.k.shape and ops.attention_portions_f32_supported(q, cache.k, ctx.portion_tiles)
               and ctx.attention_in_tiles((n_heads, head_dim, window))):
             ops.attention_portions_f32(q, ctx.portion_tiles, ctx.n_portion_tiles, cache.block_table, cache.k, cache.v, o,
