@@ -35,6 +35,7 @@ constexpr int MMA_WARP = SOFT_WARPS, LOAD_WARP = SOFT_WARPS + 1;
 constexpr int THREADS = SOFT_THREADS + 64;
 constexpr int MAX_SLOTS = 20;
 constexpr int Q_CHUNK = M * 64 * 2, SLOT = KB * 64 * 2;      // bytes of 64 columns of the queries, of a block's keys or values
+constexpr int MAX_MIX = 512;                        // numbers of the mixing matrix that a CTA keeps
 constexpr int STALE = 8;                            // powers of two that a row's maximum may grow before O is scaled
 
 struct Control {
@@ -43,6 +44,7 @@ struct Control {
   uint64_t x_full[4];                               // exchange between the two warps of the same rows
   uint64_t drained;                                 // abort path only
   float row_max[2][2][M];                           // [block & 1][half][row]
+  float talk[MAX_MIX];                              // the mixing matrix's rows of the CTA's heads
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -56,7 +58,7 @@ struct WideArgs {
   void* out;
   int* status;
   int ldq, qhs, subs, n_tiles, max_pages, n_pages, page, Hq, Hkv, Hv, Dk, Dv, window, chunk, ldg, ldo, ohs, keep_first, gate_cols;
-  int HG, steps, chunks, v_chunks, lo_tmem, slots, shared_v, tmem_cols, vec_out;
+  int HG, steps, chunks, v_chunks, lo_tmem, slots, shared_v, tmem_cols, vec_out, mix_fast;
   float scale, softcap;
 };
 
@@ -152,6 +154,8 @@ attention_wide_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const _
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_v) : "memory");
   }
+  if (a.mix_fast)
+    for (int e = threadIdx.x; e < HG * a.Hq; e += THREADS) sm.talk[e] = a.talk[h0 * a.Hq + e];
   if (warp == MMA_WARP) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem_base)),
                  "r"(a.tmem_cols) : "memory");
@@ -174,25 +178,7 @@ attention_wide_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const _
       const int n_c = min(room, a.chunks - c0), per_row = n_c * 16;
       if (c0 > 0) __syncthreads();
       if (threadIdx.x < SOFT_THREADS) {
-#pragma unroll 4
-        for (int e = threadIdx.x; e < M * per_row; e += SOFT_THREADS) {
-          const int r = e / per_row, col = c0 * 64 + (e - r * per_row) * 4;
-          const int tq = r >> hg_shift, h = h0 + (r & (HG - 1));
-          float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (tq < nq) {
-            const float* qt = q + (size_t)(t0 + tq) * a.ldq;
-            if (a.talk != nullptr) {
-              const int c = col / a.Dk, d = col - c * a.Dk;
-              if (c < a.Hkv)
-                for (int i = 0; i < rep; ++i) {
-                  const float w = __ldg(a.talk + h * a.Hq + c * rep + i);
-                  const float4 u = *reinterpret_cast<const float4*>(qt + (size_t)(c * rep + i) * a.qhs + d);
-                  v.x = fmaf(w, u.x, v.x); v.y = fmaf(w, u.y, v.y); v.z = fmaf(w, u.z, v.z); v.w = fmaf(w, u.w, v.w);
-                }
-            } else if (col < a.Dk) {
-              v = *reinterpret_cast<const float4*>(qt + (size_t)h * a.qhs + col);
-            }
-          }
+        auto put = [&](int r, int col, const float4& v) {      // four columns of a row, as halves
           const float f[4] = {v.x, v.y, v.z, v.w};
           __nv_bfloat162 hi[2], lo[2];
 #pragma unroll
@@ -206,6 +192,75 @@ attention_wide_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const _
           *reinterpret_cast<uint2*>(s_hi + j * Q_CHUNK + at) = *reinterpret_cast<const uint2*>(hi);
           uint8_t* dst = j < a.lo_tmem ? ring + (j - c0) * Q_CHUNK : s_lo + (j - a.lo_tmem) * Q_CHUNK;
           *reinterpret_cast<uint2*>(dst + at) = *reinterpret_cast<const uint2*>(lo);
+        };
+        // Every thread asks for eight pieces before it uses the first: one after the other (a store of the one in front of the
+        // load of the next) they were half of the kernel's time.
+        if (a.mix_fast) {      // a piece of all heads of a key head gives a piece of each of the CTA's rows of its token
+          const int items = TQ * 16 * n_c;
+          for (int e0 = threadIdx.x; e0 < items; e0 += 2 * SOFT_THREADS) {
+            float4 u[2][4];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+              const int e = e0 + k * SOFT_THREADS, x = e / (TQ * 16), y = e - x * (TQ * 16), tq = y >> 4, col = (c0 + x) * 64 + (y & 15) * 4;
+              const int c = col / a.Dk, d = col - c * a.Dk;
+              const bool in = e < items && tq < nq && c < a.Hkv;
+              const float* qt = q + (size_t)(t0 + tq) * a.ldq + (size_t)(c * rep) * a.qhs + d;
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                u[k][i] = in && i < rep ? *reinterpret_cast<const float4*>(qt + (size_t)i * a.qhs) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+              const int e = e0 + k * SOFT_THREADS, x = e / (TQ * 16), y = e - x * (TQ * 16), tq = y >> 4, col = (c0 + x) * 64 + (y & 15) * 4;
+              const int c = min(col / a.Dk, a.Hkv - 1);
+              if (e >= items) continue;
+              for (int hh = 0; hh < HG; ++hh) {
+                const float* w = sm.talk + hh * a.Hq + c * rep;
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                  const float f = i < rep ? w[i] : 0.f;
+                  if (i < rep) {
+                    v.x = fmaf(f, u[k][i].x, v.x); v.y = fmaf(f, u[k][i].y, v.y);
+                    v.z = fmaf(f, u[k][i].z, v.z); v.w = fmaf(f, u[k][i].w, v.w);
+                  }
+                }
+                put(tq * HG + hh, col, v);
+              }
+            }
+          }
+        } else if (a.talk == nullptr) {
+          const int items = M * per_row;
+          for (int e0 = threadIdx.x; e0 < items; e0 += 8 * SOFT_THREADS) {
+            float4 u[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              const int e = e0 + k * SOFT_THREADS, r = e / per_row, col = c0 * 64 + (e - r * per_row) * 4, tq = r >> hg_shift;
+              u[k] = e < items && tq < nq && col < a.Dk
+                         ? *reinterpret_cast<const float4*>(q + (size_t)(t0 + tq) * a.ldq + (size_t)(h0 + (r & (HG - 1))) * a.qhs + col)
+                         : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              const int e = e0 + k * SOFT_THREADS, r = e / per_row;
+              if (e < items) put(r, c0 * 64 + (e - r * per_row) * 4, u[k]);
+            }
+          }
+        } else {
+          for (int e = threadIdx.x; e < M * per_row; e += SOFT_THREADS) {
+            const int r = e / per_row, col = c0 * 64 + (e - r * per_row) * 4;
+            const int tq = r >> hg_shift, h = h0 + (r & (HG - 1)), c = col / a.Dk, d = col - c * a.Dk;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (tq < nq && c < a.Hkv) {
+              const float* qt = q + (size_t)(t0 + tq) * a.ldq;
+              for (int i = 0; i < rep; ++i) {
+                const float w = __ldg(a.talk + h * a.Hq + c * rep + i);
+                const float4 u = *reinterpret_cast<const float4*>(qt + (size_t)(c * rep + i) * a.qhs + d);
+                v.x = fmaf(w, u.x, v.x); v.y = fmaf(w, u.y, v.y); v.z = fmaf(w, u.z, v.z); v.w = fmaf(w, u.w, v.w);
+              }
+            }
+            put(r, col, v);
+          }
         }
       }
       __syncthreads();
@@ -611,6 +666,7 @@ MLXB_EXPORT int mlxb_attention_wide_tcgen05(int out_f32, const float* q, int ldq
   a.HG = p.HG; a.steps = p.steps; a.chunks = p.chunks; a.v_chunks = p.v_chunks; a.lo_tmem = p.lo_tmem; a.slots = p.slots;
   a.shared_v = shared_v; a.tmem_cols = p.tmem_cols;
   a.vec_out = ((uintptr_t)out & 15) == 0 && (long long)ldo * size % 16 == 0 && (long long)ohs * size % 16 == 0;
+  a.mix_fast = talk != nullptr && Hq / Hkv <= 4 && p.HG * Hq <= MAX_MIX;
   a.scale = scale; a.softcap = softcap;
   const dim3 grid((unsigned)n_tiles * subs, Hq / p.HG);
   static SharedLimit limits[2];
