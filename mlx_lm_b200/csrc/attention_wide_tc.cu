@@ -82,6 +82,7 @@ attention_wide_tc_kernel(const float* q, int ldq, int qhs, const int* __restrict
   const int t0 = t_first + sub * TQ, pos0 = tiles[4 * tile + 3] + sub * TQ;
   const int h0 = blockIdx.y * HG, rep = Hq / Hkv, cv = h0 / rep;
   const int* bt = block_table + (size_t)bt_row * max_pages;
+  const int shift = __ffs(page) - 1;
   int lo_min = 0;                                            // first visible key of the first token: the smallest of the CTA
   if (window > 0 && pos0 - window + 1 > lo_min) lo_min = pos0 - window + 1;
   if (chunk > 0 && (pos0 / chunk) * chunk > lo_min) lo_min = (pos0 / chunk) * chunk;
@@ -128,11 +129,11 @@ attention_wide_tc_kernel(const float* q, int ldq, int qhs, const int* __restrict
       const int c = col / seg, d = col - c * seg;
       const __nv_bfloat16* src = nullptr;
       if ((j >= lo_min || j < keep_first) && j <= p_max && c < n_seg) {
-        const int lp = j / page;
+        const int lp = j >> shift;
         const int pg = lp < max_pages ? bt[lp] : -1;
         if (pg >= n_pages) atomicOr(status, MLXB_ST_PAGE_RANGE);
         else if (pg < 0) atomicOr(status, MLXB_ST_POSITION_RANGE);     // a key inside the range has no page
-        else src = k_pool + (((size_t)pg * Hkv + (talk ? c : cv)) * page + (j % page)) * krs + d;
+        else src = k_pool + (((size_t)pg * Hkv + (talk ? c : cv)) * page + (j & (page - 1))) * krs + d;
       }
       if (src) cp_async16(dK + jj * ldk + col, src);
       else *reinterpret_cast<uint4*>(dK + jj * ldk + col) = make_uint4(0u, 0u, 0u, 0u);
@@ -144,9 +145,9 @@ attention_wide_tc_kernel(const float* q, int ldq, int qhs, const int* __restrict
         const int jj = e / per_v, col = (e - jj * per_v) * 8, j = j0 + jj;
         const __nv_bfloat16* src = nullptr;
         if ((j >= lo_min || j < keep_first) && j <= p_max) {
-          const int lp = j / page;
+          const int lp = j >> shift;
           const int pg = lp < max_pages ? bt[lp] : -1;
-          if (pg >= 0 && pg < n_pages) src = v_pool + (((size_t)pg * Hv + cv / (Hkv / Hv)) * page + (j % page)) * vrs + col;
+          if (pg >= 0 && pg < n_pages) src = v_pool + (((size_t)pg * Hv + cv / (Hkv / Hv)) * page + (j & (page - 1))) * vrs + col;
         }
         if (src) cp_async16(dV + jj * ldv + col, src);
         else *reinterpret_cast<uint4*>(dV + jj * ldv + col) = make_uint4(0u, 0u, 0u, 0u);
@@ -160,7 +161,7 @@ attention_wide_tc_kernel(const float* q, int ldq, int qhs, const int* __restrict
   const int rows_used = nq * HG;                             // rows 0 .. rows_used - 1 carry a (token, head)
   if (vec_q && !talk) {
     // four columns an access and four accesses on their way together: one column at a time each store waited for its load
-    // (single rows of 32 heads of 288: 28.1 us a launch, LATENT_ROWS this way)
+    // (single rows of 32 heads of 288: 28.1 us a launch, 17.0 this way)
     const int per_row = DkE / 4, n = rows_used * per_row;
     for (int e0 = tid; e0 < n; e0 += 4 * THREADS) {
       float4 v[4];
@@ -402,7 +403,8 @@ attention_wide_tc_kernel(const float* q, int ldq, int qhs, const int* __restrict
 //   softmax      a warp a head; weights rounded to bfloat16 and summed as rounded
 //   values       warp w: every eighth tile of 8 columns of all value heads
 // Bound by latency: loads, four phases and their barriers, then the merge.  4 rows of 32 heads of 64 at 400 positions: 111 us with
-// mixed queries (most of it the mixing, a column at a time), TALK_ROWS us this way with the merge.
+// mixed queries (most of it the mixing, a column at a time), 24 us this way with the merge (33 with every piece of a key looking its
+// page up and dividing its way to a column).
 constexpr int TR_MAXH = 64, TR_ITEMS = 16;
 struct TalkRows { int ldq, ldk, ldv, ldp; long long smem; };
 static __host__ __device__ inline TalkRows talk_rows_layout(int Hq, int G, int Dk, int Dv) {
@@ -419,6 +421,7 @@ attention_talk_rows_kernel(const float* q, int ldq_g, int qhs, const int* __rest
                            const __nv_bfloat16* gate, int ldg, TO* __restrict__ out, int ldo, int ohs, int* __restrict__ status, int bps,
                            int n_rel, float* __restrict__ scratch, int keep_first, int gate_cols) {
   extern __shared__ __align__(16) unsigned char tc_smem[];
+  __shared__ int sRow[TC_N];
   const TalkRows L = talk_rows_layout(Hq, G, Dk, Dv);
   constexpr int LS = TC_N + TC_SPAD;
   float* sT = reinterpret_cast<float*>(tc_smem);                            // [Hq][Hq]
@@ -465,29 +468,46 @@ attention_talk_rows_kernel(const float* q, int ldq_g, int qhs, const int* __rest
   k_pool = after_wait(k_pool);
   v_pool = after_wait(v_pool);
   gate = after_wait(gate);
-  // a thread a piece of 16 bytes, zeros where the row does not see the key or a page is missing
-  auto load_tile = [&](__nv_bfloat16* dst, int ld, const __nv_bfloat16* pool, int width, int rs, int j0, bool report) {
+  // The rows of a block's keys in head 0 of their pages (-1: the row does not see the key, or its page is missing), looked up once by
+  // a thread a key; then a thread a piece of 16 bytes, of the same column for all of its keys where a key's pieces divide the threads.
+  const int shift = __ffs(page) - 1;
+  auto load_tile = [&](__nv_bfloat16* dst, int ld, const __nv_bfloat16* pool, int width, int rs) {
     const int per_head = width / 8, per_key = G * per_head;
-    for (int e = tid; e < TC_N * per_key; e += TC_THREADS) {
-      const int jj = e / per_key, x = e - jj * per_key, c = x / per_head, d = (x - c * per_head) * 8, j = j0 + jj;
-      const __nv_bfloat16* src = nullptr;
-      if ((j >= lo || j < keep_first) && j <= p_max) {
-        const int lp = j / page;
-        const int pg = lp < max_pages ? bt[lp] : -1;
-        if (pg >= 0 && pg < n_pages) src = pool + (((size_t)pg * G + c) * page + (j % page)) * rs + d;
-        else if (report) atomicOr(status, pg >= n_pages ? MLXB_ST_PAGE_RANGE : MLXB_ST_POSITION_RANGE);
-      }
+    auto piece = [&](int jj, int c, int d) {
+      const int row = sRow[jj];
       __nv_bfloat16* to = dst + jj * ld + c * width + d;
-      if (src) cp_async16(to, src);
+      if (row >= 0) cp_async16(to, pool + (size_t)(row + c * page) * rs + d);
       else *reinterpret_cast<uint4*>(to) = make_uint4(0u, 0u, 0u, 0u);
+    };
+    if ((per_key & (per_key - 1)) == 0 && per_key <= TC_THREADS) {
+      const int x = tid & (per_key - 1), c = x / per_head, d = (x - c * per_head) * 8, step = TC_THREADS / per_key;
+#pragma unroll 4
+      for (int jj = tid / per_key; jj < TC_N; jj += step) piece(jj, c, d);
+    } else {
+      for (int e = tid; e < TC_N * per_key; e += TC_THREADS) {
+        const int jj = e / per_key, x = e - jj * per_key, c = x / per_head;
+        piece(jj, c, (x - c * per_head) * 8);
+      }
     }
   };
   auto load_block = [&](int j0) {
-    load_tile(sK, L.ldk, k_pool, Dk, krs, j0, true);
-    load_tile(sV, L.ldv, v_pool, Dv, vrs, j0, false);
+    if (tid < TC_N) {
+      const int j = j0 + tid;
+      int row = -1;
+      if ((j >= lo || j < keep_first) && j <= p_max) {
+        const int lp = j >> shift;
+        const int pg = lp < max_pages ? bt[lp] : -1;
+        if (pg < 0 || pg >= n_pages) atomicOr(status, pg < 0 ? MLXB_ST_POSITION_RANGE : MLXB_ST_PAGE_RANGE);
+        else row = pg * G * page + (j & (page - 1));
+      }
+      sRow[tid] = row;
+    }
+    __syncthreads();
+    load_tile(sK, L.ldk, k_pool, Dk, krs);
+    load_tile(sV, L.ldv, v_pool, Dv, vrs);
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  load_block(j_start);
+  load_block(j_start);      // (its barrier: the queries' rows below are nobody else's)
   {
     const float* qt = q + (size_t)t * ldq_g;
     const int per_row = Dk / 4;
@@ -792,7 +812,7 @@ MLXB_EXPORT int mlxb_attention_wide_tc(int out_f32, const float* q, int ldq, int
   TcPlan pl;
   const int shared_v = v_pool == k_pool;
   if (window <= 0) keep_first = 0;           // without a window every earlier position is visible anyway
-  if (talk && tile_q == 1 && !shared_v && page > 0 && (page & (page - 1)) == 0 && qhs >= Dk && ohs >= Dv &&
+  if (talk && tile_q == 1 && !shared_v && page > 0 && (long long)n_pages * Hkv * page < (1LL << 31) && (page & (page - 1)) == 0 && qhs >= Dk && ohs >= Dv &&
       talk_rows_take(q, ldq, qhs, Hq, Hkv, Hv, Dk, Dv, krs, vrs, softcap))
     return out_f32 ? launch_talk_rows<float>(q, ldq, qhs, tiles, n_tiles, block_table, max_pages, n_pages, page, Hq, Hkv, Dk, Dv, krs, vrs,
                                              window, chunk, scale, talk, k_pool, v_pool, gate, ldg, out, ldo, ohs, status, scratch, max_len,
