@@ -9,14 +9,16 @@
 // the four steps of h h last, and the block's sum is added, rounded to nearest, to a sum in registers.  One order for every
 // tile width and number of rows, so a row's result does not depend on how many other rows the call has.
 //
+// 737 rows, 24 layers of 1024 x 4096: 3072 x 1024 35 us, 1024 x 1024 25, 4096 x 1024 65, 1024 x 4096 81 (FMA tiles: 196 to 288); eight
+// warps taking the numbers apart instead of sixteen: 43, 30, 76, 98 (they wait for what they read most of the time).
 // What bounds it: six products of 128 x BN x 64 a block, and as much shared memory traffic as they need; the FMA pipes, which
 // would be three times as busy as the tensor cores for the same product, only take the numbers apart.
 //
 // Per CTA, over 128 x BN tiles (persistent, BN = 128 or 64):
-//   warps 0-7    read the next block of A and W with 16-byte loads (registers hold a block while the one before is at work),
+//   warps 0-15   read the next block of A and W with 16-byte loads (registers hold a block while the one before is at work),
 //                take it apart and store the six planes, 128-byte swizzled, into one of two buffers
-//   warp 16      issues the 24 products of a block, commits the buffer back and the accumulator forward (two of them)
-//   warps 8-15   add the accumulator of every block to their sums (64 columns of a row each at BN = 128); after the last
+//   warp 24      issues the 24 products of a block, commits the buffer back and the accumulator forward (two of them)
+//   warps 16-23  add the accumulator of every block to their sums (64 columns of a row each at BN = 128); after the last
 //                block bias, activation and residual, and out through shared memory as whole sectors
 // An output that is not finite is computed again by its warp with plain FMAs: parts of an infinity, or of a number that
 // bfloat16 rounds to one, make sums that say nothing.
@@ -31,11 +33,11 @@
 MLXB_DEFINE_LAST_ERROR()
 
 constexpr int BM = 128, BK = 64;
-constexpr int SPLIT_WARPS = 8, SUM_WARPS = 8, MMA_WARP = SPLIT_WARPS + SUM_WARPS;
-// whole groups of four warps, which registers are handed out to: 2 x 104 + 2 x 112 + 48 are the 5 x 96 of the launch
+constexpr int SPLIT_WARPS = 16, SUM_WARPS = 8, MMA_WARP = SPLIT_WARPS + SUM_WARPS;
+// whole groups of four warps, which registers are handed out to: 4 x 64 + 2 x 96 + 48 of the 7 x 72 of the launch
 constexpr int THREADS = 32 * (MMA_WARP + 4);
-constexpr int SPLIT_REGS = 104, SUM_REGS = 112, MMA_REGS = 48;
-static_assert(SPLIT_WARPS * SPLIT_REGS + SUM_WARPS * SUM_REGS + 4 * MMA_REGS == 20 * 96, "a larger sum would wait forever");
+constexpr int SPLIT_REGS = 64, SUM_REGS = 96, MMA_REGS = 48;
+static_assert(SPLIT_WARPS * SPLIT_REGS + SUM_WARPS * SUM_REGS + 4 * MMA_REGS <= 28 * 72, "a larger sum would wait forever");
 template <int R>
 __device__ __forceinline__ void more_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
 template <int R>
@@ -80,17 +82,14 @@ __device__ __forceinline__ void put_parts(const float4& v, char* plane0, uint32_
   *reinterpret_cast<uint2*>(plane0 + 2 * plane_bytes + at) = make_uint2(l[0], l[1]);
 }
 
-// 32 columns of a row's accumulator and the wait for them in one statement: between two the compiler may put additions of
+// 16 columns of a row's accumulator and the wait for them in one statement: between two the compiler may put additions of
 // registers that the load has not written yet.
-__device__ __forceinline__ void tmem_get32(uint32_t taddr, uint32_t (&r)[32]) {
+__device__ __forceinline__ void tmem_get16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\ttcgen05.wait::ld.sync.aligned;"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\ttcgen05.wait::ld.sync.aligned;"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr) : "memory");
 }
 
@@ -141,9 +140,9 @@ linear_split_kernel(const float* A, const float* __restrict__ W, const float* __
   const uint32_t tmem_base = sm.tmem_base;
 
   if (warp < SPLIT_WARPS) {
-    more_registers<SPLIT_REGS>();
-    // 16 threads take the 64 k of a row, four each: a thread has rows tr, tr + 16, ... of A and of W
-    constexpr int AR = BM / 16, WR = BN / 16;
+    fewer_registers<SPLIT_REGS>();
+    // 16 threads take the 64 k of a row, four each: a thread has rows tr, tr + ROWS, ... of A and of W
+    constexpr int ROWS = 2 * SPLIT_WARPS, AR = BM / ROWS, WR = BN / ROWS;
     const int tr = threadIdx.x >> 4, tk = (threadIdx.x & 15) * 4;
     float4 av[AR], wv[WR];
     int tile = blockIdx.x, kb = 0;                     // the block that is asked for next
@@ -153,20 +152,20 @@ linear_split_kernel(const float* A, const float* __restrict__ W, const float* __
       const bool in = tile < n_tiles && k < K;
       const float* p = W + (size_t)n0 * K + k;
 #pragma unroll
-      for (int i = 0; i < WR; ++i) wv[i] = in && n0 + 16 * i < N ? *reinterpret_cast<const float4*>(p + (size_t)(16 * i) * K) : zero;
+      for (int i = 0; i < WR; ++i) wv[i] = in && n0 + ROWS * i < N ? *reinterpret_cast<const float4*>(p + (size_t)(ROWS * i) * K) : zero;
     };
     auto fetch_a = [&]() {
       const int m0 = tile_m0(tile) + tr, k = kb * BK + tk;
       const bool in = tile < n_tiles && k < K;
       const float* p = A + (size_t)m0 * lda + k;
 #pragma unroll
-      for (int i = 0; i < AR; ++i) av[i] = in && m0 + 16 * i < M ? *reinterpret_cast<const float4*>(p + (size_t)(16 * i) * lda) : zero;
+      for (int i = 0; i < AR; ++i) av[i] = in && m0 + ROWS * i < M ? *reinterpret_cast<const float4*>(p + (size_t)(ROWS * i) * lda) : zero;
     };
     fetch_w();
     pdl_wait();                                        // A (and the residual) come from the kernel before
     A = after_wait(A);
     fetch_a();
-    // rows 16 apart have the same place in their group of eight: one swizzle for all of a thread's pieces
+    // rows ROWS apart have the same place in their group of eight: one swizzle for all of a thread's pieces
     const uint32_t at = (uint32_t)tr * 128 + (((uint32_t)(tk >> 3) ^ (tr & 7)) << 4) + (tk & 4) * 2;
     int it = 0;
     for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
@@ -179,10 +178,10 @@ linear_split_kernel(const float* A, const float* __restrict__ W, const float* __
         if (++kb == blocks) { kb = 0; tile += gridDim.x; }
         // one operand's next block is on its way while the other's is taken apart
 #pragma unroll
-        for (int i = 0; i < WR; ++i) put_parts(wv[i], pw, BN * BK * 2, at + i * 16 * 128);
+        for (int i = 0; i < WR; ++i) put_parts(wv[i], pw, BN * BK * 2, at + i * ROWS * 128);
         fetch_w();
 #pragma unroll
-        for (int i = 0; i < AR; ++i) put_parts(av[i], pa, BM * BK * 2, at + i * 16 * 128);
+        for (int i = 0; i < AR; ++i) put_parts(av[i], pa, BM * BK * 2, at + i * ROWS * 128);
         fetch_a();
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
@@ -241,11 +240,11 @@ linear_split_kernel(const float* A, const float* __restrict__ W, const float* __
         if (!mbar_wait_warp(&sm.acc_full[b], (it >> 1) & 1, abort_flag)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-        for (int c = 0; c < COLS; c += 32) {
-          uint32_t r[32];
-          tmem_get32(taddr + (uint32_t)(b * BN + c), r);
+        for (int c = 0; c < COLS; c += 16) {
+          uint32_t r[16];
+          tmem_get16(taddr + (uint32_t)(b * BN + c), r);
 #pragma unroll
-          for (int i = 0; i < 32; ++i) sum[c + i] += __uint_as_float(r[i]);
+          for (int i = 0; i < 16; ++i) sum[c + i] += __uint_as_float(r[i]);
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
