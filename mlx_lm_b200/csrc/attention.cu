@@ -226,11 +226,13 @@ MLXB_EXPORT int mlxb_attention_generic(int dtype, const void* q, int ldq, const 
 }
 
 // ---------------------------------------------------------------- portions, float32
-// 64 queries of one head a block of 128 threads, 64 keys at a time (blocks counted from position 0, so a row's order of
+// 64 queries of one head a block of 256 threads, 64 keys at a time (blocks counted from position 0, so a row's order of
 // additions does not depend on where a step begins): scores, online softmax and the sum over the values in float32 FMAs, every
-// operand read from shared memory as 16-byte pieces of eight queries by four keys (or DP / 16 value columns) a thread.  One warp
+// operand read from shared memory as 16-byte pieces of four queries by four keys (or DP / 16 value columns) a thread; the block's
+// keys and values were asked for while the one before was at work.  One warp
 // per (row, head), which the kernel above is, reads every key and value again for every query: 527 us for prompts of 301,
-// 253 and 183 tokens and 16 heads of 64, where the additions take 5.
+// 253 and 183 tokens and 16 heads of 64, where the additions take 5.  What bounds it is latency: such a step has one or two blocks an
+// SM.  Four warps of eight queries a thread, the keys asked for where they were needed: 80.4 us; eight of four: 57.1.
 // A thread fetches one key of a block (its page is looked up a block ahead), and pieces of it.
 
 constexpr int AP_Q = 64, AP_LD = AP_Q + 4;       // queries and keys of a block; floats between rows of transposed operands
@@ -245,12 +247,12 @@ struct PortionMemory {
 
 // DP: the head size rounded up to 32, 64 or 128 (zeros beyond it).
 template <int DP>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(256)
 attention_portions_f32_kernel(const float* q, int ldq, const int4* __restrict__ tiles, const int* __restrict__ block_table,
                               int max_pages, int n_pages, int page, int Hq, int Hkv, int Dh, int window, float scale,
                               const float* k_pool, const float* v_pool, float* __restrict__ out, int ldo, int* __restrict__ status,
                               const float* __restrict__ sinks) {
-  constexpr int VD = DP / 16, PIECES = DP / 8;    // value columns a thread adds up; 16-byte pieces of its key it fetches
+  constexpr int VD = DP / 16, PIECES = DP / 16;   // value columns a thread adds up; 16-byte pieces of its key it fetches
   extern __shared__ __align__(16) char ap_sm[];
   PortionMemory<DP>& sm = *reinterpret_cast<PortionMemory<DP>*>(ap_sm);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -264,8 +266,8 @@ attention_portions_f32_kernel(const float* q, int ldq, const int4* __restrict__ 
   }
   const int h = blockIdx.y, hk = h / (Hq / Hkv), row0 = tile.x + half * AP_Q, pos0 = tile.w + half * AP_Q;
   const int* bt = block_table + (size_t)tile.z * max_pages;
-  const int tx = lane & 15, ty = 2 * warp + (lane >> 4);          // keys (or columns) 4 tx .., queries 8 ty ..
-  const int key = (lane & 15) + 16 * warp, piece = lane >> 4;     // what this thread fetches
+  const int tx = lane & 15, ty = 2 * warp + (lane >> 4);          // keys (or columns) 4 tx .., queries 4 ty ..
+  const int key = (lane & 15) + 16 * (warp & 3), piece = (lane >> 4) + 2 * (warp >> 2);     // what this thread fetches
   const int last = pos0 + nq - 1, lo = window > 0 ? max(0, pos0 - window + 1) : 0;
   const int j_first = lo / AP_Q * AP_Q;
   auto page_of = [&](int j) { return (j <= last && j / page < max_pages) ? bt[j / page] : -1; };
@@ -276,31 +278,24 @@ attention_portions_f32_kernel(const float* q, int ldq, const int4* __restrict__ 
   v_pool = after_wait(v_pool);
 #pragma unroll
   for (int i = 0; i < PIECES; ++i) {
-    const int d = 4 * (piece + 2 * i);
+    const int d = 4 * (piece + 4 * i);
     float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
     if (key < nq && d < Dh) u = *reinterpret_cast<const float4*>(q + (size_t)(row0 + key) * ldq + h * Dh + d);
     sm.q[d][key] = u.x * scale; sm.q[d + 1][key] = u.y * scale; sm.q[d + 2][key] = u.z * scale; sm.q[d + 3][key] = u.w * scale;
   }
-  float m[8], l[8], o[8][VD];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    m[i] = -INFINITY;
-    l[i] = 0.f;
-#pragma unroll
-    for (int d = 0; d < VD; ++d) o[i][d] = 0.f;
-  }
-  for (int j0 = j_first; j0 <= last; j0 += AP_Q) {
+  float4 kq[PIECES], vq[PIECES];
+  bool have;
+  auto fetch = [&](int j0) {
     const int j = j0 + key;
     if (pg >= n_pages || pg < 0) {
       if (j <= last && j >= lo) atomicOr(status, pg < 0 ? MLXB_ST_POSITION_RANGE : MLXB_ST_PAGE_RANGE);   // a key in the range has no page
       pg = -1;
     }
-    const bool have = pg >= 0;
+    have = pg >= 0;
     const size_t at = have ? (((size_t)pg * Hkv + hk) * page + (j & (page - 1))) * Dh : 0;
-    float4 kq[PIECES], vq[PIECES];
 #pragma unroll
     for (int i = 0; i < PIECES; ++i) {
-      const int d = 4 * (piece + 2 * i);
+      const int d = 4 * (piece + 4 * i);
       kq[i] = vq[i] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (have && d < Dh) {
         kq[i] = *reinterpret_cast<const float4*>(k_pool + at + d);
@@ -308,10 +303,21 @@ attention_portions_f32_kernel(const float* q, int ldq, const int4* __restrict__ 
       }
     }
     pg = page_of(j + AP_Q);
-    const bool any_missing = __syncthreads_or(!have && j <= last);     // also: the block before has been read
+  };
+  fetch(j_first);
+  float m[4], l[4], o[4][VD];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    m[i] = -INFINITY;
+    l[i] = 0.f;
+#pragma unroll
+    for (int d = 0; d < VD; ++d) o[i][d] = 0.f;
+  }
+  for (int j0 = j_first; j0 <= last; j0 += AP_Q) {
+    const bool any_missing = __syncthreads_or(!have && j0 + key <= last);     // also: the block before has been read
 #pragma unroll
     for (int i = 0; i < PIECES; ++i) {
-      const int d = 4 * (piece + 2 * i);
+      const int d = 4 * (piece + 4 * i);
       sm.k[d][key] = kq[i].x; sm.k[d + 1][key] = kq[i].y; sm.k[d + 2][key] = kq[i].z; sm.k[d + 3][key] = kq[i].w;
       *reinterpret_cast<float4*>(&sm.v[key][d]) = vq[i];
     }
@@ -323,25 +329,25 @@ attention_portions_f32_kernel(const float* q, int ldq, const int4* __restrict__ 
         bad |= !(fabsf(vq[i].x) < INFINITY && fabsf(vq[i].y) < INFINITY && fabsf(vq[i].z) < INFINITY && fabsf(vq[i].w) < INFINITY);
     }
     bad = __syncthreads_or(bad);
-    float s[8][4];
+    if (j0 + AP_Q <= last) fetch(j0 + AP_Q);
+    float s[4][4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int e = 0; e < 4; ++e) s[i][e] = 0.f;
 #pragma unroll 8
     for (int d = 0; d < DP; ++d) {
-      float a[8], b[4];
-      *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(&sm.q[d][8 * ty]);
-      *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(&sm.q[d][8 * ty + 4]);
+      float a[4], b[4];
+      *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(&sm.q[d][4 * ty]);
       *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(&sm.k[d][4 * tx]);
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int e = 0; e < 4; ++e) s[i][e] = fmaf(a[i], b[e], s[i][e]);
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int pq = pos0 + 8 * ty + i;
+    for (int i = 0; i < 4; ++i) {
+      const int pq = pos0 + 4 * ty + i;
       float top = -INFINITY;
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
@@ -372,21 +378,18 @@ attention_portions_f32_kernel(const float* q, int ldq, const int4* __restrict__ 
       for (int d = 0; d < VD; ++d) o[i][d] *= corr;
     }
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      *reinterpret_cast<float4*>(&sm.p[4 * tx + e][8 * ty]) = make_float4(s[0][e], s[1][e], s[2][e], s[3][e]);
-      *reinterpret_cast<float4*>(&sm.p[4 * tx + e][8 * ty + 4]) = make_float4(s[4][e], s[5][e], s[6][e], s[7][e]);
-    }
+    for (int e = 0; e < 4; ++e)
+      *reinterpret_cast<float4*>(&sm.p[4 * tx + e][4 * ty]) = make_float4(s[0][e], s[1][e], s[2][e], s[3][e]);
     __syncwarp();          // a warp reads back the probabilities of its own queries
     const int nk = min(AP_Q, last - j0 + 1);
     auto add_values = [&](int jj, auto some) {       // some: only to the queries that see the key
-      float a[8], b[VD];
-      *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(&sm.p[jj][8 * ty]);
-      *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(&sm.p[jj][8 * ty + 4]);
+      float a[4], b[VD];
+      *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(&sm.p[jj][4 * ty]);
 #pragma unroll
       for (int d = 0; d < VD; d += 2) *reinterpret_cast<float2*>(b + d) = *reinterpret_cast<const float2*>(&sm.v[jj][VD * tx + d]);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int ahead = j0 + jj - (pos0 + 8 * ty + i);
+      for (int i = 0; i < 4; ++i) {
+        const int ahead = j0 + jj - (pos0 + 4 * ty + i);
         if (decltype(some)::value && (ahead > 0 || (window > 0 && ahead <= -window))) continue;
 #pragma unroll
         for (int d = 0; d < VD; ++d) o[i][d] = fmaf(a[i], b[d], o[i][d]);
@@ -401,8 +404,8 @@ attention_portions_f32_kernel(const float* q, int ldq, const int4* __restrict__ 
     }
   }
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int qi = 8 * ty + i;
+  for (int i = 0; i < 4; ++i) {
+    const int qi = 4 * ty + i;
     if (qi >= nq) continue;
     float total = l[i];
     if (sinks && m[i] != -INFINITY) total += expf(sinks[h] - m[i]);   // the sink: a term of the denominator without a value
@@ -427,7 +430,7 @@ MLXB_EXPORT int mlxb_attention_portions_f32(const float* q, int ldq, const int* 
   auto go = [&](auto kernel, size_t smem, SharedLimit& limit) {
     const cudaError_t e = limit.raise(kernel, smem);
     if (e != cudaSuccess) return mlxb_fail((int)e, "attention: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
-    launch_pdl(kernel, dim3(2 * n_tiles, Hq), dim3(128), smem, stream, q, ldq, (const int4*)tiles, block_table, max_pages, n_pages,
+    launch_pdl(kernel, dim3(2 * n_tiles, Hq), dim3(256), smem, stream, q, ldq, (const int4*)tiles, block_table, max_pages, n_pages,
                page, Hq, Hkv, Dh, window, scale, k_pool, v_pool, out, ldo, status, sinks);
     return mlxb_check_launch("attention (float32 portions)");
   };
