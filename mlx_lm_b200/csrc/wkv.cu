@@ -19,18 +19,9 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "recurrent_tiles.cuh"
 
 MLXB_DEFINE_LAST_ERROR()
-
-// Rows t0 .. t1-1 that belong to request r (they come first in the range).  Every thread of the block calls it.
-__device__ __forceinline__ int run_length(const int* __restrict__ token_req, int t0, int t1, int r) {
-  int n = 0;
-  for (int base = t0; base < t1; base += blockDim.x) {
-    const int t = base + threadIdx.x;
-    n += __syncthreads_count(t < t1 && token_req[t] == r);
-  }
-  return n;
-}
 
 template <typename T>
 __global__ void token_shift_mix_kernel(const T* x, int ldx, const float* __restrict__ mu, int n_mix, int D,
@@ -231,36 +222,6 @@ __device__ __forceinline__ f32x2 twice(float v) {
 }
 __device__ __forceinline__ float sum2(f32x2 v) { return __uint_as_float((unsigned)v) + __uint_as_float((unsigned)(v >> 32)); }
 
-// Job `job` of the step: chunk c of request r, in the order of the requests; base: chunks before the request's last ones, of the
-// requests before it (where its states between chunks are kept).  r = -1: there are fewer jobs.  A whole warp calls it.
-struct ChunkJob { int r, c, base; };
-__device__ __forceinline__ ChunkJob find_job(const int* __restrict__ req_first_token, int n_requests, int job) {
-  const int lane = threadIdx.x & 31;
-  ChunkJob out = {-1, 0, 0};
-  int before = 0;
-  for (int r0 = 0; r0 < n_requests; r0 += 32) {
-    const int r = r0 + lane;
-    const int mine = r < n_requests ? (req_first_token[r + 1] - req_first_token[r] + WC_Q - 1) / WC_Q : 0;
-    int jobs = mine, kept = mine > 0 ? mine - 1 : 0;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int u = __shfl_up_sync(0xffffffffu, jobs, o), w = __shfl_up_sync(0xffffffffu, kept, o);
-      if (lane >= o) { jobs += u; kept += w; }
-    }
-    const unsigned hit = __ballot_sync(0xffffffffu, before + jobs > job);
-    if (hit) {
-      const int src = __ffs(hit) - 1;
-      out.r = r0 + src;
-      out.c = job - before - __shfl_sync(0xffffffffu, jobs - mine, src);
-      out.base += __shfl_sync(0xffffffffu, kept - (mine > 0 ? mine - 1 : 0), src);
-      return out;
-    }
-    before += __shfl_sync(0xffffffffu, jobs, 31);
-    out.base += __shfl_sync(0xffffffffu, kept, 31);
-  }
-  return out;
-}
-
 template <int NS>
 struct WkvMemory {
   static constexpr int NP = NS * WK_SEG;
@@ -283,7 +244,7 @@ wkv_chunks_kernel(const T* rkv, int ld, int r_off, int k_off, int v_off, const f
   const int s = tid % NS, col = 2 * (tid / NS);      // rows 16 s .. of columns col, col + 1 of the slice
   const bool valid = v0 + col < V;                   // (V is even)
   pdl_trigger();
-  const ChunkJob job = find_job(req_first_token, n_requests, blockIdx.y);
+  const ChunkJob job = find_job(req_first_token, nullptr, n_requests, blockIdx.y, WC_Q);
   const int t_first = job.r >= 0 ? req_first_token[job.r] : 0, t_end = job.r >= 0 ? req_first_token[job.r + 1] : 0;
   const int n = run_length(token_req, t_first, t_end, job.r);
   const bool last = (job.c + 1) * WC_Q >= n;

@@ -153,6 +153,15 @@ class StepContext:
             self._choices[recurrence] = ops.chunk_rule(*recurrence, runs, sms=ops.sm_count())
         return self._choices[recurrence]
 
+    def chunks_side_by_side(self, recurrence: tuple) -> bool:
+        """Whether the runs in chunks go through a part's ``chunked_recurrence`` in two passes (see ``ops.chunks_side_by_side``)."""
+        if self.dtype != torch.bfloat16 or not self.portions:
+            return False
+        key = ("side by side", recurrence)
+        if key not in self._choices:
+            self._choices[key] = ops.chunks_side_by_side(*recurrence, tuple(n for _, n in self.portions), sms=ops.sm_count())
+        return self._choices[key]
+
     def attention_in_tiles(self, attention: tuple) -> bool:
         """Whether float32 portions run in tiles (see ``ops.attention_portions_f32_pays``)."""
         if not self.portions:
@@ -459,6 +468,7 @@ class Engine:
             ctx._tables = [view(f"table{g}", R * W).view(R, W) for g in range(len(mgr.kv_groups))]
             logits = self._run(ctx, (T, R, L_rows, n_single_rows, n_tiles, ctx.stream, dev.data_ptr())
                                + tuple(ctx.chunk_rule(c) for c in self._recurrences)
+                               + tuple(ctx.chunks_side_by_side(c) for c in self._recurrences)
                                + tuple(ctx.attention_in_tiles(a) for a in self._attentions))
         except BaseException:
             # The step did not run to its end: its positions are not part of the requests.  The pages taken for

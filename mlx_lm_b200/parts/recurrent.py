@@ -167,7 +167,10 @@ class GatedDeltaMixer(Mixer):
                 self.n_kv_heads, ctx.stream)
         rule = ctx.chunk_rule(self.chunked_recurrence)
         if rule is not None:
-            ops.gated_delta_chunks(*args, requests=ctx.portion_requests, rule=rule)
+            scratch = None
+            if ctx.chunks_side_by_side(self.chunked_recurrence):
+                scratch = ctx.ws.flat("delta_chunks", ops.gated_delta_chunks_scratch(T, ctx.portion_requests.numel(), H), torch.float32)
+            ops.gated_delta_chunks(*args, requests=ctx.portion_requests, rule=rule, scratch=scratch)
         if rule is not ops.CHUNKS or ctx.n_single:
             ops.gated_delta_scan(*args, max_run=0 if rule is None else 1, rule=rule or ops.CHUNKS)
         g = ctx.ws.get("delta_gated", T, self.v_width, x.dtype)
