@@ -1155,10 +1155,13 @@ def chunks_side_by_side(kind: str, n_heads: int, state_rows: int, columns: int, 
     Microseconds: the one kernel takes 10 a chunk of the longest run and wave of blocks; of the two passes the second 4, the first 8 a wave
     of its blocks (a chunk and head each, two on an SM), and a launch 5.  Measured, 16 heads of 64 x 64, one kernel and two: two runs
     of 1024 rows 162 and 106, one of 200 43 and 35, of 128 23.3 and 24.8, four of 64 13.7 and 23.8, eight of 100 44.8 and 40.2, eight of
-    500 164 and 136; 32 heads, four of 256 85 and 74."""
+    500 164 and 136; 32 heads, four of 256 85 and 74.  A chunk and head leaves 50 KB of scratch memory between the passes: at most 8192 of
+    them (0.4 GB)."""
     if kind != "delta" or not runs or state_rows > DELTA_CHUNK_ROWS:
         return False
     chunks = [-(-n // 64) for n in runs]
+    if sum(chunks) * n_heads > 8192:
+        return False
     waves = -(-len(runs) * n_heads * -(-columns // 32) // sms)
     first = -(-sum(chunks) * n_heads // (2 * sms))
     return waves * 10 * max(chunks) > 5 + 8 * first + waves * 4 * max(chunks)

@@ -13,3 +13,4 @@ def test_long_runs_of_few_states_go_in_two_passes():
 def test_what_has_no_two_passes_takes_none():
     assert not ops.chunks_side_by_side("delta", 16, 65, 64, (1024,))       # no chunked kernel for such states
     assert not ops.chunks_side_by_side("mamba2", 32, 128, 64, (1024,))
+    assert not ops.chunks_side_by_side(*DELTA, (40000,))                   # their scratch memory has a limit
