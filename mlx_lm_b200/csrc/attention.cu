@@ -605,7 +605,8 @@ attention_decode_kernel(const T* __restrict__ q, int ldq, const int* __restrict_
   float qv[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) qv[i] = 0.f;
-  if (active) {
+  if (active && !beside) load8<T>(q_now + (size_t)t * ldq + h * Dh + d0, qv);      // through L1: every group of threads reads the same row
+  if (active && beside) {
     Raw8<T> qr;
     qr.load_fresh(q_now + (size_t)t * ldq + h * Dh + d0);
     qr.get(qv);
