@@ -562,9 +562,10 @@ attention_decode_kernel(const T* __restrict__ q, int ldq, const int* __restrict_
   }
   Raw8<T> kr[U], vr[U];
   bool ok[U];
-  // All key and value rows of batch `it`; the page ids were fetched one batch ahead.  With `early`, the
-  // row's own position is left for fetch_own(): it is not in memory yet.
-  auto fetch = [&](int it, bool early) {
+  // All key and value rows of batch `it`; the page ids were fetched one batch ahead.  The row's own position, in whichever batch it
+  // is, is left for fetch_own(): the kernel before this one writes it while this one runs, so it is read after the wait and past L1
+  // (a load that promises read-only memory may be served from before the write).
+  auto fetch = [&](int it) {
     int pg[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -581,7 +582,7 @@ attention_decode_kernel(const T* __restrict__ q, int ldq, const int* __restrict_
         if (j == 0) atomicOr(status, pg[u] < 0 ? MLXB_ST_POSITION_RANGE : MLXB_ST_PAGE_RANGE);
         ok[u] = false;
       }
-      if (ok[u] && active && !(early && key == p)) {
+      if (ok[u] && active && key != p) {
         const size_t off = (((size_t)pg[u] * Hkv + hk) * page + (key & (page - 1))) * Dh + d0;
         kr[u].load(k_pool + off);
         vr[u].load(v_pool + off);
@@ -591,9 +592,10 @@ attention_decode_kernel(const T* __restrict__ q, int ldq, const int* __restrict_
       }
     }
   };
-  fetch(0, true);
-  int own_pg = -1;   // page of the row's own position, if it belongs to this chunk's first batch
-  if (p >= k_begin && p < k_end && p - k_begin < GROUPS * U) {
+  fetch(0);
+  const int own_it = p < k_end ? (p - k_begin) / (GROUPS * U) : -1;      // the batch of the row's own position, and its page
+  int own_pg = -1;
+  if (own_it >= 0) {
     const int lp = p >> shift;
     own_pg = lp < max_pages ? bt[lp] : -1;
   }
@@ -611,8 +613,9 @@ attention_decode_kernel(const T* __restrict__ q, int ldq, const int* __restrict_
     qr.load_fresh(q_now + (size_t)t * ldq + h * Dh + d0);
     qr.get(qv);
   }
-  if (own_pg >= 0 && own_pg < n_pages && active && (p - k_begin) % GROUPS == grp) {
-    const int u_own = (p - k_begin) / GROUPS;
+  auto fetch_own = [&](int it) {
+    if (it != own_it || own_pg < 0 || own_pg >= n_pages || !active || (p - k_begin) % GROUPS != grp) return;
+    const int u_own = (p - k_begin) / GROUPS - it * U;
     const size_t off = (((size_t)own_pg * Hkv + hk) * page + (p & (page - 1))) * Dh + d0;
 #pragma unroll
     for (int u = 0; u < U; ++u)
@@ -620,12 +623,16 @@ attention_decode_kernel(const T* __restrict__ q, int ldq, const int* __restrict_
         kr[u].load_fresh(k_now + off);
         vr[u].load_fresh(v_now + off);
       }
-  }
+  };
+  fetch_own(0);
 #pragma unroll
   for (int i = 0; i < 8; ++i) qv[i] *= scale;
 
   for (int it = 0; it < iters; ++it) {
-    if (it > 0) fetch(it, false);   // these rows are older than this step, whichever pointer they are read through
+    if (it > 0) {
+      fetch(it);
+      fetch_own(it);
+    }
     float sc[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
