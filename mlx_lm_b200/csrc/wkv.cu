@@ -230,13 +230,14 @@ struct WkvMemory {
   float bonus[WK_CHUNK];      // sum_k r u k of the token
 };
 
-// kept: [chunks before last ones][H][V][K] states (W S_0 + L of a run's first chunk, L of the others), then [..][H][K] products W.
+// kept: [chunks before last ones][H][V][K] states (the first pass leaves the state after a run's first chunk, L of the others; then the
+// state after each), then [..][H][K] products W.
 template <typename T, int NS, bool FIRST>
 __global__ void __launch_bounds__(32 * NS)
 wkv_chunks_kernel(const T* rkv, int ld, int r_off, int k_off, int v_off, const float* d_raw, int ldd, const float* __restrict__ u,
                   float* state, const int* __restrict__ slots, const int* __restrict__ token_req,
                   const int* __restrict__ req_first_token, int n_requests, float* o, int ldo, int H, int V, float* kept,
-                  float* products) {
+                  float* products, bool states_ready) {
   extern __shared__ __align__(16) char wc_sm[];
   WkvMemory<NS>* sm = reinterpret_cast<WkvMemory<NS>*>(wc_sm);      // two: the next tokens are staged beside these
   constexpr int K = NS * WK_NPT, THREADS = 32 * NS, PER_TOK = K / 8;
@@ -372,11 +373,12 @@ wkv_chunks_kernel(const T* rkv, int ld, int r_off, int k_off, int v_off, const f
     for (int i = 0; i < 8; ++i) S[0][i] = S[1][i] = 0ull;
   } else if (FIRST) {
     load_state(pool);
-  } else {            // the run's state after its first chunk, then through the chunks up to this one
-    const float* L = kept + (size_t)job.base * state_size + at;
-    const float* W = products + ((size_t)job.base * H + h) * K + s * WK_NPT;
+  } else {            // the run's state after its first chunk (or, with states_ready, after the one before), then through the chunks up to this one
+    const int from = states_ready ? job.c - 1 : 0;
+    const float* L = kept + (size_t)(job.base + from) * state_size + at;
+    const float* W = products + ((size_t)(job.base + from) * H + h) * K + s * WK_NPT;
     load_state(L);
-    for (int c = 1; c < job.c; ++c) {
+    for (int c = from + 1; c < job.c; ++c) {
       L += state_size;
       W += (size_t)H * K;
 #pragma unroll
@@ -481,9 +483,55 @@ wkv_chunks_kernel(const T* rkv, int ld, int r_off, int k_off, int v_off, const f
   }
 }
 
-// Floats of scratch memory for mlxb_wkv_chunks: states and products of the chunks before a run's last one.
-MLXB_EXPORT long long mlxb_wkv_chunks_scratch(int n_tokens, int H, int K, int V) {
-  return (long long)(n_tokens / WC_Q) * H * K * (V + 1);
+// Between the passes, in steps with long runs: the state after every chunk of a run in place of what the first pass left of it, so that
+// the second pass does not walk through all of a run's chunks for each of them (as many reads as chunks squared).  A block has 1024
+// numbers of a (request, head); the same arithmetic in the same order.  16 heads of 64, one run of 2048 rows 107 us without and 86 with
+// it, of 8192 622 and 311, of 131072 97 and 15 ms; one of 512 rows 55 and 64, eight of 200 60 and 74.
+constexpr int WC_LONG = 4096;  // rows of a step from which it pays: the launch takes up to 14 us, a run of as many rows gains more
+constexpr int WS_AHEAD = 8;    // chunks that are asked for together
+__global__ void __launch_bounds__(256)
+wkv_states_kernel(const int* __restrict__ token_req, const int* __restrict__ req_first_token, float* kept, const float* products, int H,
+                  int V, int K) {
+  const int h = blockIdx.x, r = blockIdx.y, lane = threadIdx.x & 31;
+  pdl_trigger();
+  const int n = run_length(token_req, req_first_token[r], req_first_token[r + 1], r);
+  int base = 0;      // kept states of the requests before
+  for (int i = lane; i < r; i += 32) {
+    const int len = req_first_token[i + 1] - req_first_token[i];
+    base += len > WC_Q ? (len - 1) / WC_Q : 0;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) base += __shfl_xor_sync(0xffffffffu, base, o);
+  const int at = (blockIdx.z * 256 + threadIdx.x) * 4, size = V * K, last = (n - 1) / WC_Q;      // chunks 0 .. last - 1 are kept
+  pdl_wait();
+  if (at >= size || last < 2) return;
+  kept = after_wait(kept);
+  products = after_wait(products);
+  float* L = kept + ((size_t)base * H + h) * size + at;
+  const float* W = products + ((size_t)base * H + h) * K + at % K;
+  const size_t next = (size_t)H * size, next_w = (size_t)H * K;
+  float4 S = *reinterpret_cast<const float4*>(L);
+  for (int c = 1; c < last; c += WS_AHEAD) {
+    float4 l[WS_AHEAD], w[WS_AHEAD];
+#pragma unroll
+    for (int i = 0; i < WS_AHEAD; ++i) {
+      if (c + i >= last) continue;
+      l[i] = *reinterpret_cast<const float4*>(L + (size_t)(c + i) * next);
+      w[i] = *reinterpret_cast<const float4*>(W + (size_t)(c + i) * next_w);
+    }
+#pragma unroll
+    for (int i = 0; i < WS_AHEAD; ++i) {
+      if (c + i >= last) continue;
+      S = make_float4(fmaf(w[i].x, S.x, l[i].x), fmaf(w[i].y, S.y, l[i].y), fmaf(w[i].z, S.z, l[i].z), fmaf(w[i].w, S.w, l[i].w));
+      *reinterpret_cast<float4*>(L + (size_t)(c + i) * next) = S;
+    }
+  }
+}
+
+// Floats of scratch memory for mlxb_wkv_chunks: states and products of the chunks before a run's last one, about as much as the step's
+// outputs in float32 (V + 1 floats a key channel for every 64 rows).
+MLXB_EXPORT long long mlxb_wkv_chunks_scratch(int long_rows, int H, int K, int V) {
+  return (long long)(long_rows / WC_Q) * H * K * (V + 1);
 }
 
 // What the kernels take: states of 16, 32, ... 256 rows and an even number of columns, 16-byte rows of r, k and the decay.
@@ -500,21 +548,22 @@ MLXB_EXPORT int mlxb_wkv_scan(int dtype, const void* rkv, int ld, int r_off, int
                               const int* req_first_token, float* o, int ldo, int H, int K, int V, int n_requests,
                               cudaStream_t stream);
 
-// The arguments of mlxb_wkv_scan, the step's rows, and scratch memory of mlxb_wkv_chunks_scratch floats (16-byte aligned).  Sizes
-// that the kernels do not take go token by token.
+// The arguments of mlxb_wkv_scan, and scratch memory of mlxb_wkv_chunks_scratch floats (16-byte aligned).  long_rows: at least the rows
+// of the step beyond the first of every request.  Sizes that the kernels do not take, and more chunks than a grid has, go token by token.
 MLXB_EXPORT int mlxb_wkv_chunks(int dtype, const void* rkv, int ld, int r_off, int k_off, int v_off, const float* d_raw, int ldd,
                                 const float* u, float* state, const int* slots, const int* token_req, const int* req_first_token,
-                                float* o, int ldo, int H, int K, int V, int n_requests, int n_tokens, float* scratch,
+                                float* o, int ldo, int H, int K, int V, int n_requests, int long_rows, float* scratch,
                                 cudaStream_t stream) {
-  if (n_requests <= 0 || n_tokens <= 0) return 0;
+  if (n_requests <= 0 || long_rows < 0) return 0;
   const int size = dtype == MLXB_F32 ? 4 : 2;
-  if (!chunks_take(rkv, size, ld, r_off, k_off, v_off, d_raw, ldd, state, o, ldo, K, V) || ((uintptr_t)scratch & 15) || H <= 0)
+  const long long jobs = (long long)long_rows / WC_Q + n_requests;
+  if (!chunks_take(rkv, size, ld, r_off, k_off, v_off, d_raw, ldd, state, o, ldo, K, V) || ((uintptr_t)scratch & 15) || H <= 0 ||
+      jobs > 65535 || (long long)V * K > 65535 * 1024LL)
     return mlxb_wkv_scan(dtype, rkv, ld, r_off, k_off, v_off, d_raw, ldd, u, state, slots, token_req, req_first_token, o, ldo, H, K, V,
                          n_requests, stream);
-  const long long jobs = (long long)n_tokens / WC_Q + n_requests;
-  if (jobs > 65535 || (V + WC_VB - 1) / WC_VB > 65535) return mlxb_fail(MLXB_BAD_ARG, "wkv_chunks: %d rows of %d requests, %d columns", n_tokens, n_requests, V);
-  float* products = scratch + (size_t)(n_tokens / WC_Q) * H * V * K;
+  float* products = scratch + (size_t)(long_rows / WC_Q) * H * V * K;
   const dim3 grid(H, (unsigned)jobs, (V + WC_VB - 1) / WC_VB);
+  const bool states_ready = long_rows >= WC_LONG;
   auto run = [&](auto type, auto ns) {
     using T = decltype(type);
     constexpr int NS = decltype(ns)::value;
@@ -524,12 +573,16 @@ MLXB_EXPORT int mlxb_wkv_chunks(int dtype, const void* rkv, int ld, int r_off, i
       const cudaError_t e = limit.raise(kernel, smem);
       if (e != cudaSuccess) return mlxb_fail((int)e, "wkv_chunks: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
       launch_pdl(kernel, grid, dim3(32 * NS), smem, stream, (const T*)rkv, ld, r_off, k_off, v_off, d_raw, ldd, u, state, slots,
-                 token_req, req_first_token, n_requests, o, ldo, H, V, scratch, products);
+                 token_req, req_first_token, n_requests, o, ldo, H, V, scratch, products, states_ready);
       return mlxb_check_launch("wkv_chunks");
     };
     if (int e = go(wkv_chunks_kernel<T, NS, true>, limits[0])) return e;
-    // a run of more than one chunk: not with fewer rows than that
-    if (n_tokens <= WC_Q) return 0;
+    if (long_rows < WC_Q) return 0;                      // no run of two chunks
+    if (states_ready) {
+      launch_pdl(wkv_states_kernel, dim3(H, n_requests, (V * K + 1023) / 1024), dim3(256), 0, stream, token_req, req_first_token, scratch,
+                 (const float*)products, H, V, K);
+      if (int e = mlxb_check_launch("wkv_chunks (states)")) return e;
+    }
     return go(wkv_chunks_kernel<T, NS, false>, limits[1]);
   };
   auto by_rows = [&](auto type) {

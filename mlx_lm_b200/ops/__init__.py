@@ -1925,23 +1925,24 @@ def wkv_scan(rkv, r_off: int, k_off: int, v_off: int, decay_raw, bonus, state, s
           stream)
 
 
-def wkv_chunks_scratch(n_tokens: int, n_heads: int, state_rows: int, columns: int) -> int:
-    """Floats of scratch memory for ``wkv_chunks`` over ``n_tokens`` rows."""
+def wkv_chunks_scratch(long_rows: int, n_heads: int, state_rows: int, columns: int) -> int:
+    """Floats of scratch memory for ``wkv_chunks`` over ``long_rows`` rows."""
     f, _ = _fn("wkv", "mlxb_wkv_chunks_scratch", [c_int] * 4)
     f.restype = ctypes.c_longlong
-    return int(f(n_tokens, n_heads, state_rows, columns))
+    return int(f(long_rows, n_heads, state_rows, columns))
 
 
 def wkv_chunks(rkv, r_off: int, k_off: int, v_off: int, decay_raw, bonus, state, slots, token_req, req_first_token, o,
-               n_heads: int, scratch, stream) -> None:
-    """``wkv_scan`` with the chunks of 64 rows of a request's run side by side (csrc/wkv.cu).  ``scratch``: float32, at least
-    ``wkv_chunks_scratch`` elements."""
+               n_heads: int, scratch, stream, long_rows: Optional[int] = None) -> None:
+    """``wkv_scan`` with the chunks of 64 rows of a request's run side by side (csrc/wkv.cu).  ``long_rows``: the step's rows without
+    those of requests that bring a single one (default: all).  ``scratch``: float32, at least ``wkv_chunks_scratch`` elements."""
     args = _wkv_args(rkv, r_off, k_off, v_off, decay_raw, bonus, state, slots, token_req, req_first_token, o, n_heads, "wkv_chunks")
     _need(scratch, torch.float32, "wkv_chunks scratch")
     T, (_, H, V, K) = rkv.shape[0], state.shape
-    if scratch.numel() < wkv_chunks_scratch(T, H, K, V):
-        raise KernelError(f"wkv_chunks: {scratch.numel()} floats of scratch memory for {T} rows")
-    _call("wkv", "mlxb_wkv_chunks", _WKV_ARGS[:-1] + [c_int, c_void_p, c_void_p], *args, T, _p(scratch), stream)
+    rows = T if long_rows is None else int(long_rows)
+    if not 0 <= rows <= T or scratch.numel() < wkv_chunks_scratch(rows, H, K, V):
+        raise KernelError(f"wkv_chunks: {scratch.numel()} floats of scratch memory for {rows} of {T} rows")
+    _call("wkv", "mlxb_wkv_chunks", _WKV_ARGS[:-1] + [c_int, c_void_p, c_void_p], *args, rows, _p(scratch), stream)
 
 
 # --------------------------------------------------------------------------

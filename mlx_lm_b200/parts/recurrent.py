@@ -254,9 +254,9 @@ class WKVMixer(Mixer):
         o = ctx.ws.get("wkv_o", T, HD, torch.float32)
         ops.label(self.name + ".scan", 6.0 * T * HD * self.dim, x.element_size() * 3.0 * T * HD + 8.0 * T * HD
                   + 8.0 * min(T, ctx.n_requests) * HD * self.dim)
-        scratch = ctx.ws.flat("wkv_states", ops.wkv_chunks_scratch(T, self.n_heads, self.dim, self.dim), torch.float32)
+        scratch = ctx.ws.flat("wkv_states", ops.wkv_chunks_scratch(ctx.n_portion, self.n_heads, self.dim, self.dim), torch.float32)
         ops.wkv_chunks(rkvg, 0, HDp, 2 * HDp, decay, self.bonus, rule.state, rule.slots, ctx.token_req, ctx.req_first_token,
-                       o, self.n_heads, scratch, ctx.stream)
+                       o, self.n_heads, scratch, ctx.stream, long_rows=ctx.n_portion)
         gated = ctx.ws.get("wkv_gated", T, HD, x.dtype)
         ops.label(self.name + ".norm", 8.0 * T * HD, (4.0 + 2 * x.element_size()) * T * HD)
         ops.rmsnorm(o, self.norm_w, gated, self.eps, ctx.stream, groups=self.n_heads, gate=rkvg[:, 3 * HDp:3 * HDp + HD],

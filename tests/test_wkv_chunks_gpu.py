@@ -25,6 +25,7 @@ def reference(r, k, v, d, u, S):
     (2, 64, 64, [1, 63, 64, 65, 128, 129, 300]),      # around a chunk, several chunks
     (3, 16, 16, [70, 1, 200]), (2, 32, 34, [130, 17]), (1, 128, 70, [65, 192]), (1, 256, 130, [66, 5]),
     (2, 64, 64, [1] * 40 + [100] + [1] * 7),          # requests beyond a warp's lanes
+    (1, 64, 64, [1] * 33 + [577, 64, 3700, 1]),       # the states of all chunks before the second pass
     (2, 48, 48, [70, 3]), (2, 64, 63, [70, 3]),       # token by token: rows that are no power of two, odd columns
 ])
 def test_wkv_chunks(dtype, H, K, V, runs):
@@ -47,9 +48,10 @@ def test_wkv_chunks(dtype, H, K, V, runs):
     first = i32(first[:-1] + [T + pad])               # rows that pad the step belong to nobody
     before, scan_pool = pool.clone(), pool.clone()
     o, by_token = (torch.full((T + pad, H * V), 7.0, device=DEV) for _ in range(2))
-    scratch = torch.full((max(4, ops.wkv_chunks_scratch(T + pad, H, K, V)),), float("nan"), device=DEV)
+    long_rows = T + pad - n                           # all but the first of every request
+    scratch = torch.full((max(4, ops.wkv_chunks_scratch(long_rows, H, K, V)),), float("nan"), device=DEV)
     args = (rkv, 0, Kp, 2 * Kp, d, u)
-    ops.wkv_chunks(*args, pool, i32(slots), token_req, first, o, H, scratch, ops.current_stream())
+    ops.wkv_chunks(*args, pool, i32(slots), token_req, first, o, H, scratch, ops.current_stream(), long_rows=long_rows)
     ops.wkv_scan(*args, scan_pool, i32(slots), token_req, first, by_token, H, ops.current_stream())
     at = 0
     for i, m in enumerate(runs):
@@ -65,6 +67,24 @@ def test_wkv_chunks(dtype, H, K, V, runs):
     assert bool((o[T:] == 7.0).all())
     rest = [s for s in range(n + 3) if s not in slots]
     assert torch.equal(pool[rest], before[rest])
+
+
+def test_wkv_chunks_of_a_run_beside_others():
+    """A run's bits do not depend on the step's rows, with the states of all chunks made before the second pass or walked through by it."""
+    from mlx_lm_b200 import ops
+    H, K, runs = 2, 64, [700, 3600]
+    g = torch.Generator(device=DEV).manual_seed(5)
+    randn = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    rkv, d, u = randn(sum(runs), 3 * H * K), randn(sum(runs), H * K), randn(H, K)
+    outs = []
+    for T, first in ((700, [0, 700]), (4300, [0, 700, 4300])):
+        n = len(first) - 1
+        o, pool = torch.empty(T, H * K, device=DEV), torch.zeros(n, H, K, K, device=DEV)
+        scratch = torch.empty(ops.wkv_chunks_scratch(T, H, K, K), device=DEV)
+        ops.wkv_chunks(rkv[:T], 0, H * K, 2 * H * K, d[:T], u, pool, i32(list(range(n))),
+                       i32([0] * 700 + [1] * (T - 700)), i32(first), o, H, scratch, ops.current_stream())
+        outs.append((o[:700], pool[0]))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
 
 
 def test_wkv_chunks_keep_what_is_not_finite_to_the_rows_behind_it():
