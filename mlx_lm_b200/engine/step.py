@@ -140,6 +140,9 @@ class StepContext:
         # that run in chunks, those entries' request indexes, longest first, filled up with -1 (int32)
         self.portions: Tuple[Tuple[int, int], ...] = ()
         self.portion_requests = None
+        # float32: as many rows from the first on belong to requests that bring several tokens (and to nobody), those behind them to
+        # requests that bring one; 0 in bfloat16, where the two kinds may stand in any order
+        self.leading_portion_rows = 0
         self._choices: Dict[tuple, object] = {}
         self._tables: List[torch.Tensor] = []
         self._slots: Optional[torch.Tensor] = None
@@ -364,6 +367,12 @@ class Engine:
             if L_rows:
                 L_rows = (L_rows + 7) // 8 * 8
         T = sum(span) + n_fake + n_pad_rows
+        # The order the entries' rows stand in.  In float32 linear layers run the rows of portions and single rows through different
+        # kernels, whichever others share the step: the portions come first (with the rows without a request right behind them).
+        order = list(range(n_real))
+        portions_first = self.model.dtype == torch.float32 and n_portions > 0
+        if portions_first:
+            order.sort(key=lambda i: len(entries[i].tokens) == 1)
         n_listed = R - n_single_rows if n_portions and self._recurrences else 0
         mixed = 0 < n_single_rows < n_real + n_fake
         off, sizes = {}, [("tokens", T), ("positions", T), ("token_req", T), ("logit_rows", L_rows), ("slots", R),
@@ -383,12 +392,17 @@ class Engine:
         h[off["token_req"]: off["token_req"] + T] = -1
         try:
             t0 = 0
-            rows: List[int] = []
             single_rows: List[int] = []
             portion_rows: List[int] = []
             tiles: List[tuple] = []
             single_tiles: List[tuple] = []
-            for r, e in enumerate(entries):
+            first_rows = [0] * n_real
+            for r, i in enumerate(order):
+                e = entries[i]
+                if portions_first and r == n_portions:
+                    if mixed:
+                        portion_rows.extend(range(t0, t0 + n_pad_rows))
+                    t0 += n_pad_rows
                 n = len(e.tokens)
                 start = mgr.reserve(e.rid, n)
                 slot = mgr.requests[e.rid].slot
@@ -398,16 +412,17 @@ class Engine:
                 h[off["slots"] + r] = slot
                 h[off["req_first_token"] + r] = t0
                 h[off["req_first_position"] + r] = start
-                rows.extend(t0 + w for w in e.want)
+                first_rows[i] = t0
                 if mixed:
-                    (single_rows if n == 1 else portion_rows).extend(range(t0, t0 + span[r]))
+                    (single_rows if n == 1 else portion_rows).extend(range(t0, t0 + span[i]))
                 if n > 1:
                     tiles.extend((t0 + a, min(TQ, n - a), r, start + a) for a in range(0, n, TQ))
                 else:
                     single_tiles.append((t0, 1, r, start))
                 ctx.spans.append(RequestSpan(e.rid, slot, t0, n, start))
                 ctx.max_q_len = max(ctx.max_q_len, n)
-                t0 += span[r]
+                t0 += span[i]
+            rows = [t + w for t, e in zip(first_rows, entries) for w in e.want]
             for f in range(n_fake):                      # filler single-token entries
                 r = n_real + f
                 h[off["slots"] + r] = 0
@@ -417,7 +432,7 @@ class Engine:
                     single_rows.append(t0)
                 single_tiles.append((t0, 0, 0, 0))
                 t0 += 1
-            if mixed and n_pad_rows:
+            if mixed and n_pad_rows and not portions_first:
                 portion_rows.extend(range(t0, t0 + n_pad_rows))        # rows without a request: every kernel skips them
             for r in range(n_real + n_fake, R):                        # requests that only fill the tables up
                 h[off["slots"] + r] = 0
@@ -439,9 +454,9 @@ class Engine:
                     np.asarray(single_tiles, dtype=np.int32).reshape(-1)
             ctx.portions = tuple((s.first_position, s.n_tokens) for s in ctx.spans if s.n_tokens > 1)
             if n_listed:
-                listed = sorted((r for r, e in enumerate(entries) if len(e.tokens) > 1), key=lambda r: -len(entries[r].tokens))
+                listed = sorted((r for r, i in enumerate(order) if len(entries[i].tokens) > 1), key=lambda r: -len(entries[order[r]].tokens))
                 h[off["portion_requests"]: off["portion_requests"] + n_listed] = listed + [-1] * (n_listed - n_portions)
-            rids = [e.rid for e in entries]
+            rids = [entries[i].rid for i in order]
             for g in range(len(mgr.kv_groups)):
                 o = off[f"table{g}"]
                 h[o: o + R * W] = -1
@@ -456,6 +471,7 @@ class Engine:
             ctx.req_first_token, ctx.req_first_position = view("req_first_token", R + 1), view("req_first_position", R)
             ctx._slots = view("slots", R)
             ctx.n_single, ctx.n_portion = n_single_rows, T - n_single_rows
+            ctx.leading_portion_rows = T - n_single_rows if portions_first else 0
             if mixed:
                 ctx.single_rows = view("single_rows", n_single_rows)
                 ctx.portion_rows = view("portion_rows", T - n_single_rows)

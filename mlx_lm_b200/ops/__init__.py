@@ -352,10 +352,12 @@ def linear_split_supported(x, w, out, residual=None) -> bool:
     return not any(t is not None and t.data_ptr() % 16 for t in (x, w, out, residual))
 
 
-def linear_split_pays(M: int, N: int, K: int) -> bool:
-    """Whether ``linear_split`` takes less time than ``linear_generic``: from 17 rows on (up to 16 the few-rows kernel, 6 us at
-    1024 x 1024, to 28) and two blocks of K (20 rows, 512 x 128: 8.2 us to 10.0; 20 and 300 rows with 64 of K 6.9 and 7.7 to 6.4 and 6.9)."""
-    return M > 16 and K >= 128
+def linear_split_pays(K: int) -> bool:
+    """Whether ``linear_split`` takes less time than ``linear_generic`` for 17 rows and more: from two blocks of K on, whatever the
+    outputs (17 and 737 rows, split and generic: 1024 x 1024 24.7 to 49.4 us and 24.6 to 72.8, 1024 x 128 6.2 to 7.7 and 7.2 to 16.3,
+    64 x 512 12.7 to 21.8 and 13.3 to 25.7; with 64 of K 20 and 300 rows 6.9 and 7.7 to 6.4 and 6.9).  Up to 16 rows the generic
+    layer's few-rows kernel is the faster one (1024 x 1024: 2.7 to 6 us)."""
+    return K >= 128
 
 
 def linear_split(x, w, bias, out, status, stream, epilogue: int = EPI_NONE, residual=None) -> None:

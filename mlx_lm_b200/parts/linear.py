@@ -106,10 +106,12 @@ class Linear(Part):
         ops.row_stats(src, stats, f.eps, ctx.stream)
         return (f.colsum, stats)
 
-    def forward(self, ctx, x, out, activation=None, residual=None) -> torch.Tensor:
-        """float32: the generic kernel (true 32-bit arithmetic), or for more than a few rows the tensor cores at the same precision.  bfloat16: the weight-streaming kernel for up
-        to 64 rows, the tcgen05 kernel for more; an inner size that is no multiple of 8 (no 16-byte rows)
-        goes to the generic kernel."""
+    def forward(self, ctx, x, out, activation=None, residual=None, step_rows: bool = True) -> torch.Tensor:
+        """bfloat16: the weight-streaming kernel for up to 64 rows, the tcgen05 kernel for more; an inner size that is no multiple of 8
+        (no 16-byte rows) goes to the generic kernel.  float32: the generic kernel (true 32-bit arithmetic), but rows of requests that
+        bring several tokens go through the tensor cores at the same precision.  Which of the two a row takes, whose sums differ by
+        rounding, so depends on its own request alone and never on how many others share the step.  ``step_rows=False``: the rows
+        of ``x`` are not the step's (the wanted ones): the generic kernel."""
         epi = ACTIVATIONS[activation]
         M = x.shape[0]
         few = self.few_rows(x.shape[0])      # decided once, before the fold's argument is made for that kernel
@@ -122,17 +124,27 @@ class Linear(Part):
                                   f"Normed, not a tensor")
         fast = (x.dtype == torch.bfloat16 and self.n_in % 8 == 0 and x.stride(0) % 8 == 0
                 and x.data_ptr() % 16 == 0)
-        ops.label(self.name, 2.0 * M * self.n_in * self.n_out,
-                  self.weight.element_size() * (self.n_in * self.n_out + M * self.n_in) + out.element_size() * M * self.n_out)
+        def label(rows):
+            ops.label(self.name, 2.0 * rows * self.n_in * self.n_out, self.weight.element_size() * (self.n_in * self.n_out + rows * self.n_in)
+                      + out.element_size() * rows * self.n_out)
+        label(M)
         if fast and few:
             ops.linear_few_rows(x, self.weight, self.bias, out, ctx.stream, epilogue=epi, residual=residual, fold=fold)
         elif fast:
             ops.linear_tensor_cores(x, self.weight, self.bias, out, ctx.status, ctx.stream, epilogue=epi,
                                     residual=residual, fold=fold)
-        elif ops.linear_split_supported(x, self.weight, out, residual) and ops.linear_split_pays(M, self.n_out, self.n_in):
-            ops.linear_split(x, self.weight, self.bias, out, ctx.status, ctx.stream, epilogue=epi, residual=residual)
         else:
-            ops.linear_generic(x, self.weight, self.bias, out, ctx.stream, epilogue=epi, residual=residual)
+            n = getattr(ctx, "leading_portion_rows", 0) if step_rows and M == ctx.n_tokens else 0
+            if n and ops.linear_split_pays(self.n_in) and ops.linear_split_supported(x, self.weight, out, residual):
+                label(n)
+                ops.linear_split(x[:n], self.weight, self.bias, out[:n], ctx.status, ctx.stream, epilogue=epi,
+                                 residual=None if residual is None else residual[:n])
+            else:
+                n = 0
+            if n < M:
+                label(M - n)
+                ops.linear_generic(x[n:], self.weight, self.bias, out[n:], ctx.stream, epilogue=epi,
+                                   residual=None if residual is None else residual[n:])
         return out
 
 

@@ -141,7 +141,7 @@ class OutputHead(Part):
 
     def forward(self, ctx, x):
         out = ctx.ws.get("logits", x.shape[0], self.vocab_size, torch.float32)
-        out = self.linear.forward(ctx, x, out)
+        out = self.linear.forward(ctx, x, out, step_rows=False)
         if self.softcap:
             ops.label("head.softcap", 3.0 * out.numel(), 8.0 * out.numel())
             ops.soft_cap(out, self.softcap, ctx.stream)

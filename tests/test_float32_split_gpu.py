@@ -4,6 +4,7 @@ import math
 import pytest
 import torch
 
+from helpers import CONFIG_C, make_model_dir, random_tokens
 from test_kernels_gpu import rel_err, stream
 
 pytestmark = pytest.mark.gpu
@@ -67,3 +68,48 @@ def test_float32_linear_in_parts_of_numbers_at_the_ends(ops):
     assert bool(fine[50].any()) and bool(fine[60].any())
     for r in (0, 50, 60, 199):
         assert rel_err(out[r][fine[r]], plain[r][fine[r]]) <= 1e-6
+
+
+def test_rows_of_a_step_whatever_others_share_it(tmp_path):
+    """A float32 engine: the logits of a request that brings one token, and of one that brings several, have the same bits alone and
+    beside others, few or many, before or behind them among the step's entries."""
+    from mlx_lm_b200.engine import Engine, StepEntry
+    from mlx_lm_b200.weights import load_model
+    make_model_dir(str(tmp_path), CONFIG_C, 11, peaky=3.0)
+    model, _ = load_model(str(tmp_path), dtype="float32", device="cuda:0")
+    V, N = CONFIG_C["vocab_size"], 40
+    engine = Engine(model, page_size=16, n_pages=4 * N + 64, max_requests=N + 1)
+    for r in range(N):
+        engine.add_request(r)
+        engine.step([StepEntry(r, random_tokens(20 + r, V, r))])
+    engine.add_request("p")
+    prompt = random_tokens(270, V, 77)
+    first, rest = prompt[:170], prompt[170:]
+
+    def logits(ones, place=None, wanted=(0, 99)):
+        entries = [StepEntry(r, [3 * r + 1], [0]) for r in ones]
+        if place is not None:
+            engine.step([StepEntry("p", first)])
+            entries.insert(place, StepEntry("p", rest, list(wanted)))
+        got = engine.step(entries)
+        by, at = {}, 0
+        for e in entries:
+            by[e.rid] = got[at:at + len(e.want)].clone()
+            at += len(e.want)
+        for r in ones:
+            engine.cache.truncate(r, 20 + r)
+        engine.cache.truncate("p", 0)
+        return by
+
+    alone = {r: logits([r])[r] for r in range(N)}
+    portion = logits([], 0)["p"]
+    assert float((alone[0] - alone[1]).abs().max()) > 1e-3
+    for ones, place in ((range(16), None), (range(17), None), (range(N), None), ([5], 0), (range(17), 17), (range(N), 3), ([2, 1], 1)):
+        by = logits(list(ones), place)
+        for r in ones:
+            assert torch.equal(by[r], alone[r]), (r, len(ones), place)
+        if place is not None:
+            assert torch.equal(by["p"], portion), (len(ones), place)
+    every = logits([4], 0, range(100))["p"]                     # more wanted rows: the output head runs more rows
+    assert torch.equal(every[[0, 99]], portion)
+    engine.check_status()
