@@ -1022,27 +1022,27 @@ gated_delta_second_kernel(const __nv_bfloat16* qkv, int ldq, int q_off, int k_of
     }
 }
 
-// Floats of scratch memory for the two passes over runs of n_requests requests with n_tokens rows together.
-MLXB_EXPORT long long mlxb_gated_delta_chunks_scratch(int n_tokens, int n_requests, int H) {
-  return ((long long)n_tokens / RC_Q + n_requests) * H * (long long)(sizeof(DeltaChunk) / sizeof(float));
+// Floats of scratch memory for the two passes over runs of `jobs` chunks at most.
+MLXB_EXPORT long long mlxb_gated_delta_chunks_scratch(int jobs, int H) {
+  return (long long)jobs * H * (long long)(sizeof(DeltaChunk) / sizeof(float));
 }
 
 // The arguments of mlxb_gated_delta_scan (bfloat16 inputs, states of up to 64 rows); requests with a single row are left out.
-// scratch: null (one kernel), or memory of mlxb_gated_delta_chunks_scratch floats, 16-byte aligned (two passes).
+// scratch: null (one kernel), or memory of mlxb_gated_delta_chunks_scratch floats, 16-byte aligned (two passes).  jobs: the chunks of
+// the listed requests' rows, no fewer (their rows / 64 and a chunk a request are enough).
 MLXB_EXPORT int mlxb_gated_delta_chunks(const void* qkv, int ldq, int q_off, int k_off, int v_off, const void* b_raw, int ldb,
                                         const void* a_raw, int lda, const float* dt_bias, const float* A_log, float* state,
                                         const int* slots, const int* token_req, const int* req_first_token, float* o, int ldo, int H,
                                         int G, int K, int V, const int* requests, int n_requests, int scan_fixed, int scan_row,
-                                        int chunk_fixed, int chunk_each, int n_tokens, float* scratch, cudaStream_t stream) {
+                                        int chunk_fixed, int chunk_each, int jobs, float* scratch, cudaStream_t stream) {
   if (n_requests <= 0) return 0;
   if (H <= 0 || G <= 0 || H % G || K <= 0 || V <= 0 || K > GD_KP || n_requests > 65535)
     return mlxb_fail(MLXB_BAD_ARG, "gated_delta_chunks: %d heads over %d key heads, state %d x %d (at most %d rows)", H, G, K, V, GD_KP);
   const int vec = (((uintptr_t)qkv & 15) == 0 && ldq % 8 == 0 && q_off % 8 == 0 && k_off % 8 == 0 && v_off % 8 == 0 && K % 8 == 0 &&
                    V % 8 == 0);
   if (scratch != nullptr) {
-    const long long jobs = (long long)n_tokens / RC_Q + n_requests;
-    if (n_tokens <= 0 || jobs > 65535 || ((uintptr_t)scratch & 15))
-      return mlxb_fail(MLXB_BAD_ARG, "gated_delta_chunks: %d rows of %d requests, scratch memory not 16-byte aligned", n_tokens, n_requests);
+    if (jobs <= 0 || jobs > 65535 || ((uintptr_t)scratch & 15))
+      return mlxb_fail(MLXB_BAD_ARG, "gated_delta_chunks: %d chunks of %d requests, scratch memory 16-byte aligned", jobs, n_requests);
     static_assert(sizeof(DeltaChunk) % 16 == 0 && sizeof(DeltaSecondMemory) <= 227 * 1024, "pieces of 16 bytes; a block's shared memory");
     static SharedLimit limits[2];
     cudaError_t e = limits[0].raise(gated_delta_first_kernel, sizeof(DeltaFirstMemory));

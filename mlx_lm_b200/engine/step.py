@@ -57,13 +57,16 @@ class Workspace:
             self.generation += 1
         return buf[:rows]
 
-    def flat(self, tag: str, n: int, dtype: torch.dtype) -> torch.Tensor:
-        """Scratch memory of at least ``n`` elements whose size varies from step to step."""
+    def flat(self, tag: str, n: int, dtype: torch.dtype, most: Optional[int] = None) -> torch.Tensor:
+        """Scratch memory of at least ``n`` elements whose size varies from step to step: when it grows, to twice what it was, but not
+        beyond ``most`` elements (where the caller never asks for more)."""
         key = (tag, 0, dtype)
         buf = self._bufs.get(key)
         if buf is None or buf.numel() < n:
-            buf = torch.zeros(max(n, 1024, 2 * (buf.numel() if buf is not None else 0)), dtype=dtype,
-                              device=self.device)   # zero: ticket counters of kernels start from zero
+            room = max(n, 1024, 2 * (buf.numel() if buf is not None else 0))
+            if most is not None:
+                room = max(n, min(room, most))
+            buf = torch.zeros(room, dtype=dtype, device=self.device)   # zero: ticket counters of kernels start from zero
             self._bufs[key] = buf
             self.generation += 1
         return buf
@@ -162,8 +165,13 @@ class StepContext:
             return False
         key = ("side by side", recurrence)
         if key not in self._choices:
-            self._choices[key] = ops.chunks_side_by_side(*recurrence, tuple(n for _, n in self.portions), sms=ops.sm_count())
+            self._choices[key] = ops.chunks_side_by_side(*recurrence, tuple(n for _, n in self.portions), sms=ops.sm_count(),
+                                                         jobs=self.chunk_jobs())
         return self._choices[key]
+
+    def chunk_jobs(self) -> int:
+        """No fewer than the chunks of 64 rows of the listed requests (``portion_requests``)."""
+        return ops.delta_chunk_jobs(self.n_portion, self.portion_requests.numel())
 
     def attention_in_tiles(self, attention: tuple) -> bool:
         """Whether float32 portions run in tiles (see ``ops.attention_portions_f32_pays``)."""

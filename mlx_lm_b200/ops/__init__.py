@@ -1152,18 +1152,27 @@ def chunk_rule(kind: str, n_heads: int, state_rows: int, columns: int, runs, sms
     return CHUNKS if all(ways) else rule if any(ways) else None
 
 
-def chunks_side_by_side(kind: str, n_heads: int, state_rows: int, columns: int, runs, sms: int = 148) -> bool:
+# Chunks, heads counted, of one step in the delta rule's two passes: each leaves 50 KB between them, so 0.4 GB of scratch memory.
+DELTA_CHUNK_HEADS = 8192
+
+
+def delta_chunk_jobs(n_rows: int, n_requests: int) -> int:
+    """The most chunks of 64 rows that ``n_requests`` runs of ``n_rows`` rows together have."""
+    return n_rows // 64 + n_requests
+
+
+def chunks_side_by_side(kind: str, n_heads: int, state_rows: int, columns: int, runs, sms: int = 148, jobs: Optional[int] = None) -> bool:
     """Whether runs that go through the delta rule in chunks do so in two passes, what needs no state for all chunks side by side.
+    ``jobs``: the ``delta_chunk_jobs`` that scratch memory is for (default: of the runs); at most ``DELTA_CHUNK_HEADS`` with heads.
     Microseconds: the one kernel takes 10 a chunk of the longest run and wave of blocks; of the two passes the second 4, the first 8 a wave
     of its blocks (a chunk and head each, two on an SM), and a launch 5.  Measured, 16 heads of 64 x 64, one kernel and two: two runs
-    of 1024 rows 162 and 106, one of 200 43 and 35, of 128 23.3 and 24.8, four of 64 13.7 and 23.8, eight of 100 44.8 and 40.2, eight of
-    500 164 and 136; 32 heads, four of 256 85 and 74.  A chunk and head leaves 50 KB of scratch memory between the passes: at most 8192 of
-    them (0.4 GB)."""
+    of 1024 rows 160 and 105, one of 200 42 and 34, of 128 22.5 and 23.3, four of 64 12.9 and 22.8, eight of 100 44 and 39, eight of
+    500 162 and 133; 32 heads, four of 256 84 and 72."""
     if kind != "delta" or not runs or state_rows > DELTA_CHUNK_ROWS:
         return False
-    chunks = [-(-n // 64) for n in runs]
-    if sum(chunks) * n_heads > 8192:
+    if (delta_chunk_jobs(sum(runs), len(runs)) if jobs is None else jobs) * n_heads > DELTA_CHUNK_HEADS:
         return False
+    chunks = [-(-n // 64) for n in runs]
     waves = -(-len(runs) * n_heads * -(-columns // 32) // sms)
     first = -(-sum(chunks) * n_heads // (2 * sms))
     return waves * 10 * max(chunks) > 5 + 8 * first + waves * 4 * max(chunks)
@@ -1248,19 +1257,20 @@ def gated_delta_scan(qkv, q_off: int, k_off: int, v_off: int, b_raw, a_raw, dt_b
           _rows(o, "gated_delta o"), H, n_key_heads, K, V, slots.numel(), int(max_run), *rule, stream)
 
 
-def gated_delta_chunks_scratch(n_tokens: int, n_requests: int, n_heads: int) -> int:
-    """Floats of scratch memory for ``gated_delta_chunks`` over ``n_tokens`` rows of ``n_requests`` listed requests."""
-    f, _ = _fn("recurrent_chunks", "mlxb_gated_delta_chunks_scratch", [c_int] * 3)
+def gated_delta_chunks_scratch(jobs: int, n_heads: int) -> int:
+    """Floats of scratch memory for ``gated_delta_chunks`` over ``jobs`` chunks (``delta_chunk_jobs``)."""
+    f, _ = _fn("recurrent_chunks", "mlxb_gated_delta_chunks_scratch", [c_int] * 2)
     f.restype = ctypes.c_longlong
-    return int(f(n_tokens, n_requests, n_heads))
+    return int(f(jobs, n_heads))
 
 
 def gated_delta_chunks(qkv, q_off: int, k_off: int, v_off: int, b_raw, a_raw, dt_bias, a_log, state, slots, token_req,
                        req_first_token, o, n_heads: int, n_key_heads: int, stream, requests=None,
-                       rule: ChunkRule = CHUNKS, scratch=None) -> None:
+                       rule: ChunkRule = CHUNKS, scratch=None, jobs: Optional[int] = None) -> None:
     """``gated_delta_scan`` for the requests whose runs ``rule`` sends here, 64 rows at a time on tensor cores (bfloat16 inputs,
     csrc/recurrent_chunks.cu).  ``requests`` as for ``mamba2_chunks``.  ``scratch`` (float32, at least
-    ``gated_delta_chunks_scratch`` elements): what the chunks of a run need no state for is done for all of them side by side."""
+    ``gated_delta_chunks_scratch`` elements): what the chunks of a run need no state for is done for all of them side by side.
+    ``jobs``: no fewer chunks than the listed requests' rows have (default: as if all rows were theirs)."""
     _need(state, torch.float32, "gated_delta_chunks state")
     _need(o, torch.float32, "gated_delta_chunks o")
     for t in (qkv, b_raw, a_raw):
@@ -1269,14 +1279,15 @@ def gated_delta_chunks(qkv, q_off: int, k_off: int, v_off: int, b_raw, a_raw, dt
     if H != n_heads or o.shape[1] != H * V or not state.is_contiguous() or K > DELTA_CHUNK_ROWS:
         raise KernelError(f"gated_delta_chunks: state {tuple(state.shape)} for {n_heads} heads, o {tuple(o.shape)}")
     listed, n_listed = _requests(requests, slots, "gated_delta_chunks")
+    jobs = delta_chunk_jobs(qkv.shape[0], n_listed) if jobs is None else int(jobs)
     if scratch is not None:
         _need(scratch, torch.float32, "gated_delta_chunks scratch")
-        if scratch.numel() < gated_delta_chunks_scratch(qkv.shape[0], n_listed, H):
-            raise KernelError(f"gated_delta_chunks: {scratch.numel()} floats of scratch memory for {qkv.shape[0]} rows")
+        if scratch.numel() < gated_delta_chunks_scratch(jobs, H):
+            raise KernelError(f"gated_delta_chunks: {scratch.numel()} floats of scratch memory for {jobs} chunks")
     _call("recurrent_chunks", "mlxb_gated_delta_chunks", _GD_CHUNKS_ARGS, _p(qkv), _rows(qkv, "gated_delta qkv"),
           q_off, k_off, v_off, _p(b_raw), _rows(b_raw, "gated_delta b"), _p(a_raw), _rows(a_raw, "gated_delta a"),
           _p(dt_bias), _p(a_log), _p(state), _p(slots), _p(token_req), _p(req_first_token), _p(o),
-          _rows(o, "gated_delta o"), H, n_key_heads, K, V, listed, n_listed, *rule, qkv.shape[0], _p(scratch), stream)
+          _rows(o, "gated_delta o"), H, n_key_heads, K, V, listed, n_listed, *rule, jobs, _p(scratch), stream)
 
 
 # --------------------------------------------------------------------------

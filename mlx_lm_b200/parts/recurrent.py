@@ -169,8 +169,9 @@ class GatedDeltaMixer(Mixer):
         if rule is not None:
             scratch = None
             if ctx.chunks_side_by_side(self.chunked_recurrence):
-                scratch = ctx.ws.flat("delta_chunks", ops.gated_delta_chunks_scratch(T, ctx.portion_requests.numel(), H), torch.float32)
-            ops.gated_delta_chunks(*args, requests=ctx.portion_requests, rule=rule, scratch=scratch)
+                most = ops.gated_delta_chunks_scratch(ops.DELTA_CHUNK_HEADS // H, H)
+                scratch = ctx.ws.flat("delta_chunks", ops.gated_delta_chunks_scratch(ctx.chunk_jobs(), H), torch.float32, most=most)
+            ops.gated_delta_chunks(*args, requests=ctx.portion_requests, rule=rule, scratch=scratch, jobs=ctx.chunk_jobs())
         if rule is not ops.CHUNKS or ctx.n_single:
             ops.gated_delta_scan(*args, max_run=0 if rule is None else 1, rule=rule or ops.CHUNKS)
         g = ctx.ws.get("delta_gated", T, self.v_width, x.dtype)

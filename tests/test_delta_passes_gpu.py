@@ -15,7 +15,7 @@ def two_passes(monkeypatch):
 
     def wrapped(*a, requests=None, **k):
         n = a[9].numel() if requests is None else requests.numel()
-        scratch = torch.full((ops.gated_delta_chunks_scratch(a[0].shape[0], n, a[13]),), float("nan"), device="cuda")
+        scratch = torch.full((ops.gated_delta_chunks_scratch(ops.delta_chunk_jobs(a[0].shape[0], n), a[13]),), float("nan"), device="cuda")
         calls.append(n)
         return real(*a, requests=requests, scratch=scratch, **k)
     monkeypatch.setattr(ops, "gated_delta_chunks", wrapped)
