@@ -746,6 +746,15 @@ def sm_count() -> int:
     return _sm_count
 
 
+def rows_beside_pay(n_rows: int, n_tiles: int, n_heads: int) -> bool:
+    """Whether single rows whose kernel runs beside the portions' take less time than after one another: always, except for many rows
+    beside a few tiles of 128 queries, which then wait for the rows' blocks to leave.  Microseconds a layer, one after the other and
+    beside: 64 rows at 900 positions, 16 heads, portions of 64, 256 and 1024 rows 56.4, 60.2, 75.7 and 56.5, 57.4, 66.3; 32 rows 35.2,
+    38.9, 54.1 and 33.2, 34.0, 46.9; one row and 1024 of a portion 26.7 and 25.0; 128 rows at 400, 20 heads, and 256 68.6 and 71.3, at
+    900, 16 heads, and 128 100.8 and 103.8; but 192 rows, 20 heads, and 512 99.4 and 99.2, 128 rows, 25 heads, and 1024 136.5 and 132.2."""
+    return n_rows * n_heads < 2048 or n_tiles * n_heads >= 80
+
+
 def attention_rows(q, tiles, n_rows: int, block_table, k_pool, v_pool, out, n_heads: int, scale: float, window: int,
                    status, stream, sinks=None, beside: bool = False) -> None:
     """Attention of rows with a single query each (decode steps) on tensor cores (bfloat16,

@@ -99,7 +99,8 @@ def paged_attention(ctx, q, cache, o, n_heads: int, head_dim: int, scale: float,
     portions = (ctx.n_portion and ctx.portion_tiles is not None
                 and ops.attention_portions_supported(q.dtype, head_dim, scale))
     # rows and portions know nothing of each other: where the portions' kernel lets them, the rows run beside it
-    beside = bool(portions and ctx.n_single and ops.attention_portions_tc_supported(q, o, cache.k, cache.v))
+    beside = bool(portions and ctx.n_single and ops.attention_portions_tc_supported(q, o, cache.k, cache.v)
+                  and ops.rows_beside_pay(ctx.n_single, ctx.n_portion_tiles, n_heads))
 
     def in_portions() -> None:
         ops.attention_portions(q, ctx.portion_tiles, ctx.n_portion_tiles, cache.block_table, cache.k, cache.v, o, n_heads, scale,

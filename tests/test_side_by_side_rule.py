@@ -1,4 +1,5 @@
-"""Which runs of the gated delta rule go through it in two passes (``ops.chunks_side_by_side``)."""
+"""Which runs of the gated delta rule go through it in two passes (``ops.chunks_side_by_side``), and which single rows' attention runs
+beside that of portions (``ops.rows_beside_pay``)."""
 import torch
 
 from mlx_lm_b200 import ops
@@ -33,3 +34,8 @@ def test_scratch_memory_grows_up_to_its_limit():
     f = lambda n: ws.flat("x", n, torch.float32, most=10000).numel()
     assert [f(3000), f(3000), f(3001), f(6001), f(9000), f(10000)] == [3000, 3000, 6000, 10000, 10000, 10000]
     assert ws.flat("y", 3000, torch.float32).numel() == 3000 and ws.flat("y", 3001, torch.float32).numel() == 6000
+
+
+def test_many_rows_do_not_run_beside_few_tiles():
+    assert ops.rows_beside_pay(1, 1, 16) and ops.rows_beside_pay(64, 1, 25) and ops.rows_beside_pay(128, 8, 25)
+    assert not ops.rows_beside_pay(128, 1, 16) and not ops.rows_beside_pay(128, 2, 20)
