@@ -45,8 +45,8 @@ def test_order_of_kernels_and_of_runs(two_passes):
     one.test_every_run_goes_one_way("delta rule")
 
 
-def test_error_against_64_bits_is_no_larger(two_passes):
-    """1000 rows, random and slow: within what the one kernel is held to, twice the error of the scan in float32 or some roundings."""
+def test_error_against_64_bits_is_no_larger():
+    """1000 rows, random and slow: no further from 64 bits than the one kernel, up to the tenth that the order of roundings moves."""
     from mlx_lm_b200 import ops
     errors = {}
     for slow in (False, True):
@@ -71,13 +71,15 @@ def test_error_against_64_bits_is_no_larger(two_passes):
             u = beta[t, :, None] * (v[t] - torch.einsum("hkv,k->hv", S, k[t]))
             S = S + k[t][None, :, None] * u[:, None, :]
             want[t] = torch.einsum("hkv,k->hv", S, q[t])
-        for name, f in (("two", ops.gated_delta_chunks), ("scan", ops.gated_delta_scan)):
+        scratch = torch.empty(ops.gated_delta_chunks_scratch(ops.delta_chunk_jobs(T + 2, 1), H), device="cuda")
+        for name, f, kw in (("two", ops.gated_delta_chunks, dict(scratch=scratch)), ("one", ops.gated_delta_chunks, {}),
+                            ("scan", ops.gated_delta_scan, {})):
             state, o = torch.zeros(1, H, V, K, device="cuda"), torch.zeros(T + 2, H * V, device="cuda")
             f(qkv, 0, K, 2 * K, b, a, dt_bias, a_log, state, torch.zeros(1, dtype=torch.int32, device="cuda"), token_req, first, o, H, 1,
-              ops.current_stream())
+              ops.current_stream(), **kw)
             errors[slow, name] = (float((o[:T].view(T, H, V) - want).norm() / want.norm()),
                                   float((state[0].transpose(1, 2) - S).norm() / S.norm()))
     print(errors)
-    for slow in (False, True):      # the scan, token by token in float32, is the measure that the one kernel is held to as well
-        for two, scan in zip(errors[slow, "two"], errors[slow, "scan"]):
-            assert two < max(2 * scan, 2e-7), errors
+    for slow in (False, True):
+        for two, one_kernel in zip(errors[slow, "two"], errors[slow, "one"]):
+            assert two < 1.1 * one_kernel, errors
