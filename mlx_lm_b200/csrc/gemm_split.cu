@@ -48,6 +48,7 @@ struct Smem {
   alignas(1024) __nv_bfloat16 a[2][3][BM * BK];      // [buffer][part]
   alignas(1024) __nv_bfloat16 w[2][3][BN * BK];
   alignas(16) uint4 stage[SUM_WARPS][32 * 4];        // 64 bytes of each of a warp's 32 rows on their way out
+  uint32_t bad[SUM_WARPS][BN / 8];                   // per eight rows and 16 columns the pieces of four columns that are not finite
   uint64_t full[2], empty[2];                        // a buffer's parts are written / have been multiplied
   uint64_t acc_full[2], acc_empty[2];
   uint64_t drained;                                  // abort path only
@@ -93,12 +94,24 @@ __device__ __forceinline__ void tmem_get16(uint32_t taddr, uint32_t (&r)[16]) {
       : "r"(taddr) : "memory");
 }
 
-// A row of A times a row of W in plain float32, by a warp; the same in every lane.
-__device__ __noinline__ float plain_dot(const float* a, const float* w, int K) {
-  const int lane = threadIdx.x & 31;
-  float s = 0.f;
-  for (int k = lane; k < K; k += 32) s = fmaf(a[k], w[k], s);
-  return warp_sum(s);
+// A row of A times up to four neighbouring rows of W in plain float32, by a warp; the same in every lane.
+__device__ __noinline__ float4 plain_dots(const float* a, const float* w, int rows, int K) {
+  float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 2
+  for (int k = (threadIdx.x & 31) * 4; k < K; k += 128) {
+    const float4 x = *reinterpret_cast<const float4*>(a + k);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if (e >= rows) continue;
+      const float4 y = *reinterpret_cast<const float4*>(w + (size_t)e * K + k);
+      s[e] = fmaf(x.w, y.w, fmaf(x.z, y.z, fmaf(x.y, y.y, fmaf(x.x, y.x, s[e]))));
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) s[e] += __shfl_xor_sync(0xffffffffu, s[e], o);
+  return make_float4(s[0], s[1], s[2], s[3]);
 }
 
 __device__ __forceinline__ int stage_index(int row, int piece) { return row * 4 + (piece ^ ((row >> 1) & 3)); }
@@ -252,6 +265,7 @@ linear_split_kernel(const float* A, const float* __restrict__ W, const float* __
       }
       if (kt < blocks) break;
       const int m0 = tile_m0(t) + q * 32, n0 = tile_n0(t) + half * COLS;
+      unsigned any_bad = 0;
 #pragma unroll
       for (int c = 0; c < COLS; c += 16) {             // 64 bytes of each row at a time
 #pragma unroll
@@ -269,18 +283,10 @@ linear_split_kernel(const float* A, const float* __restrict__ W, const float* __
           const uint4 u = stg[stage_index(8 * j + o_row, o_piece)];
           float v[4] = {__uint_as_float(u.x), __uint_as_float(u.y), __uint_as_float(u.z), __uint_as_float(u.w)};
           const bool fine = fabsf(v[0]) < INFINITY && fabsf(v[1]) < INFINITY && fabsf(v[2]) < INFINITY && fabsf(v[3]) < INFINITY;
-          unsigned bad = __ballot_sync(0xffffffffu, !fine && m < M && n < N);
-          while (bad) {
-            const int src = __ffs(bad) - 1;
-            bad &= bad - 1;
-            const int mm = __shfl_sync(0xffffffffu, m, src), nn = __shfl_sync(0xffffffffu, n, src);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float s = nn + e < N ? plain_dot(A + (size_t)mm * lda, W + (size_t)(nn + e) * K, K) : 0.f;
-              if (lane == src) v[e] = s;
-            }
-          }
-          if (m >= M || n >= N) continue;
+          const unsigned bad = __ballot_sync(0xffffffffu, !fine && m < M && n < N);
+          if (lane == 0) sm.bad[warp - SPLIT_WARPS][c / 4 + j] = bad;
+          any_bad |= bad;
+          if (m >= M || n >= N || !fine) continue;
           const size_t o = (size_t)m * ldc + n;
 #pragma unroll
           for (int e = 0; e < 4; ++e) v[e] = activate<EPI, false>(v[e] + bs[e]);
@@ -298,6 +304,19 @@ linear_split_kernel(const float* A, const float* __restrict__ W, const float* __
         }
         __syncwarp();                                  // the pieces are read before the next ones overwrite them
       }
+      // What is not finite, after all the others: the sums need no registers any more (a call in the loop above cost every call 5 %).
+      for (int piece = 0; any_bad && piece < COLS / 4; ++piece)
+        for (unsigned bad = sm.bad[warp - SPLIT_WARPS][piece]; bad; bad &= bad - 1) {
+          const int src = __ffs(bad) - 1, m = m0 + 8 * (piece & 3) + (src >> 2), n = n0 + (piece >> 2) * 16 + (src & 3) * 4;
+          const float4 s = plain_dots(A + (size_t)m * lda, W + (size_t)n * K, min(4, N - n), K);
+          if (lane < 4 && n + lane < N) {
+            const size_t o = (size_t)m * ldc + n + lane;
+            const float x = lane == 0 ? s.x : lane == 1 ? s.y : lane == 2 ? s.z : s.w;
+            const float v = activate<EPI, false>(x + (bias != nullptr ? bias[n + lane] : 0.f));
+            C[o] = residual != nullptr ? v + residual[o] : v;
+          }
+        }
+      __syncwarp();
     }
   }
 

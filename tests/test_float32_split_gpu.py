@@ -70,6 +70,33 @@ def test_float32_linear_in_parts_of_numbers_at_the_ends(ops):
         assert rel_err(out[r][fine[r]], plain[r][fine[r]]) <= 1e-6
 
 
+def test_float32_linear_in_parts_with_many_rows_that_are_not_finite(ops):
+    """Every number of such rows among the 32 that a warp finishes: as in plain float32, and the other rows' bits as without them."""
+    M, N, K = 300, 150, 260
+    g = torch.Generator(device="cuda").manual_seed(6)
+    x, w = torch.randn(M, K, generator=g, device="cuda"), torch.randn(N, K, generator=g, device="cuda") / 16
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out, clean, plain = (torch.empty(M, N, device="cuda") for _ in range(3))
+    ops.linear_split(x, w, None, clean, status, stream())
+    bad = list(range(32)) + [40] + list(range(64, 71)) + list(range(97, 100)) + [130]
+    x[:32, 3], x[40], x[64:71, 259], x[97:100, 7] = math.nan, math.nan, math.inf, -math.inf
+    x[130], x[130, 1] = 0.0, 3.4e38                  # bfloat16 rounds it to infinity
+    ops.linear_split(x, w, None, out, status, stream())
+    ops.linear_generic(x, w, None, plain, stream())
+    assert int(status.item()) == 0
+    others = [r for r in range(M) if r not in bad]
+    assert torch.equal(out[others], clean[others])
+    assert torch.equal(torch.isnan(out), torch.isnan(plain)) and torch.equal(torch.isinf(out), torch.isinf(plain))
+    assert torch.equal(out[64:100][torch.isinf(plain[64:100])], plain[64:100][torch.isinf(plain[64:100])])
+    assert rel_err(out[130], plain[130]) <= 1e-6
+    b, res = torch.randn(N, generator=g, device="cuda"), torch.randn(M, N, generator=g, device="cuda")
+    inplace, want = res.clone(), res.clone()
+    ops.linear_split(x, w, b, inplace, status, stream(), epilogue=ops.EPI_GELU_NEW, residual=inplace)
+    ops.linear_generic(x, w, b, want, stream(), epilogue=ops.EPI_GELU_NEW, residual=want)
+    assert torch.equal(torch.isnan(inplace), torch.isnan(want)) and torch.equal(torch.isinf(inplace), torch.isinf(want))
+    assert rel_err(inplace[130], want[130]) <= 1e-6 and rel_err(inplace[others], want[others]) <= 1e-6
+
+
 def test_rows_of_a_step_whatever_others_share_it(tmp_path):
     """A float32 engine: the logits of a request that brings one token, and of one that brings several, have the same bits alone and
     beside others, few or many, before or behind them among the step's entries."""
