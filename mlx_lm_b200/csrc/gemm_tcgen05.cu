@@ -48,15 +48,6 @@ constexpr int EPI_WARPS = 16;                     // four per quadrant of TMEM l
 constexpr int THREADS = 64 + 32 * EPI_WARPS;
 // slices of a tile's columns over the epilogue warps of a quadrant; a tile narrower than 128 leaves warps without work
 constexpr int epi_slices(int bn) { return bn >= 128 ? EPI_WARPS / 4 : bn / 32; }
-// Polls of a barrier before a wait gives up (about a second).  A test builds this file with
-// MLXB_TEST_WAIT_TIMEOUT defined: the limit is then short, and mlxb_test_withhold_arrival(1) makes the MMA thread
-// leave out the arrival that tells the epilogue warps that a CTA's first accumulator is complete, so that their
-// wait runs out and the abort path below is taken: every role leaves its loop, the CTA waits (bounded) for
-// what it has in flight, reports MLXB_ST_WAIT_TIMEOUT, frees its tensor memory and returns.  Nothing else differs.
-#ifdef MLXB_TEST_WAIT_TIMEOUT
-__device__ int g_test_withhold_arrival = 0;
-#endif
-
 // A stage holds KB blocks of 64 of K, each a tile of its own.
 template <int BN, int STAGES, int KB, int CG>
 struct Smem {
@@ -508,15 +499,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 }
 
 // ---------------------------------------------------------------------------------------------- host side
-
-#ifdef MLXB_TEST_WAIT_TIMEOUT
-// Test builds only: switch the withheld arrival on or off for the launches that follow on this device.
-MLXB_EXPORT int mlxb_test_withhold_arrival(int on) {
-  const cudaError_t e = cudaMemcpyToSymbol(g_test_withhold_arrival, &on, sizeof(int));
-  if (e != cudaSuccess) return mlxb_fail((int)e, "withhold_arrival: %s", cudaGetErrorString(e));
-  return 0;
-}
-#endif
 
 static int make_map(CUtensorMap* map, const void* base, int rows, int cols, int ld, int box_rows) {
   const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};

@@ -6,9 +6,19 @@
 
 #include "common.cuh"
 
-// Polls of a barrier before a wait gives up (about a second); short in a test build (MLXB_TEST_WAIT_TIMEOUT).
+// Polls of a barrier before a wait gives up (about a second).  A test builds a kernel with MLXB_TEST_WAIT_TIMEOUT defined: the limit is
+// then short, and mlxb_test_withhold_arrival(1) makes the thread that issues the products leave out the arrival that tells the other
+// warps that a CTA's first accumulator is complete, so that their wait runs out and the abort path is taken: every role leaves its
+// loop, the CTA waits (bounded) for what it has in flight, reports MLXB_ST_WAIT_TIMEOUT, frees its tensor memory and returns.
 #ifdef MLXB_TEST_WAIT_TIMEOUT
 constexpr uint32_t SPIN_LIMIT = 1u << 12;
+__device__ int g_test_withhold_arrival = 0;
+// Switches the withheld arrival on or off for the launches that follow on this device.
+MLXB_EXPORT int mlxb_test_withhold_arrival(int on) {
+  const cudaError_t e = cudaMemcpyToSymbol(g_test_withhold_arrival, &on, sizeof(int));
+  if (e != cudaSuccess) return mlxb_fail((int)e, "withhold_arrival: %s", cudaGetErrorString(e));
+  return 0;
+}
 #else
 constexpr uint32_t SPIN_LIMIT = 1u << 22;
 #endif

@@ -97,6 +97,35 @@ def test_float32_linear_in_parts_with_many_rows_that_are_not_finite(ops):
     assert rel_err(inplace[130], want[130]) <= 1e-6 and rel_err(inplace[others], want[others]) <= 1e-6
 
 
+def test_a_bounded_wait_that_runs_out(ops):
+    """A build with a short limit on its waits and one arrival left out (the sums' warps are never told of the first accumulator): the
+    kernel comes back by itself and says so, and the next launch of the same library, with the switch off, is right."""
+    from ctypes import c_int, c_void_p
+    from mlx_lm_b200.ops import build
+    name = "gemm_split:MLXB_TEST_WAIT_TIMEOUT=1"
+    lib = build.load(name)
+    lib.mlxb_test_withhold_arrival.argtypes, lib.mlxb_test_withhold_arrival.restype = [c_int], c_int
+    M, N, K = 300, 200, 512
+    g = torch.Generator(device="cuda").manual_seed(2)
+    x, w = torch.randn(M, K, generator=g, device="cuda"), torch.randn(N, K, generator=g, device="cuda")
+    out, status = torch.zeros(M, N, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def launch():
+        ops._call(name, "mlxb_linear_split", [c_void_p] * 5 + [c_int] * 6 + [c_void_p, c_void_p], x.data_ptr(), w.data_ptr(), None, None,
+                  out.data_ptr(), M, N, K, K, N, ops.EPI_NONE, status.data_ptr(), stream())
+        torch.cuda.synchronize()
+
+    assert lib.mlxb_test_withhold_arrival(1) == 0
+    try:
+        launch()
+        assert int(status.item()) == ops.ST_WAIT_TIMEOUT and not out.any()
+    finally:
+        assert lib.mlxb_test_withhold_arrival(0) == 0
+    status.zero_()
+    launch()
+    assert int(status.item()) == 0 and rel_err(out, x.double() @ w.double().T) <= 5e-7
+
+
 def test_rows_of_a_step_whatever_others_share_it(tmp_path):
     """A float32 engine: the logits of a request that brings one token, and of one that brings several, have the same bits alone and
     beside others, few or many, before or behind them among the step's entries."""

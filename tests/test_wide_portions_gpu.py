@@ -125,3 +125,37 @@ def test_wide_portions_sizes():
     lat = pool(1, 576)
     assert not ok(lat, lat, 4, 576, 512)
     assert not ok(pool(2, 64), pool(2, 64), 4, 64, 64, q=q[:, 1:4093], qhs=64) and not ok(pool(2, 64), pool(2, 64), 4, 62, 64)
+
+
+def test_a_bounded_wait_that_runs_out():
+    """A build with a short limit on its waits and one arrival left out (the softmax warps are never told of a tile's first scores): the
+    kernel comes back by itself and says so, and the next launch of the same library, with the switch off, is right."""
+    from ctypes import c_int
+    from mlx_lm_b200 import ops
+    from mlx_lm_b200.ops import build
+    name = "attention_wide_tcgen05:MLXB_TEST_WAIT_TIMEOUT=1"
+    lib = build.load(name)
+    lib.mlxb_test_withhold_arrival.argtypes, lib.mlxb_test_withhold_arrival.restype = [c_int], c_int
+    H, G, d, T = 4, 2, 64, 300
+    q, keys, values, kp, vp, table, _ = case(H, G, d, d, 16, False, [0], [T], 9)
+    tiles, status = tiles_of([0], [T]), torch.zeros(1, dtype=torch.int32, device=DEV)
+    out, want = torch.zeros(T, H * d, device=DEV), torch.zeros(T, H * d, device=DEV)
+    real = ops._call
+    launch = lambda o: (ops.attention_wide_portions(q.view(T, H * d), d, tiles, len(tiles), 128, table, kp, vp, o, d, H, d, d, 0.2, status,
+                                                    ops.current_stream()), torch.cuda.synchronize())
+    launch(want)
+    assert lib.mlxb_test_withhold_arrival(1) == 0
+    try:
+        ops._call = lambda lib_name, *a: real(name, *a)
+        launch(out)
+        assert int(status.item()) == ops.ST_WAIT_TIMEOUT and not out.any()
+    finally:
+        ops._call = real
+        assert lib.mlxb_test_withhold_arrival(0) == 0
+    status.zero_()
+    try:
+        ops._call = lambda lib_name, *a: real(name, *a)
+        launch(out)
+    finally:
+        ops._call = real
+    assert int(status.item()) == 0 and torch.equal(out, want)
