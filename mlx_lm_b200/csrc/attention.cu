@@ -520,7 +520,7 @@ attention_decode_kernel(const T* __restrict__ q, int ldq, const int* __restrict_
   // tables) and the keys and values of earlier positions.  So the chain of dependent loads (request ->
   // page ids -> first batch of keys and values) goes out before the wait for that kernel, and only the
   // query and the row's own key and value are fetched after it.
-  // beside: the kernel before this one is the portions', which has waited for the one that matters (see WaitAtEnd).  A step of
+  // beside: the kernel before this one is the portions', which has waited for the one that matters (see WaitAtEnd).  In a step of
   // 31 such rows of 20 heads and a portion of 256 rows: 25.8 + 18.0 us one after the other, 33.4 side by side.
   pdl_trigger();
   const WaitAtEnd end{beside && last_block_thread()};

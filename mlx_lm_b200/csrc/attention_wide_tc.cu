@@ -161,7 +161,7 @@ attention_wide_tc_kernel(const float* q, int ldq, int qhs, const int* __restrict
   const int rows_used = nq * HG;                             // rows 0 .. rows_used - 1 carry a (token, head)
   if (vec_q && !talk) {
     // four columns an access and four accesses on their way together: one column at a time each store waited for its load
-    // (single rows of 32 heads of 288: 28.1 us a launch, 17.0 this way)
+    // (4 single rows of 32 heads of 288 at 400 positions, with the merge: 27.6 us, 17.8 this way)
     const int per_row = DkE / 4, n = rows_used * per_row;
     for (int e0 = tid; e0 < n; e0 += 4 * THREADS) {
       float4 v[4];
@@ -402,9 +402,10 @@ attention_wide_tc_kernel(const float* q, int ldq, int qhs, const int* __restrict
 //   mix          a thread a key and every fourth head
 //   softmax      a warp a head; weights rounded to bfloat16 and summed as rounded
 //   values       warp w: every eighth tile of 8 columns of all value heads
-// Bound by latency: loads, four phases and their barriers, then the merge.  4 rows of 32 heads of 64 at 400 positions: 111 us with
-// mixed queries (most of it the mixing, a column at a time), 24 us this way with the merge (33 with every piece of a key looking its
-// page up and dividing its way to a column).
+// Bound by latency: loads, four phases and their barriers, then the merge (ncu: 3.5 % of the SMs' throughput, instructions issued in
+// 20 % of the cycles, short-scoreboard stalls first).  32 heads of 64 at 400 positions with the merge, mixed queries (most of it the mixing,
+// a column at a time) and this way: 1 row 22.5 and 20.0 us, 4 rows 40.8 and 20.2, 8 rows 70.8 and 20.4; 16 heads, 8 rows 18.5 and 13.7.
+// Up to 8 key heads of 64 fit the shared memory; designs with more go on with mixed queries.
 constexpr int TR_MAXH = 64, TR_ITEMS = 16;
 struct TalkRows { int ldq, ldk, ldv, ldp; long long smem; };
 static __host__ __device__ inline TalkRows talk_rows_layout(int Hq, int G, int Dk, int Dv) {

@@ -8,8 +8,8 @@
 // What bounds it is a tile's chain of blocks: S = Q K^T is DkE / 16 steps of two products 128 x 64 x 16 (hi and lo), O += P V
 // another 4 Dv / 64, and the softmax of 128 x 64 scores; so a block's products run during the softmax of the block before, and
 // keys arrive two blocks ahead.  With mma.sync (attention_wide_tc.cu) a CTA of 64 rows reads a fragment of shared memory for every
-// product.  2027 rows in portions of 731, 683 and 613, mma.sync and here: mixed scores of 16 heads 294 and 88 us, of 32 heads 1524 and
-// 223, latent rows 251 and 110 (16 heads), 440 and 192 (32).  A tile takes 20 us and 3 to 4 a block of keys.
+// product.  2027 rows in portions of 731, 683 and 613, mma.sync and here, inputs in L2: mixed scores of 16 heads 245 and 82 us, of 32
+// heads 1342 and 217, latent rows 200 and 83 (16 heads), 394 and 168 (32).  A tile takes 20 us and 3 to 4 a block of keys.
 //
 //   warp 9       producer: the pages of a block, a TMA copy per page and chunk of 64 columns, into a ring of 8 KB slots
 //                ([64 keys][64 columns], 128-byte swizzle)
@@ -21,8 +21,10 @@
 //                result depends on (weights and their sum refer to the same maximum), each row by itself
 //
 // Keys of a block that no query of the tile sees (behind the window, beyond the last position) are there as zeros among the values:
-// the softmax warps clear them, so that a value that is not finite reaches no row that does not see it, nor one of a page's next
-// request.  The order of additions for a row depends on its position only.
+// the softmax warps clear them, so that what earlier owners left in a page reaches nobody.  Keys that some query of the tile sees must
+// have finite values: to the others they are zero times the value, so an infinity or a NaN spoils the up to 128 / HG - 1 tokens
+// of the same request before it in its tile (as with mma.sync, whose tiles have 64 rows).  The order of additions for a row depends on
+// its position only.  Weights are 2^x by ex2.approx (two units in the last place) before they are rounded to bfloat16.
 //
 // Every wait on an mbarrier is bounded (tcgen05.cuh); after the limit all roles leave their loops, the copies and products in
 // flight are waited for, bounded, and MLXB_ST_WAIT_TIMEOUT is reported.

@@ -2,8 +2,9 @@
 //   C[M,N] = epilogue(A[M,K] . W[N,K]^T + bias[N]) (+ residual[M,N])
 // A and W are float32 or bfloat16 (one dtype for both); products and sums are
 // float32 FMAs; C is that dtype or float32, and the residual has C's dtype.
-// This is the whole matrix path of the float32 engine, and the fallback of
-// the bfloat16 engine for shapes its tensor-core kernels refuse.
+// In the float32 engine these kernels take single rows, the output head and
+// inner sizes below 128 (gemm_split.cu the rows of longer runs); they are the
+// fallback of the bfloat16 engine for shapes its tensor-core kernels refuse.
 //
 // Every output element adds k in order within segments of SEG = 128, and the segments' sums in order: one order for
 // every kernel, tile and number of rows, so a row's result does not depend on how many other rows the call has.  (A

@@ -1,18 +1,21 @@
 // Linear layer of float32 rows on the 5th-generation tensor cores, at float32's precision:
 //   C[M,N] = epilogue(A[M,K] . W[N,K]^T + bias[N]) (+ residual[M,N]),  all of them float32
 //
-// Every operand is the sum of three bfloat16 numbers, x = h + m + l (24 bits together, nothing of x is lost; h is cut off, m
-// rounded, so that l has either sign), and a product of two operands is the six products of such parts that reach 24 bits:
-// h h, h m, m h, h l, l h, m m (what is left out, m l and l m, is 2^-23 of the product at most and as often above as below).  The tensor core's products are exact; what
+// Every operand is the sum of three bfloat16 numbers, x = h + m + l (24 bits together, nothing of x is lost down to 2^-110, below which
+// l, and then m, ends with bfloat16's range; h is cut off, m rounded, so that l has either sign), and a product of two operands is
+// the six products of such parts that reach 24 bits: h h, h m, m h, h l, l h, m m.  What is left out, m l, l m and l l, is up to 2^-22 of
+// the product where both mantissas are at their worst, 2^-25.4 in the mean square, and as often above as below: less than the rounding
+// of a running sum by each FMA.  The tensor core's products are exact; what
 // it adds to its accumulator it cuts off instead of rounding, so no sum is left to it for long: a block of 64 of K starts a
 // fresh accumulator, the five small products of all its steps go in first, when the accumulator is 2^-8 of what it will be,
 // the four steps of h h last, and the block's sum is added, rounded to nearest, to a sum in registers.  One order for every
-// tile width and number of rows, so a row's result does not depend on how many other rows the call has.
+// tile width and number of rows, so a row's result does not depend on how many other rows go through this kernel; it differs by rounding
+// from the FMA kernels', and which of them a row takes depends on its own request alone (parts/linear.py).
 //
-// 737 rows, 24 layers of 1024 x 4096: 3072 x 1024 35 us, 1024 x 1024 25, 4096 x 1024 65, 1024 x 4096 81 (FMA tiles: 196 to 288); eight
+// 737 rows, weights from DRAM: 3072 x 1024 35 us, 1024 x 1024 24, 4096 x 1024 64, 1024 x 4096 79 (FMA tiles: 144, 73, 212, 278); eight
 // warps taking the numbers apart instead of sixteen: 43, 30, 76, 98 (they wait for what they read most of the time).
-// What bounds it: six products of 128 x BN x 64 a block, and as much shared memory traffic as they need; the FMA pipes, which
-// would be three times as busy as the tensor cores for the same product, only take the numbers apart.
+// What bounds it is reading the operands and taking them apart: 4096 x 1024 issues instructions in 70 % of all cycles, its tensor pipes
+// are busy in 25 %, shared memory in 30 %.
 //
 // Per CTA, over 128 x BN tiles (persistent, BN = 128 or 64):
 //   warps 0-15   read the next block of A and W with 16-byte loads (registers hold a block while the one before is at work),
@@ -20,8 +23,8 @@
 //   warp 24      issues the 24 products of a block, commits the buffer back and the accumulator forward (two of them)
 //   warps 16-23  add the accumulator of every block to their sums (64 columns of a row each at BN = 128); after the last
 //                block bias, activation and residual, and out through shared memory as whole sectors
-// An output that is not finite is computed again by its warp with plain FMAs: parts of an infinity, or of a number that
-// bfloat16 rounds to one, make sums that say nothing.
+// Outputs that are not finite are computed again by their warp with plain FMAs, after all others of its tile: parts of an infinity, or
+// sums beyond float32's range on the way, say nothing.  One row of NaN among 737 takes 4096 x 1024 from 63 to 80 us, all rows to 1.7 ms.
 //
 // Every wait on an mbarrier is bounded (tcgen05.cuh): after the limit all roles leave their loops, the CTA waits, bounded, for the
 // products in flight, reports MLXB_ST_WAIT_TIMEOUT, frees its tensor memory and returns.
@@ -378,6 +381,9 @@ MLXB_EXPORT int mlxb_linear_split(const float* A, const float* W, const float* b
   const char* want = getenv("MLXB_SPLIT_BN");      // experiments and tests
   const long long rows = (M + BM - 1) / BM, sms = mlxb_sm_count();
   const long long wide = (rows * ((N + 127) / 128) + sms - 1) / sms, narrow = (rows * ((N + 63) / 64) + sms - 1) / sms;
+  // Waves of wide tiles against waves of narrow ones, us: one and one 35 and 26 (64 x 3072 x 1024), two and three 65.7 and 64.3 (737 x
+  // 4096 x 1024) and 92 and 94 (2048 x 1600 x 1600), two and four 65.8 and 84 (1024 x 4096 x 1024), three and six 93 and 120 (2048 x 3072
+  // x 1024), one and two 33.5 and 42.3 (2048 x 1024 x 1024): the line lies where both take the same.
   const bool take_wide = want ? atoi(want) == 128 : wide * 100 <= narrow * 62;
   if (take_wide) return launch<128>(A, W, bias, residual, C, M, N, K, lda, ldc, epi, status, stream);
   return launch<64>(A, W, bias, residual, C, M, N, K, lda, ldc, epi, status, stream);

@@ -20,8 +20,8 @@
 // columns a thread asks for all that it has of a row at once (16-byte accesses, the weights before the wait for the kernel before)
 // and keeps it in registers between the sum and the result; parts of up to 512 columns take a warp each, wider ones a block.  The
 // kernels that read a column at a time, and the row again for the result, serve what is left.  Rows of 1024, norm and update: 6.3 and 6.75
-// us in a decode step of 8 rows, now 2.1 both; 2048 rows 15.8 and 9.7, now 5.65 and 5.7.  Squares are added in pairs: one chain of FMAs
-// moved a bfloat16 model of sharp attention from 0.12 to 0.20 off.
+// us in a decode step of 8 rows, now 2.1 both; 2048 rows 15.8 and 9.7, now 5.65 and 5.7.  The norms add squares in pairs (one chain of
+// FMAs moved a bfloat16 model of sharp attention from 0.12 to 0.20 off); the updates add theirs in one chain a thread.
 #include "common.cuh"
 
 MLXB_DEFINE_LAST_ERROR()

@@ -15,7 +15,8 @@
 // in row slots[r] of a float32 pool ([slots, H, V, K]: a head's state column by column), read at the start of the
 // run and written back at its end.  A thread holds 16 consecutive rows of one column in registers; the NS threads of
 // a column are neighbouring lanes and add their partial sums by shuffles; 16 tokens at a time are staged in shared
-// memory.  The order of additions for a token depends on the layer's sizes only.
+// memory.  Token by token the order of additions for a token depends on the layer's sizes only; in chunks (wkv_chunks below, which
+// the engine's sizes take) also on where its run begins, that is on how a prompt was cut into steps, in float32 as in bfloat16.
 #include <type_traits>
 
 #include "common.cuh"
@@ -194,13 +195,15 @@ wkv_scan_kernel(const T* rkv, int ld, int r_off, int k_off, int v_off, const flo
 // ---------------------------------------------------------------- the recurrence in chunks
 
 // Token by token a run is a chain as long as it is, on as many SMs as there are (request, head) pairs: 731, 683 and 613 rows of 16
-// heads took 440 us (in chunks 98; a decode step of 8 requests 34 and 11).  The state is linear in the state before, channel by channel: over a chunk of rows, S_end = W S_0 + L with W
+// heads of 64 took 217 us with the next tokens fetched ahead (474 without, as the scan above is), in chunks 90; a decode step of 8
+// requests 9.2 and 7.0.  The state is linear in the state before, channel by channel: over a chunk of rows, S_end = W S_0 + L with W
 // the product of the chunk's decays (one number a key channel) and L the state that the chunk leaves of an empty one.  So the
 // chunks of a run are walked side by side:
 //   first pass   chunk 0 of a run as a scan, with its outputs; of every other chunk but the last L and W
 //   second pass  every chunk after the first: its state from the chunks before, then the scan with its outputs
-// in float32 like the scan, in the same order within a chunk.  What bounds it then is the FMAs and the loads of r, k, w that feed
-// them, so a thread has two columns (32 numbers of the state) and multiplies pairs of channels (fma.rn.f32x2).
+// in float32 like the scan, in the same order within a chunk.  What bounds it then is the loads of r, k, w from shared memory that feed
+// the FMAs (shared memory busy in 35 and 39 % of the cycles, ten warps an SM), so a thread has two columns (32
+// numbers of the state) and multiplies pairs of channels (fma.rn.f32x2).
 constexpr int WC_Q = 64;       // rows of a chunk
 constexpr int WC_VB = 64;      // columns of a block: NS threads for every two of them
 

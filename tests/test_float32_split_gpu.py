@@ -20,8 +20,9 @@ def ops():
 @pytest.mark.parametrize("M,N,K", [(1, 64, 256), (17, 7, 4), (127, 65, 60), (128, 128, 64), (129, 130, 68), (300, 200, 1000),
                                    (257, 1030, 260), (1100, 512, 128), (64, 3072, 132), (40, 24, 4100)])
 def test_float32_linear_in_parts(ops, M, N, K, width, monkeypatch):
-    """What is left out of a product is 2^-25 of it, a block of 64 of K takes four cut-off sums of 2^-23 at most, the blocks' sums K / 64
-    roundings of 2^-24: a few 1e-7 over the whole result at most; the same bits for both tile widths and however many rows."""
+    """What is left out of a product is 2^-25.4 of it in the mean square (2^-22 at worst) and of either sign, a block of 64 of K takes four
+    cut-off sums of 2^-23 at most, the blocks' sums K / 64 roundings of 2^-24: a few 1e-7 over the whole result at most; the same bits for
+    both tile widths and however many rows of this kernel."""
     monkeypatch.setenv("MLXB_SPLIT_BN", width)
     g = torch.Generator(device="cuda").manual_seed(M + N + K)
     draw = lambda *s: torch.randn(*s, generator=g, device="cuda")
