@@ -22,6 +22,8 @@
 // kernels that read a column at a time, and the row again for the result, serve what is left.  Rows of 1024, norm and update: 6.3 and 6.75
 // us in a decode step of 8 rows, now 2.1 both; 2048 rows 15.8 and 9.7, now 5.65 and 5.7.  The norms add squares in pairs (one chain of
 // FMAs moved a bfloat16 model of sharp attention from 0.12 to 0.20 off); the updates add theirs in one chain a thread.
+#include <type_traits>
+
 #include "common.cuh"
 
 MLXB_DEFINE_LAST_ERROR()
@@ -138,44 +140,57 @@ rmsnorm_parts_kernel(const TI* x, int ldx, const float* __restrict__ w, float of
 
 // Wider parts (or whole rows), four columns a thread and step: a block per part, the part in registers, the weights asked for before
 // the wait.  NV * 4 * blockDim.x columns at most.
-template <typename TI, typename TO, int NV>
+enum { WHOLE_ROWS, PARTS, GATED_PARTS };      // WHOLE_ROWS: with a weight, without a gate
+template <typename TI, typename TO, int NV, int FORM>
 __global__ void __launch_bounds__(512)
 rmsnorm_rows_kernel(const TI* x, int ldx, const int* __restrict__ rows, int n_src_rows, const float* __restrict__ w, float offset,
-                    int period, const TO* gate, int ldg, int gate_mode, TO* __restrict__ out, int ldo, int Dg, float eps) {
+                    int w_step, const TO* gate, int ldg, int gate_mode, TO* __restrict__ out, int ldo, int Dg, float eps) {
+  constexpr bool GATED = FORM == GATED_PARTS;
   __shared__ float red[33];
-  const int r = blockIdx.x, g = blockIdx.y;
+  const int r = blockIdx.x, g = FORM == WHOLE_ROWS ? 0 : blockIdx.y;
   const int src = rows ? rows[r] : r;
   const bool there = src >= 0 && src < n_src_rows;
-  const int w0 = g * Dg % period;      // (a part's weights are neighbours: the period is the width or the part's)
-  float wv[NV][4], v[NV][4], gv[NV][4];
+  float wv[NV][4], v[NV][4], gv[GATED ? NV : 1][4];
+  if (FORM != WHOLE_ROWS) {
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const int c = (i * blockDim.x + threadIdx.x) * 4;
+    for (int i = 0; i < NV; ++i)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) wv[i][e] = v[i][e] = gv[i][e] = 0.f;
-    if (c < Dg && w) load4(w + w0 + c, wv[i]);
+      for (int e = 0; e < 4; ++e) wv[i][e] = 0.f;
+  }
+  if (FORM == WHOLE_ROWS || w) {
+    w += g * w_step;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int c = (i * blockDim.x + threadIdx.x) * 4;
+      if (c < Dg) load4(w + c, wv[i]);
+    }
   }
   pdl_wait();
   pdl_trigger();
   x = after_wait(x);
-  gate = after_wait(gate);
+  if (GATED) gate = after_wait(gate);
   float s = 0.f;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int c = (i * blockDim.x + threadIdx.x) * 4;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[i][e] = 0.f;
+    if (GATED)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) gv[GATED ? i : 0][e] = 0.f;
     if (c < Dg && there) {
       load4(x + (size_t)src * ldx + (size_t)g * Dg + c, v[i]);
-      if (gate_mode) load4(gate + (size_t)src * ldg + (size_t)g * Dg + c, gv[i]);
+      if (GATED) load4(gate + (size_t)src * ldg + (size_t)g * Dg + c, gv[GATED ? i : 0]);
     }
   }
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
+    if (GATED && gate_mode == 1)
 #pragma unroll
-    for (int e = 0; e < 4; ++e)
-      if (gate_mode == 1) v[i][e] *= silu_f(gv[i][e]);
+      for (int e = 0; e < 4; ++e) v[i][e] *= silu_f(gv[GATED ? i : 0][e]);
     s += squares(v[i]);
   }
-  const float rinv = 1.f / sqrtf(block_sum(s, red) / (float)Dg + eps);
+  const float total = block_sum(s, red), rinv = there ? 1.f / sqrtf(total / (float)Dg + eps) : 0.f;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int c = (i * blockDim.x + threadIdx.x) * 4;
@@ -183,8 +198,7 @@ rmsnorm_rows_kernel(const TI* x, int ldx, const int* __restrict__ rows, int n_sr
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       v[i][e] = v[i][e] * rinv * (offset + wv[i][e]);
-      if (gate_mode == 2) v[i][e] *= silu_f(gv[i][e]);
-      if (!there) v[i][e] = 0.f;
+      if (GATED && gate_mode == 2) v[i][e] *= silu_f(gv[GATED ? i : 0][e]);
     }
     store4(out + (size_t)r * ldo + (size_t)g * Dg + c, v[i]);
   }
@@ -192,9 +206,9 @@ rmsnorm_rows_kernel(const TI* x, int ldx, const int* __restrict__ rows, int n_sr
 
 constexpr int RR_MAX = 4 * 512 * 4;      // columns of a part that a block holds
 
-// Threads of a block with a part of Dg columns: the fewest that have it in two steps each, up to 512.
+// Threads of a block with a part of Dg columns: the fewest that have it in two steps each, up to 512 (a warp for up to 128 columns).
 static int rows_threads(int Dg) {
-  int threads = 64;
+  int threads = Dg <= 128 ? 32 : 64;
   while (threads < 512 && Dg / 4 > threads * 2) threads *= 2;
   return threads;
 }
@@ -202,13 +216,21 @@ template <typename TI, typename TO>
 static void launch_rows(const TI* x, int ldx, const int* rows, int n_src_rows, const float* w, float offset, int period, const TO* gate,
                         int ldg, int gate_mode, TO* out, int ldo, int R, int Dg, int groups, float eps, cudaStream_t stream) {
   const int threads = rows_threads(Dg), nv = (Dg / 4 + threads - 1) / threads;
+  const int w_step = period == Dg ? 0 : Dg;      // a part's weights are neighbours: the period is the width or the part's
   auto go = [&](auto kernel) {
-    launch_pdl(kernel, dim3(R, groups), dim3(threads), 0, stream, x, ldx, rows, n_src_rows, w, offset, period, gate, ldg, gate_mode, out,
+    launch_pdl(kernel, dim3(R, groups), dim3(threads), 0, stream, x, ldx, rows, n_src_rows, w, offset, w_step, gate, ldg, gate_mode, out,
                ldo, Dg, eps);
   };
-  if (nv <= 1) go(rmsnorm_rows_kernel<TI, TO, 1>);
-  else if (nv <= 2) go(rmsnorm_rows_kernel<TI, TO, 2>);
-  else go(rmsnorm_rows_kernel<TI, TO, 4>);
+  // (a gate's registers in every instance took 4096 rows of 4096 from 17.0 to 30.6 us, the parts' indexes to 18.6)
+  auto by_steps = [&](auto form) {
+    constexpr int FORM = decltype(form)::value;
+    if (nv <= 1) go(rmsnorm_rows_kernel<TI, TO, 1, FORM>);
+    else if (nv <= 2) go(rmsnorm_rows_kernel<TI, TO, 2, FORM>);
+    else go(rmsnorm_rows_kernel<TI, TO, 4, FORM>);
+  };
+  if (gate_mode) by_steps(std::integral_constant<int, GATED_PARTS>{});
+  else if (groups > 1 || !w) by_steps(std::integral_constant<int, PARTS>{});
+  else by_steps(std::integral_constant<int, WHOLE_ROWS>{});
 }
 
 // x_f32: x is float32 (else it has out_dtype); w may be null (the offset is then the factor).
@@ -302,24 +324,23 @@ __global__ void residual_update_kernel(float* x, int ldx, const float* y1, const
   }
 }
 
-// Four columns a thread and step, all of a row's operands in registers: NV * 4 * blockDim.x columns at most.
-template <typename TO, int NV>
+// Four columns a thread and step, all of a row's operands in registers: NV * 4 * blockDim.x columns at most.  NORMED: with a weight or
+// two (a sum without any waits for nobody: 4096 rows of 64 took 5.0 us with the norms' code beside it, 4.7 without).
+template <typename TO, int NV, bool NORMED>
 __global__ void __launch_bounds__(512)
 residual_update_rows_kernel(float* x, int ldx, const float* y1, const float* __restrict__ w1, const float* y2,
                             const float* __restrict__ w2, int ldy, float scale, float eps, TO* __restrict__ cast_out, int ldc, int D) {
-  __shared__ float red[33], red2[33];
   const int r = blockIdx.x;
-  float wa[NV][4], wb[NV][4], a[NV][4], b[NV][4], xv[NV][4];
+  float wa[NORMED ? NV : 1][4], wb[NORMED ? NV : 1][4], a[NV][4], b[NV][4], xv[NV][4];
+  if (NORMED) {
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const int c = (i * blockDim.x + threadIdx.x) * 4;
+    for (int i = 0; i < NV; ++i) {
+      const int c = (i * blockDim.x + threadIdx.x) * 4, k = NORMED ? i : 0;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      wa[i][e] = wb[i][e] = 1.f;
-      a[i][e] = b[i][e] = xv[i][e] = 0.f;
+      for (int e = 0; e < 4; ++e) wa[k][e] = wb[k][e] = 1.f;
+      if (c < D && w1) load4(w1 + c, wa[k]);
+      if (c < D && w2) load4(w2 + c, wb[k]);
     }
-    if (c < D && w1) load4(w1 + c, wa[i]);
-    if (c < D && w2) load4(w2 + c, wb[i]);
   }
   pdl_wait();
   pdl_trigger();
@@ -329,25 +350,30 @@ residual_update_rows_kernel(float* x, int ldx, const float* y1, const float* __r
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int c = (i * blockDim.x + threadIdx.x) * 4;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) a[i][e] = b[i][e] = xv[i][e] = 0.f;
     if (c >= D) continue;
     load4(y1 + (size_t)r * ldy + c, a[i]);
     if (y2) load4(y2 + (size_t)r * ldy + c, b[i]);
     load4(x + (size_t)r * ldx + c, xv[i]);
   }
-  auto normed = [&](float (&v)[NV][4], const float (&w)[NV][4], float* memory) {
-    float s = 0.f;
+  if constexpr (NORMED) {
+    __shared__ float red[33], red2[33];
+    auto normed = [&](float (&v)[NV][4], const float (&w)[NV][4], float* memory) {
+      float s = 0.f;
 #pragma unroll
-    for (int i = 0; i < NV; ++i)
+      for (int i = 0; i < NV; ++i)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) s = fmaf(v[i][e], v[i][e], s);
-    const float f = 1.f / sqrtf(block_sum(s, memory) / (float)D + eps);
+        for (int e = 0; e < 4; ++e) s = fmaf(v[i][e], v[i][e], s);
+      const float f = 1.f / sqrtf(block_sum(s, memory) / (float)D + eps);
 #pragma unroll
-    for (int i = 0; i < NV; ++i)
+      for (int i = 0; i < NV; ++i)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) v[i][e] = v[i][e] * f * w[i][e];
-  };
-  if (w1) normed(a, wa, red);
-  if (y2 && w2) normed(b, wb, red2);
+        for (int e = 0; e < 4; ++e) v[i][e] = v[i][e] * f * w[i][e];
+    };
+    if (w1) normed(a, wa, red);
+    if (y2 && w2) normed(b, wb, red2);
+  }
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int c = (i * blockDim.x + threadIdx.x) * 4;
@@ -376,9 +402,14 @@ MLXB_EXPORT int mlxb_residual_update(int cast_dtype, float* x, int ldx, const fl
       auto go = [&](auto kernel) {
         launch_pdl(kernel, dim3(R), dim3(threads), 0, stream, x, ldx, y1, w1, y2, w2, ldy, scale, eps, (TO*)cast_out, ldc, D);
       };
-      if (nv <= 1) go(residual_update_rows_kernel<TO, 1>);
-      else if (nv <= 2) go(residual_update_rows_kernel<TO, 2>);
-      else go(residual_update_rows_kernel<TO, 4>);
+      auto by_steps = [&](auto normed) {
+        constexpr bool NORMED = decltype(normed)::value;
+        if (nv <= 1) go(residual_update_rows_kernel<TO, 1, NORMED>);
+        else if (nv <= 2) go(residual_update_rows_kernel<TO, 2, NORMED>);
+        else go(residual_update_rows_kernel<TO, 4, NORMED>);
+      };
+      if (w1 || (y2 && w2)) by_steps(std::true_type{});
+      else by_steps(std::false_type{});
     };
     if (cast_dtype == MLXB_F32) by(float{});
     else by(__nv_bfloat16{});
