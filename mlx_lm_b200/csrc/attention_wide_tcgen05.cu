@@ -177,6 +177,9 @@ attention_wide_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const _
   {
     const float* q = after_wait(a.q);
     const int room = a.slots / 2;                                  // chunks of queries that fit the ring
+    // Rows of no token are zeros, but with a cap the last token's: capping a score of zero is a quotient of zero, 370 cycles, and a tile
+    // with such rows took twice its time (130 tokens at 1900 positions, 8 heads of 64: 272 us, 133 this way).
+    const int n_rows = a.softcap > 0.f ? TQ : nq;
     for (int c0 = 0; c0 < a.chunks; c0 += room) {
       const int n_c = min(room, a.chunks - c0), per_row = n_c * 16;
       if (c0 > 0) __syncthreads();
@@ -206,8 +209,8 @@ attention_wide_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const _
             for (int k = 0; k < 2; ++k) {
               const int e = e0 + k * SOFT_THREADS, x = e / (TQ * 16), y = e - x * (TQ * 16), tq = y >> 4, col = (c0 + x) * 64 + (y & 15) * 4;
               const int c = col / a.Dk, d = col - c * a.Dk;
-              const bool in = e < items && tq < nq && c < a.Hkv;
-              const float* qt = q + (size_t)(t0 + tq) * a.ldq + (size_t)(c * rep) * a.qhs + d;
+              const bool in = e < items && tq < n_rows && c < a.Hkv;
+              const float* qt = q + (size_t)(t0 + min(tq, nq - 1)) * a.ldq + (size_t)(c * rep) * a.qhs + d;
 #pragma unroll
               for (int i = 0; i < 4; ++i)
                 u[k][i] = in && i < rep ? *reinterpret_cast<const float4*>(qt + (size_t)i * a.qhs) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -239,8 +242,8 @@ attention_wide_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const _
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
               const int e = e0 + k * SOFT_THREADS, r = e / per_row, col = c0 * 64 + (e - r * per_row) * 4, tq = r >> hg_shift;
-              u[k] = e < items && tq < nq && col < a.Dk
-                         ? *reinterpret_cast<const float4*>(q + (size_t)(t0 + tq) * a.ldq + (size_t)(h0 + (r & (HG - 1))) * a.qhs + col)
+              u[k] = e < items && tq < n_rows && col < a.Dk
+                         ? *reinterpret_cast<const float4*>(q + (size_t)(t0 + min(tq, nq - 1)) * a.ldq + (size_t)(h0 + (r & (HG - 1))) * a.qhs + col)
                          : make_float4(0.f, 0.f, 0.f, 0.f);
             }
 #pragma unroll
@@ -254,8 +257,8 @@ attention_wide_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const _
             const int r = e / per_row, col = c0 * 64 + (e - r * per_row) * 4;
             const int tq = r >> hg_shift, h = h0 + (r & (HG - 1)), c = col / a.Dk, d = col - c * a.Dk;
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (tq < nq && c < a.Hkv) {
-              const float* qt = q + (size_t)(t0 + tq) * a.ldq;
+            if (tq < n_rows && c < a.Hkv) {
+              const float* qt = q + (size_t)(t0 + min(tq, nq - 1)) * a.ldq;
               for (int i = 0; i < rep; ++i) {
                 const float w = __ldg(a.talk + h * a.Hq + c * rep + i);
                 const float4 u = *reinterpret_cast<const float4*>(qt + (size_t)(c * rep + i) * a.qhs + d);
